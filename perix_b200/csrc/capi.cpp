@@ -137,7 +137,7 @@ size_t ctx_bytes(const pxb_ctx *c) {
     s += bufsz(bt.clouds) + bufsz(bt.tasks) + bufsz(bt.off) + bufsz(bt.nbr) + bufsz(bt.pos) + bufsz(bt.vol) +
          bufsz(bt.ops) + bufsz(bt.degenerate) + bufsz(bt.counters) + bufsz(bt.defect);
     const CsrState &k = c->csr;
-    s += bufsz(k.rowptr) + bufsz(k.cols) + bufsz(k.slot) + bufsz(k.diag) + bufsz(k.kvals) + bufsz(k.rhs) +
+    s += bufsz(k.rowptr) + bufsz(k.cols) + bufsz(k.slot) + bufsz(k.bpos) + bufsz(k.spos) + bufsz(k.xpos) + bufsz(k.diag) + bufsz(k.kvals) + bufsz(k.rhs) +
          bufsz(k.u) + bufsz(k.uold) + bufsz(k.fnode) + bufsz(k.mnode);
     s += bufsz(c->ch.rev) + bufsz(c->ch.lap) + bufsz(c->ch.ghost) + bufsz(c->ch.lrv) + bufsz(c->ch.bfl) +
          bufsz(c->scratch);
@@ -1876,46 +1876,76 @@ extern "C" int pxb_epf_force_adjoint(pxb_ctx *c, const double *u, const double *
 
 // ============================================================================================== CSR assembly
 namespace pxb {
-// the slot map, diagonal slots, exact-pattern flags and value buffers of the pattern in c->csr (rowptr, cols, ndof,
-// nnz set on the device)
-int csr_finish(pxb_ctx *c, const char *who) {
+// the block positions (exact block patterns) or the slot map, the diagonal slots and the value buffers of the pattern
+// in c->csr (rowptr, cols, ndof, nnz set on the device); verify: the rows come from the caller and are checked
+int csr_finish(pxb_ctx *c, const char *who, bool verify) {
     CsrState &k = c->csr;
-    const int ndof = k.ndof;
-    const size_t rows = (size_t)c->g.n * ndof;
-    PXB_TRY(dev_alloc(c, k.slot, sizeof(int) * (size_t)std::max(1LL, c->g.nb) * ndof * ndof));
-    PXB_TRY(dev_alloc(c, k.diag, sizeof(int) * (size_t)c->g.n * ndof * ndof));
-    PXB_TRY(dev_alloc(c, k.extra, sizeof(int) * (size_t)c->g.n * ndof * ndof));
+    const int ndof = k.ndof, n = c->g.n;
+    const size_t rows = (size_t)n * ndof, nb = (size_t)std::max(1LL, c->g.nb);
+    PXB_TRY(dev_alloc(c, k.diag, sizeof(int) * (size_t)n * ndof * ndof));
     void *tmp = nullptr;
     PXB_TRY(scratch(c, 8, &tmp));
     PXB_CUDA_TRY(cudaMemsetAsync(tmp, 0, 8, c->stream));
-    CsrMapArgs a;
-    a.n = c->g.n;
-    a.ndof = ndof;
-    a.off = c->g.off.as<int>();
-    a.nbr = c->g.nbr.as<int>();
-    a.rowptr = k.rowptr.as<int>();
-    a.cols = k.cols.as<int>();
-    a.slot = k.slot.as<int>();
-    a.diag = k.diag.as<int>();
-    a.missing = static_cast<int *>(tmp);
-    a.inexact = static_cast<int *>(tmp) + 1;
-    a.mirror = c->g.mirror.p ? c->g.mirror.as<int>() : nullptr;
-    a.extra = k.extra.as<int>();
-    launch_csr_map(a, c->stream);
-    PXB_TRY(check_launch(c, "csr_map"));
+    k.mmax = c->g.max_family + 2;  // own block, family, a mirror outside it
+    k.exact = false;
     int flags[2] = {0, 0};
-    PXB_TRY(d2h(c, flags, tmp, 8));
-    PXB_TRY(sync(c));
-    const int missing = flags[0];
-    k.exact = flags[1] == 0;
-    if (missing) return fail(PXB_ERR_INVALID, std::string(who) + ": pattern lacks " + std::to_string(missing) +
-                                                  " entries required by the families");
+    if (k.mmax <= kBlockMax) {
+        PXB_TRY(dev_alloc(c, k.bpos, nb));
+        PXB_TRY(dev_alloc(c, k.spos, (size_t)n));
+        PXB_TRY(dev_alloc(c, k.xpos, sizeof(int16_t) * (size_t)n));
+        BlockMapArgs m;
+        m.n = n;
+        m.ndof = ndof;
+        m.verify = verify ? 1 : 0;
+        m.nnz = k.nnz;
+        m.off = c->g.off.as<int>();
+        m.nbr = c->g.nbr.as<int>();
+        m.rowptr = k.rowptr.as<int>();
+        m.cols = k.cols.as<int>();
+        m.mirror = c->g.mirror.p ? c->g.mirror.as<int>() : nullptr;
+        m.bpos = k.bpos.as<uint8_t>();
+        m.spos = k.spos.as<uint8_t>();
+        m.xpos = k.xpos.as<int16_t>();
+        m.diag = k.diag.as<int>();
+        m.inexact = static_cast<int *>(tmp);
+        PXB_CUDA_TRY(launch_block_map(m, c->stream));
+        PXB_TRY(check_launch(c, "block map"));
+        PXB_TRY(d2h(c, flags, tmp, 4));
+        PXB_TRY(sync(c));
+        k.exact = flags[0] == 0;
+    }
+    if (!k.exact) {
+        k.bpos.release();
+        k.spos.release();
+        k.xpos.release();
+        PXB_TRY(dev_alloc(c, k.slot, sizeof(int) * nb * ndof * ndof));
+        CsrMapArgs a;
+        a.n = n;
+        a.ndof = ndof;
+        a.off = c->g.off.as<int>();
+        a.nbr = c->g.nbr.as<int>();
+        a.rowptr = k.rowptr.as<int>();
+        a.cols = k.cols.as<int>();
+        a.slot = k.slot.as<int>();
+        a.diag = k.diag.as<int>();
+        a.missing = static_cast<int *>(tmp) + 1;
+        launch_csr_map(a, c->stream);
+        PXB_TRY(check_launch(c, "csr_map"));
+        PXB_TRY(d2h(c, flags, tmp, 8));
+        PXB_TRY(sync(c));
+        if (flags[1]) return fail(PXB_ERR_INVALID, std::string(who) + ": pattern lacks " + std::to_string(flags[1]) +
+                                                       " entries required by the families");
+    }
     PXB_TRY(dev_alloc(c, k.kvals, sizeof(double) * (size_t)k.nnz));
     PXB_TRY(dev_alloc(c, k.rhs, sizeof(double) * rows));
     PXB_TRY(dev_alloc(c, k.u, sizeof(double) * rows));
     PXB_TRY(dev_alloc(c, k.uold, sizeof(double) * rows));
     k.ready = true;
     return PXB_OK;
+}
+
+BlockPattern block_pattern(const CsrState &k) {
+    return {k.bpos.as<uint8_t>(), k.spos.as<uint8_t>(), k.xpos.as<int16_t>()};
 }
 }  // namespace pxb
 
@@ -1935,7 +1965,7 @@ extern "C" int pxb_csr_set_pattern(pxb_ctx *c, int ndof, const int *rowptr, cons
         PXB_TRY(dev_upload(c, k.bcol, k.h_bcol.data(), sizeof(int) * std::max<size_t>(1, k.h_bcol.size())));
         k.blocked2 = true;
     }
-    return csr_finish(c, "pxb_csr_set_pattern");
+    return csr_finish(c, "pxb_csr_set_pattern", true);
 }
 
 extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
@@ -1988,7 +2018,7 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     a.cols = k.cols.as<int>();
     PXB_CUDA_TRY(launch_pattern_fill(a, c->stream));
     c->launches++;
-    PXB_TRY(csr_finish(c, "pxb_csr_build_pattern"));
+    PXB_TRY(csr_finish(c, "pxb_csr_build_pattern", false));
     if (nnz) *nnz = total;
     return PXB_OK;
 }
@@ -2040,7 +2070,8 @@ extern "C" int pxb_assemble_scalar_d(pxb_ctx *c, int type, double coef, double f
     a.uold = uold_d;
     a.kvals = kvals_d;
     a.rhs = rhs_d;
-    launch_assemble_scalar(a, c->stream);
+    if (k.exact) PXB_CUDA_TRY(launch_scalar_block(a, block_pattern(k), c->stream));
+    else PXB_CUDA_TRY(launch_assemble_scalar(a, c->stream));
     return check_launch(c, "assemble_scalar");
 }
 
@@ -2158,15 +2189,12 @@ static int ch_args(pxb_ctx *c, double kappa, double chi, double dt, const double
     a.rowptr = k.rowptr.as<int>();
     a.slot = k.slot.as<int>();
     a.diag = k.diag.as<int>();
-    a.extra = k.exact ? k.extra.as<int>() : nullptr;
     a.u = u_d;
     a.uold = uold_d;
     a.kvals = kvals_d;
     a.rhs = rhs_d;
-    if (c->ch.lrv.p && c->ch.bfl.p) {
-        a.lrv = c->ch.lrv.as<double>();
-        a.bfl = c->ch.bfl.as<uint8_t>();
-    }
+    a.lrv = c->ch.lrv.as<double>();
+    a.bfl = c->ch.bfl.as<uint8_t>();
     return PXB_OK;
 }
 
@@ -2175,7 +2203,8 @@ extern "C" int pxb_assemble_ch_d(pxb_ctx *c, double kappa, double chi, double dt
     if (!mnode_d || !u_d || !uold_d || !kvals_d || !rhs_d) return fail(PXB_ERR_INVALID, "pxb_assemble_ch: NULL buffer");
     ChAsmArgs a;
     PXB_TRY(ch_args(c, kappa, chi, dt, mnode_d, u_d, uold_d, kvals_d, rhs_d, a, "pxb_assemble_ch"));
-    launch_assemble_ch(a, c->stream);
+    if (c->csr.exact) PXB_CUDA_TRY(launch_ch_block(a, block_pattern(c->csr), c->stream));
+    else PXB_CUDA_TRY(launch_assemble_ch(a, c->stream));
     return check_launch(c, "assemble_ch");
 }
 
@@ -2234,7 +2263,10 @@ extern "C" int pxb_assemble_stress_ch_d(pxb_ctx *c, const pxb_stress_ch_params *
     a.uold = uold_d;
     a.kvals = kvals_d;
     a.rhs = rhs_d;
-    PXB_CUDA_TRY(launch_assemble_stress_ch(a, c->stream));
+    a.lrv = c->ch.lrv.as<double>();
+    a.bfl = c->ch.bfl.as<uint8_t>();
+    if (k.exact) PXB_CUDA_TRY(launch_stress_ch_block(a, block_pattern(k), k.mmax, c->stream));
+    else PXB_CUDA_TRY(launch_assemble_stress_ch(a, c->stream));
     return check_launch(c, "assemble_stress_ch");
 }
 
@@ -2314,7 +2346,8 @@ extern "C" int pxb_assemble_cached_d(pxb_ctx *c, const pxb_cached_params *p, con
     a.uold = uold_d;
     a.kvals = kvals_d;
     a.rhs = rhs_d;
-    PXB_CUDA_TRY(launch_assemble_cached(a, c->stream));
+    if (k.exact) PXB_CUDA_TRY(launch_cached_block(a, block_pattern(k), k.mmax, c->stream));
+    else PXB_CUDA_TRY(launch_assemble_cached(a, c->stream));
     return check_launch(c, "assemble_cached");
 }
 
@@ -2356,32 +2389,8 @@ extern "C" int pxb_assemble_ch(pxb_ctx *c, double kappa, double chi, double dt, 
     PXB_TRY(h2d(c, k.mnode.p, mnode, sizeof(double) * n));
     PXB_TRY(h2d(c, k.u.p, u, sizeof(double) * 2 * n));
     PXB_TRY(h2d(c, k.uold.p, uold, sizeof(double) * 2 * n));
-    ChAsmArgs a;
-    a.n = c->g.n;
-    a.kappa = kappa;
-    a.chi = chi;
-    a.dt = dt;
-    a.off = c->g.off.as<int>();
-    a.nbr = c->g.nbr.as<int>();
-    a.rev = c->ch.rev.as<int>();
-    a.lap = c->ch.lap.as<double>();
-    a.vol = c->g.vol.as<double>();
-    a.mnode = k.mnode.as<double>();
-    a.ghost = c->ch.ghost.p ? c->ch.ghost.as<char>() : nullptr;
-    a.rowptr = k.rowptr.as<int>();
-    a.slot = k.slot.as<int>();
-    a.diag = k.diag.as<int>();
-    a.extra = k.exact ? k.extra.as<int>() : nullptr;
-    a.u = k.u.as<double>();
-    a.uold = k.uold.as<double>();
-    a.kvals = k.kvals.as<double>();
-    a.rhs = k.rhs.as<double>();
-    if (c->ch.lrv.p && c->ch.bfl.p) {
-        a.lrv = c->ch.lrv.as<double>();
-        a.bfl = c->ch.bfl.as<uint8_t>();
-    }
-    launch_assemble_ch(a, c->stream);
-    PXB_TRY(check_launch(c, "assemble_ch"));
+    PXB_TRY(pxb_assemble_ch_d(c, kappa, chi, dt, k.mnode.as<double>(), k.u.as<double>(), k.uold.as<double>(),
+                              k.kvals.as<double>(), k.rhs.as<double>()));
     PXB_TRY(d2h(c, kvals, k.kvals.p, sizeof(double) * (size_t)k.nnz));
     PXB_TRY(d2h(c, rhs, k.rhs.p, sizeof(double) * 2 * n));
     return sync(c);

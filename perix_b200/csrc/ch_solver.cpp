@@ -362,8 +362,9 @@ extern "C" int pxb_ch_gradient(pxb_ctx *c, const pxb_ch_run_params *p, const dou
         // A = (K - J_M)^T at (U_n, U_{n-1}): fold the mobility derivative into K, then transpose the values
         PXB_TRY(assemble(r, Un, Un - rows));
         const ChAdjArgs fa = adj_args(r, Un, nullptr, nullptr);
-        PXB_TRY(check(c, launch_ch_fold_mobility(fa, c->csr.slot.as<int>(), c->csr.diag.as<int>(), h.kv.as<double>(),
-                                                 c->stream),
+        PXB_TRY(check(c, launch_ch_fold_mobility(fa, c->csr.slot.as<int>(), c->csr.rowptr.as<int>(),
+                                                 c->csr.exact ? c->csr.bpos.as<uint8_t>() : nullptr,
+                                                 c->csr.diag.as<int>(), h.kv.as<double>(), c->stream),
                       "ch mobility fold"));
         PXB_TRY(check(c, launch_gather_values(c->csr.nnz, c->csr.tperm.as<int>(), h.kv.as<double>(), h.kvt.as<double>(),
                                               c->stream),

@@ -44,21 +44,6 @@ __global__ void csr_map_kernel(CsrMapArgs a) {
                 }
             }
         }
-        if (a.extra) {
-            // the mirror block, when the mirror node is not a family member, and whether the rows hold anything else
-            const int m = a.mirror ? a.mirror[i] - 1 : -1;
-            bool in_fam = m == i;
-            for (int t = a.off[i]; t < a.off[i + 1] && m >= 0 && !in_fam; ++t) in_fam = a.nbr[t] == m;
-            const bool extra = m >= 0 && !in_fam;
-            const int width = nd * (1 + (a.off[i + 1] - a.off[i]) + (extra ? 1 : 0));
-            for (int r = 0; r < nd; ++r) {
-                const int row = i * nd + r;
-                const int lo = a.rowptr[row], hi = a.rowptr[row + 1];
-                if (hi - lo != width) atomicAdd(a.inexact, 1);
-                for (int c = 0; c < nd; ++c)
-                    a.extra[(size_t)i * nd * nd + r * nd + c] = extra ? find_slot(a.cols, lo, hi, m * nd + c) : -1;
-            }
-        }
     }
 }
 
@@ -151,7 +136,7 @@ __global__ void __launch_bounds__(256) assemble_stress_ch_kernel(StressChAsmArgs
         double uI[ND];
 #pragma unroll
         for (int b = 0; b < ND; ++b) uI[b] = a.u[rb + b];
-        const double Vi = a.vol[i], Mi = a.mnode[i];
+        const double Vi = a.vol[i], Mi = a.mnode[i], iV = 1.0 / Vi;
         double R[ND], S[NK];
 #pragma unroll
         for (int b = 0; b < ND; ++b) R[b] = 0.0;
@@ -165,15 +150,12 @@ __global__ void __launch_bounds__(256) assemble_stress_ch_kernel(StressChAsmArgs
 #pragma unroll
             for (int d = 0; d < DIM; ++d) G1[d] = g * op[sl[d]];
             const double Gxx = g * op[sl[3]], Gxy = g * op[sl[4]], Gyy = g * op[sl[5]];
-            const bool ghostJ = a.ghost && a.ghost[j];
+            const uint8_t f = a.bfl[t];
+            const bool ghostJ = f & 1;
             const double g2A = a.lap[t];
             double coeff_c = 0.0;
-            if (!ghostJ) {
-                const int r = a.rev[t];
-                const double w = (r >= 0 && Vi > 0.0) ? 0.5 * (Mi * g2A + (a.vol[j] / Vi) * a.mnode[j] * a.lap[r])
-                                                      : Mi * g2A;
-                coeff_c = -w;
-            }
+            if (!ghostJ)
+                coeff_c = (f & 2) && Vi > 0.0 ? species_flux(Mi, g2A, a.lrv[t], iV, a.mnode[j]) : -(Mi * g2A);
             const double kappaLap = ghostJ ? 0.0 : a.kappa * g2A;
             double k[NK];
             k[0] = coeff_c;
@@ -462,16 +444,8 @@ __global__ void __launch_bounds__(256) assemble_ch_kernel(ChAsmArgs a) {
         const int i = base + grp;
         const bool act = i < a.n;
         const int rc = 2 * i, rm = 2 * i + 1;
-        if (act) {
-            if (a.extra) {  // exact pattern: every other entry of the two rows is written below
-                if (gl < 4) {
-                    const int e = a.extra[(size_t)i * 4 + gl];
-                    if (e >= 0) a.kvals[e] = 0.0;
-                }
-            } else {
-                for (int s = a.rowptr[rc] + gl; s < a.rowptr[rm + 1]; s += LPN) a.kvals[s] = 0.0;
-            }
-        }
+        if (act)
+            for (int s = a.rowptr[rc] + gl; s < a.rowptr[rm + 1]; s += LPN) a.kvals[s] = 0.0;
         __syncwarp();
         double c = 0.0, mu = 0.0, Vi = 0.0, Mi = 0.0;
         int b0 = 0, b1 = 0;
@@ -483,30 +457,16 @@ __global__ void __launch_bounds__(256) assemble_ch_kernel(ChAsmArgs a) {
             b0 = a.off[i];
             b1 = a.off[i + 1];
         }
+        const double iV = 1.0 / Vi;
         double rcs = 0.0, rms = 0.0, k12 = 0.0, k21 = 0.0;
         for (int t = b0 + gl; t < b1; t += LPN) {
             const int j = __ldg(a.nbr + t);
             const double g2 = a.lap[t];
             double coeff_c = 0.0, coeff_mu = 0.0;
-            if (a.lrv) {  // the geometry's bond-order streams: only the mobility and u of j are gathered
-                const uint8_t f = a.bfl[t];
-                if (!(f & 1)) {
-                    double w;
-                    if ((f & 2) && Vi > 0.0) w = 0.5 * (Mi * g2 + (a.lrv[t] / Vi) * a.mnode[j]);
-                    else w = Mi * g2;
-                    coeff_c = -w;
-                    coeff_mu = a.kappa * g2;
-                }
-            } else {
-                const bool ghostJ = a.ghost && a.ghost[j];
-                if (!ghostJ) {
-                    const int r = a.rev[t];
-                    double w;
-                    if (r >= 0 && Vi > 0.0) w = 0.5 * (Mi * g2 + (a.vol[j] / Vi) * a.mnode[j] * a.lap[r]);
-                    else w = Mi * g2;
-                    coeff_c = -w;
-                    coeff_mu = a.kappa * g2;
-                }
+            const uint8_t f = a.bfl[t];  // the geometry's bond-order streams: only the mobility and u of j are gathered
+            if (!(f & 1)) {
+                coeff_c = (f & 2) && Vi > 0.0 ? species_flux(Mi, g2, a.lrv[t], iV, a.mnode[j]) : -(Mi * g2);
+                coeff_mu = a.kappa * g2;
             }
             rcs += coeff_c * (a.u[2 * (size_t)j + 1] - mu);  // u may be only 8-byte aligned (a caller's pointer)
             rms += coeff_mu * (a.u[2 * (size_t)j] - c);

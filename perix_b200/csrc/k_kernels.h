@@ -317,11 +317,29 @@ struct CsrMapArgs {
     int *slot = nullptr;   // [nb*ndof*ndof]
     int *diag = nullptr;   // [n*ndof*ndof]
     int *missing = nullptr;
-    const int *mirror = nullptr;  // 1-based mirror bulk node, 0 none (may be NULL)
-    int *extra = nullptr;         // [n*ndof*ndof] slots of the mirror block when it is not a family member, else -1
-    int *inexact = nullptr;       // rows holding entries beyond own block + family + mirror block
 };
 cudaError_t launch_csr_map(const CsrMapArgs &a, cudaStream_t s);
+// Exact block patterns (k_csr_block.cu): the rows of a node hold one list of at most kBlockMax column nodes (own,
+// family, mirror), sorted, each expanded to ndof columns.  Entry (row i ndof + r, column j ndof + c) of bond t lies
+// at rowptr[i ndof] + r W + bpos[t] ndof + c, W = rowptr[i ndof + 1] - rowptr[i ndof].
+constexpr int kBlockMax = 256;
+struct BlockMapArgs {
+    int n = 0, ndof = 1;
+    int verify = 0;  // check the rows too (a caller's pattern; the device-built one is of this form)
+    long long nnz = 0;
+    const int *off = nullptr, *nbr = nullptr, *rowptr = nullptr, *cols = nullptr;
+    const int *mirror = nullptr;  // 1-based mirror bulk node, 0 none (may be NULL)
+    uint8_t *bpos = nullptr;      // [nb] block position of bond t's neighbour in its node's list
+    uint8_t *spos = nullptr;      // [n] position of the node's own block
+    int16_t *xpos = nullptr;      // [n] position of a mirror block outside the family, -1 none
+    int *diag = nullptr;          // [n*ndof*ndof] slots of the diagonal block
+    int *inexact = nullptr;       // += nodes whose rows are of another form
+};
+cudaError_t launch_block_map(const BlockMapArgs &a, cudaStream_t s);
+struct BlockPattern {
+    const uint8_t *bpos = nullptr, *spos = nullptr;
+    const int16_t *xpos = nullptr;
+};
 
 struct ScalarAsmArgs {
     int n = 0, dim = 2, nop = 0, type = 0, mixed = 0;
@@ -339,10 +357,11 @@ struct ScalarAsmArgs {
     double *kvals = nullptr, *rhs = nullptr;
 };
 cudaError_t launch_assemble_scalar(const ScalarAsmArgs &a, cudaStream_t s);
+// the same on an exact block pattern (below, mmax: its longest block list)
+cudaError_t launch_scalar_block(const ScalarAsmArgs &a, const BlockPattern &bp, cudaStream_t s);
 
 struct ChAsmArgs {
     int n = 0;
-    const int *extra = nullptr;  // exact pattern: mirror-block slots to clear (rows are not zeroed first)
     double kappa = 0, chi = 0, dt = 1;
     const int *off = nullptr, *nbr = nullptr, *rev = nullptr;
     const double *lap = nullptr, *vol = nullptr, *mnode = nullptr;
@@ -350,13 +369,14 @@ struct ChAsmArgs {
     const int *rowptr = nullptr, *slot = nullptr, *diag = nullptr;
     const double *u = nullptr, *uold = nullptr;
     double *kvals = nullptr, *rhs = nullptr;
-    // optional bond-order streams of the fixed geometry (launch_ch_bond_streams): lrv[t] = vol[j] lap[rev t] (0
-    // without a reverse bond) and bfl[t] = (ghost j) | 2 (reverse bond exists); with them the kernel gathers only
-    // the neighbour's mobility and u
+    // bond-order streams of the fixed geometry (launch_ch_bond_streams): lrv[t] = vol[j] lap[rev t] (0 without a
+    // reverse bond) and bfl[t] = (ghost j) | 2 (reverse bond exists); with them a bond gathers only the neighbour's
+    // mobility and u
     const double *lrv = nullptr;
     const uint8_t *bfl = nullptr;
 };
 cudaError_t launch_assemble_ch(const ChAsmArgs &a, cudaStream_t s);
+cudaError_t launch_ch_block(const ChAsmArgs &a, const BlockPattern &bp, cudaStream_t s);
 cudaError_t launch_ch_bond_streams(int n, const int *off, const int *nbr, const int *rev, const double *lap,
                                    const double *vol, const char *ghost, double *lrv, uint8_t *bfl, cudaStream_t s);
 // Stress-coupled Cahn-Hilliard (rows c, mu, u_x, u_y[, u_z] per node; ndof = dim + 2): the device twin of
@@ -374,11 +394,14 @@ struct StressChAsmArgs {
     const uint8_t *degenerate = nullptr;
     const double *health = nullptr;     // [nb] frozen bond health (NULL: every bond intact)
     const double *vel = nullptr;        // [n*dim] committed velocity (inertia when rho > 0)
+    const double *lrv = nullptr;        // ChAsmArgs::lrv / bfl
+    const uint8_t *bfl = nullptr;
     const int *rowptr = nullptr, *slot = nullptr, *diag = nullptr;
     const double *u = nullptr, *uold = nullptr;
     double *kvals = nullptr, *rhs = nullptr;
 };
 cudaError_t launch_assemble_stress_ch(const StressChAsmArgs &a, cudaStream_t s);
+cudaError_t launch_stress_ch_block(const StressChAsmArgs &a, const BlockPattern &bp, int mmax, cudaStream_t s);
 // Implicit PDDO dynamic fracture (rows u per node; ndof = dim): the device twin of the reference's
 // cachedAssembleKernel (src/PDSystem/CudaAssembleKernels.cu:880-1024) on the FP64 order-2 operator cache.
 // nodecache[i*ncache + a] = committed velocity, bondcache[t*nbcache] = frozen bond health.
@@ -396,6 +419,7 @@ struct CachedAsmArgs {
     double *kvals = nullptr, *rhs = nullptr;
 };
 cudaError_t launch_assemble_cached(const CachedAsmArgs &a, cudaStream_t s);
+cudaError_t launch_cached_block(const CachedAsmArgs &a, const BlockPattern &bp, int mmax, cudaStream_t s);
 // Output projections of the explicit state (k_project.cu; ExplicitPDDOFracElement.cpp:324-405).  Outputs may be
 // NULL; stress and strain are 3x3 row-major per node.  sl = operator slots of d/dx, d/dy, d/dz.
 struct ProjectArgs {
@@ -467,8 +491,10 @@ cudaError_t launch_gather_values(long long nnz, const int *perm, const double *v
 // the whole solve A x = b (x from 0) as one cooperative kernel; the outcome is in *a.sc when it ends
 cudaError_t launch_bicg_solve(const BicgArgs &a, double tol, int max_its, cudaStream_t s);
 // K' = K - J_M in place on the (c, c) entries of bulk rows, J_M the mobility derivative the Picard Jacobian omits
-// (the adjoint operator is K'^T); slot: bond slot map, diag: diagonal slots of the 2-dof pattern
-cudaError_t launch_ch_fold_mobility(const ChAdjArgs &a, const int *slot, const int *diag, double *kv, cudaStream_t s);
+// (the adjoint operator is K'^T); the (c, c_j) entry of bond t is slot[4 t], or, with bpos (an exact block pattern,
+// slot unused), rowptr[2 i] + 2 bpos[t]; diag: diagonal slots of the 2-dof pattern
+cudaError_t launch_ch_fold_mobility(const ChAdjArgs &a, const int *slot, const int *rowptr, const uint8_t *bpos,
+                                    const int *diag, double *kv, cudaStream_t s);
 // per-node lambda_mu dF_mu/dkappa
 cudaError_t launch_ch_dkappa(const ChAdjArgs &a, cudaStream_t s);
 struct ChEnergyArgs {

@@ -153,8 +153,8 @@ __device__ __forceinline__ double mob_prime(double c, double M0) {
 //   K'[c_i, c_i] -= M'(c_i) sum_t -(paired ? g2_t / 2 : g2_t) (mu_j - mu_i),
 //   K'[c_i, c_j] -= M'(c_j) (-1/2) (V_j / V_i) g2_rev(t) (mu_j - mu_i)   (paired bonds),
 // paired = the bond has a reverse and V_i > 0.  Each bond slot belongs to one bond, so the updates do not collide.
-__global__ void __launch_bounds__(256) ch_fold_mobility_kernel(ChAdjArgs a, const int *slot, const int *diag,
-                                                               double *kv) {
+__global__ void __launch_bounds__(256) ch_fold_mobility_kernel(ChAdjArgs a, const int *slot, const int *rowptr,
+                                                               const uint8_t *bpos, const int *diag, double *kv) {
     constexpr int WPB = 256 / kWarp;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -169,17 +169,19 @@ __global__ void __launch_bounds__(256) ch_fold_mobility_kernel(ChAdjArgs a, cons
             const int r = a.rev[t];
             const bool paired = r >= 0 && Vi > 0.0;
             acc += -(paired ? 0.5 : 1.0) * a.lap[t] * dmu;
+            const int q = bpos ? rowptr[2 * i] + 2 * bpos[t] : slot[4 * (size_t)t];
             if (paired)
-                kv[slot[4 * (size_t)t]] -= mob_prime(a.u[2 * (size_t)j], a.M0) * (-0.5 * (a.vol[j] / Vi) * a.lap[r] * dmu);
+                kv[q] -= mob_prime(a.u[2 * (size_t)j], a.M0) * (-0.5 * (a.vol[j] / Vi) * a.lap[r] * dmu);
         }
         acc = group_sum<kWarp>(acc);
         if (lane == 0) kv[diag[4 * (size_t)i]] -= mob_prime(a.u[2 * (size_t)i], a.M0) * acc;
     }
 }
 
-cudaError_t launch_ch_fold_mobility(const ChAdjArgs &a, const int *slot, const int *diag, double *kv, cudaStream_t s) {
+cudaError_t launch_ch_fold_mobility(const ChAdjArgs &a, const int *slot, const int *rowptr, const uint8_t *bpos,
+                                    const int *diag, double *kv, cudaStream_t s) {
     const int g = (a.n + 7) / 8;
-    ch_fold_mobility_kernel<<<g > 0 ? g : 1, 256, 0, s>>>(a, slot, diag, kv);
+    ch_fold_mobility_kernel<<<g > 0 ? g : 1, 256, 0, s>>>(a, slot, rowptr, bpos, diag, kv);
     return cudaGetLastError();
 }
 

@@ -125,6 +125,12 @@ __device__ __forceinline__ double cd_next(double u, double up, double acc, doubl
     return __dadd_rn(__dsub_rn(__dmul_rn(2.0, u), up), __dmul_rn(dt2, acc));
 }
 
+// Cahn-Hilliard species flux of a bond, -0.5 (M_i g2_ij + (V_j g2_ji / V_i) M_j) with lrv = V_j g2_ji and iV = 1 / V_i
+// (one rounding order everywhere: the two terms may nearly cancel)
+__device__ __forceinline__ double species_flux(double Mi, double g2, double lrv, double iV, double Mj) {
+    return -0.5 * __fma_rn(__dmul_rn(lrv, iV), Mj, __dmul_rn(Mi, g2));
+}
+
 // ---- compensated FP32 accumulation (Knuth two-sum) ---------------------------------------------------------
 struct CompF {
     float s, c;

@@ -180,17 +180,19 @@ struct CsrState {
     int ndof = 1;
     long long nnz = 0;
     DevBuf rowptr, cols;
-    DevBuf slot;       // int32 [nb*ndof*ndof]: CSR slot of (row i*ndof+a, col j*ndof+b) for bond t
     DevBuf diag;       // int32 [n*ndof*ndof]: slot of the diagonal block entries
-    // exact pattern (every row = own block + family blocks + mirror block): the assembly kernels then write every
-    // entry once instead of zeroing the rows first; extra = slots of a mirror block outside the family (-1 none)
+    // exact block pattern (k_csr_block.cu): every row of a node = own block + family blocks + mirror block, at most
+    // kBlockMax of them; block positions of the bonds, the nodes and the mirrors outside their families
     bool exact = false;
+    int mmax = 0;  // longest block list
+    DevBuf bpos, spos, xpos;
+    // any other pattern: int32 [nb*ndof*ndof] CSR slot of (row i*ndof+a, col j*ndof+b) for bond t (k_csr.cu)
+    DevBuf slot;
     // ndof 2 and rows 2i, 2i+1 share one list of column pairs (2j, 2j+1): the block view (block_view) and, built on
     // first use by an adjoint solve, the block view of the transpose with its value permutation
     bool blocked2 = false, transposed = false;
     std::vector<int> h_bptr, h_bcol;
     DevBuf bptr, bcol, tbptr, tbcol, tperm;
-    DevBuf extra;      // int32 [n*ndof*ndof]
     DevBuf kvals, rhs, u, uold, fnode, mnode;
 };
 
