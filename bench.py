@@ -522,9 +522,11 @@ def read_traffic(kind, prec, variant=None):
 
 
 def kernel_name(dim, prec, tuned):
-    """The step kernel the autotuner picked (variants 0-2 lane groups, 3-4 CSR tiles, 5 and up TMA-staged)."""
+    """The step kernel the autotuner picked (variants 0-2 lane groups, 3-4 CSR tiles, 5-16 TMA-staged, 17-20 sliced)."""
     v, lpn = tuned["variant"], tuned["lanes_per_node"]
     mixed = "true" if prec == "mixed" else "false"
+    if v >= 17:
+        return "pxb::epf_sliced_kernel<%d,%s,...> (variant %d)" % (dim, mixed, v)
     if v >= 5:
         return "pxb::epf_tma_kernel<%d,%s,LPN=%d,...> (variant %d)" % (dim, mixed, lpn, v)
     if v >= 3:

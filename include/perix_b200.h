@@ -183,8 +183,8 @@ int pxb_epf_setup(pxb_ctx *ctx, int precision, double C11, double C12, double C6
 /* Variable horizon: every bond breaks at its own critical stretch s_c(0.5 (delta_i + delta_j)) from the fracture
  * energy G0, Young's modulus E and (2D) plane stress (ExplicitPDDOFracElement.cpp:254-261 with
  * FractureCriterion.h:30-43), instead of the uniform sc of pxb_epf_setup.  Needs pxb_set_node_horizons; call after
- * pxb_epf_setup.  The staged step kernels do not read per-bond thresholds: their variants then run the lane-group
- * kernel. */
+ * pxb_epf_setup.  The staged and sliced step kernels do not read per-bond thresholds: their variants then run the
+ * lane-group kernel. */
 int pxb_epf_set_variable_horizon_stretch(pxb_ctx *ctx, double G0, double E, int plane_stress);
 /* One rate evaluation at u (N*dim): damage then force, a = (L+b)/rho (the reference CUDA entry
  * assembleExplicitPDDOFracAccel).  *n_broken = bonds that broke in this call. */
@@ -301,11 +301,13 @@ int pxb_epf_set_constants(pxb_ctx *ctx, double C11, double C12, double C66, doub
 int pxb_epf_snapshot(pxb_ctx *ctx);
 int pxb_epf_restore(pxb_ctx *ctx);
 /* Schedule variants of the explicit kernel: 0-2 lane groups (lanes per node x bonds per lane per pass), 3-4
- * CSR-stream tiles, 5 and up TMA-staged tiles (time step only; the other modes of a staged variant run
- * variant 1).  pxb_epf_variant_count() gives their number.  pxb_epf_autotune times every variant that fits
- * for `steps` steps from a private copy of the current state (L2 flushed before each step), restores the
- * state, selects the fastest and caches the choice per problem signature (dim, precision, nodes, bonds,
- * largest family); use_cache=1 returns a cached choice without timing.  ms_per_variant (may be NULL;
+ * CSR-stream tiles, 5-16 TMA-staged tiles, 17-20 sliced (time step and rate call only; the other modes of a staged or
+ * sliced variant run variant 1).  A sliced variant keeps a second, neighbour-sorted copy of the bond streams (about
+ * 54 bytes a bond in 3D FP64, 30 mixed), built when it is first selected; without room for it pxb_epf_set_variant
+ * fails with PXB_ERR_OOM and the autotuners skip it.  pxb_epf_variant_count() gives their number.  pxb_epf_autotune
+ * times every variant that fits for `steps` steps from a private copy of the current state (L2 flushed before each
+ * step), restores the state, selects the fastest and caches the choice per problem signature (dim, precision, nodes,
+ * bonds, largest family); use_cache=1 returns a cached choice without timing.  ms_per_variant (may be NULL;
  * pxb_epf_variant_count() entries) receives the mean step time of each variant, -1 for one that does not fit. */
 int pxb_epf_variant_count(void);
 int pxb_epf_autotune(pxb_ctx *ctx, int steps, size_t flush_bytes, int use_cache, int *best, float *ms_per_variant);

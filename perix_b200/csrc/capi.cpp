@@ -128,7 +128,8 @@ size_t ctx_bytes(const pxb_ctx *c) {
     s += bufsz(c->ops.ops) + bufsz(c->ops.degenerate) + bufsz(c->ops.defect) + bufsz(c->ops.yeff);
     const EpfState &e = c->epf;
     s += bufsz(e.G) + bufsz(e.P) + bufsz(e.xib) + bufsz(e.health) + bufsz(e.u[0]) + bufsz(e.u[1]) + bufsz(e.accel) + bufsz(e.counters) +
-         bufsz(e.umax) + bufsz(e.tsched) + bufsz(e.sc_bond);
+         bufsz(e.umax) + bufsz(e.tsched) + bufsz(e.sc_bond) + bufsz(e.sl_row0) + bufsz(e.sl_word) + bufsz(e.sl_P) +
+         bufsz(e.sl_src);
     s += bufsz(e.adj_ckpt) + bufsz(e.adj_seg) + bufsz(e.adj_p[0]) + bufsz(e.adj_p[1]) + bufsz(e.adj_A) + bufsz(e.adj_R) +
          bufsz(e.adj_W) + bufsz(e.adj_t) + bufsz(e.adj_dC) + bufsz(e.adj_umax) + bufsz(e.adj_GR) + bufsz(e.adj_HR) + bufsz(e.adj_u0) + bufsz(e.adj_SG) + bufsz(e.adj_UW);
     s += bufsz(e.bc.own) + bufsz(e.bc.src_off) + bufsz(e.bc.tgt) + bufsz(e.bc.comp) + bufsz(e.bc.form) +
@@ -735,6 +736,110 @@ static EpfArgs epf_args(pxb_ctx *c) {
     return a;
 }
 
+// ---- the sliced step's streams ----------------------------------------------------------------------------------
+namespace pxb {
+namespace {
+
+bool runs_sliced(const EpfState &e) { return epf_is_sliced(e.variant) && !e.sc_bond.p; }
+
+int sliced_build(pxb_ctx *c) {
+    EpfState &e = c->epf;
+    const Geometry &g = c->g;
+    const int n = g.n, slices = (n + 31) / 32;
+    std::vector<int> row0((size_t)slices + 1, 0);
+    for (int s = 0; s < slices; ++s) {
+        int rows = 0;
+        for (int i = 32 * s; i < std::min(n, 32 * s + 32); ++i)
+            rows = std::max(rows, g.h_off[(size_t)i + 1] - g.h_off[(size_t)i]);
+        if (row0[(size_t)s] > (1 << 25) - rows)  // 32-bit entry indices
+            return fail(PXB_ERR_UNSUPPORTED, "sliced step: more than 2^30 stream entries");
+        row0[(size_t)s + 1] = row0[(size_t)s] + rows;
+    }
+    const size_t entries = 32 * (size_t)std::max(1, row0.back());
+    const int nc = g.dim == 3 ? 6 : 3;
+    const bool mixed = e.precision == PXB_MIXED;
+    int st = dev_upload(c, e.sl_row0, row0.data(), sizeof(int) * row0.size());
+    if (st == PXB_OK) st = dev_alloc(c, e.sl_word, sizeof(int) * (entries + 32 * kSlicedSlack));
+    if (st == PXB_OK) st = dev_alloc(c, e.sl_src, sizeof(uint16_t) * entries);
+    if (st == PXB_OK) st = dev_alloc(c, e.sl_P, (mixed ? 4 : 8) * (size_t)nc * entries);
+    if (st != PXB_OK) {
+        for (DevBuf *b : {&e.sl_row0, &e.sl_word, &e.sl_src, &e.sl_P}) b->release();
+        return st;
+    }
+    int idbits = 1;
+    while (idbits < 31 && (n - 1) >> idbits) ++idbits;
+    const int qbits = std::min(7, 31 - idbits);
+    static_assert(kSlicedClasses == 1 << 7, "length classes");
+    e.sl_shift = 31 - qbits;
+    unsigned long long *key = e.counters.as<unsigned long long>() + 5;  // the set-up's scratch counter
+    PXB_CUDA_TRY(cudaMemsetAsync(key, 0, sizeof(*key), c->stream));
+    PXB_CUDA_TRY(launch_sliced_rank(n, g.dim, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, e.sl_row0.as<int>(),
+                                    e.sl_src.as<uint16_t>(), key, c->stream));
+    unsigned long long k2 = 0;
+    PXB_TRY(d2h(c, &k2, key, sizeof(k2)));
+    PXB_TRY(sync(c));  // (row0 leaves scope here too)
+    double r2 = 0.0;
+    std::memcpy(&r2, &k2, sizeof(double));
+    e.sl_step = std::isfinite(r2) ? std::sqrt(r2) / (1 << qbits) : 0.0;
+    PXB_CUDA_TRY(launch_sliced_fill(n, g.dim, mixed, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, e.sl_row0.as<int>(),
+                                    e.sl_src.as<uint16_t>(), e.sl_shift, e.sl_step > 0.0 ? 1.0 / e.sl_step : 0.0,
+                                    (1 << qbits) - 1, e.P.p, (long long)g.ldb, e.sl_word.as<int>(), e.sl_P.p, c->stream));
+    c->launches += 2;
+    e.sl_ready = true;
+    e.sl_P_stale = false;
+    e.sl_stale = true;
+    return PXB_OK;
+}
+
+SlicedArgs sliced_args(const EpfState &e) {
+    SlicedArgs s;
+    s.row0 = e.sl_row0.as<int>();
+    s.word = e.sl_word.as<int>();
+    s.P = e.sl_P.p;
+    s.src = e.sl_src.as<uint16_t>();
+    s.shift = e.sl_shift;
+    const double m = e.sc * (1.0 - 1.0e-6) - 1.0e-12;
+    s.clear = m > 0.0 ? m * m * e.sl_step * e.sl_step : 0.0;
+    return s;
+}
+
+}  // namespace
+
+int epf_ready(pxb_ctx *c) {
+    EpfState &e = c->epf;
+    if (!runs_sliced(e)) return PXB_OK;
+    const Geometry &g = c->g;
+    if (!e.sl_ready) PXB_TRY(sliced_build(c));
+    if (e.sl_P_stale) {
+        PXB_CUDA_TRY(launch_sliced_fill(g.n, g.dim, e.precision == PXB_MIXED, g.off.as<int>(), g.nbr.as<int>(), g.pos.p,
+                                        e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(), 0, 0.0, 0, e.P.p, (long long)g.ldb,
+                                        nullptr, e.sl_P.p, c->stream));
+        c->launches++;
+        e.sl_P_stale = false;
+    }
+    if (e.sl_stale) {
+        PXB_CUDA_TRY(launch_sliced_health(g.n, g.off.as<int>(), e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(),
+                                          e.health.as<uint8_t>(), e.sl_word.as<int>(), c->stream));
+        c->launches++;
+        e.sl_stale = false;
+    }
+    return PXB_OK;
+}
+
+cudaError_t epf_launch(pxb_ctx *c, const EpfArgs &a, int mode, int variant, cudaStream_t s) {
+    EpfState &e = c->epf;
+    const bool mixed = e.precision == PXB_MIXED;
+    if (epf_is_sliced(variant) && !a.sc_bond && !e.sc_bond.p && (mode == EPF_STEP || (mode == EPF_RATE && a.accel))) {
+        if (!e.sl_ready) return cudaErrorNotReady;
+        EpfArgs r = a;
+        r.rate = mode == EPF_RATE ? 1 : 0;
+        return launch_epf_sliced(r, sliced_args(e), c->g.dim, mixed, variant - 5 - kEpfTmaConfigs, s);
+    }
+    if (a.damage && mode != EPF_FORCE_FROZEN) e.sl_stale = true;
+    return launch_epf(a, c->g.dim, mixed, mode, variant, s);
+}
+}  // namespace pxb
+
 extern "C" int pxb_epf_setup(pxb_ctx *c, int precision, double C11, double C12, double C66, double rho,
                              const double *b, double sc, int tension_only, const uint8_t *health0) {
     PXB_TRY(need_geometry(c, "pxb_epf_setup"));
@@ -845,7 +950,7 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
     const size_t nd = (size_t)c->g.n * c->g.dim;
     unsigned long long *cnt = e.counters.as<unsigned long long>();
     // (a per-bond critical stretch runs the lane-group kernel, which computes every node: no chunking then)
-    if (pinned && e.rate_K > 1 && epf_is_tma(e.variant) && !e.sc_bond.p) {
+    if (pinned && e.rate_K > 1 && e.variant >= 5 && !e.sc_bond.p) {
         // pieces of u go up on one stream, each chunk's kernel starts once its neighbours' piece is there, and each
         // chunk's acceleration goes down on another stream while the next chunk computes
         const int K = e.rate_K, dim = c->g.dim;
@@ -879,7 +984,7 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
             err = cudaStreamWaitEvent(s, ev[2 + e.rate_need[(size_t)k]], 0);
             a.node0 = b[k];
             a.n = b[k + 1];
-            if (err == cudaSuccess) err = launch_epf(a, dim, e.precision == PXB_MIXED, EPF_RATE, e.variant, s);
+            if (err == cudaSuccess) err = epf_launch(c, a, EPF_RATE, e.variant, s);
             if (err == cudaSuccess) err = cudaEventRecord(ev[2 + K + k], s);
             if (err == cudaSuccess) err = cudaStreamWaitEvent(e.rate_down, ev[2 + K + k], 0);
             if (err == cudaSuccess)
@@ -901,7 +1006,7 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
     EpfArgs a = epf_args(c);
     a.u = e.u[e.cur].as<double>();
     a.accel = e.accel.as<double>();
-    err = launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_RATE, e.variant, s);
+    err = epf_launch(c, a, EPF_RATE, e.variant, s);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(accel, e.accel.p, sizeof(double) * nd, cudaMemcpyDeviceToHost, s);
     if (err == cudaSuccess)
@@ -951,6 +1056,8 @@ extern "C" int pxb_epf_rate(pxb_ctx *c, const double *u, double *accel, long lon
     EpfState &e = c->epf;
     PXB_TRY(ensure_pinned(e.rate_h, sizeof(unsigned long long) * 5));
     PXB_TRY(rate_plan(c));
+    PXB_TRY(epf_ready(c));
+    if (!runs_sliced(e)) e.sl_stale = true;  // (a replayed graph does not pass epf_launch)
     // pinned buffers that the previous call used too, with the same schedule: replay (or capture) the call as one
     // graph; otherwise (first call with these buffers or this schedule, or pageable memory) queue the operations
     // one by one, which also gives a kernel its first, uncaptured launch
@@ -1210,7 +1317,7 @@ extern "C" int pxb_epf_start(pxb_ctx *c, const double *u0, const double *v0, dou
     a.v0 = dv0;
     a.dt = dt;
     a.dt2 = 0.5 * dt * dt;
-    launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_START, e.variant, c->stream);
+    epf_launch(c, a, EPF_START, e.variant, c->stream);
     PXB_TRY(check_launch(c, "epf start"));
     PXB_TRY(sync(c));
     e.dt = dt;
@@ -1257,7 +1364,7 @@ static int launch_step(pxb_ctx *c, int par, int q, cudaStream_t s, bool pdl = fa
     step_args(c, par, &a);
     a.step_in_chunk = q;
     a.pdl = pdl ? 1 : 0;
-    const cudaError_t err = launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_STEP, e.variant, s);
+    const cudaError_t err = epf_launch(c, a, EPF_STEP, e.variant, s);
     if (err != cudaSuccess) return cuda_fail(err, "epf step launch");
     return PXB_OK;
 }
@@ -1322,6 +1429,8 @@ extern "C" int pxb_epf_advance(pxb_ctx *c, int nsteps, int chunk, int *bad_step)
         destroy_graphs(e);
         e.graph_chunk = chunk;
     }
+    PXB_TRY(epf_ready(c));
+    if (!runs_sliced(e)) e.sl_stale = true;  // (a replayed graph does not pass epf_launch)
     int done = 0;
     std::vector<unsigned long long> keys((size_t)chunk);
     while (done < nsteps) {
@@ -1368,6 +1477,7 @@ static int single_step(pxb_ctx *c, double dtA, int *bad_step) {
     th[0] = t_new;
     PXB_TRY(h2d(c, e.tsched.p, th, sizeof(double)));
     PXB_CUDA_TRY(cudaMemsetAsync(e.umax.p, 0, sizeof(unsigned long long), c->stream));
+    PXB_TRY(epf_ready(c));
     EpfArgs a;
     PXB_TRY(step_args(c, e.cur, &a));
     a.step_in_chunk = 0;
@@ -1375,7 +1485,7 @@ static int single_step(pxb_ctx *c, double dtA, int *bad_step) {
     a.var_step = dtA == e.dt_prev ? 0 : 1;
     a.cv_rho = dtA / e.dt_prev;
     a.cv_w = 0.5 * dtA * (dtA + e.dt_prev);
-    const cudaError_t err = launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_STEP, e.variant, c->stream);
+    const cudaError_t err = epf_launch(c, a, EPF_STEP, e.variant, c->stream);
     if (err != cudaSuccess) return cuda_fail(err, "epf variable step launch");
     c->launches++;
     unsigned long long key = 0;
@@ -1460,6 +1570,7 @@ extern "C" int pxb_epf_set_state(pxb_ctx *c, const double *u, const double *u_pr
     if (u) PXB_TRY(h2d(c, e.u[e.cur].p, u, sizeof(double) * nd));
     if (u_prev) PXB_TRY(h2d(c, e.u[e.cur ^ 1].p, u_prev, sizeof(double) * nd));
     if (health) PXB_TRY(h2d(c, e.health.p, health, (size_t)c->g.nb));
+    if (health) e.sl_stale = true;
     e.t = t;
     if (u && u_prev) e.started = true;
     return sync(c);
@@ -1487,7 +1598,7 @@ extern "C" int pxb_epf_force_frozen_d(pxb_ctx *c, const double *u_d, double *a_d
     a.u = u_d;
     a.accel = a_d;
     a.damage = 0;
-    launch_epf(a, c->g.dim, c->epf.precision == PXB_MIXED, EPF_FORCE_FROZEN, c->epf.variant, c->stream);
+    epf_launch(c, a, EPF_FORCE_FROZEN, c->epf.variant, c->stream);
     return check_launch(c, "epf force (frozen mask)");
 }
 
@@ -1534,6 +1645,7 @@ extern "C" int pxb_epf_set_constants(pxb_ctx *c, double C11, double C12, double 
     e.C12 = C12;
     e.C66 = C66;
     e.rho = rho;
+    e.sl_P_stale = true;
     PXB_CUDA_TRY(launch_navier_pack(e.G.p, e.P.p, (long long)c->g.ldb, c->g.dim, e.precision == PXB_MIXED, C11, C12,
                                     C66, c->stream));
     return check_launch(c, "navier pack");
@@ -1592,7 +1704,7 @@ int adj_step(pxb_ctx *c, double *cur, double *other, const double *tsched, int q
     a.damage = 0;
     a.sc_bond = nullptr;
     a.pdl = 0;
-    const cudaError_t err = launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_STEP, e.variant, c->stream);
+    const cudaError_t err = epf_launch(c, a, EPF_STEP, e.variant, c->stream);
     if (err != cudaSuccess) return cuda_fail(err, "adjoint forward step");
     c->launches++;
     return PXB_OK;
@@ -1676,6 +1788,7 @@ extern "C" int pxb_epf_record_d(pxb_ctx *c, const double *u0_d, const double *v0
         return fail(PXB_ERR_INVALID, "pxb_epf_record_d: need u0, dt > 0, nsteps >= 0");
     EpfState &e = c->epf;
     e.rec_steps = -1;
+    PXB_TRY(epf_ready(c));
     const size_t nd = (size_t)c->g.n * c->g.dim, bytes = sizeof(double) * nd;
     // every state kept when checkpoint_every <= 0 or covers the run: the reverse sweep then recomputes nothing
     const bool all = checkpoint_every <= 0 || checkpoint_every >= nsteps;
@@ -1710,7 +1823,7 @@ extern "C" int pxb_epf_record_d(pxb_ctx *c, const double *u0_d, const double *v0
         a.dt2 = 0.5 * dt * dt;
         a.damage = 0;
         a.sc_bond = nullptr;
-        const cudaError_t err = launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_START, 1, c->stream);
+        const cudaError_t err = epf_launch(c, a, EPF_START, 1, c->stream);
         if (err != cudaSuccess) return cuda_fail(err, "recorded start");
         c->launches++;
         PXB_TRY(d2d(P[0], u0_d, bytes));
@@ -1751,6 +1864,7 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
         return fail(PXB_ERR_STATE, "pxb_epf_adjoint_recorded_d: no recorded forward loop (pxb_epf_record_d)");
     if (!ubar_N_d || !u0bar_d) return fail(PXB_ERR_INVALID, "pxb_epf_adjoint_recorded_d: need dJ/du^N and dJ/du0");
     PXB_TRY(ensure_grev(c));
+    PXB_TRY(epf_ready(c));  // (recomputed segments)
     struct SgOff {  // the reverse-only kernel is used inside this sweep only
         EpfState &e;
         ~SgOff() { e.adj_sg_on = false; }

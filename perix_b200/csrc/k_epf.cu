@@ -932,7 +932,8 @@ static cudaError_t launch_dm(const EpfArgs &a, int mode, int variant, cudaStream
     }
 }
 
-bool epf_is_tma(int variant) { return variant >= 5; }
+bool epf_is_tma(int variant) { return variant >= 5 && variant < 5 + kEpfTmaConfigs; }
+bool epf_is_sliced(int variant) { return variant >= 5 + kEpfTmaConfigs; }
 
 int epf_tma_maxb(int dim, int variant, int max_family) {
     const int nt = epf_tma_tile_nodes(dim, variant - 5);
@@ -942,6 +943,7 @@ int epf_tma_maxb(int dim, int variant, int max_family) {
 
 cudaError_t launch_epf(const EpfArgs &a, int dim, bool mixed, int mode, int variant, cudaStream_t s) {
     if (a.sc_bond && epf_is_tma(variant)) variant = 1;  // per-bond critical stretch: the lane-group kernels read it
+    if (epf_is_sliced(variant)) variant = 1;            // (the modes the sliced kernel does not implement)
     if (epf_is_tma(variant)) {
         if (mode == EPF_STEP) return launch_epf_tma(a, dim, mixed, variant - 5, s);
         if (mode == EPF_RATE && a.accel) {
@@ -957,15 +959,17 @@ cudaError_t launch_epf(const EpfArgs &a, int dim, bool mixed, int mode, int vari
 
 int epf_lanes_per_node(int dim, int variant) {
     if (epf_is_tma(variant)) return epf_tma_lanes(dim, variant - 5);
+    if (epf_is_sliced(variant)) return 1;
     return dim == 3 ? kLpn3[variant] : kLpn2[variant];
 }
 
 int epf_tile_nodes(int dim, int variant) {
-    if (epf_is_tma(variant)) return 0;
+    if (variant >= 5) return 0;
     return dim == 3 ? kTile3[variant] : kTile2[variant];
 }
 
 bool epf_variant_fits(int dim, int variant, int max_family) {
+    if (epf_is_sliced(variant)) return max_family <= 0xffff;
     if (epf_is_tma(variant)) {
         const int maxb = epf_tma_maxb(dim, variant, max_family);
         return epf_tma_smem(dim, false, variant - 5, maxb) <= 227u * 1024u;

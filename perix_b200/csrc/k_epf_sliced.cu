@@ -1,0 +1,483 @@
+// explicit_pddo_frac step on a sliced, neighbour-sorted copy of the bond streams.
+//
+// What bounds the step is memory: 53 bytes a bond in 3D FP64 (29 mixed), and the gathers of the neighbours'
+// displacements.  The lanes-per-node kernels (k_epf.cu, k_epf_tma.cu) read the streams in family order, where the 32
+// lanes of a warp gather 32 unrelated rows of u, three 8-byte loads each, and wait for them with 16-24 warps an SM.
+// Here a slice is 32 consecutive nodes, a lane a node, and row k of a slice holds the k-th bond of every node with the
+// families sorted by neighbour id.  On a lattice the k-th neighbours of consecutive nodes are consecutive nodes, so a
+// gather is one run of u; on any mesh the coefficients and ids are read as full 256- and 128-byte lines, whose
+// addresses depend on nothing, so several rows are in flight a warp without shared memory, barriers or waits.
+//
+// A bond's word is (broken << 31 | q << shift | neighbour): q is its length in units of step = r_max / 2^(31 - shift),
+// rounded down (at most 7 bits, what the ids leave of 31).  A bond whose relative displacement satisfies
+// |e|^2 < (s_c (1 - 1e-6) - 1e-12)^2 (q step)^2 holds under either criterion, whatever its direction, because its stretch is
+// at most |e| / |xi|; only the others gather the position for the reference's test, so every decision is the
+// reference's.  (The bound with the mesh's shortest bond in place of q step, the staged kernels' test, clears few
+// bonds once the strain passes a third of s_c at a horizon of three spacings.)
+// The health bytes stay the truth: a bond that breaks is written there and in its word, and the words are brought up to
+// date (sliced_health_kernel) before a step whenever anything else may have written health.
+// KW warps share a slice's rows (their sums meet in shared memory), so that a mesh of few slices still fills the chip.
+// B200, a state with strains about the threshold: the 44.2 M-bond slab 550 -> 352 us a step in FP64 (2.36 GB of streams:
+// 6.7 TB/s, the measured copy rate) and 451 -> 246 us mixed (5.2 TB/s; latency and issue, at 24 warps an SM), against
+// the best staged configuration; the 2.25 M-bond plate in a captured loop 21.0 -> 16.1 us FP64, 16.1 -> 13.6 us mixed.
+#include <type_traits>
+
+#include "k_kernels.h"
+#include "pxb_common.cuh"
+
+namespace pxb {
+
+namespace {
+
+
+__device__ __forceinline__ unsigned long long stream_policy(bool evict) {
+    unsigned long long p;
+    if (evict) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ double ld_stream(const double *p, unsigned long long pol) {
+    double v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ float ld_stream(const float *p, unsigned long long pol) {
+    float v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    return v;
+}
+// a bond's word: a step writes the words of the bonds it breaks, so no read-only path
+__device__ __forceinline__ int ld_word(const int *p, unsigned long long pol) {
+    int v;
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    return v;
+}
+
+// whether an intact bond clearly holds: a squared comparison in contracted arithmetic, whose rounding is far inside
+// the 1e-6 r^2 band folded into hi / lo (a zero-length bond is never tested and holds)
+template <int DIM, typename PosT>
+__device__ __forceinline__ bool clearly_holds(const PosT &xi, const PosT &xj, const double *e, double hi, double lo,
+                                              bool tension_only) {
+    double x[DIM];
+    x[0] = xj.x - xi.x;
+    x[1] = xj.y - xi.y;
+    if constexpr (DIM == 3) x[2] = xj.z - xi.z;
+    double r2 = 0.0, y2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const double y = x[d] + e[d];
+        r2 = fma(x[d], x[d], r2);
+        y2 = fma(y, y, y2);
+    }
+    return (y2 < hi * r2 && (tension_only || y2 > lo * r2)) || !(r2 > 0.0);
+}
+
+// whether it breaks, in the reference's rounding where the squared comparison is within 1e-6 r^2 of the threshold
+// (ExplicitPDDOFracElement.cpp:239-299)
+template <int DIM, typename PosT>
+__device__ __forceinline__ bool breaks(const PosT &xi, const PosT &xj, const double *e, const EpfArgs &a) {
+    const double x0 = __dsub_rn(xj.x, xi.x), x1 = __dsub_rn(xj.y, xi.y);
+    const double y0 = __dadd_rn(x0, e[0]), y1 = __dadd_rn(x1, e[1]);
+    double r2 = __dadd_rn(__dmul_rn(x0, x0), __dmul_rn(x1, x1)), y2 = __dadd_rn(__dmul_rn(y0, y0), __dmul_rn(y1, y1));
+    if constexpr (DIM == 3) {
+        const double x2 = __dsub_rn(xj.z, xi.z), yz = __dadd_rn(x2, e[2]);
+        r2 = __dadd_rn(r2, __dmul_rn(x2, x2));
+        y2 = __dadd_rn(y2, __dmul_rn(yz, yz));
+    }
+    if (!(r2 > 0.0)) return false;
+    const double band = 1.0e-6 * r2, qh = y2 - a.sc_hi2 * r2, ql = a.sc_lo2 * r2 - y2;
+    if (qh > band || (!a.tension_only && ql > band)) return true;
+    if (qh < -band && (a.tension_only || ql < -band)) return false;
+    const double r = sqrt(r2), s = __ddiv_rn(__dsub_rn(sqrt(y2), r), r);
+    return (a.tension_only ? s : fabs(s)) > a.sc;
+}
+
+template <int DIM, typename GT>
+__device__ __forceinline__ void add_force(const GT *g, const double *e, double *L) {
+    if constexpr (DIM == 3) {
+        L[0] = fma((double)g[0], e[0], fma((double)g[3], e[1], fma((double)g[4], e[2], L[0])));
+        L[1] = fma((double)g[3], e[0], fma((double)g[1], e[1], fma((double)g[5], e[2], L[1])));
+        L[2] = fma((double)g[4], e[0], fma((double)g[5], e[1], fma((double)g[2], e[2], L[2])));
+    } else {
+        L[0] = fma((double)g[0], e[0], fma((double)g[2], e[1], L[0]));
+        L[1] = fma((double)g[2], e[0], fma((double)g[1], e[1], L[1]));
+    }
+}
+
+template <int DIM>
+__device__ __forceinline__ void load_u(const double *u, size_t i, double *v) {
+    if constexpr (DIM == 2) {
+        const double2 w = __ldg(reinterpret_cast<const double2 *>(u) + i);
+        v[0] = w.x;
+        v[1] = w.y;
+    } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[d] = __ldg(u + i * 3 + d);
+    }
+}
+
+}  // namespace
+
+// KW warps a slice, SPB slices a block, U rows in flight a lane.  The loop has no bounds of its own: short families are
+// padded with broken words and zero coefficients (0.1 % of a 2D lattice's entries, 0.4-2 % in 3D), and the words are
+// read U rows ahead, past the slice's end if need be (kSlicedSlack rows after the last slice).
+template <int DIM, bool MIXED, int KW, int SPB, int U, int MINB>
+__global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs a, SlicedArgs sl) {
+    using GT = typename std::conditional<MIXED, float, double>::type;
+    using PosT = typename Vec<DIM>::T;
+    constexpr int NC = DIM == 3 ? 6 : 3;
+    static_assert(U <= kSlicedSlack, "words are read U rows ahead");
+    __shared__ double part[SPB][KW > 1 ? KW - 1 : 1][DIM][32];
+    __shared__ double clear[2 * kSlicedClasses];  // by word >> shift: |e|^2 below it clearly holds; broken: nothing does
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, sub = wib / KW, w = wib % KW;
+    const int slice = a.node0 / 32 + blockIdx.x * SPB + sub;
+    const int i = slice * 32 + lane;
+    const bool act = i < a.n;
+    const bool rate = a.rate != 0;
+    int r0 = 0, rows = 0;
+    if (slice * 32 < a.n) {
+        r0 = __ldg(sl.row0 + slice);
+        rows = __ldg(sl.row0 + slice + 1) - r0;
+    }
+    for (int q = threadIdx.x; q < 2 * kSlicedClasses; q += KW * SPB * 32)
+        clear[q] = q >> (31 - sl.shift) ? -1.0 : a.damage ? sl.clear * (double)(q * q) : __longlong_as_double(0x7ff0000000000000LL);
+    const int kb = rows * w / KW, ke = rows * (w + 1) / KW;
+    const GT *P = static_cast<const GT *>(sl.P) + ((size_t)(r0 + kb) * NC * 32 + lane);
+    const int *W = sl.word + ((size_t)(r0 + kb) * 32 + lane);
+    const unsigned long long pol = stream_policy(a.evict_first);
+    const unsigned idmask = (1u << sl.shift) - 1u;
+    const PosT *pos = static_cast<const PosT *>(a.pos);
+    const double hi = a.sc_hi2 - 1.0e-6, lo = a.sc_lo2 + 1.0e-6;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // (words and u are written by the step before)
+    double ui[DIM], up[DIM], L[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) ui[d] = up[d] = L[d] = 0.0;
+    unsigned own_bits = 0;
+    int e0 = 0, e1 = 0;
+    int wd[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) wd[q] = ld_word(W + q * 32, pol);
+    if (act) {
+        load_u<DIM>(a.u, i, ui);
+        if (w == 0 && !rate) {
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) up[d] = a.u_other[(size_t)i * DIM + d];
+            if (a.bc_own) own_bits = __ldg(a.bc_own + i);
+            if (a.bc_off) {
+                e0 = __ldg(a.bc_off + i);
+                e1 = __ldg(a.bc_off + i + 1);
+            }
+        }
+    }
+    unsigned broken = 0;
+    // N rows whose words are in wd: coefficients and displacements, the words U rows on, then the arithmetic
+    auto pass = [&](auto count) {
+        constexpr int N = decltype(count)::value;
+        GT p[N][NC];
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) p[q][c] = ld_stream(P + (q * NC + c) * 32, pol);
+        double e[N][DIM];
+#pragma unroll
+        for (int q = 0; q < N; ++q) load_u<DIM>(a.u, (unsigned)wd[q] & idmask, e[q]);
+        int wn[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) wn[q] = ld_word(W + (U + q) * 32, pol);
+        bool hold[N], open = false;  // open: intact bonds that the clear test does not decide
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            double ee = 0.0;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                e[q][d] = __dsub_rn(e[q][d], ui[d]);
+                ee = fma(e[q][d], e[q][d], ee);
+            }
+            hold[q] = ee < clear[(unsigned)wd[q] >> sl.shift];
+            open = open || (!hold[q] && wd[q] >= 0);
+        }
+        unsigned late = 0;
+        if (__any_sync(kFull, open)) {  // these rows' positions, all at once
+            const PosT xi = ldg_vec(pos + (act ? i : 0));
+            PosT xj[N];
+#pragma unroll
+            for (int q = 0; q < N; ++q) xj[q] = ldg_vec(pos + ((unsigned)wd[q] & idmask));
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+                if (!hold[q] && wd[q] >= 0) {
+                    hold[q] = clearly_holds<DIM>(xi, xj[q], e[q], hi, lo, a.tension_only);
+                    if (!hold[q]) late |= 1u << q;
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+            if (hold[q]) add_force<DIM>(p[q], e[q], L);
+        // the few bonds near the threshold or past it, everything read again (nothing of the fast path is kept for them)
+        while (late) {
+            const int q = __ffs(late) - 1;
+            late &= late - 1;
+            const int wq = ld_word(W + q * 32, pol), j = (unsigned)wq & idmask;
+            double ej[DIM];
+            load_u<DIM>(a.u, j, ej);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) ej[d] = __dsub_rn(ej[d], ui[d]);
+            if (a.damage && breaks<DIM>(ldg_vec(pos + i), ldg_vec(pos + j), ej, a)) {
+                const size_t at = (size_t)(W + q * 32 - sl.word);
+                sl.word[at] = wq | (int)0x80000000u;
+                a.health[__ldg(a.off + i) + sl.src[at]] = 0;
+                ++broken;
+            } else {
+                GT g[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) g[c] = __ldg(P + (q * NC + c) * 32);
+                add_force<DIM>(g, ej, L);
+            }
+        }
+        P += N * NC * 32;
+        W += N * 32;
+        if constexpr (N == U) {
+#pragma unroll
+            for (int q = 0; q < U; ++q) wd[q] = wn[q];
+        } else {  // (the last rows, one at a time: the words move up)
+#pragma unroll
+            for (int q = 0; q + 1 < U; ++q) wd[q] = wd[q + 1];
+        }
+    };
+    int k = kb;
+    for (; k + U <= ke; k += U) pass(std::integral_constant<int, U>{});
+    if constexpr (U > 1)
+        for (; k < ke; ++k) pass(std::integral_constant<int, 1>{});
+    if (__any_sync(kFull, broken != 0)) {
+        broken = __reduce_add_sync(kFull, broken);
+        if (lane == 0 && a.n_broken) atomicAdd(a.n_broken, (unsigned long long)broken);
+    }
+    if constexpr (KW > 1) {
+        if (w > 0)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) part[sub][w - 1][d][lane] = L[d];
+        __syncthreads();
+        if (w > 0) return;
+#pragma unroll
+        for (int q = 0; q < KW - 1; ++q)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) L[d] += part[sub][q][d][lane];
+    }
+    double umax = 0.0, un[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const double acc = __ddiv_rn(__dadd_rn(L[d], a.b[d]), a.rho);
+        un[d] = 0.0;
+        if (act && rate) a.accel[(size_t)i * DIM + d] = acc;
+        if (act && !rate) {
+            un[d] = cd_next(ui[d], up[d], acc, a.dt2, a.var_step, a.cv_rho, a.cv_w);
+            if (!((own_bits >> d) & 1u)) {
+                a.u_other[(size_t)i * DIM + d] = un[d];
+                umax = max_nan(umax, fabs(un[d]));
+            }
+        }
+    }
+    if (rate) return;
+    const double t_new = e1 > e0 ? a.t_sched[a.step_in_chunk] : 0.0;
+    for (int q = e0; q < e1; ++q) {  // the BC entries that read this node's new value (see EpfArgs)
+        const int comp = a.bc_comp[q], form = a.bc_form[q];
+        const double g1 = __dadd_rn(a.bc_val[q], __dmul_rn(a.bc_vel[q], t_new));
+        double own = un[0];
+#pragma unroll
+        for (int d = 1; d < DIM; ++d)
+            if (comp == d) own = un[d];
+        double v;
+        if (form == 0) v = own;
+        else if (form == 1) v = g1;
+        else if (form == 2) v = __dsub_rn(__dmul_rn(2.0, g1), own);
+        else v = __dsub_rn(__dmul_rn(2.0, g1), __dadd_rn(a.bc_val2[q], __dmul_rn(a.bc_vel2[q], t_new)));
+        a.u_other[(size_t)a.bc_tgt[q] * DIM + comp] = v;
+        umax = max_nan(umax, fabs(v));
+    }
+    umax = group_max_nan<kWarp>(umax);
+    if (lane == 0 && a.umax) {
+        const unsigned long long key = dbl_key(umax);
+        volatile unsigned long long *m = a.umax + a.step_in_chunk;
+        if (key > *m) atomicMax(a.umax + a.step_in_chunk, key);  // most slices find a larger value there
+    }
+}
+
+// ---- building the slices ----------------------------------------------------------------------------------------
+// Warp per node: bond b of the family goes to row rank(b) of the node's column, ranked by (neighbour id, b);
+// rmax_key: the largest squared bond length (bit pattern, zeroed by the caller).
+template <int DIM>
+__global__ void __launch_bounds__(256) sliced_rank_kernel(int n, const int *off, const int *nbr, const void *posv,
+                                                          const int *row0, uint16_t *src, unsigned long long *rmax_key) {
+    using PosT = typename Vec<DIM>::T;
+    const PosT *pos = static_cast<const PosT *>(posv);
+    const int lane = threadIdx.x & 31;
+    double rmax = 0.0;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        const int b0 = off[i], len = off[i + 1] - b0;
+        const PosT xi = pos[i];
+        uint16_t *dst = src + (size_t)row0[i >> 5] * 32 + (i & 31);
+        for (int c = 0; c < len; c += kWarp) {
+            const int b = c + lane;
+            const int j = b < len ? nbr[b0 + b] : 0;
+            int rank = 0;
+            for (int o = 0; o < len; ++o) {
+                const int x = __ldg(nbr + b0 + o);
+                rank += (x < j || (x == j && o < b)) ? 1 : 0;
+            }
+            if (b < len) {
+                dst[(size_t)rank * 32] = (uint16_t)b;
+                const PosT xj = pos[j];
+                double r2 = (xj.x - xi.x) * (xj.x - xi.x) + (xj.y - xi.y) * (xj.y - xi.y);
+                if constexpr (DIM == 3) r2 += (xj.z - xi.z) * (xj.z - xi.z);
+                rmax = fmax(rmax, r2);
+            }
+        }
+    }
+    rmax = group_max<kWarp>(rmax);
+    if (lane == 0) atomicMax(rmax_key, dbl_key(rmax));
+}
+
+// Warp per slice: the words (without the broken bit of real bonds) and the coefficients, row by row
+template <int DIM, typename GT>
+__global__ void __launch_bounds__(256) sliced_fill_kernel(int n, const int *off, const int *nbr, const void *posv,
+                                                          const int *row0, const uint16_t *src, int shift, double inv_step,
+                                                          int qmax, const GT *Pc, long long ldb, int *word, GT *P) {
+    using PosT = typename Vec<DIM>::T;
+    constexpr int NC = DIM == 3 ? 6 : 3;
+    const PosT *pos = static_cast<const PosT *>(posv);
+    const int lane = threadIdx.x & 31, nsl = (n + 31) / 32;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nsl; s += (gridDim.x * blockDim.x) >> 5) {
+        const int r0 = row0[s], rows = row0[s + 1] - r0, i = s * 32 + lane;
+        const int b0 = i < n ? off[i] : 0, len = i < n ? off[i + 1] - b0 : 0;
+        PosT xi{};
+        if (i < n) xi = pos[i];
+        for (int k = 0; k < rows; ++k) {
+            const size_t at = (size_t)(r0 + k) * 32 + lane;
+            const int t = b0 + (k < len ? src[at] : 0);
+            if (word) {
+                int w = (int)0x80000000u | (i < n ? i : 0);
+                if (k < len) {
+                    const int j = nbr[t];
+                    const PosT xj = pos[j];
+                    double r2 = (xj.x - xi.x) * (xj.x - xi.x) + (xj.y - xi.y) * (xj.y - xi.y);
+                    if constexpr (DIM == 3) r2 += (xj.z - xi.z) * (xj.z - xi.z);
+                    // rounded down with a margin far above the rounding of r: q step never exceeds the length
+                    const int q = min(qmax, (int)(sqrt(r2) * inv_step * (1.0 - 1.0e-9)));
+                    w = j | q << shift;
+                }
+                word[at] = w;
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                P[((size_t)(r0 + k) * NC + c) * 32 + lane] = k < len ? Pc[(size_t)c * ldb + t] : GT(0);
+        }
+    }
+}
+
+// Warp per slice: the words' broken bits from the health bytes
+__global__ void __launch_bounds__(256) sliced_health_kernel(int n, const int *off, const int *row0, const uint16_t *src,
+                                                            const uint8_t *health, int *word) {
+    const int lane = threadIdx.x & 31, nsl = (n + 31) / 32;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nsl; s += (gridDim.x * blockDim.x) >> 5) {
+        const int r0 = row0[s], i = s * 32 + lane;
+        const int b0 = i < n ? off[i] : 0, len = i < n ? off[i + 1] - b0 : 0;
+#pragma unroll 4
+        for (int k = 0; k < len; ++k) {
+            const size_t at = (size_t)(r0 + k) * 32 + lane;
+            const int w = word[at], v = (w & 0x7fffffff) | (health[b0 + src[at]] ? 0 : (int)0x80000000u);
+            if (v != w) word[at] = v;
+        }
+    }
+}
+
+namespace {
+int slice_grid(int n) {
+    const int g = ((n + 31) / 32 + 7) / 8;
+    return g < 1 ? 1 : (g < 148 * 8 ? g : 148 * 8);
+}
+
+template <int DIM, bool MIXED, int KW, int SPB, int U, int MINB>
+cudaError_t launch_sliced(const EpfArgs &a, const SlicedArgs &sl, cudaStream_t s) {
+    auto k = epf_sliced_kernel<DIM, MIXED, KW, SPB, U, MINB>;
+    const int slices = (a.n - a.node0 + 31) / 32, grid = (slices + SPB - 1) / SPB;
+    if (grid <= 0) return cudaSuccess;
+    epf_note_shape(LaunchShape{grid, KW * SPB * 32, 0});
+    if (a.pdl && !a.rate) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(KW * SPB * 32);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k, a, sl);
+        if (e != cudaSuccess) return e;
+    } else {
+        k<<<grid, KW * SPB * 32, 0, s>>>(a, sl);
+    }
+    return cudaGetLastError();
+}
+
+// Sliced configurations (the autotuner picks): warps a slice, slices a block, rows in flight, minimum resident blocks.
+// Measured in a captured 50-step loop, FP64 / mixed us a step: the 44.2 M-bond slab 4,1,2,6 352 / 246, 4,1,3,4 359 / 278,
+// 4,1,1,8 356 / 269, 8,1,2,3 412 / 285; the 2.25 M-bond plate 4,1,2,8 16.1 / 13.6, 2,2,4,5 16.4 / 13.7, 2,2,2,8 16.9 /
+// 14.2, 1,4,2,8 23.5 / 20.3.  The last of each dimension, eight warps a slice, is for meshes of a few hundred slices.
+template <int DIM, bool MIXED>
+cudaError_t launch_cfg(const EpfArgs &a, const SlicedArgs &sl, int which, cudaStream_t s) {
+    if constexpr (DIM == 3) {
+        switch (which) {
+            case 0: return launch_sliced<3, MIXED, 4, 1, 2, 6>(a, sl, s);
+            case 1: return launch_sliced<3, MIXED, 4, 1, 3, 4>(a, sl, s);
+            case 2: return launch_sliced<3, MIXED, 4, 1, 1, 8>(a, sl, s);
+            default: return launch_sliced<3, MIXED, 8, 1, 1, 4>(a, sl, s);
+        }
+    } else {
+        switch (which) {
+            case 0: return launch_sliced<2, MIXED, 4, 1, 2, 8>(a, sl, s);
+            case 1: return launch_sliced<2, MIXED, 2, 2, 4, 5>(a, sl, s);
+            case 2: return launch_sliced<2, MIXED, 2, 2, 2, 8>(a, sl, s);
+            default: return launch_sliced<2, MIXED, 8, 1, 2, 4>(a, sl, s);
+        }
+    }
+}
+}  // namespace
+
+cudaError_t launch_epf_sliced(const EpfArgs &a, const SlicedArgs &sl, int dim, bool mixed, int which, cudaStream_t s) {
+    if (!sl.word || !sl.P || !sl.row0 || !sl.src) return cudaErrorInvalidValue;
+    if (dim == 3) return mixed ? launch_cfg<3, true>(a, sl, which, s) : launch_cfg<3, false>(a, sl, which, s);
+    return mixed ? launch_cfg<2, true>(a, sl, which, s) : launch_cfg<2, false>(a, sl, which, s);
+}
+
+cudaError_t launch_sliced_rank(int n, int dim, const int *off, const int *nbr, const void *pos, const int *row0, uint16_t *src,
+                               unsigned long long *rmax_key, cudaStream_t s) {
+    const int g = (n + 7) / 8 < 148 * 8 ? (n + 7) / 8 : 148 * 8;
+    if (dim == 3) sliced_rank_kernel<3><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, rmax_key);
+    else sliced_rank_kernel<2><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, rmax_key);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sliced_fill(int n, int dim, bool mixed, const int *off, const int *nbr, const void *pos, const int *row0,
+                               const uint16_t *src, int shift, double inv_step, int qmax, const void *Pc, long long ldb,
+                               int *word, void *P, cudaStream_t s) {
+    const int g = slice_grid(n);
+    if (dim == 3) {
+        if (mixed) sliced_fill_kernel<3, float><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const float *)Pc, ldb, word, (float *)P);
+        else sliced_fill_kernel<3, double><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const double *)Pc, ldb, word, (double *)P);
+    } else {
+        if (mixed) sliced_fill_kernel<2, float><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const float *)Pc, ldb, word, (float *)P);
+        else sliced_fill_kernel<2, double><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const double *)Pc, ldb, word, (double *)P);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sliced_health(int n, const int *off, const int *row0, const uint16_t *src, const uint8_t *health, int *word,
+                                 cudaStream_t s) {
+    sliced_health_kernel<<<slice_grid(n), 256, 0, s>>>(n, off, row0, src, health, word);
+    return cudaGetLastError();
+}
+
+}  // namespace pxb

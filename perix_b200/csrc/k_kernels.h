@@ -177,8 +177,11 @@ struct EpfArgs {
     double e2_hold = 0;
 };
 // schedule variants of the explicit kernel (lanes per node x bonds per lane per pass); see k_epf.cu
-constexpr int kEpfTmaConfigs = 16;                // staged (TMA) configurations per dimension
-constexpr int kEpfVariants = 5 + kEpfTmaConfigs;  // 0-2 lane groups, 3-4 CSR tiles, 5.. staged
+constexpr int kEpfTmaConfigs = 12;                // staged (TMA) configurations per dimension
+constexpr int kEpfSlicedConfigs = 4;              // sliced configurations per dimension (k_epf_sliced.cu)
+// 0-2 lane groups, 3-4 CSR tiles, then staged, then sliced
+constexpr int kEpfVariants = 5 + kEpfTmaConfigs + kEpfSlicedConfigs;
+// (a sliced variant is launched by launch_epf_sliced; here its START and FORCE_FROZEN modes run variant 1)
 cudaError_t launch_epf(const EpfArgs &a, int dim, bool mixed, int mode, int variant, cudaStream_t s);
 // P[c][t] from G[c][t] (t < ldb, SoA stride ldb): 2D p11 = C11 Gxx + C66 Gyy, p22 = C66 Gxx + C11 Gyy,
 // pxy = (C12 + C66) Gxy; 3D p11/p22/p33 and (C12 + C66) times Gxy, Gxz, Gyz
@@ -196,6 +199,7 @@ int epf_tile_nodes(int dim, int variant);
 bool epf_variant_fits(int dim, int variant, int max_family);
 // TMA-staged step (k_epf_tma.cu): STEP mode only; `which` selects one of kEpfTmaConfigs configurations
 bool epf_is_tma(int variant);
+bool epf_is_sliced(int variant);
 int epf_tma_maxb(int dim, int variant, int max_family);
 int epf_tma_tile_nodes(int dim, int which);
 size_t epf_tma_smem(int dim, bool mixed, int which, int maxb);
@@ -206,9 +210,35 @@ struct LaunchShape {
     int grid, block;
     size_t smem;
 };
-LaunchShape epf_tma_last_shape();
+LaunchShape epf_last_shape();
+void epf_note_shape(const LaunchShape &shape);
 // an empty kernel with the given launch shape (the fixed cost of a launch, timed like a step)
 cudaError_t launch_empty(int grid, int block, size_t smem, cudaStream_t s);
+
+// The sliced step's streams (k_epf_sliced.cu): slice s = nodes 32 s .. 32 s + 31, its rows row0[s] .. row0[s + 1] - 1
+// hold their k-th bonds by neighbour id, entry (row, lane) at 32 row + lane, coefficient c at 32 (nc row + c) + lane.
+constexpr int kSlicedClasses = 128, kSlicedSlack = 8;
+struct SlicedArgs {
+    const int *row0 = nullptr;
+    int *word = nullptr;            // broken << 31 | length class << shift | neighbour; kSlicedSlack rows of room at the end
+    const void *P = nullptr;        // packed Navier coefficients (float when mixed)
+    const uint16_t *src = nullptr;  // the bond's place in its family
+    int shift = 31;  // 31 - the bits of the length classes (at most kSlicedClasses)
+    double clear = 0;  // |e|^2 < clear q^2 clears a bond of length class q: ((s_c (1 - 1e-6) - 1e-12) step)^2
+};
+// STEP, or RATE with EpfArgs::rate set (node0 a multiple of 32); which: one of kEpfSlicedConfigs configurations
+cudaError_t launch_epf_sliced(const EpfArgs &a, const SlicedArgs &sl, int dim, bool mixed, int which, cudaStream_t s);
+// src from the families, and the largest squared bond length as an atomicMax over its bit pattern (zeroed before)
+cudaError_t launch_sliced_rank(int n, int dim, const int *off, const int *nbr, const void *pos, const int *row0, uint16_t *src,
+                               unsigned long long *rmax_key, cudaStream_t s);
+// the words of intact bonds (length class = floor(length inv_step), at most qmax; word NULL: left as they are) and the
+// coefficients from the bond-ordered ones (SoA stride ldb)
+cudaError_t launch_sliced_fill(int n, int dim, bool mixed, const int *off, const int *nbr, const void *pos, const int *row0,
+                               const uint16_t *src, int shift, double inv_step, int qmax, const void *Pc, long long ldb,
+                               int *word, void *P, cudaStream_t s);
+// the words' broken bits from the health bytes
+cudaError_t launch_sliced_health(int n, const int *off, const int *row0, const uint16_t *src, const uint8_t *health, int *word,
+                                 cudaStream_t s);
 
 struct EpfAdjArgs {
     int n = 0;

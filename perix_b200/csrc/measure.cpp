@@ -25,7 +25,7 @@ extern "C" int pxb_epf_time_steps(pxb_ctx *c, int nsteps, size_t flush_bytes, in
 extern "C" int pxb_epf_launch_floor(pxb_ctx *c, size_t flush_bytes, int reps, float *ms, int *grid, int *block,
                                     size_t *smem) {
     if (!c || reps <= 0 || !ms) return fail(PXB_ERR_INVALID, "pxb_epf_launch_floor: bad arguments");
-    const LaunchShape sh = epf_tma_last_shape();
+    const LaunchShape sh = epf_last_shape();
     if (sh.grid <= 0) return fail(PXB_ERR_STATE, "pxb_epf_launch_floor: no staged step launched yet");
     Events ev;
     PXB_TRY(ev.make(2 * (size_t)reps));

@@ -120,6 +120,13 @@ struct EpfState {
     DevBuf G;          // SoA Navier operators [c][ldb], double or float (c = 3 in 2D, 6 in 3D)
     DevBuf P;          // SoA packed Navier coefficients [c][ldb] (same type): the staged step kernels' stream
     DevBuf xib;        // mixed: FP32 reference bond vectors [dim][ldb] (the staged kernels' stretch pre-test)
+    // the sliced step's copy of the streams (k_epf_sliced.cu), built when a sliced variant is first selected: rows of
+    // the slices, words, coefficients, places in the family; sl_P_stale: the constants changed since they were filled,
+    // sl_stale: something other than a sliced launch may have written health since the words' broken bits were set
+    DevBuf sl_row0, sl_word, sl_P, sl_src;
+    bool sl_ready = false, sl_P_stale = false, sl_stale = true;
+    int sl_shift = 31;
+    double sl_step = 0.0;
     DevBuf sc_bond;    // variable horizon: per-bond critical stretch s_c(0.5 (delta_i + delta_j)) [ldb]
     // explicit-loop adjoint (pxb_epf_adjoint_d): checkpoints, a segment's states, the two ping-pong states, the
     // adjoint vectors A (dJ/du^n), R (dJ/du^{n-1} carried), W (BC-transposed A), step times, dC accumulator
@@ -258,5 +265,9 @@ int sync(pxb_ctx *c);
 int check_launch(pxb_ctx *c, const char *what);
 size_t ctx_bytes(const pxb_ctx *c);
 int l2_flush(pxb_ctx *c, size_t bytes);  // writes `bytes` through the L2 on the context stream (0: nothing)
+// the explicit kernel of schedule `variant` (mode EpfMode) on stream s; a sliced variant must be ready (epf_ready)
+cudaError_t epf_launch(pxb_ctx *c, const EpfArgs &a, int mode, int variant, cudaStream_t s);
+// before launches of the current variant on the context stream: a sliced variant's streams built and up to date
+int epf_ready(pxb_ctx *c);
 int wait_failure(pxb_ctx *c, unsigned int werr, const char *what);  // report (and clear) a staged wait that ran out
 }  // namespace pxb

@@ -77,6 +77,7 @@ int load_state(pxb_ctx *c, const Snapshot &s) {
     PXB_TRY(d2d(c, e.u[0].p, s.u0.p, s.u0.bytes));
     PXB_TRY(d2d(c, e.u[1].p, s.u1.p, s.u1.bytes));
     PXB_TRY(d2d(c, e.health.p, s.health.p, s.health.bytes));
+    e.sl_stale = true;
     e.cur = s.cur;
     e.t = s.t;
     e.step = s.step;
@@ -102,11 +103,12 @@ int timed_steps(pxb_ctx *c, int nsteps, size_t flush_bytes, int restore_every, c
         PXB_CUDA_TRY(cudaStreamSynchronize(c->stream));
         th[0] = e.t + e.dt;
         PXB_TRY(h2d(c, e.tsched.p, th, sizeof(double)));
+        PXB_TRY(epf_ready(c));
         PXB_TRY(flush_l2(c, flush_bytes, g_flush));
         EpfArgs a;
         PXB_TRY(step_args(c, e.cur, &a));
         PXB_CUDA_TRY(cudaEventRecord(ev.ev[2 * (size_t)s], c->stream));
-        const cudaError_t err = launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_STEP, e.variant, c->stream);
+        const cudaError_t err = epf_launch(c, a, EPF_STEP, e.variant, c->stream);
         if (err != cudaSuccess) return cuda_fail(err, "epf step launch");
         c->launches++;
         PXB_CUDA_TRY(cudaEventRecord(ev.ev[2 * (size_t)s + 1], c->stream));
@@ -120,6 +122,15 @@ int timed_steps(pxb_ctx *c, int nsteps, size_t flush_bytes, int restore_every, c
     if (werr) return wait_failure(c, werr, "explicit step");
     for (int s = 0; s < nsteps; ++s) PXB_CUDA_TRY(cudaEventElapsedTime(&ms[s], ev.ev[2 * (size_t)s], ev.ev[2 * (size_t)s + 1]));
     return PXB_OK;
+}
+
+// makes `variant` the context's schedule; a sliced one that cannot be built leaves the schedule as it was
+int select_variant(pxb_ctx *c, int variant) {
+    const int before = c->epf.variant;
+    c->epf.variant = variant;
+    const int st = epf_ready(c);
+    if (st != PXB_OK) c->epf.variant = before;
+    return st;
 }
 
 // process-wide cache of autotuned schedule choices, keyed by problem signature
@@ -165,8 +176,7 @@ extern "C" int pxb_epf_set_variant(pxb_ctx *c, int variant) {
     if (variant < 0 || variant >= kEpfVariants) return fail(PXB_ERR_INVALID, "pxb_epf_set_variant: no such variant");
     if (!epf_variant_fits(c->g.dim, variant, c->g.max_family))
         return fail(PXB_ERR_UNSUPPORTED, "pxb_epf_set_variant: families too large for this tile size");
-    c->epf.variant = variant;
-    return PXB_OK;
+    return select_variant(c, variant);
 }
 
 extern "C" int pxb_epf_variant_count(void) { return kEpfVariants; }
@@ -186,8 +196,7 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
     if (steps <= 0) return fail(PXB_ERR_INVALID, "pxb_epf_autotune: steps must be > 0");
     const std::string key = signature(c);
     auto hit = g_tuned.find(key);
-    if (use_cache && hit != g_tuned.end()) {
-        c->epf.variant = hit->second;
+    if (use_cache && hit != g_tuned.end() && select_variant(c, hit->second) == PXB_OK) {
         if (best) *best = hit->second;
         return PXB_OK;
     }
@@ -201,7 +210,10 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
             if (ms_per_variant) ms_per_variant[v] = -1.f;
             continue;
         }
-        c->epf.variant = v;
+        if (select_variant(c, v) != PXB_OK) {  // no room for its streams
+            if (ms_per_variant) ms_per_variant[v] = -1.f;
+            continue;
+        }
         // two untimed steps first: a kernel's first launch in a process also loads its module
         PXB_TRY(load_state(c, keep));
         PXB_TRY(timed_steps(c, 2, 0, 0, nullptr, ms.data()));
@@ -235,8 +247,7 @@ extern "C" int pxb_epf_autotune_rate(pxb_ctx *c, const double *u, int reps, int 
     EpfState &e = c->epf;
     const std::string key = signature(c) + ":rate";
     auto hit = g_tuned.find(key);
-    if (use_cache && hit != g_tuned.end()) {
-        e.variant = hit->second;
+    if (use_cache && hit != g_tuned.end() && select_variant(c, hit->second) == PXB_OK) {
         if (best) *best = hit->second;
         return PXB_OK;
     }
@@ -248,7 +259,9 @@ extern "C" int pxb_epf_autotune_rate(pxb_ctx *c, const double *u, int reps, int 
     PXB_TRY(h2d(c, e.u[e.cur].p, u, sizeof(double) * (size_t)c->g.n * c->g.dim));
     auto restore = [&]() -> int {
         PXB_TRY(d2d(c, e.health.p, health.p, health.bytes));
-        return d2d(c, e.counters.p, counters.p, counters.bytes);
+        e.sl_stale = true;
+        PXB_TRY(d2d(c, e.counters.p, counters.p, counters.bytes));
+        return epf_ready(c);
     };
     Events ev;
     PXB_TRY(ev.make(2 * (size_t)reps));
@@ -260,14 +273,17 @@ extern "C" int pxb_epf_autotune_rate(pxb_ctx *c, const double *u, int reps, int 
             if (ms_per_variant) ms_per_variant[v] = -1.f;
             continue;
         }
-        e.variant = v;
+        if (select_variant(c, v) != PXB_OK) {  // no room for its streams
+            if (ms_per_variant) ms_per_variant[v] = -1.f;
+            continue;
+        }
         EpfArgs a;
         PXB_TRY(rate_args(c, &a));
         // one untimed launch first: a kernel's first launch in a process also loads its module
         for (int r = -1; r < reps; ++r) {
             PXB_TRY(restore());
             if (r >= 0) PXB_CUDA_TRY(cudaEventRecord(ev.ev[2 * (size_t)r], c->stream));
-            const cudaError_t err = launch_epf(a, c->g.dim, e.precision == PXB_MIXED, EPF_RATE, v, c->stream);
+            const cudaError_t err = epf_launch(c, a, EPF_RATE, v, c->stream);
             if (err != cudaSuccess) return cuda_fail(err, "rate autotune launch");
             c->launches++;
             if (r >= 0) PXB_CUDA_TRY(cudaEventRecord(ev.ev[2 * (size_t)r + 1], c->stream));
