@@ -307,7 +307,8 @@ int pxb_epf_restore(pxb_ctx *ctx);
  * fails with PXB_ERR_OOM and the autotuners skip it.  pxb_epf_variant_count() gives their number.  pxb_epf_autotune
  * times every variant that fits for `steps` steps from a private copy of the current state (L2 flushed before each
  * step), restores the state, selects the fastest and caches the choice per problem signature (dim, precision, nodes,
- * bonds, largest family); use_cache=1 returns a cached choice without timing.  ms_per_variant (may be NULL;
+ * bonds, largest family); where the streams fit in the L2, the schedules within a tenth of the fastest are timed in a
+ * captured loop as well, and the fastest there is selected; use_cache=1 returns a cached choice without timing.  ms_per_variant (may be NULL;
  * pxb_epf_variant_count() entries) receives the mean step time of each variant, -1 for one that does not fit. */
 int pxb_epf_variant_count(void);
 int pxb_epf_autotune(pxb_ctx *ctx, int steps, size_t flush_bytes, int use_cache, int *best, float *ms_per_variant);

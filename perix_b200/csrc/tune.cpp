@@ -133,6 +133,26 @@ int select_variant(pxb_ctx *c, int variant) {
     return st;
 }
 
+// milliseconds of a captured run of kLoopSteps steps of the current schedule from `from` (the better of two)
+constexpr int kLoopSteps = 24;
+int loop_time(pxb_ctx *c, const Snapshot &from, float *ms) {
+    Events ev;
+    PXB_TRY(ev.make(2));
+    *ms = 1e30f;
+    for (int r = 0; r < 3; ++r) {  // the first one captures
+        PXB_TRY(load_state(c, from));
+        PXB_TRY(epf_ready(c));
+        PXB_CUDA_TRY(cudaEventRecord(ev.ev[0], c->stream));
+        PXB_TRY(pxb_epf_advance(c, kLoopSteps, kLoopSteps, nullptr));
+        PXB_CUDA_TRY(cudaEventRecord(ev.ev[1], c->stream));
+        PXB_TRY(sync(c));
+        float t = 0.f;
+        PXB_CUDA_TRY(cudaEventElapsedTime(&t, ev.ev[0], ev.ev[1]));
+        if (r > 0) *ms = std::min(*ms, t);
+    }
+    return PXB_OK;
+}
+
 // process-wide cache of autotuned schedule choices, keyed by problem signature
 std::map<std::string, int> g_tuned;
 
@@ -202,7 +222,7 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
     }
     Snapshot keep;
     PXB_TRY(save_state(c, keep));
-    std::vector<float> ms((size_t)std::max(steps, 2));
+    std::vector<float> ms((size_t)std::max(steps, 2)), mean_ms(kEpfVariants, 1e30f);
     float best_ms = 1e30f;
     int best_v = c->epf.variant;
     for (int v = 0; v < kEpfVariants; ++v) {
@@ -223,7 +243,20 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
         for (int k = 0; k < steps; ++k) mean += ms[(size_t)k];
         mean /= (float)steps;
         if (ms_per_variant) ms_per_variant[v] = mean;
+        mean_ms[(size_t)v] = mean;
         if (mean < best_ms) { best_ms = mean; best_v = v; }
+    }
+    // Streams that stay in L2 from one step to the next: a run's captured steps are faster than the flushed ones timed
+    // above, and not by the same factor for every schedule (the 2.25 M-bond plate, mixed: 24.5 and 25.3 us flushed, 13.6
+    // and 16.1 us in the loop).  The schedules within a tenth of the best are timed in a loop too, and that decides.
+    if (!c->epf.evict_first && flush_bytes > 0) {
+        float loop_best = 1e30f;
+        for (int v = 0; v < kEpfVariants; ++v) {
+            float t = 0.f;
+            if (mean_ms[(size_t)v] > 1.1f * best_ms || select_variant(c, v) != PXB_OK) continue;
+            if (loop_time(c, keep, &t) != PXB_OK) break;  // (a run that blows up within the loop: the flushed choice stands)
+            if (t < loop_best) { loop_best = t; best_v = v; }
+        }
     }
     PXB_TRY(load_state(c, keep));
     PXB_TRY(sync(c));
