@@ -277,13 +277,13 @@ int pxb_epf_record_d(pxb_ctx *ctx, const double *u0_d, const double *v0_d, doubl
 int pxb_epf_set_rate_chunks(pxb_ctx *ctx, int chunks);
 /* The reverse sweep's bond-force adjoint kernel: 0 a kernel that streams both the forward and the reverse bonds'
  * operators; 1 the reverse-only kernel: the frozen mask's own-bond operator sums are formed once per sweep, dJ/dC
- * is summed over the reverse bonds, and one operator stream is read per step; 2, 3, 4 (and -1, the default: 4) the
- * reverse-only kernel with the tiles' ids, reverse health and node rows staged by bulk copies through a
- * shared-memory ring (bounded waits: a wait that runs out fails the sweep with PXB_ERR_CUDA) and each reverse
- * bond's source node gathered as one interleaved (u, adjoint) row, in three launch configurations (3D: 2, 1 or 3
- * reverse bonds a lane per pass at 16 lanes a node; 2D: 4, 4 or 8 lanes a node).  The reverse-only
- * kernels apply when every bond has its reverse (symmetric families); other meshes fall back to 0.  Results agree
- * to rounding.  No counterpart in the reference. */
+ * is summed over the reverse bonds, and one operator stream is read per step; 2, 3, 4 the reverse-only kernel with the
+ * tiles' ids, reverse health and node rows staged by bulk copies through a shared-memory ring (bounded waits: a wait that
+ * runs out fails the sweep with PXB_ERR_CUDA) and each reverse bond's source node gathered as one interleaved (u, adjoint)
+ * row, in three launch configurations (3D: 2, 1 or 3 reverse bonds a lane per pass at 16 lanes a node; 2D: 4, 4 or 8 lanes
+ * a node); 5 (and -1, the default) the reverse-only sums on the slices of the sliced step, with a neighbour-sorted copy of
+ * the reverse operators (without room for it: 4).  The reverse-only kernels apply when every bond has its reverse
+ * (symmetric families); other meshes fall back to 0.  Results agree to rounding.  No counterpart in the reference. */
 int pxb_epf_set_adjoint_schedule(pxb_ctx *ctx, int schedule);
 /* The reverse sweep of the last pxb_epf_record_d (PXB_ERR_STATE when there is none); arguments as pxb_epf_adjoint_d. */
 int pxb_epf_adjoint_recorded_d(pxb_ctx *ctx, const double *ubar_N_d, const double *ubar_Nm1_d, double *u0bar_d,
@@ -301,8 +301,8 @@ int pxb_epf_set_constants(pxb_ctx *ctx, double C11, double C12, double C66, doub
 int pxb_epf_snapshot(pxb_ctx *ctx);
 int pxb_epf_restore(pxb_ctx *ctx);
 /* Schedule variants of the explicit kernel: 0-2 lane groups (lanes per node x bonds per lane per pass), 3-4
- * CSR-stream tiles, 5-16 TMA-staged tiles, 17-20 sliced (time step and rate call only; the other modes of a staged or
- * sliced variant run variant 1).  A sliced variant keeps a second, neighbour-sorted copy of the bond streams (about
+ * CSR-stream tiles, 5-16 TMA-staged tiles, 17-20 sliced (time step and rate call, in FP64 the start and the frozen
+ * force too; the other modes of a staged or sliced variant run variant 1).  A sliced variant keeps a second, neighbour-sorted copy of the bond streams (about
  * 54 bytes a bond in 3D FP64, 30 mixed), built when it is first selected; without room for it pxb_epf_set_variant
  * fails with PXB_ERR_OOM and the autotuners skip it.  pxb_epf_variant_count() gives their number.  pxb_epf_autotune
  * times every variant that fits for `steps` steps from a private copy of the current state (L2 flushed before each

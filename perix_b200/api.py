@@ -411,7 +411,8 @@ class Context:
 
     def epf_set_adjoint_schedule(self, schedule):
         """The recorded reverse sweep's kernel: -1 default, 0 both operator streams, 1 reverse-only, 2-4 reverse-only
-        staged through shared memory in three launch configurations (pxb_epf_set_adjoint_schedule)."""
+        staged through shared memory in three launch configurations, 5 reverse-only on the slices
+        (pxb_epf_set_adjoint_schedule)."""
         _check(self.L.pxb_epf_set_adjoint_schedule(self.h, int(schedule)))
 
     def gbuild(self, order=2, precision=FP64, allow_degenerate=False):

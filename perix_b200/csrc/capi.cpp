@@ -129,7 +129,7 @@ size_t ctx_bytes(const pxb_ctx *c) {
     const EpfState &e = c->epf;
     s += bufsz(e.G) + bufsz(e.P) + bufsz(e.xib) + bufsz(e.health) + bufsz(e.u[0]) + bufsz(e.u[1]) + bufsz(e.accel) + bufsz(e.counters) +
          bufsz(e.umax) + bufsz(e.tsched) + bufsz(e.sc_bond) + bufsz(e.sl_row0) + bufsz(e.sl_word) + bufsz(e.sl_P) +
-         bufsz(e.sl_src);
+         bufsz(e.sl_src) + bufsz(e.sl_GR) + bufsz(e.sl_aword);
     s += bufsz(e.adj_ckpt) + bufsz(e.adj_seg) + bufsz(e.adj_p[0]) + bufsz(e.adj_p[1]) + bufsz(e.adj_A) + bufsz(e.adj_R) +
          bufsz(e.adj_W) + bufsz(e.adj_t) + bufsz(e.adj_dC) + bufsz(e.adj_umax) + bufsz(e.adj_GR) + bufsz(e.adj_HR) + bufsz(e.adj_u0) + bufsz(e.adj_SG) + bufsz(e.adj_UW);
     s += bufsz(e.bc.own) + bufsz(e.bc.src_off) + bufsz(e.bc.tgt) + bufsz(e.bc.comp) + bufsz(e.bc.form) +
@@ -551,8 +551,8 @@ extern "C" int pxb_gbuild_set_schedule(pxb_ctx *c, int schedule) {
     return PXB_OK;
 }
 
-// the recorded sweep's adjoint schedule in effect (-1: the staged reverse-only kernel, schedule 4)
-static int adj_sched(const pxb_ctx *c) { return c->adj_schedule < 0 ? 4 : c->adj_schedule; }
+// the recorded sweep's adjoint schedule asked for (-1: the sliced reverse-only kernel, schedule 5)
+static int adj_sched(const pxb_ctx *c) { return c->adj_schedule < 0 ? 5 : c->adj_schedule; }
 
 extern "C" int pxb_epf_set_rate_chunks(pxb_ctx *c, int chunks) {
     if (!c) return fail(PXB_ERR_INVALID, "pxb_epf_set_rate_chunks: NULL context");
@@ -565,7 +565,7 @@ extern "C" int pxb_epf_set_rate_chunks(pxb_ctx *c, int chunks) {
 
 extern "C" int pxb_epf_set_adjoint_schedule(pxb_ctx *c, int schedule) {
     if (!c) return fail(PXB_ERR_INVALID, "pxb_epf_set_adjoint_schedule: NULL context");
-    if (schedule < -1 || schedule > 4) return fail(PXB_ERR_INVALID, "pxb_epf_set_adjoint_schedule: -1 .. 4");
+    if (schedule < -1 || schedule > 5) return fail(PXB_ERR_INVALID, "pxb_epf_set_adjoint_schedule: -1 .. 5");
     c->adj_schedule = schedule;
     return PXB_OK;
 }
@@ -742,9 +742,13 @@ namespace {
 
 bool runs_sliced(const EpfState &e) { return epf_is_sliced(e.variant) && !e.sc_bond.p; }
 
-int sliced_build(pxb_ctx *c) {
+size_t sliced_entries(const EpfState &e) { return e.sl_src.bytes / sizeof(uint16_t); }
+
+// slices, places in the families and length classes of the geometry
+int sliced_topology(pxb_ctx *c) {
     EpfState &e = c->epf;
     const Geometry &g = c->g;
+    if (e.sl_src.p) return PXB_OK;
     const int n = g.n, slices = (n + 31) / 32;
     std::vector<int> row0((size_t)slices + 1, 0);
     for (int s = 0; s < slices; ++s) {
@@ -756,14 +760,10 @@ int sliced_build(pxb_ctx *c) {
         row0[(size_t)s + 1] = row0[(size_t)s] + rows;
     }
     const size_t entries = 32 * (size_t)std::max(1, row0.back());
-    const int nc = g.dim == 3 ? 6 : 3;
-    const bool mixed = e.precision == PXB_MIXED;
-    int st = dev_upload(c, e.sl_row0, row0.data(), sizeof(int) * row0.size());
-    if (st == PXB_OK) st = dev_alloc(c, e.sl_word, sizeof(int) * (entries + 32 * kSlicedSlack));
-    if (st == PXB_OK) st = dev_alloc(c, e.sl_src, sizeof(uint16_t) * entries);
-    if (st == PXB_OK) st = dev_alloc(c, e.sl_P, (mixed ? 4 : 8) * (size_t)nc * entries);
+    PXB_TRY(dev_alloc(c, e.sl_src, sizeof(uint16_t) * entries));
+    const int st = dev_upload(c, e.sl_row0, row0.data(), sizeof(int) * row0.size());
     if (st != PXB_OK) {
-        for (DevBuf *b : {&e.sl_row0, &e.sl_word, &e.sl_src, &e.sl_P}) b->release();
+        e.sl_src.release();
         return st;
     }
     int idbits = 1;
@@ -775,19 +775,56 @@ int sliced_build(pxb_ctx *c) {
     PXB_CUDA_TRY(cudaMemsetAsync(key, 0, sizeof(*key), c->stream));
     PXB_CUDA_TRY(launch_sliced_rank(n, g.dim, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, e.sl_row0.as<int>(),
                                     e.sl_src.as<uint16_t>(), key, c->stream));
+    c->launches++;
     unsigned long long k2 = 0;
     PXB_TRY(d2h(c, &k2, key, sizeof(k2)));
     PXB_TRY(sync(c));  // (row0 leaves scope here too)
     double r2 = 0.0;
     std::memcpy(&r2, &k2, sizeof(double));
     e.sl_step = std::isfinite(r2) ? std::sqrt(r2) / (1 << qbits) : 0.0;
-    PXB_CUDA_TRY(launch_sliced_fill(n, g.dim, mixed, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, e.sl_row0.as<int>(),
-                                    e.sl_src.as<uint16_t>(), e.sl_shift, e.sl_step > 0.0 ? 1.0 / e.sl_step : 0.0,
-                                    (1 << qbits) - 1, e.P.p, (long long)g.ldb, e.sl_word.as<int>(), e.sl_P.p, c->stream));
-    c->launches += 2;
+    return PXB_OK;
+}
+
+// words and coefficients (bond-ordered source Pc; rev: the reverse bonds') of the slices; word NULL: coefficients only
+int sliced_fill(pxb_ctx *c, const void *Pc, const int *rev, int *word, void *P) {
+    EpfState &e = c->epf;
+    const Geometry &g = c->g;
+    PXB_CUDA_TRY(launch_sliced_fill(g.n, g.dim, e.precision == PXB_MIXED, g.off.as<int>(), g.nbr.as<int>(), g.pos.p,
+                                    e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(), e.sl_shift,
+                                    e.sl_step > 0.0 ? 1.0 / e.sl_step : 0.0, (1 << (31 - e.sl_shift)) - 1, Pc,
+                                    (long long)g.ldb, rev, word, P, c->stream));
+    c->launches++;
+    return PXB_OK;
+}
+
+int sliced_alloc(pxb_ctx *c, DevBuf &word, DevBuf &P) {
+    const EpfState &e = c->epf;
+    const size_t entries = sliced_entries(e), nc = c->g.dim == 3 ? 6 : 3;
+    int st = dev_alloc(c, word, sizeof(int) * (entries + 32 * kSlicedSlack));
+    if (st == PXB_OK) st = dev_alloc(c, P, (e.precision == PXB_MIXED ? 4 : 8) * nc * entries);
+    if (st != PXB_OK) {
+        word.release();
+        P.release();
+    }
+    return st;
+}
+
+int sliced_build(pxb_ctx *c) {
+    EpfState &e = c->epf;
+    PXB_TRY(sliced_topology(c));
+    PXB_TRY(sliced_alloc(c, e.sl_word, e.sl_P));
+    PXB_TRY(sliced_fill(c, e.P.p, nullptr, e.sl_word.as<int>(), e.sl_P.p));
     e.sl_ready = true;
     e.sl_P_stale = false;
     e.sl_stale = true;
+    return PXB_OK;
+}
+
+int sliced_health(pxb_ctx *c, const int *rev, int *word) {
+    EpfState &e = c->epf;
+    PXB_CUDA_TRY(launch_sliced_health(c->g.n, c->g.off.as<int>(), e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(),
+                                      e.health.as<uint8_t>(), rev, word, c->stream));
+    c->launches++;
     return PXB_OK;
 }
 
@@ -808,31 +845,27 @@ SlicedArgs sliced_args(const EpfState &e) {
 int epf_ready(pxb_ctx *c) {
     EpfState &e = c->epf;
     if (!runs_sliced(e)) return PXB_OK;
-    const Geometry &g = c->g;
     if (!e.sl_ready) PXB_TRY(sliced_build(c));
-    if (e.sl_P_stale) {
-        PXB_CUDA_TRY(launch_sliced_fill(g.n, g.dim, e.precision == PXB_MIXED, g.off.as<int>(), g.nbr.as<int>(), g.pos.p,
-                                        e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(), 0, 0.0, 0, e.P.p, (long long)g.ldb,
-                                        nullptr, e.sl_P.p, c->stream));
-        c->launches++;
-        e.sl_P_stale = false;
-    }
-    if (e.sl_stale) {
-        PXB_CUDA_TRY(launch_sliced_health(g.n, g.off.as<int>(), e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(),
-                                          e.health.as<uint8_t>(), e.sl_word.as<int>(), c->stream));
-        c->launches++;
-        e.sl_stale = false;
-    }
+    if (!e.sl_P_stale && !e.sl_stale) return PXB_OK;
+    if (e.sl_P_stale) PXB_TRY(sliced_fill(c, e.P.p, nullptr, nullptr, e.sl_P.p));
+    if (e.sl_stale) PXB_TRY(sliced_health(c, nullptr, e.sl_word.as<int>()));
+    // (captured by a caller, these launches have not run: the next call queues them again)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PXB_CUDA_TRY(cudaStreamIsCapturing(c->stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone) e.sl_P_stale = e.sl_stale = false;
     return PXB_OK;
 }
 
 cudaError_t epf_launch(pxb_ctx *c, const EpfArgs &a, int mode, int variant, cudaStream_t s) {
     EpfState &e = c->epf;
     const bool mixed = e.precision == PXB_MIXED;
-    if (epf_is_sliced(variant) && !a.sc_bond && !e.sc_bond.p && (mode == EPF_STEP || (mode == EPF_RATE && a.accel))) {
+    // (mixed: START and FORCE_FROZEN stay with the lane-group kernel, which forms its coefficients from the FP32 operators
+    // in FP64; the packed ones are rounded once more)
+    if (epf_is_sliced(variant) && !e.sc_bond.p && (mode == EPF_STEP || mode == EPF_RATE || !mixed)) {
         if (!e.sl_ready) return cudaErrorNotReady;
         EpfArgs r = a;
-        r.rate = mode == EPF_RATE ? 1 : 0;
+        r.rate = mode == EPF_STEP ? kEpfStep : mode == EPF_START ? kEpfStart : kEpfRate;
+        if (mode == EPF_FORCE_FROZEN) r.damage = 0;
         return launch_epf_sliced(r, sliced_args(e), c->g.dim, mixed, variant - 5 - kEpfTmaConfigs, s);
     }
     if (a.damage && mode != EPF_FORCE_FROZEN) e.sl_stale = true;
@@ -1311,6 +1344,7 @@ extern "C" int pxb_epf_start(pxb_ctx *c, const double *u0, const double *v0, dou
         PXB_TRY(h2d(c, tmp, v0, sizeof(double) * nd));
         dv0 = static_cast<const double *>(tmp);
     }
+    PXB_TRY(epf_ready(c));
     EpfArgs a = epf_args(c);
     a.u = e.u[0].as<double>();
     a.u_other = e.u[1].as<double>();
@@ -1594,11 +1628,15 @@ extern "C" int pxb_epf_broken_count(pxb_ctx *c, long long *n_broken) {
 extern "C" int pxb_epf_force_frozen_d(pxb_ctx *c, const double *u_d, double *a_d) {
     PXB_TRY(need_epf(c, "pxb_epf_force_frozen"));
     if (!u_d || !a_d) return fail(PXB_ERR_INVALID, "pxb_epf_force_frozen: NULL buffer");
+    PXB_TRY(epf_ready(c));
     EpfArgs a = epf_args(c);
     a.u = u_d;
     a.accel = a_d;
     a.damage = 0;
-    epf_launch(c, a, EPF_FORCE_FROZEN, c->epf.variant, c->stream);
+    // (the sliced kernel reads 2D displacements as 16-byte pairs)
+    const bool pairs = c->g.dim == 3 || (reinterpret_cast<uintptr_t>(u_d) & 15u) == 0;
+    const cudaError_t err = epf_launch(c, a, EPF_FORCE_FROZEN, pairs ? c->epf.variant : 1, c->stream);
+    if (err != cudaSuccess) return cuda_fail(err, "epf force (frozen mask)");
     return check_launch(c, "epf force (frozen mask)");
 }
 
@@ -1741,6 +1779,19 @@ int adj_kernel(pxb_ctx *c, const double *u, const double *w, double scale, doubl
     a.c_o = c_o;
     a.rout = rout;
     if (e.adj_sg_on) a.SG = e.adj_SG.as<double>();
+    if (e.adj_sliced) {
+        a.evict_first = e.evict_first ? 1 : 0;
+        a.UW = uw;
+        a.dC = e.adj_dC.as<double>() + 4;
+        SlicedArgs sl;
+        sl.row0 = e.sl_row0.as<int>();
+        sl.word = e.sl_aword.as<int>();
+        sl.P = e.sl_GR.p;
+        sl.shift = e.sl_shift;
+        const cudaError_t err = launch_adjoint_sliced(a, sl, c->g.dim, e.precision == PXB_MIXED, c->stream);
+        if (err != cudaSuccess) return cuda_fail(err, "sliced adjoint step");
+        return check_launch(c, "sliced adjoint step");
+    }
     const bool aligned = ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(w) |
                            reinterpret_cast<uintptr_t>(rin)) & 15u) == 0;
     if (staged && e.adj_sg_on && adj_sched(c) >= 2 && rin && aligned) {
@@ -1749,8 +1800,8 @@ int adj_kernel(pxb_ctx *c, const double *u, const double *w, double scale, doubl
         if (e.wait_tries >= 0) a.wait_tries = e.wait_tries;
         a.evict_first = e.evict_first ? 1 : 0;
         a.UW = uw;
-        const cudaError_t err = launch_epf_adjoint_tma(a, c->g.dim, e.precision == PXB_MIXED, adj_sched(c) - 2,
-                                                       c->stream);
+        const cudaError_t err = launch_epf_adjoint_tma(a, c->g.dim, e.precision == PXB_MIXED,
+                                                       std::min(adj_sched(c), 4) - 2, c->stream);
         if (err != cudaSuccess) return cuda_fail(err, "staged adjoint step");
         return check_launch(c, "staged adjoint step");
     }
@@ -1813,17 +1864,17 @@ extern "C" int pxb_epf_record_d(pxb_ctx *c, const double *u0_d, const double *v0
         return PXB_OK;
     };
     PXB_TRY(d2d(e.adj_u0.p, u0_d, bytes));
-    // start: u^{-1} = u0 - dt v0 + dt^2/2 a(u0) with the frozen mask (the START mode of the lane-group kernel)
+    // start: u^{-1} = u0 - dt v0 + dt^2/2 a(u0) with the frozen mask
     {
         EpfArgs a = epf_args(c);
-        a.u = u0_d;
+        a.u = e.adj_u0.as<double>();  // (the context's copy: the caller's may be aligned to 8 bytes only)
         a.u_other = P[1];
         a.v0 = v0_d;
         a.dt = dt;
         a.dt2 = 0.5 * dt * dt;
         a.damage = 0;
         a.sc_bond = nullptr;
-        const cudaError_t err = epf_launch(c, a, EPF_START, 1, c->stream);
+        const cudaError_t err = epf_launch(c, a, EPF_START, e.variant, c->stream);
         if (err != cudaSuccess) return cuda_fail(err, "recorded start");
         c->launches++;
         PXB_TRY(d2d(P[0], u0_d, bytes));
@@ -1863,40 +1914,56 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
     if (e.rec_steps < 0)
         return fail(PXB_ERR_STATE, "pxb_epf_adjoint_recorded_d: no recorded forward loop (pxb_epf_record_d)");
     if (!ubar_N_d || !u0bar_d) return fail(PXB_ERR_INVALID, "pxb_epf_adjoint_recorded_d: need dJ/du^N and dJ/du0");
-    PXB_TRY(ensure_grev(c));
     PXB_TRY(epf_ready(c));  // (recomputed segments)
-    struct SgOff {  // the reverse-only kernel is used inside this sweep only
+    struct SgOff {  // the reverse-only kernels are used inside this sweep only
         EpfState &e;
-        ~SgOff() { e.adj_sg_on = false; }
+        ~SgOff() { e.adj_sg_on = e.adj_sliced = false; }
     } sg_off{e};
-    e.adj_sg_on = false;
-    if (e.adj_GR.p) {  // the frozen mask in reverse-bond order, for this sweep
-        PXB_TRY(dev_alloc(c, e.adj_HR, (size_t)std::max(1LL, c->g.ldb)));  // to ldb: the staged kernel's copies
-        PXB_CUDA_TRY(cudaMemsetAsync(e.adj_HR.p, 0, e.adj_HR.bytes, c->stream));
-        PXB_CUDA_TRY(launch_reverse_health(e.health.as<uint8_t>(), c->g.rev.as<int>(), e.adj_HR.as<uint8_t>(), c->g.nb,
-                                           c->stream));
-        PXB_TRY(check_launch(c, "reverse health"));
-        // the own bonds' operator sums under the frozen mask: with every bond's reverse present, the reverse-only
-        // kernel then reads one operator stream per step instead of two (the missing count uses counter slot 5)
-        const int nc = c->g.dim == 3 ? 6 : 3;
-        if (adj_sched(c) != 0 &&
-            dev_alloc(c, e.adj_SG, sizeof(double) * nc * (size_t)std::max(1, c->g.n)) == PXB_OK) {
-            unsigned int *miss = reinterpret_cast<unsigned int *>(e.counters.as<unsigned long long>() + 5);
-            PXB_CUDA_TRY(cudaMemsetAsync(miss, 0, sizeof(unsigned int), c->stream));
-            PXB_CUDA_TRY(launch_own_sums(c->g.n, c->g.dim, e.precision == PXB_MIXED, c->g.off.as<int>(),
-                                         c->g.rev.as<int>(), e.health.as<uint8_t>(), e.G.p, (long long)c->g.ldb,
-                                         e.adj_SG.as<double>(), miss, c->stream));
-            PXB_TRY(check_launch(c, "own sums"));
-            unsigned int nmiss = 1;
-            PXB_TRY(d2h(c, &nmiss, miss, sizeof(nmiss)));
-            PXB_CUDA_TRY(cudaStreamSynchronize(c->stream));
-            e.adj_sg_on = nmiss == 0;
-            // the staged kernel's interleaved (u, w) gather rows (without room for them it gathers u and w apart)
-            if (!e.adj_sg_on || adj_sched(c) < 2 ||
-                dev_alloc(c, e.adj_UW, sizeof(double) * 2 * c->g.dim * (size_t)std::max(1, c->g.n)) != PXB_OK)
-                e.adj_UW.release();
+    e.adj_sg_on = e.adj_sliced = false;
+    PXB_TRY(ensure_rev(c));
+    // the own bonds' operator sums under the frozen mask: with every bond's reverse present, the reverse-only kernels
+    // then read one operator stream per step instead of two (the missing count uses counter slot 5)
+    const int nc = c->g.dim == 3 ? 6 : 3;
+    bool sums = false;
+    if (adj_sched(c) != 0 && dev_alloc(c, e.adj_SG, sizeof(double) * nc * (size_t)std::max(1, c->g.n)) == PXB_OK) {
+        unsigned int *miss = reinterpret_cast<unsigned int *>(e.counters.as<unsigned long long>() + 5);
+        PXB_CUDA_TRY(cudaMemsetAsync(miss, 0, sizeof(unsigned int), c->stream));
+        PXB_CUDA_TRY(launch_own_sums(c->g.n, c->g.dim, e.precision == PXB_MIXED, c->g.off.as<int>(),
+                                     c->g.rev.as<int>(), e.health.as<uint8_t>(), e.G.p, (long long)c->g.ldb,
+                                     e.adj_SG.as<double>(), miss, c->stream));
+        PXB_TRY(check_launch(c, "own sums"));
+        unsigned int nmiss = 1;
+        PXB_TRY(d2h(c, &nmiss, miss, sizeof(nmiss)));
+        PXB_CUDA_TRY(cudaStreamSynchronize(c->stream));
+        sums = nmiss == 0;
+    }
+    if (sums && adj_sched(c) == 5) {  // the slices' reverse streams (without room for them: schedule 4)
+        bool built = e.sl_GR.p && e.sl_aword.p;
+        if (!built && c->g.max_family <= 0xffff && sliced_topology(c) == PXB_OK &&
+            sliced_alloc(c, e.sl_aword, e.sl_GR) == PXB_OK) {
+            PXB_TRY(sliced_fill(c, e.G.p, c->g.rev.as<int>(), e.sl_aword.as<int>(), e.sl_GR.p));
+            built = true;
+        }
+        if (built) {
+            PXB_TRY(sliced_health(c, c->g.rev.as<int>(), e.sl_aword.as<int>()));
+            e.adj_sliced = e.adj_sg_on = true;
         }
     }
+    if (!e.adj_sliced) {
+        PXB_TRY(ensure_grev(c));
+        if (e.adj_GR.p) {  // the frozen mask in reverse-bond order, for this sweep
+            PXB_TRY(dev_alloc(c, e.adj_HR, (size_t)std::max(1LL, c->g.ldb)));  // to ldb: the staged kernel's copies
+            PXB_CUDA_TRY(cudaMemsetAsync(e.adj_HR.p, 0, e.adj_HR.bytes, c->stream));
+            PXB_CUDA_TRY(launch_reverse_health(e.health.as<uint8_t>(), c->g.rev.as<int>(), e.adj_HR.as<uint8_t>(), c->g.nb,
+                                               c->stream));
+            PXB_TRY(check_launch(c, "reverse health"));
+            e.adj_sg_on = sums;
+        }
+    }
+    // the interleaved (u, w) gather rows of the staged and sliced kernels (without room for them they gather u and w apart)
+    if (!e.adj_sg_on || adj_sched(c) < 2 ||
+        dev_alloc(c, e.adj_UW, sizeof(double) * 2 * c->g.dim * (size_t)std::max(1, c->g.n)) != PXB_OK)
+        e.adj_UW.release();
     const size_t nd = (size_t)c->g.n * c->g.dim, bytes = sizeof(double) * nd;
     const int nsteps = e.rec_steps, K = e.rec_K;
     const double dt = e.rec_dt, dt2 = dt * dt;
@@ -1906,8 +1973,8 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
     PXB_TRY(dev_alloc(c, e.adj_W, bytes + 64));
     if (adj_sched(c) >= 2)  // the staged adjoint's wait-failure word
         PXB_CUDA_TRY(cudaMemsetAsync(e.counters.as<unsigned long long>() + 2, 0, sizeof(unsigned int), c->stream));
-    PXB_TRY(dev_alloc(c, e.adj_dC, 4 * sizeof(double)));
-    PXB_CUDA_TRY(cudaMemsetAsync(e.adj_dC.p, 0, 4 * sizeof(double), c->stream));
+    PXB_TRY(dev_alloc(c, e.adj_dC, (4 + 3 * kDcSlots) * sizeof(double)));  // the result, then the sliced kernel's slots
+    PXB_CUDA_TRY(cudaMemsetAsync(e.adj_dC.p, 0, e.adj_dC.bytes, c->stream));
     auto d2d = [&](void *dst, const void *src, size_t b) -> int {
         PXB_CUDA_TRY(cudaMemcpyAsync(dst, src, b, cudaMemcpyDeviceToDevice, c->stream));
         return PXB_OK;
@@ -1948,7 +2015,7 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
             PXB_TRY(adj_kernel(c, uq, W, dt2, 1.0, Rv, 2.0, A, -1.0, Rv, true, uw));
         }
     }
-    if (adj_sched(c) >= 2) {  // a staged wait that ran out fails the sweep
+    if (adj_sched(c) >= 2 && !e.adj_sliced) {  // a staged wait that ran out fails the sweep
         unsigned int werr = 0;
         PXB_TRY(d2h(c, &werr, e.counters.as<unsigned long long>() + 2, sizeof(unsigned int)));
         PXB_TRY(sync(c));
@@ -1956,6 +2023,10 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
     }
     // the start: dJ/du0 = A + R + (da/du)^T (dt^2/2 R), dJ/dv0 = -dt R
     PXB_TRY(adj_kernel(c, e.adj_u0.as<double>(), Rv, 0.5 * dt2, 1.0, A, 1.0, u0bar_d, -dt, v0bar_d));
+    if (e.adj_sliced) {
+        PXB_CUDA_TRY(launch_dc_collect(e.adj_dC.as<double>() + 4, e.adj_dC.as<double>(), c->stream));
+        PXB_TRY(check_launch(c, "dC collect"));
+    }
     if (dC_d) PXB_TRY(d2d(dC_d, e.adj_dC.p, 3 * sizeof(double)));
     return PXB_OK;
 }

@@ -53,11 +53,11 @@ __device__ __forceinline__ int ld_word(const int *p, unsigned long long pol) {
     return v;
 }
 
-// whether an intact bond clearly holds: a squared comparison in contracted arithmetic, whose rounding is far inside
-// the 1e-6 r^2 band folded into hi / lo (a zero-length bond is never tested and holds)
+// an intact bond by the squared comparison in contracted arithmetic: 1 holds, -1 breaks, 0 within 1e-6 r^2 of the
+// threshold (the contraction's rounding is far inside that band; a zero-length bond is never tested and holds)
 template <int DIM, typename PosT>
-__device__ __forceinline__ bool clearly_holds(const PosT &xi, const PosT &xj, const double *e, double hi, double lo,
-                                              bool tension_only) {
+__device__ __forceinline__ int verdict(const PosT &xi, const PosT &xj, const double *e, double hi2, double lo2,
+                                       bool tension_only) {
     double x[DIM];
     x[0] = xj.x - xi.x;
     x[1] = xj.y - xi.y;
@@ -69,7 +69,9 @@ __device__ __forceinline__ bool clearly_holds(const PosT &xi, const PosT &xj, co
         r2 = fma(x[d], x[d], r2);
         y2 = fma(y, y, y2);
     }
-    return (y2 < hi * r2 && (tension_only || y2 > lo * r2)) || !(r2 > 0.0);
+    const double band = 1.0e-6 * r2, qh = fma(-hi2, r2, y2), ql = fma(lo2, r2, -y2);
+    if (!(r2 > 0.0) || (qh < -band && (tension_only || ql < -band))) return 1;
+    return qh > band || (!tension_only && ql > band) ? -1 : 0;
 }
 
 // whether it breaks, in the reference's rounding where the squared comparison is within 1e-6 r^2 of the threshold
@@ -133,7 +135,7 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
     const int slice = a.node0 / 32 + blockIdx.x * SPB + sub;
     const int i = slice * 32 + lane;
     const bool act = i < a.n;
-    const bool rate = a.rate != 0;
+    const bool step = a.rate == kEpfStep;
     int r0 = 0, rows = 0;
     if (slice * 32 < a.n) {
         r0 = __ldg(sl.row0 + slice);
@@ -147,7 +149,6 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
     const unsigned long long pol = stream_policy(a.evict_first);
     const unsigned idmask = (1u << sl.shift) - 1u;
     const PosT *pos = static_cast<const PosT *>(a.pos);
-    const double hi = a.sc_hi2 - 1.0e-6, lo = a.sc_lo2 + 1.0e-6;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
     for (int q = 0; q < U; ++q) wd[q] = ld_word(W + q * 32, pol);
     if (act) {
         load_u<DIM>(a.u, i, ui);
-        if (w == 0 && !rate) {
+        if (w == 0 && step) {
 #pragma unroll
             for (int d = 0; d < DIM; ++d) up[d] = a.u_other[(size_t)i * DIM + d];
             if (a.bc_own) own_bits = __ldg(a.bc_own + i);
@@ -173,6 +174,13 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
         }
     }
     unsigned broken = 0;
+    // a bond breaks: in its word and in the health bytes
+    auto break_bond = [&](const int *at, int wq) {
+        const size_t k = (size_t)(at - sl.word);
+        sl.word[k] = wq | (int)0x80000000u;
+        a.health[__ldg(a.off + i) + sl.src[k]] = 0;
+        return 1u;
+    };
     // N rows whose words are in wd: coefficients and displacements, the words U rows on, then the arithmetic
     auto pass = [&](auto count) {
         constexpr int N = decltype(count)::value;
@@ -208,14 +216,16 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
 #pragma unroll
             for (int q = 0; q < N; ++q)
                 if (!hold[q] && wd[q] >= 0) {
-                    hold[q] = clearly_holds<DIM>(xi, xj[q], e[q], hi, lo, a.tension_only);
-                    if (!hold[q]) late |= 1u << q;
+                    const int v = a.damage ? verdict<DIM>(xi, xj[q], e[q], a.sc_hi2, a.sc_lo2, a.tension_only) : 1;
+                    hold[q] = v > 0;
+                    if (v == 0) late |= 1u << q;
+                    if (v < 0) broken += break_bond(W + q * 32, wd[q]);
                 }
         }
 #pragma unroll
         for (int q = 0; q < N; ++q)
             if (hold[q]) add_force<DIM>(p[q], e[q], L);
-        // the few bonds near the threshold or past it, everything read again (nothing of the fast path is kept for them)
+        // the few bonds near the threshold, everything read again (nothing of the fast path is kept for them)
         while (late) {
             const int q = __ffs(late) - 1;
             late &= late - 1;
@@ -224,11 +234,8 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
             load_u<DIM>(a.u, j, ej);
 #pragma unroll
             for (int d = 0; d < DIM; ++d) ej[d] = __dsub_rn(ej[d], ui[d]);
-            if (a.damage && breaks<DIM>(ldg_vec(pos + i), ldg_vec(pos + j), ej, a)) {
-                const size_t at = (size_t)(W + q * 32 - sl.word);
-                sl.word[at] = wq | (int)0x80000000u;
-                a.health[__ldg(a.off + i) + sl.src[at]] = 0;
-                ++broken;
+            if (breaks<DIM>(ldg_vec(pos + i), ldg_vec(pos + j), ej, a)) {
+                broken += break_bond(W + q * 32, wq);
             } else {
                 GT g[NC];
 #pragma unroll
@@ -270,8 +277,12 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
     for (int d = 0; d < DIM; ++d) {
         const double acc = __ddiv_rn(__dadd_rn(L[d], a.b[d]), a.rho);
         un[d] = 0.0;
-        if (act && rate) a.accel[(size_t)i * DIM + d] = acc;
-        if (act && !rate) {
+        if (act && a.rate == kEpfRate) a.accel[(size_t)i * DIM + d] = acc;
+        if (act && a.rate == kEpfStart) {
+            const double v = a.v0 ? a.v0[(size_t)i * DIM + d] : 0.0;
+            a.u_other[(size_t)i * DIM + d] = __dadd_rn(__dsub_rn(ui[d], __dmul_rn(a.dt, v)), __dmul_rn(a.dt2, acc));
+        }
+        if (act && step) {
             un[d] = cd_next(ui[d], up[d], acc, a.dt2, a.var_step, a.cv_rho, a.cv_w);
             if (!((own_bits >> d) & 1u)) {
                 a.u_other[(size_t)i * DIM + d] = un[d];
@@ -279,7 +290,7 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
             }
         }
     }
-    if (rate) return;
+    if (!step) return;
     const double t_new = e1 > e0 ? a.t_sched[a.step_in_chunk] : 0.0;
     for (int q = e0; q < e1; ++q) {  // the BC entries that read this node's new value (see EpfArgs)
         const int comp = a.bc_comp[q], form = a.bc_form[q];
@@ -301,6 +312,177 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
         const unsigned long long key = dbl_key(umax);
         volatile unsigned long long *m = a.umax + a.step_in_chunk;
         if (key > *m) atomicMax(a.umax + a.step_in_chunk, key);  // most slices find a larger value there
+    }
+}
+
+// ---- the reverse-only adjoint step on the slices -----------------------------------------------------------------
+// The sums of epf_adjoint_tma_kernel (k_epf_tma.cu) with a lane a node: row k of a slice holds the reverse operators of
+// the nodes' k-th bonds (sl.P: G in reverse-bond order) and words whose broken bit is the reverse bond's health.  Per bond
+// with source node j, L = abar_j and e = u_m - u_j, the force adjoint is split by constant,
+//   a1 = (g_d L_d),  a2 = the mixed-derivative part of L,  a3 = ((tr g - g_d) L_d),
+//   P(g) L = C11 a1 + (C12 + C66) a2 + C66 a3,   dC11 = a1.e,  dC12 = a2.e,  dC66 = (a2 + a3).e,
+// so scale / rho multiplies the nodes' sums once.  11.2 M bonds in 3D FP64 (0.60 GB): 138 us a step staged, 102 us here
+// (5.9 TB/s of the 6.5 a copy reaches).  dC: per-block sums into one of kDcSlots slots (an
+// address taking three atomics a block would serialise them), added up by dc_collect_kernel.
+template <int DIM>
+__device__ __forceinline__ void split_force(const double *g, const double *L, double *a1, double *a2, double *a3) {
+    if constexpr (DIM == 3) {
+        a2[0] = fma(g[4], L[2], g[3] * L[1]);
+        a2[1] = fma(g[5], L[2], g[3] * L[0]);
+        a2[2] = fma(g[5], L[1], g[4] * L[0]);
+        a3[0] = (g[1] + g[2]) * L[0];
+        a3[1] = (g[0] + g[2]) * L[1];
+        a3[2] = (g[0] + g[1]) * L[2];
+    } else {
+        a2[0] = g[2] * L[1];
+        a2[1] = g[2] * L[0];
+        a3[0] = g[1] * L[0];
+        a3[1] = g[0] * L[1];
+    }
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) a1[d] = g[d] * L[d];
+}
+
+template <int DIM, bool MIXED, int KW, int SPB, int U, int MINB>
+__global__ void __launch_bounds__(KW * SPB * 32, MINB) adjoint_sliced_kernel(EpfAdjArgs a, SlicedArgs sl) {
+    using GT = typename std::conditional<MIXED, float, double>::type;
+    constexpr int NC = DIM == 3 ? 6 : 3;
+    static_assert(U <= kSlicedSlack, "words are read U rows ahead");
+    __shared__ double part[SPB][KW > 1 ? KW - 1 : 1][DIM][32];
+    __shared__ double s_dC[KW * SPB][3];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, sub = wib / KW, w = wib % KW;
+    const int slice = blockIdx.x * SPB + sub, m = slice * 32 + lane;
+    const bool act = m < a.n;
+    int r0 = 0, rows = 0;
+    if (slice * 32 < a.n) {
+        r0 = __ldg(sl.row0 + slice);
+        rows = __ldg(sl.row0 + slice + 1) - r0;
+    }
+    const int kb = rows * w / KW, ke = rows * (w + 1) / KW;
+    const GT *P = static_cast<const GT *>(sl.P) + ((size_t)(r0 + kb) * NC * 32 + lane);
+    const int *W = sl.word + ((size_t)(r0 + kb) * 32 + lane);
+    const unsigned long long pol = stream_policy(a.evict_first);
+    const unsigned idmask = (1u << sl.shift) - 1u;
+    int wd[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) wd[q] = ld_word(W + q * 32, pol);
+    double um[DIM], F[DIM], dC[3] = {0.0, 0.0, 0.0};  // F: the force sums with the constants in
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) um[d] = F[d] = 0.0;
+    if (act) load_u<DIM>(a.u, m, um);
+    const double ac = a.C12 + a.C66;
+    auto pass = [&](auto count) {
+        constexpr int N = decltype(count)::value;
+        GT p[N][NC];
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) p[q][c] = ld_stream(P + (q * NC + c) * 32, pol);
+        double uj[N][DIM], L[N][DIM];
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            const unsigned j = (unsigned)wd[q] & idmask;
+            if (a.UW) {  // one interleaved row (u_j, abar_j): DIM 16-byte loads
+                const double2 *row = reinterpret_cast<const double2 *>(a.UW) + (size_t)j * DIM;
+                double r[2 * DIM];
+#pragma unroll
+                for (int h = 0; h < DIM; ++h) {
+                    const double2 v = __ldg(row + h);
+                    r[2 * h] = v.x;
+                    r[2 * h + 1] = v.y;
+                }
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) {
+                    uj[q][d] = r[d];
+                    L[q][d] = r[DIM + d];
+                }
+            } else {
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) {
+                    uj[q][d] = __ldg(a.u + (size_t)j * DIM + d);
+                    L[q][d] = __ldg(a.abar + (size_t)j * DIM + d);
+                }
+            }
+        }
+        int wn[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) wn[q] = ld_word(W + (U + q) * 32, pol);
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+            if (wd[q] >= 0) {
+                double g[NC], a1[DIM], a2[DIM], a3[DIM];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) g[c] = (double)p[q][c];
+                split_force<DIM>(g, L[q], a1, a2, a3);
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) {
+                    const double e = um[d] - uj[q][d];
+                    F[d] = fma(a.C11, a1[d], fma(ac, a2[d], fma(a.C66, a3[d], F[d])));
+                    dC[0] = fma(a1[d], e, dC[0]);
+                    dC[1] = fma(a2[d], e, dC[1]);
+                    dC[2] = fma(a3[d], e, dC[2]);
+                }
+            }
+        P += N * NC * 32;
+        W += N * 32;
+        if constexpr (N == U) {
+#pragma unroll
+            for (int q = 0; q < U; ++q) wd[q] = wn[q];
+        } else {
+#pragma unroll
+            for (int q = 0; q + 1 < U; ++q) wd[q] = wd[q + 1];
+        }
+    };
+    int k = kb;
+    for (; k + U <= ke; k += U) pass(std::integral_constant<int, U>{});
+    if constexpr (U > 1)
+        for (; k < ke; ++k) pass(std::integral_constant<int, 1>{});
+#pragma unroll
+    for (int q = 0; q < 3; ++q) dC[q] = group_sum<kWarp>(dC[q]);
+    if (lane == 0) {
+        s_dC[wib][0] = dC[0];
+        s_dC[wib][1] = dC[1];
+        s_dC[wib][2] = dC[1] + dC[2];
+    }
+    if constexpr (KW > 1)
+        if (w > 0)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) part[sub][w - 1][d][lane] = F[d];
+    __syncthreads();
+    const double lscale = a.scale * a.inv_rho;
+    if (threadIdx.x < 3 && a.dC) {
+        double s = 0.0;
+        for (int q = 0; q < KW * SPB; ++q) s += s_dC[q][threadIdx.x];
+        atomicAdd(a.dC + 3 * (blockIdx.x % kDcSlots) + threadIdx.x, lscale * s);
+    }
+    if (w > 0 || !act) return;
+    if constexpr (KW > 1)
+#pragma unroll
+        for (int q = 0; q < KW - 1; ++q)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) F[d] += part[sub][q][d][lane];
+    // the own bonds' term - P(SG_m) abar_m, then the central difference's transpose
+    double sg[NC], wm[DIM], a1[DIM], a2[DIM], a3[DIM];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) sg[c] = __ldg(a.SG + (size_t)m * NC + c);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) wm[d] = a.abar[(size_t)m * DIM + d];
+    split_force<DIM>(sg, wm, a1, a2, a3);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const double own = fma(a.C11, a1[d], fma(ac, a2[d], a.C66 * a3[d]));
+        const size_t k2 = (size_t)m * DIM + d;
+        const double r = a.rin ? a.rin[k2] : 0.0;
+        a.ubar[k2] = a.c_r * r + a.c_w * wm[d] + lscale * (F[d] - own);
+        if (a.rout) a.rout[k2] = a.c_o * wm[d];
+    }
+}
+
+__global__ void dc_collect_kernel(const double *slots, double *dC) {
+    if (threadIdx.x < 3) {
+        double s = dC[threadIdx.x];
+        for (int k = 0; k < kDcSlots; ++k) s += slots[3 * k + threadIdx.x];
+        dC[threadIdx.x] = s;
     }
 }
 
@@ -339,11 +521,13 @@ __global__ void __launch_bounds__(256) sliced_rank_kernel(int n, const int *off,
     if (lane == 0) atomicMax(rmax_key, dbl_key(rmax));
 }
 
-// Warp per slice: the words (without the broken bit of real bonds) and the coefficients, row by row
+// Warp per slice: the words (without the broken bit of real bonds) and the coefficients, row by row; rev: those of the
+// reverse bonds
 template <int DIM, typename GT>
 __global__ void __launch_bounds__(256) sliced_fill_kernel(int n, const int *off, const int *nbr, const void *posv,
                                                           const int *row0, const uint16_t *src, int shift, double inv_step,
-                                                          int qmax, const GT *Pc, long long ldb, int *word, GT *P) {
+                                                          int qmax, const GT *Pc, long long ldb, const int *rev, int *word,
+                                                          GT *P) {
     using PosT = typename Vec<DIM>::T;
     constexpr int NC = DIM == 3 ? 6 : 3;
     const PosT *pos = static_cast<const PosT *>(posv);
@@ -369,33 +553,52 @@ __global__ void __launch_bounds__(256) sliced_fill_kernel(int n, const int *off,
                 }
                 word[at] = w;
             }
+            const int tc = k >= len ? -1 : (rev ? rev[t] : t);
 #pragma unroll
             for (int c = 0; c < NC; ++c)
-                P[((size_t)(r0 + k) * NC + c) * 32 + lane] = k < len ? Pc[(size_t)c * ldb + t] : GT(0);
+                P[((size_t)(r0 + k) * NC + c) * 32 + lane] = tc >= 0 ? Pc[(size_t)c * ldb + tc] : GT(0);
         }
     }
 }
 
-// Warp per slice: the words' broken bits from the health bytes
+// The words' broken bits from the health bytes (rev: those of the reverse bonds): four warps a slice, eight rows in
+// flight a lane (a warp a slice and a row at a time, each row waited for a chain of two or three loads: 147 us for
+// 11.2 M bonds with rev, 70 us now)
 __global__ void __launch_bounds__(256) sliced_health_kernel(int n, const int *off, const int *row0, const uint16_t *src,
-                                                            const uint8_t *health, int *word) {
+                                                            const uint8_t *health, const int *rev, int *word) {
+    constexpr int U = 8, KW = 4;
     const int lane = threadIdx.x & 31, nsl = (n + 31) / 32;
-    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nsl; s += (gridDim.x * blockDim.x) >> 5) {
-        const int r0 = row0[s], i = s * 32 + lane;
+    for (int x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < nsl * KW; x += (gridDim.x * blockDim.x) >> 5) {
+        const int s = x / KW, w = x % KW, r0 = row0[s], rows = row0[s + 1] - r0, i = s * 32 + lane;
         const int b0 = i < n ? off[i] : 0, len = i < n ? off[i + 1] - b0 : 0;
-#pragma unroll 4
-        for (int k = 0; k < len; ++k) {
-            const size_t at = (size_t)(r0 + k) * 32 + lane;
-            const int w = word[at], v = (w & 0x7fffffff) | (health[b0 + src[at]] ? 0 : (int)0x80000000u);
-            if (v != w) word[at] = v;
+        const int ke = min(len, rows * (w + 1) / KW);
+        for (int k = rows * w / KW; k < ke; k += U) {
+            int t[U], v[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const size_t at = (size_t)(r0 + k + q) * 32 + lane;
+                t[q] = k + q < ke ? b0 + (int)src[at] : -1;
+                v[q] = k + q < ke ? word[at] : 0;
+            }
+            if (rev)
+#pragma unroll
+                for (int q = 0; q < U; ++q) t[q] = t[q] >= 0 ? __ldg(rev + t[q]) : -1;
+            uint8_t h[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) h[q] = t[q] >= 0 ? health[t[q]] : (uint8_t)0;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int x2 = (v[q] & 0x7fffffff) | (h[q] ? 0 : (int)0x80000000u);
+                if (k + q < ke && x2 != v[q]) word[(size_t)(r0 + k + q) * 32 + lane] = x2;
+            }
         }
     }
 }
 
 namespace {
-int slice_grid(int n) {
-    const int g = ((n + 31) / 32 + 7) / 8;
-    return g < 1 ? 1 : (g < 148 * 8 ? g : 148 * 8);
+int slice_grid(long long n) {
+    const long long g = ((n + 31) / 32 + 7) / 8;
+    return (int)(g < 1 ? 1 : (g < 148 * 8 ? g : 148 * 8));
 }
 
 template <int DIM, bool MIXED, int KW, int SPB, int U, int MINB>
@@ -404,7 +607,7 @@ cudaError_t launch_sliced(const EpfArgs &a, const SlicedArgs &sl, cudaStream_t s
     const int slices = (a.n - a.node0 + 31) / 32, grid = (slices + SPB - 1) / SPB;
     if (grid <= 0) return cudaSuccess;
     epf_note_shape(LaunchShape{grid, KW * SPB * 32, 0});
-    if (a.pdl && !a.rate) {
+    if (a.pdl && a.rate == kEpfStep) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)grid);
         cfg.blockDim = dim3(KW * SPB * 32);
@@ -452,6 +655,24 @@ cudaError_t launch_epf_sliced(const EpfArgs &a, const SlicedArgs &sl, int dim, b
     return mixed ? launch_cfg<2, true>(a, sl, which, s) : launch_cfg<2, false>(a, sl, which, s);
 }
 
+template <int DIM, bool MIXED, int KW, int SPB, int U, int MINB>
+static cudaError_t launch_adj(const EpfAdjArgs &a, const SlicedArgs &sl, cudaStream_t s) {
+    const int grid = ((a.n + 31) / 32 + SPB - 1) / SPB;
+    adjoint_sliced_kernel<DIM, MIXED, KW, SPB, U, MINB><<<grid > 0 ? grid : 1, KW * SPB * 32, 0, s>>>(a, sl);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_sliced(const EpfAdjArgs &a, const SlicedArgs &sl, int dim, bool mixed, cudaStream_t s) {
+    if (!sl.word || !sl.P || !sl.row0 || !a.SG) return cudaErrorInvalidValue;
+    if (dim == 3) return mixed ? launch_adj<3, true, 4, 1, 2, 5>(a, sl, s) : launch_adj<3, false, 4, 1, 2, 5>(a, sl, s);
+    return mixed ? launch_adj<2, true, 4, 1, 2, 6>(a, sl, s) : launch_adj<2, false, 4, 1, 2, 6>(a, sl, s);
+}
+
+cudaError_t launch_dc_collect(const double *slots, double *dC, cudaStream_t s) {
+    dc_collect_kernel<<<1, 32, 0, s>>>(slots, dC);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_sliced_rank(int n, int dim, const int *off, const int *nbr, const void *pos, const int *row0, uint16_t *src,
                                unsigned long long *rmax_key, cudaStream_t s) {
     const int g = (n + 7) / 8 < 148 * 8 ? (n + 7) / 8 : 148 * 8;
@@ -462,21 +683,21 @@ cudaError_t launch_sliced_rank(int n, int dim, const int *off, const int *nbr, c
 
 cudaError_t launch_sliced_fill(int n, int dim, bool mixed, const int *off, const int *nbr, const void *pos, const int *row0,
                                const uint16_t *src, int shift, double inv_step, int qmax, const void *Pc, long long ldb,
-                               int *word, void *P, cudaStream_t s) {
+                               const int *rev, int *word, void *P, cudaStream_t s) {
     const int g = slice_grid(n);
     if (dim == 3) {
-        if (mixed) sliced_fill_kernel<3, float><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const float *)Pc, ldb, word, (float *)P);
-        else sliced_fill_kernel<3, double><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const double *)Pc, ldb, word, (double *)P);
+        if (mixed) sliced_fill_kernel<3, float><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const float *)Pc, ldb, rev, word, (float *)P);
+        else sliced_fill_kernel<3, double><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const double *)Pc, ldb, rev, word, (double *)P);
     } else {
-        if (mixed) sliced_fill_kernel<2, float><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const float *)Pc, ldb, word, (float *)P);
-        else sliced_fill_kernel<2, double><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const double *)Pc, ldb, word, (double *)P);
+        if (mixed) sliced_fill_kernel<2, float><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const float *)Pc, ldb, rev, word, (float *)P);
+        else sliced_fill_kernel<2, double><<<g, 256, 0, s>>>(n, off, nbr, pos, row0, src, shift, inv_step, qmax, (const double *)Pc, ldb, rev, word, (double *)P);
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_sliced_health(int n, const int *off, const int *row0, const uint16_t *src, const uint8_t *health, int *word,
-                                 cudaStream_t s) {
-    sliced_health_kernel<<<slice_grid(n), 256, 0, s>>>(n, off, row0, src, health, word);
+cudaError_t launch_sliced_health(int n, const int *off, const int *row0, const uint16_t *src, const uint8_t *health,
+                                 const int *rev, int *word, cudaStream_t s) {
+    sliced_health_kernel<<<slice_grid(4LL * n), 256, 0, s>>>(n, off, row0, src, health, rev, word);
     return cudaGetLastError();
 }
 

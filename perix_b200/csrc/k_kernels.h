@@ -123,6 +123,7 @@ cudaError_t launch_apply_batch(const BatchArgs &a, bool mixed, int variant, int 
 // ---------------------------------------------------------------------------------------- explicit fracture
 enum EpfMode { EPF_RATE = 0, EPF_START = 1, EPF_STEP = 2, EPF_FORCE_FROZEN = 3 };
 
+constexpr int kEpfStep = 0, kEpfRate = 1, kEpfStart = 2;  // EpfArgs::rate
 struct EpfArgs {
     int n = 0;
     long long nb = 0;
@@ -158,7 +159,7 @@ struct EpfArgs {
     unsigned long long *n_broken = nullptr; // broken-bond counter
     int maxb = 0;                           // TMA variants: staged bonds per tile (multiple of 32)
     unsigned int *err = nullptr;            // TMA variants: pipeline waits that ran out
-    int rate = 0;                           // TMA variants: RATE mode (accel out; u_other and BCs unused)
+    int rate = 0;  // TMA and sliced variants: kEpfStep, kEpfRate (accel out; u_other and BCs unused), kEpfStart (sliced only)
     int node0 = 0;  // TMA variants: the launch computes nodes [node0, n) (node0 a multiple of 64; RATE mode only)
     // TMA variants, STEP mode: launch with programmatic stream serialisation, so that inside a captured loop of
     // steps the next step's blocks start their set-up while this step's last blocks finish (host-side only)
@@ -181,7 +182,7 @@ constexpr int kEpfTmaConfigs = 12;                // staged (TMA) configurations
 constexpr int kEpfSlicedConfigs = 4;              // sliced configurations per dimension (k_epf_sliced.cu)
 // 0-2 lane groups, 3-4 CSR tiles, then staged, then sliced
 constexpr int kEpfVariants = 5 + kEpfTmaConfigs + kEpfSlicedConfigs;
-// (a sliced variant is launched by launch_epf_sliced; here its START and FORCE_FROZEN modes run variant 1)
+// (a sliced variant is launched by launch_epf_sliced)
 cudaError_t launch_epf(const EpfArgs &a, int dim, bool mixed, int mode, int variant, cudaStream_t s);
 // P[c][t] from G[c][t] (t < ldb, SoA stride ldb): 2D p11 = C11 Gxx + C66 Gyy, p22 = C66 Gxx + C11 Gyy,
 // pxy = (C12 + C66) Gxy; 3D p11/p22/p33 and (C12 + C66) times Gxy, Gxz, Gyz
@@ -235,10 +236,11 @@ cudaError_t launch_sliced_rank(int n, int dim, const int *off, const int *nbr, c
 // coefficients from the bond-ordered ones (SoA stride ldb)
 cudaError_t launch_sliced_fill(int n, int dim, bool mixed, const int *off, const int *nbr, const void *pos, const int *row0,
                                const uint16_t *src, int shift, double inv_step, int qmax, const void *Pc, long long ldb,
-                               int *word, void *P, cudaStream_t s);
-// the words' broken bits from the health bytes
-cudaError_t launch_sliced_health(int n, const int *off, const int *row0, const uint16_t *src, const uint8_t *health, int *word,
-                                 cudaStream_t s);
+                               const int *rev, int *word, void *P, cudaStream_t s);
+// the words' broken bits from the health bytes.  rev (both): the coefficients / health of the reverse bonds (0 and broken
+// where there is none)
+cudaError_t launch_sliced_health(int n, const int *off, const int *row0, const uint16_t *src, const uint8_t *health,
+                                 const int *rev, int *word, cudaStream_t s);
 
 struct EpfAdjArgs {
     int n = 0;
@@ -282,6 +284,11 @@ cudaError_t launch_epf_adjoint(const EpfAdjArgs &a, int dim, bool mixed, int gri
 // node / bonds per pass / occupancy configuration.
 cudaError_t launch_epf_adjoint_tma(const EpfAdjArgs &a, int dim, bool mixed, int which, cudaStream_t s);
 int epf_adj_tma_maxb(int dim, int max_family);
+// The same step on the slices: sl.P the operators (not packed) in reverse-bond order, sl.word with the reverse bonds'
+// health, sl.src unused; dC receives per-block sums in kDcSlots slots of three, which launch_dc_collect adds up
+constexpr int kDcSlots = 64;
+cudaError_t launch_adjoint_sliced(const EpfAdjArgs &a, const SlicedArgs &sl, int dim, bool mixed, cudaStream_t s);
+cudaError_t launch_dc_collect(const double *slots, double *dC, cudaStream_t s);
 // SG[m][c] = sum_{t in fam(m), health[t]} G[c][t] (nc = 3 in 2D, 6 in 3D, FP64 sums); missing[0] += the bonds
 // without a reverse bond (rev t < 0)
 cudaError_t launch_own_sums(int n, int dim, bool mixed, const int *off, const int *rev, const uint8_t *health,

@@ -123,7 +123,8 @@ struct EpfState {
     // the sliced step's copy of the streams (k_epf_sliced.cu), built when a sliced variant is first selected: rows of
     // the slices, words, coefficients, places in the family; sl_P_stale: the constants changed since they were filled,
     // sl_stale: something other than a sliced launch may have written health since the words' broken bits were set
-    DevBuf sl_row0, sl_word, sl_P, sl_src;
+    // sl_GR, sl_aword: the reverse sweep's (operators in reverse-bond order; words whose broken bits are the reverse bonds')
+    DevBuf sl_row0, sl_word, sl_P, sl_src, sl_GR, sl_aword;
     bool sl_ready = false, sl_P_stale = false, sl_stale = true;
     int sl_shift = 31;
     double sl_step = 0.0;
@@ -137,6 +138,7 @@ struct EpfState {
     bool adj_GR_none = false;  // no room for adj_GR: the adjoint kernel gathers the reverse bonds' operators
     DevBuf adj_SG;             // per-node sums of the healthy own bonds' operators (rebuilt by every reverse sweep)
     DevBuf adj_UW;             // the staged adjoint's gather rows (u, w) interleaved, [n][2 dim] (empty: apart)
+    bool adj_sliced = false;   // inside a reverse sweep on the slices
     bool adj_sg_on = false;    // inside a reverse sweep whose families all have reverse bonds: reverse-only kernel
     // the recorded forward loop (pxb_epf_record_d): rec_steps < 0 when there is none; rec_all: every state kept
     double rec_dt = 0.0;
@@ -238,8 +240,9 @@ struct pxb_ctx {
     size_t mem_limit = 0;  // device bytes the context may hold (0: no limit beyond the GPU's)
     int gbuild_schedule = -1;  // g-build: -1 by problem, 0 lane groups, 1 one warp per node, 2 the same with
                                // its products on the FP64 tensor cores
-    int adj_schedule = -1;     // recorded reverse sweep: -1 default (4), 0 both operator streams, 1 reverse-only,
-                               // 2-4 reverse-only staged (bulk-copy ring) in three launch configurations
+    int adj_schedule = -1;     // recorded reverse sweep: -1 default (5; 4 without room for its streams), 0 both operator
+                               // streams, 1 reverse-only, 2-4 reverse-only staged (bulk-copy ring) in three launch
+                               // configurations, 5 reverse-only on the slices
     int rate_chunks = -1;      // pipelined rate call: -1 by mesh size, 1 off, 2..8 node chunks
     cudaStream_t own = nullptr;
     cudaStream_t stream = nullptr;

@@ -222,7 +222,7 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
     }
     Snapshot keep;
     PXB_TRY(save_state(c, keep));
-    std::vector<float> ms((size_t)std::max(steps, 2)), mean_ms(kEpfVariants, 1e30f);
+    std::vector<float> ms((size_t)std::max(steps, 2)), step_ms(kEpfVariants, 1e30f);
     float best_ms = 1e30f;
     int best_v = c->epf.variant;
     for (int v = 0; v < kEpfVariants; ++v) {
@@ -243,8 +243,9 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
         for (int k = 0; k < steps; ++k) mean += ms[(size_t)k];
         mean /= (float)steps;
         if (ms_per_variant) ms_per_variant[v] = mean;
-        mean_ms[(size_t)v] = mean;
-        if (mean < best_ms) { best_ms = mean; best_v = v; }
+        std::nth_element(ms.begin(), ms.begin() + steps / 2, ms.begin() + steps);
+        step_ms[(size_t)v] = ms[(size_t)(steps / 2)];  // the median decides: one late step must not
+        if (step_ms[(size_t)v] < best_ms) { best_ms = step_ms[(size_t)v]; best_v = v; }
     }
     // Streams that stay in L2 from one step to the next: a run's captured steps are faster than the flushed ones timed
     // above, and not by the same factor for every schedule (the 2.25 M-bond plate, mixed: 24.5 and 25.3 us flushed, 13.6
@@ -253,7 +254,7 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
         float loop_best = 1e30f;
         for (int v = 0; v < kEpfVariants; ++v) {
             float t = 0.f;
-            if (mean_ms[(size_t)v] > 1.1f * best_ms || select_variant(c, v) != PXB_OK) continue;
+            if (step_ms[(size_t)v] > 1.1f * best_ms || select_variant(c, v) != PXB_OK) continue;
             if (loop_time(c, keep, &t) != PXB_OK) break;  // (a run that blows up within the loop: the flushed choice stands)
             if (t < loop_best) { loop_best = t; best_v = v; }
         }

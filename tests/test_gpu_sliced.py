@@ -160,3 +160,56 @@ def test_no_room_for_the_copy():
         c.epf_advance(1)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("keep", [0, 3])
+@pytest.mark.parametrize("dim,shape", [(2, (4, 8)), (2, (23, 29)), (3, (5, 5, 5)), (3, (7, 6, 9))])
+def test_sliced_adjoint_matches_reverse_only_kernel(ctx, dim, shape, keep, precision):
+    """The reverse sweep on the slices (adjoint schedule 5) against the unstaged reverse-only kernel (1), with a health
+    mask that differs between a bond and its reverse.  With k as in _bound but over the larger of the operators' row and
+    column sums, the adjoint's magnitude and the difference of the two sweeps grow along the transposed central difference
+    as M_{n+1} <= (2 + k) M_n + M_{n-1} and d_{n+1} <= (2 + k) d_n + d_{n-1} + (m + 10) eps (2 + k) M_n; dC adds one term a
+    bond and step in trees of fewer than 256 levels."""
+    import ctypes
+    import torch
+    steps = 7
+    u0, off, dt, C = _setup(ctx, dim, shape, sc=0.0, precision=precision)
+    x, vol, off, ids, h = _mesh(dim, shape)
+    ctx.gbuild(2, 0)
+    g = np.abs(ctx.get_ops())[:, dim:].sum(1)
+    i = np.repeat(np.arange(len(off) - 1), np.diff(off))
+    row, col = np.zeros(len(off) - 1), np.zeros(len(off) - 1)
+    np.add.at(row, i, g)
+    np.add.at(col, ids - 1, g)
+    k = 2 * dt * dt * (C[0] + C[1] + 2 * C[2]) * max(row.max(), col.max()) / 2440.0
+    dev = torch.device("cuda", 0)
+    ctx.set_stream(torch.cuda.current_stream(dev).cuda_stream)
+    rng = np.random.default_rng(3)
+    u = torch.tensor(u0, device=dev)
+    gN = torch.tensor(rng.standard_normal(u0.size), device=dev)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    out = []
+    for v, schedule in ((6, 1), (17, 5)):
+        ctx.epf_set_variant(6)
+        assert ctx.L.pxb_epf_record_d(ctx.h, p(u), None, ctypes.c_double(dt), steps, keep, None, None) == 0
+        ctx.epf_set_adjoint_schedule(schedule)
+        ub, vb = torch.empty_like(u), torch.empty_like(u)
+        dC = torch.zeros(3, dtype=torch.float64, device=dev)
+        assert ctx.L.pxb_epf_adjoint_recorded_d(ctx.h, p(gN), None, p(ub), p(vb), p(dC)) == 0
+        out.append((ub.cpu().numpy(), vb.cpu().numpy(), dC.cpu().numpy()))
+    ctx.epf_set_adjoint_schedule(-1)
+    ctx.set_stream(None)
+    m = int(np.diff(off).max())
+    M, Mp, d, dp = float(gN.abs().max()), 0.0, 0.0, 0.0
+    terms, emax = 0.0, 2 * float(u.abs().max()) * (2 + k) ** steps
+    for _ in range(steps + 1):
+        terms += 4 * dim * dt * dt / 2440.0 * g.sum() * M * emax
+        d, dp = (2 + k) * d + dp + (m + 10) * EPS * (2 + k) * M, d
+        M, Mp = (2 + k) * M + Mp, M
+    (ua, va, ca), (ub, vb, cb) = out
+    assert np.abs(ua - ub).max() <= d and np.abs(va - vb).max() <= dt * d
+    assert np.abs(ca - cb).max() <= 256 * EPS * terms + terms * d / M
+    # and far closer than that in practice: the bounds above are for the worst case
+    assert np.linalg.norm(ua - ub) <= 1e-10 * np.linalg.norm(ua)
+    assert np.abs(ca - cb).max() <= 1e-9 * np.abs(ca).max()
