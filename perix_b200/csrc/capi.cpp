@@ -72,6 +72,12 @@ static int malloc_dev(void **p, size_t bytes) {
 
 int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
     if (b.p && b.bytes == bytes) return PXB_OK;
+    // the adjoint's optional scratch makes room for what has to be there
+    if (c && c->ops.bond.p && &b != &c->ops.bond && bytes > b.bytes) {
+        size_t free_b = 0, total_b = 0;
+        const bool over = c->mem_limit && ctx_bytes(c) - b.bytes + bytes > c->mem_limit;
+        if (over || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > free_b)) c->ops.bond.release();
+    }
     if (c && c->mem_limit && bytes > b.bytes && ctx_bytes(c) - b.bytes + bytes > c->mem_limit)
         return fail(PXB_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes would exceed the context's " +
                                      std::to_string(c->mem_limit) + "-byte limit (pxb_ctx_set_memory_limit)");
@@ -125,7 +131,7 @@ size_t ctx_bytes(const pxb_ctx *c) {
     size_t s = 0;
     const Geometry &g = c->g;
     s += bufsz(g.off) + bufsz(g.nbr) + bufsz(g.pos) + bufsz(g.vol) + bufsz(g.mirror) + bufsz(g.layer) + bufsz(g.rev);
-    s += bufsz(c->ops.ops) + bufsz(c->ops.degenerate) + bufsz(c->ops.defect) + bufsz(c->ops.yeff);
+    s += bufsz(c->ops.ops) + bufsz(c->ops.degenerate) + bufsz(c->ops.defect) + bufsz(c->ops.yeff) + bufsz(c->ops.bond);
     const EpfState &e = c->epf;
     s += bufsz(e.G) + bufsz(e.P) + bufsz(e.xib) + bufsz(e.health) + bufsz(e.u[0]) + bufsz(e.u[1]) + bufsz(e.accel) + bufsz(e.counters) +
          bufsz(e.umax) + bufsz(e.tsched) + bufsz(e.sc_bond) + bufsz(e.sl_row0) + bufsz(e.sl_word) + bufsz(e.sl_P) +
@@ -235,6 +241,7 @@ extern "C" int pxb_ctx_destroy(pxb_ctx *c) {
     cudaStreamSynchronize(c->stream);
     drop_snapshot(c);
     destroy_graphs(c->epf);
+    if (c->bond_ev) cudaEventDestroy(c->bond_ev);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
     return PXB_OK;
@@ -636,6 +643,22 @@ extern "C" int pxb_apply(pxb_ctx *c, const double *u, int nk, const int *slots, 
     return sync(c);
 }
 
+// Scratch of the two-pass transpose, or NULL for the one-pass kernel: where the operator row has no kernels of
+// its own, when the memory (limit) does not hold it, and under stream capture, whose graph would keep a pointer
+// to a buffer that the context may give up.
+static double *adjoint_scratch(pxb_ctx *c, const ApplyArgs &a) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!apply_has_rows(a) || c->g.nb == 0 || cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess ||
+        cap != cudaStreamCaptureStatusNone)
+        return nullptr;
+    const size_t need = sizeof(double) * (size_t)c->g.nb;
+    if (c->ops.bond.bytes != need && dev_alloc(c, c->ops.bond, need) != PXB_OK) return nullptr;
+    if (!c->bond_ev && cudaEventCreateWithFlags(&c->bond_ev, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+    if (c->bond_stream && c->bond_stream != c->stream && cudaStreamWaitEvent(c->stream, c->bond_ev, 0) != cudaSuccess)
+        return nullptr;
+    return c->ops.bond.as<double>();
+}
+
 extern "C" int pxb_apply_adjoint_d(pxb_ctx *c, const double *ybar_d, int nk, const int *slots, double *ubar_d) {
     ApplyArgs a;
     PXB_TRY(apply_args(c, nk, slots, a, "pxb_apply_adjoint"));
@@ -672,8 +695,15 @@ extern "C" int pxb_apply_adjoint_d(pxb_ctx *c, const double *ybar_d, int nk, con
         for (int s = 0; s < p.next; ++s) a.slots[s] = p.ext[s];
         a.u = p.yeff;
     }
-    launch_apply_adjoint(a, c->ops.precision == PXB_MIXED, grid_nodes(a.n, kApplyThreads), c->stream);
-    return check_launch(c, "apply_adjoint");
+    double *bond = adjoint_scratch(c, a);
+    launch_apply_adjoint(a, c->ops.precision == PXB_MIXED, bond, grid_nodes(a.n, kApplyThreads), c->stream);
+    PXB_TRY(check_launch(c, "apply_adjoint"));
+    if (bond) {
+        c->launches++;
+        PXB_CUDA_TRY(cudaEventRecord(c->bond_ev, c->stream));
+        c->bond_stream = c->stream;
+    }
+    return PXB_OK;
 }
 
 extern "C" int pxb_apply_adjoint(pxb_ctx *c, const double *ybar, int nk, const int *slots, double *ubar) {

@@ -11,6 +11,7 @@ namespace pxb {
 
 constexpr int kMaxK = 20;
 
+// Any operator row and slot list; rows of 2, 3, 5 and 9 operators go to apply_rows_kernel below instead.
 // MIXED: FP32-stored operators widened to FP64 for the products and sums (HBM-bound: the arithmetic is free);
 // with a.defect (mixed, order 2) every requested second derivative is corrected by the first-moment defect of
 // its stored operator, D^k -= sum_m defect[k][m] D^m, the first derivatives D^m being summed alongside.
@@ -87,6 +88,8 @@ cudaError_t launch_apply_adjoint_prep(const AdjPrepArgs &p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// One pass, no scratch: rows of other lengths, and every row where the scratch of the two passes below is not to be
+// had (memory, stream capture).
 template <bool MIXED>
 __global__ void __launch_bounds__(kApplyThreads) apply_adjoint_kernel(ApplyArgs a) {
     constexpr int WPB = kApplyThreads / kWarp;
@@ -121,15 +124,174 @@ __global__ void __launch_bounds__(kApplyThreads) apply_adjoint_kernel(ApplyArgs 
     }
 }
 
+// ---- operator rows of a size known at compile time ---------------------------------------------------------
+// Operators of first and second order (2 and 5 in 2D, 3 and 9 in 3D) and of third order in 2D (9): LPN lanes a
+// node stride its family, so that a warp's loads cover consecutive operator rows and every sector of a row is
+// used by the loads issued with it, and one butterfly over the group closes each sum.  `used` masks the
+// operators that some slot asks for; a slot list in any order, with repeats, is met by selecting from the sums.
+// What bounds both kernels is the operator stream (72 bytes a bond in 3D FP64), read once.
+// 124,416 nodes, 14.2 million bonds, 9 FP64 operators (1.08 GB): 190 us, 0.87 of the measured copy rate; the warp a
+// node over a run-time slot list (apply_kernel) 431 us.
+template <int NOP>
+__device__ __forceinline__ double pick(const double (&v)[NOP], int k) {
+    double r = v[0];
+#pragma unroll
+    for (int q = 1; q < NOP; ++q) r = k == q ? v[q] : r;
+    return r;
+}
+
+template <bool MIXED, int NOP, int LPN>
+__global__ void __launch_bounds__(kApplyThreads) apply_rows_kernel(ApplyArgs a, unsigned int used) {
+    using GT = typename std::conditional<MIXED, float, double>::type;
+    const int q = (blockIdx.x * kApplyThreads + threadIdx.x) / LPN;
+    const int gl = threadIdx.x & (LPN - 1);
+    const bool act = q < a.n;
+    const int i = act ? q : a.n - 1;
+    const int b0 = a.off[i], b1 = act ? a.off[i + 1] : b0;
+    const double ui = a.u[i];
+    const GT *ops = static_cast<const GT *>(a.ops);
+    double acc[NOP];
+#pragma unroll
+    for (int k = 0; k < NOP; ++k) acc[k] = 0.0;
+    for (int t = b0 + gl; t < b1; t += LPN) {
+        const double du = __ldg(a.u + __ldg(a.nbr + t)) - ui;
+        const GT *g = ops + (size_t)t * NOP;
+#pragma unroll
+        for (int k = 0; k < NOP; ++k)
+            if (used >> k & 1u) acc[k] = fma((double)__ldg(g + k), du, acc[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < NOP; ++k) acc[k] = group_sum<LPN>(acc[k]);
+    for (int s = gl; s < a.nk && act; s += LPN) {
+        const int k = a.slots[s];
+        double v = pick<NOP>(acc, k);
+        if (MIXED && a.defect && k >= a.dim) {
+            const float *dv = a.defect + ((size_t)i * (NOP - a.dim) + (k - a.dim)) * a.dim;
+            for (int m = 0; m < a.dim; ++m) v -= (double)__ldg(dv + m) * pick<NOP>(acc, m);
+        }
+        a.out[(size_t)i * a.nk + s] = v;
+    }
+}
+
+// Transpose in two passes.  The first streams the operators in their own order and keeps one scalar a bond,
+// s_t = sum_k g^k_t ybar_i^k (8 bytes), and the node's -sum_t s_t in out; the second adds the s of the reverse
+// bonds.  Gathering the reverse bonds' operator rows instead reads 72 bytes a bond a second time, out of order.
+// Same mesh: 197 + 61 us (1.19 and 0.17 GB) against 717 us for the gather of rows (apply_adjoint_kernel).
+template <bool MIXED, int NOP, int LPN>
+__global__ void __launch_bounds__(kApplyThreads) adjoint_bonds_kernel(ApplyArgs a, unsigned int used, double *bond) {
+    using GT = typename std::conditional<MIXED, float, double>::type;
+    const int q = (blockIdx.x * kApplyThreads + threadIdx.x) / LPN;
+    const int gl = threadIdx.x & (LPN - 1);
+    const bool act = q < a.n;
+    const int i = act ? q : a.n - 1;
+    const int b0 = a.off[i], b1 = act ? a.off[i + 1] : b0;
+    const GT *ops = static_cast<const GT *>(a.ops);
+    double y[NOP];
+#pragma unroll
+    for (int k = 0; k < NOP; ++k) y[k] = 0.0;
+    for (int s = 0; s < a.nk; ++s) {
+        const double v = __ldg(a.u + (size_t)i * a.nk + s);
+#pragma unroll
+        for (int k = 0; k < NOP; ++k) y[k] += a.slots[s] == k ? v : 0.0;
+    }
+    double own = 0.0;
+    for (int t = b0 + gl; t < b1; t += LPN) {
+        const GT *g = ops + (size_t)t * NOP;
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < NOP; ++k)
+            if (used >> k & 1u) v = fma((double)__ldg(g + k), y[k], v);
+        bond[t] = v;
+        own += v;
+    }
+    own = group_sum<LPN>(own);
+    if (act && gl == 0) a.out[i] = -own;
+}
+
+template <int LPN>
+__global__ void __launch_bounds__(kApplyThreads) adjoint_gather_kernel(ApplyArgs a, const double *bond) {
+    const int q = (blockIdx.x * kApplyThreads + threadIdx.x) / LPN;
+    const int gl = threadIdx.x & (LPN - 1);
+    const bool act = q < a.n;
+    const int i = act ? q : a.n - 1;
+    const int b0 = a.off[i], b1 = act ? a.off[i + 1] : b0;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int t = b0 + gl; t < b1; t += LPN) {
+        const int r = __ldg(a.rev + t);
+        if (r >= 0) acc += __ldg(bond + r);
+    }
+    acc = group_sum<LPN>(acc);
+    if (act && gl == 0) a.out[i] += acc;
+}
+
+static unsigned int used_ops(const ApplyArgs &a) {
+    unsigned int m = 0;
+    for (int s = 0; s < a.nk; ++s) m |= 1u << a.slots[s];
+    if (a.defect)
+        for (int s = 0; s < a.nk; ++s)
+            if (a.slots[s] >= a.dim) m |= (1u << a.dim) - 1u;
+    return m;
+}
+
+template <int LPN>
+static int rows_grid(int n) {
+    return (int)(((long long)n * LPN + kApplyThreads - 1) / kApplyThreads);
+}
+
+template <bool MIXED, int NOP, int LPN>
+static cudaError_t rows_forward(const ApplyArgs &a, cudaStream_t s) {
+    apply_rows_kernel<MIXED, NOP, LPN><<<rows_grid<LPN>(a.n), kApplyThreads, 0, s>>>(a, used_ops(a));
+    return cudaGetLastError();
+}
+
+template <bool MIXED, int NOP, int LPN>
+static cudaError_t rows_adjoint(const ApplyArgs &a, double *bond, cudaStream_t s) {
+    ApplyArgs b = a;
+    b.defect = nullptr;  // already transposed into ybar
+    adjoint_bonds_kernel<MIXED, NOP, LPN><<<rows_grid<LPN>(a.n), kApplyThreads, 0, s>>>(b, used_ops(b), bond);
+    adjoint_gather_kernel<LPN><<<rows_grid<LPN>(a.n), kApplyThreads, 0, s>>>(b, bond);
+    return cudaGetLastError();
+}
+
+// `f(mixed, nop, lanes)` for an operator row with a kernel of its own; false: the general kernels
+template <typename F>
+static bool with_rows(const ApplyArgs &a, bool mixed, F f) {
+    auto lanes = [&](auto nop) {
+        using N = decltype(nop);
+        if (a.dim == 3) mixed ? f(std::true_type{}, N{}, std::integral_constant<int, 16>{}) : f(std::false_type{}, N{}, std::integral_constant<int, 16>{});
+        else mixed ? f(std::true_type{}, N{}, std::integral_constant<int, 8>{}) : f(std::false_type{}, N{}, std::integral_constant<int, 8>{});
+    };
+    switch (a.nop) {
+        case 2: lanes(std::integral_constant<int, 2>{}); return true;
+        case 3: lanes(std::integral_constant<int, 3>{}); return true;
+        case 5: lanes(std::integral_constant<int, 5>{}); return true;
+        case 9: lanes(std::integral_constant<int, 9>{}); return true;
+        default: return false;
+    }
+}
+
+bool apply_has_rows(const ApplyArgs &a) { return a.nop == 2 || a.nop == 3 || a.nop == 5 || a.nop == 9; }
+
 cudaError_t launch_apply(const ApplyArgs &a, bool mixed, int grid, cudaStream_t s) {
     if (a.nk > kMaxK) return cudaErrorInvalidValue;
+    cudaError_t e = cudaSuccess;
+    if (with_rows(a, mixed, [&](auto mx, auto nop, auto lpn) {
+            e = rows_forward<decltype(mx)::value, decltype(nop)::value, decltype(lpn)::value>(a, s);
+        }))
+        return e;
     if (mixed) apply_kernel<true><<<grid, kApplyThreads, 0, s>>>(a);
     else apply_kernel<false><<<grid, kApplyThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_apply_adjoint(const ApplyArgs &a, bool mixed, int grid, cudaStream_t s) {
+cudaError_t launch_apply_adjoint(const ApplyArgs &a, bool mixed, double *bond, int grid, cudaStream_t s) {
     if (a.nk > kMaxK) return cudaErrorInvalidValue;
+    cudaError_t e = cudaSuccess;
+    if (bond && with_rows(a, mixed, [&](auto mx, auto nop, auto lpn) {
+            e = rows_adjoint<decltype(mx)::value, decltype(nop)::value, decltype(lpn)::value>(a, bond, s);
+        }))
+        return e;
     if (mixed) apply_adjoint_kernel<true><<<grid, kApplyThreads, 0, s>>>(a);
     else apply_adjoint_kernel<false><<<grid, kApplyThreads, 0, s>>>(a);
     return cudaGetLastError();

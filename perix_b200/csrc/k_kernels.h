@@ -325,7 +325,9 @@ struct ApplyArgs {
     int dim = 2;
 };
 cudaError_t launch_apply(const ApplyArgs &a, bool mixed, int grid, cudaStream_t s);
-cudaError_t launch_apply_adjoint(const ApplyArgs &a, bool mixed, int grid, cudaStream_t s);
+bool apply_has_rows(const ApplyArgs &a);  // the operator row has kernels of its own
+// bond: one double a bond of scratch for the two-pass transpose, NULL for the kernel that needs none
+cudaError_t launch_apply_adjoint(const ApplyArgs &a, bool mixed, double *bond, int grid, cudaStream_t s);
 struct AdjPrepArgs {
     int n = 0, dim = 2, nop = 0, nk = 0, next = 0;
     int slots[32], ext[32];

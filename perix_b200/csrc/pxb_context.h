@@ -88,6 +88,7 @@ struct OpsCache {
     DevBuf degenerate;  // uint8 [n]
     DevBuf defect;      // mixed, order 2: double [n][(nop - dim) * dim] first-moment defects (GBuildArgs::defect)
     DevBuf yeff;        // adjoint with defects: transposed-correction ybar (grown on demand)
+    DevBuf bond;        // adjoint: one double a bond between its two passes (optional, given up when memory is short)
     std::vector<int> pqr;
 };
 
@@ -237,6 +238,9 @@ struct BatchState {
 
 struct pxb_ctx {
     int device = 0;
+    // last use of ops.bond: another stream's use waits for it
+    cudaEvent_t bond_ev = nullptr;
+    cudaStream_t bond_stream = nullptr;
     size_t mem_limit = 0;  // device bytes the context may hold (0: no limit beyond the GPU's)
     int gbuild_schedule = -1;  // g-build: -1 by problem, 0 lane groups, 1 one warp per node, 2 the same with
                                // its products on the FP64 tensor cores
