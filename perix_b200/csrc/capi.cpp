@@ -70,14 +70,25 @@ static int malloc_dev(void **p, size_t bytes) {
     return cuda_fail(e, "cudaMalloc");
 }
 
+// What the context can do without gives way to what has to be there: the field transpose's scratch, then the
+// implicit run's slices (both are built again by a use that finds the memory).
+static void make_room(pxb_ctx *c, const DevBuf &b, size_t bytes) {
+    CsrState &k = c->csr;
+    auto short_of = [&]() {
+        if (c->mem_limit && ctx_bytes(c) - b.bytes + bytes > c->mem_limit) return true;
+        size_t free_b = 0, total_b = 0;
+        return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > free_b;
+    };
+    if (c->ops.bond.p && &b != &c->ops.bond && short_of()) c->ops.bond.release();
+    if (k.sl_pair.p && &b != &k.sl_pair && &b != &k.sl_col && &b != &k.sl_row0 && short_of()) {
+        k.sl_pair.release();
+        k.sl_col.release();
+    }
+}
+
 int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
     if (b.p && b.bytes == bytes) return PXB_OK;
-    // the adjoint's optional scratch makes room for what has to be there
-    if (c && c->ops.bond.p && &b != &c->ops.bond && bytes > b.bytes) {
-        size_t free_b = 0, total_b = 0;
-        const bool over = c->mem_limit && ctx_bytes(c) - b.bytes + bytes > c->mem_limit;
-        if (over || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > free_b)) c->ops.bond.release();
-    }
+    if (c && bytes > b.bytes) make_room(c, b, bytes);
     if (c && c->mem_limit && bytes > b.bytes && ctx_bytes(c) - b.bytes + bytes > c->mem_limit)
         return fail(PXB_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes would exceed the context's " +
                                      std::to_string(c->mem_limit) + "-byte limit (pxb_ctx_set_memory_limit)");
@@ -145,7 +156,8 @@ size_t ctx_bytes(const pxb_ctx *c) {
          bufsz(bt.ops) + bufsz(bt.degenerate) + bufsz(bt.counters) + bufsz(bt.defect);
     const CsrState &k = c->csr;
     s += bufsz(k.rowptr) + bufsz(k.cols) + bufsz(k.slot) + bufsz(k.bpos) + bufsz(k.spos) + bufsz(k.xpos) + bufsz(k.diag) + bufsz(k.kvals) + bufsz(k.rhs) +
-         bufsz(k.u) + bufsz(k.uold) + bufsz(k.fnode) + bufsz(k.mnode);
+         bufsz(k.u) + bufsz(k.uold) + bufsz(k.fnode) + bufsz(k.mnode) + bufsz(k.sl_row0) + bufsz(k.sl_col) +
+         bufsz(k.sl_pair);
     s += bufsz(c->ch.rev) + bufsz(c->ch.lap) + bufsz(c->ch.ghost) + bufsz(c->ch.lrv) + bufsz(c->ch.bfl) +
          bufsz(c->scratch);
     return s;

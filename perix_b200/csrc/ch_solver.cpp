@@ -33,6 +33,7 @@ struct RunCtx {
     int n;
     long long rows;
     pxb_ch_run_params p;
+    bool slices = false;  // Newton systems on slices, else as CSR values
 };
 
 int need_ch_run(pxb_ctx *c, const char *who) {
@@ -54,25 +55,110 @@ int check(pxb_ctx *c, cudaError_t e, const char *what) {
     return PXB_OK;
 }
 
-int alloc_run(RunCtx &r) {
+// the transposed block view and value permutation of the pattern, and room for K^T (adjoint solves)
+int ensure_transpose(pxb_ctx *c) {
+    CsrState &k = c->csr;
+    if (!k.transposed) {
+        if (k.h_bptr.empty()) {  // a pattern built on the device: its block view comes to the host once
+            k.h_bptr.resize((size_t)c->g.n + 1);
+            PXB_TRY(d2h(c, k.h_bptr.data(), k.bptr.p, sizeof(int) * k.h_bptr.size()));
+            PXB_TRY(sync(c));
+            k.h_bcol.resize((size_t)k.h_bptr.back());
+            if (!k.h_bcol.empty()) PXB_TRY(d2h(c, k.h_bcol.data(), k.bcol.p, sizeof(int) * k.h_bcol.size()));
+            PXB_TRY(sync(c));
+        }
+        std::vector<int> tbptr, tbcol, perm;
+        block_transpose(c->g.n, k.h_bptr, k.h_bcol, tbptr, tbcol, perm);
+        PXB_TRY(dev_upload(c, k.tbptr, tbptr.data(), sizeof(int) * tbptr.size()));
+        PXB_TRY(dev_upload(c, k.tbcol, tbcol.data(), sizeof(int) * std::max<size_t>(1, tbcol.size())));
+        PXB_TRY(dev_upload(c, k.tperm, perm.data(), sizeof(int) * std::max<size_t>(1, perm.size())));
+        PXB_TRY(sync(c));
+        k.transposed = true;
+    }
+    return dev_alloc(c, c->ch.kvt, sizeof(double) * (size_t)k.nnz);
+}
+
+// Slices of an exact pattern (k_bicg.cu), built by the pattern's first run; false when there is no memory for them
+bool ensure_slices(pxb_ctx *c, int *status) {
+    CsrState &k = c->csr;
+    const Geometry &g = c->g;
+    *status = PXB_OK;
+    if (!k.exact) return false;
+    if (k.sl_pair.p) return true;
+    const int ns = (g.n + 31) / 32;
+    std::vector<int> row0((size_t)ns + 1, 0);
+    for (int s = 0; s < ns; ++s) {
+        int w = 0;
+        for (int i = 32 * s; i < std::min(g.n, 32 * (s + 1)); ++i)  // a bulk row holds its own block and its family's
+            if (g.h_mirror.empty() || g.h_mirror[(size_t)i] <= 0)
+                w = std::max(w, g.h_off[(size_t)i + 1] - g.h_off[(size_t)i] + 1);
+        row0[(size_t)s + 1] = row0[(size_t)s] + w;
+    }
+    const size_t cells = 32 * (size_t)std::max(1, row0[(size_t)ns]);
+    if (dev_alloc(c, k.sl_row0, sizeof(int) * row0.size()) != PXB_OK ||
+        dev_alloc(c, k.sl_col, sizeof(int) * cells) != PXB_OK || dev_alloc(c, k.sl_pair, 16 * cells) != PXB_OK) {
+        k.sl_row0.release();
+        k.sl_col.release();
+        k.sl_pair.release();
+        return false;
+    }
+    ChSlices m;
+    m.n = g.n;
+    m.row0 = k.sl_row0.as<int>();
+    m.col = k.sl_col.as<int>();
+    m.pair = k.sl_pair.as<double2>();
+    m.mirror = g.mirror.p ? g.mirror.as<int>() : nullptr;
+    m.bptr = k.bptr.as<int>();
+    m.bcol = k.bcol.as<int>();
+    *status = h2d(c, k.sl_row0.p, row0.data(), sizeof(int) * row0.size());
+    if (*status == PXB_OK) *status = check(c, launch_ch_slices_fill(m, c->stream), "ch slices");
+    if (*status == PXB_OK) *status = sync(c);  // row0 is this function's
+    if (*status != PXB_OK) k.sl_pair.release();
+    return *status == PXB_OK;
+}
+
+// `values`: the CSR values too
+int alloc_buffers(RunCtx &r, bool values) {
     pxb_ctx *c = r.c;
     ChState &h = c->ch;
     const size_t rows = (size_t)r.rows, n = (size_t)r.n;
+    if (values) PXB_TRY(dev_alloc(c, h.kv, sizeof(double) * (size_t)c->csr.nnz));
     PXB_TRY(dev_alloc(c, h.U, sizeof(double) * rows));
     PXB_TRY(dev_alloc(c, h.Uold, sizeof(double) * rows));
     PXB_TRY(dev_alloc(c, h.dU, sizeof(double) * rows));
     PXB_TRY(dev_alloc(c, h.rhs, sizeof(double) * rows));
-    PXB_TRY(dev_alloc(c, h.kv, sizeof(double) * (size_t)c->csr.nnz));
     PXB_TRY(dev_alloc(c, h.mnode, sizeof(double) * n));
     PXB_TRY(dev_alloc(c, h.binv, sizeof(double) * 4 * n));
     PXB_TRY(dev_alloc(c, h.red, sizeof(double) * (size_t)(dot_scratch_doubles() + 8)));
     PXB_TRY(dev_alloc(c, h.nodal, sizeof(double) * 2 * n));
     for (auto &w : h.w) PXB_TRY(dev_alloc(c, w, sizeof(double) * rows));
     PXB_TRY(dev_alloc(c, h.bicg, kBicgScalarBytes + sizeof(double) * 6 * kBicgParts));
+    return PXB_OK;
+}
+
+// `solve`: Newton systems; `states`: states a gradient keeps (0: no gradient, no transposed system)
+int alloc_run(RunCtx &r, bool solve, size_t states) {
+    pxb_ctx *c = r.c;
+    ChState &h = c->ch;
+    const size_t n = (size_t)r.n, hist = sizeof(double) * (size_t)r.rows * states;
+    if (solve) {
+        int st = PXB_OK;
+        r.slices = ensure_slices(c, &st);
+        PXB_TRY(st);
+    }
+    PXB_TRY(alloc_buffers(r, states > 0 || (solve && !r.slices)));
+    if (states > 0) {
+        PXB_TRY(dev_alloc(c, h.hist, hist));
+        PXB_TRY(ensure_transpose(c));
+    }
     PXB_TRY(ensure_pinned(h.bicg_h, kBicgScalarBytes + sizeof(double) * kHostDots));
     if (h.ones.bytes < sizeof(double) * n) {
         std::vector<double> one(n, 1.0);
         PXB_TRY(dev_upload(c, h.ones, one.data(), sizeof(double) * n));
+    }
+    if (r.slices && !c->csr.sl_pair.p) {  // they made room for what has to be there
+        r.slices = false;
+        PXB_TRY(dev_alloc(c, h.kv, sizeof(double) * (size_t)c->csr.nnz));
     }
     return PXB_OK;
 }
@@ -126,14 +212,10 @@ ChAdjArgs adj_args(RunCtx &r, const double *U, const double *x, double *y) {
 // Right-preconditioned BiCGStab for A x = b (x starts at 0) on the device, one cooperative kernel (k_bicg.cu); A = K
 // (ch.kv) or, for adjoint solves, K'^T (ch.kvt through the transposed block view); the block-Jacobi inverse of A must
 // be in ch.binv.  Launches only; bicg_outcome reads the result after the caller's next synchronisation.
-int bicgstab_launch(RunCtx &r, bool adjoint, const double *b, double *x) {
-    pxb_ctx *c = r.c;
-    ChState &h = c->ch;
+BicgArgs bicg_args(RunCtx &r, const double *b, double *x) {
+    ChState &h = r.c->ch;
     BicgArgs a;
     a.n = r.n;
-    a.bptr = (adjoint ? c->csr.tbptr : c->csr.bptr).as<int>();
-    a.bcol = (adjoint ? c->csr.tbcol : c->csr.bcol).as<int>();
-    a.val = (adjoint ? h.kvt : h.kv).as<double>();
     a.binv = h.binv.as<double>();
     a.b = b;
     a.x = x;
@@ -150,6 +232,16 @@ int bicgstab_launch(RunCtx &r, bool adjoint, const double *b, double *x) {
     a.vh[1] = h.w[10].as<double>();
     a.sc = h.bicg.as<BicgScalars>();
     a.part = reinterpret_cast<double *>(h.bicg.as<char>() + kBicgScalarBytes);
+    return a;
+}
+
+int bicgstab_launch(RunCtx &r, bool adjoint, const double *b, double *x) {
+    pxb_ctx *c = r.c;
+    ChState &h = c->ch;
+    BicgArgs a = bicg_args(r, b, x);
+    a.bptr = (adjoint ? c->csr.tbptr : c->csr.bptr).as<int>();
+    a.bcol = (adjoint ? c->csr.tbcol : c->csr.bcol).as<int>();
+    a.val = (adjoint ? h.kvt : h.kv).as<double>();
     PXB_TRY(check(c, launch_bicg_solve(a, r.p.lin_rtol, r.p.lin_max, c->stream), "bicgstab"));
     return PXB_OK;
 }
@@ -169,12 +261,16 @@ int queue_readback(pxb_ctx *c, int ndots) {
     return PXB_OK;
 }
 
+int bicg_timeout() {
+    return fail(PXB_ERR_CUDA, "CH linear solve: a grid barrier of the BiCGStab kernel timed out");
+}
+
 int bicg_outcome(ChState &h, int *its, double *relres) {
     const BicgScalars *hs = host_outcome(h);
     *its = hs->its;
     *relres = hs->relres;
     if (hs->status == kBicgDone) return PXB_OK;
-    if (hs->abort) return fail(PXB_ERR_CUDA, "CH linear solve: a grid barrier of the BiCGStab kernel timed out");
+    if (hs->abort) return bicg_timeout();
     const char *why = hs->status == kBicgBreakdown ? " (breakdown)" : "";
     return fail(PXB_ERR_STATE, "CH linear solve: BiCGStab stopped at relative residual " + std::to_string(*relres) +
                                    " after " + std::to_string(*its) + " iterations" + why);
@@ -187,27 +283,54 @@ int dot_into(RunCtx &r, long long len, const double *a, const double *b, int k) 
     return check(c, launch_dot(len, a, b, red, dev_dots(c->ch) + k, c->stream), "dot");
 }
 
-// the transposed block view and value permutation of the pattern, and room for K^T (adjoint solves)
-int ensure_transpose(pxb_ctx *c) {
-    CsrState &k = c->csr;
-    if (!k.transposed) {
-        if (k.h_bptr.empty()) {  // a pattern built on the device: its block view comes to the host once
-            k.h_bptr.resize((size_t)c->g.n + 1);
-            PXB_TRY(d2h(c, k.h_bptr.data(), k.bptr.p, sizeof(int) * k.h_bptr.size()));
-            PXB_TRY(sync(c));
-            k.h_bcol.resize((size_t)k.h_bptr.back());
-            if (!k.h_bcol.empty()) PXB_TRY(d2h(c, k.h_bcol.data(), k.bcol.p, sizeof(int) * k.h_bcol.size()));
-            PXB_TRY(sync(c));
-        }
-        std::vector<int> tbptr, tbcol, perm;
-        block_transpose(c->g.n, k.h_bptr, k.h_bcol, tbptr, tbcol, perm);
-        PXB_TRY(dev_upload(c, k.tbptr, tbptr.data(), sizeof(int) * tbptr.size()));
-        PXB_TRY(dev_upload(c, k.tbcol, tbcol.data(), sizeof(int) * std::max<size_t>(1, tbcol.size())));
-        PXB_TRY(dev_upload(c, k.tperm, perm.data(), sizeof(int) * std::max<size_t>(1, perm.size())));
-        PXB_TRY(sync(c));
-        k.transposed = true;
-    }
-    return dev_alloc(c, c->ch.kvt, sizeof(double) * (size_t)k.nnz);
+// one Newton iteration on the slices: the system at (U, Uold), then the solve and update in one kernel.  The outcome
+// (|F|, solve, update and state norms) is in host_outcome; `stop`: |F| that ends the step, `only_norm`: |F| only.
+int newton_iteration(RunCtx &r, double *U, const double *Uold, double stop, bool only_norm) {
+    pxb_ctx *c = r.c;
+    ChState &h = c->ch;
+    const CsrState &k = c->csr;
+    ChSystemArgs s;
+    s.n = r.n;
+    s.kappa = r.p.kappa;
+    s.chi = r.p.chi;
+    s.dt = r.p.dt;
+    s.M0 = r.p.M0;
+    s.off = c->g.off.as<int>();
+    s.nbr = c->g.nbr.as<int>();
+    s.mirror = c->g.mirror.p ? c->g.mirror.as<int>() : nullptr;
+    s.row0 = k.sl_row0.as<int>();
+    s.lap = h.lap.as<double>();
+    s.lrv = h.lrv.as<double>();
+    s.vol = c->g.vol.as<double>();
+    s.bfl = h.bfl.as<uint8_t>();
+    s.bpos = k.bpos.as<uint8_t>();
+    s.spos = k.spos.as<uint8_t>();
+    s.u = U;
+    s.uold = Uold;
+    s.pair = k.sl_pair.as<double2>();
+    s.binv = h.binv.as<double>();
+    s.rhs = h.rhs.as<double>();
+    s.sc = h.bicg.as<BicgScalars>();
+    PXB_TRY(check(c, launch_ch_system(s, c->stream), "ch system"));
+    BicgArgs a = bicg_args(r, h.rhs.as<double>(), h.dU.as<double>());
+    a.r0 = h.rhs.as<double>();  // the shadow residual is the right-hand side, which no phase writes
+    ChSlices m;
+    m.n = r.n;
+    m.row0 = s.row0;
+    m.col = k.sl_col.as<int>();
+    m.pair = s.pair;
+    m.mirror = s.mirror;
+    m.d0 = -(1.0 / r.p.dt);
+    m.g0 = ghost_scale(r.p.dt);
+    ChNewton nw;
+    nw.u = U;
+    nw.stop = stop;
+    nw.only_norm = only_norm ? 1 : 0;
+    nw.tol = r.p.lin_rtol;
+    nw.max_its = r.p.lin_max;
+    PXB_TRY(check(c, launch_ch_newton(a, m, nw, c->stream), "ch newton"));
+    PXB_TRY(queue_readback(c, 0));
+    return sync(c);
 }
 
 // one backward-Euler step: U (in: initial guess, out: converged state) from Uold
@@ -216,10 +339,17 @@ int newton_step(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) 
     ChState &h = c->ch;
     double res0 = -1.0;
     for (int it = 0; it <= r.p.newton_max; ++it) {
-        PXB_TRY(assemble(r, U, Uold));
-        double ff = 0.0;
-        PXB_TRY(dotp(r, r.rows, h.rhs.as<double>(), h.rhs.as<double>(), &ff));
-        const double res = std::sqrt(ff);
+        double res = 0.0;
+        if (r.slices) {
+            PXB_TRY(newton_iteration(r, U, Uold, it > 0 ? r.p.newton_rtol * res0 : 0.0, it == r.p.newton_max));
+            if (host_outcome(h)->abort) return bicg_timeout();
+            res = host_outcome(h)->bnorm;
+        } else {
+            PXB_TRY(assemble(r, U, Uold));
+            double ff = 0.0;
+            PXB_TRY(dotp(r, r.rows, h.rhs.as<double>(), h.rhs.as<double>(), &ff));
+            res = std::sqrt(ff);
+        }
         if (!std::isfinite(res)) return fail(PXB_ERR_BLOWUP, "CH Newton: non-finite residual");
         if (it == 0) res0 = res;
         st->max_residual = std::max(st->max_residual, it == 0 ? 0.0 : res / std::max(res0, 1e-300));
@@ -228,21 +358,24 @@ int newton_step(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) 
             return PXB_OK;
         }
         if (it == r.p.newton_max) break;
-        PXB_TRY(check(c, launch_block_inv(r.n, c->csr.diag.as<int>(), h.kv.as<double>(), false, h.binv.as<double>(),
-                                          c->stream),
-                      "block inverse"));
-        PXB_TRY(bicgstab_launch(r, false, h.rhs.as<double>(), h.dU.as<double>()));
-        PXB_TRY(dot_into(r, r.rows, h.dU.as<double>(), h.dU.as<double>(), 0));
-        PXB_TRY(dot_into(r, r.rows, U, U, 1));
-        PXB_TRY(check(c, launch_axpby(r.rows, 1.0, h.dU.as<double>(), 1.0, U, c->stream), "update"));
-        PXB_TRY(queue_readback(c, 2));
-        PXB_TRY(sync(c));
+        if (!r.slices) {
+            PXB_TRY(check(c, launch_block_inv(r.n, c->csr.diag.as<int>(), h.kv.as<double>(), false, h.binv.as<double>(),
+                                              c->stream),
+                          "block inverse"));
+            PXB_TRY(bicgstab_launch(r, false, h.rhs.as<double>(), h.dU.as<double>()));
+            PXB_TRY(dot_into(r, r.rows, h.dU.as<double>(), h.dU.as<double>(), 0));
+            PXB_TRY(dot_into(r, r.rows, U, U, 1));
+            PXB_TRY(check(c, launch_axpby(r.rows, 1.0, h.dU.as<double>(), 1.0, U, c->stream), "update"));
+            PXB_TRY(queue_readback(c, 2));
+            PXB_TRY(sync(c));
+        }
         int lits = 0;
         double lres = 0.0;
         PXB_TRY(bicg_outcome(h, &lits, &lres));
         st->lin_iters += lits;
         st->max_lin_relres = std::max(st->max_lin_relres, lres);
-        const double dd = host_dots(h)[0], uu = host_dots(h)[1];
+        const double dd = r.slices ? host_outcome(h)->dd : host_dots(h)[0];
+        const double uu = r.slices ? host_outcome(h)->uu : host_dots(h)[1];
         // an update at the rounding level of the state ends the iteration (the residual of a small step can sit
         // at its evaluation floor, far above newton_rtol times its initial value)
         if (std::sqrt(dd) <= kUpdateTol * std::sqrt(uu)) {
@@ -316,7 +449,7 @@ extern "C" int pxb_ch_run(pxb_ctx *c, const pxb_ch_run_params *p, const double *
                           pxb_ch_run_stats *stats) {
     PXB_TRY(validate(c, p, c0, "pxb_ch_run"));
     RunCtx r{c, c->g.n, 2LL * c->g.n, *p};
-    PXB_TRY(alloc_run(r));
+    PXB_TRY(alloc_run(r, true, 0));
     ChState &h = c->ch;
     pxb_ch_run_stats st{};
     PXB_TRY(initial_state(r, c0, h.U.as<double>()));
@@ -339,10 +472,9 @@ extern "C" int pxb_ch_gradient(pxb_ctx *c, const pxb_ch_run_params *p, const dou
                                double *dE_dc0, pxb_ch_run_stats *stats) {
     PXB_TRY(validate(c, p, c0, "pxb_ch_gradient"));
     RunCtx r{c, c->g.n, 2LL * c->g.n, *p};
-    PXB_TRY(alloc_run(r));
+    PXB_TRY(alloc_run(r, true, (size_t)p->nsteps + 1));
     ChState &h = c->ch;
     const size_t rows = (size_t)r.rows;
-    PXB_TRY(dev_alloc(c, h.hist, sizeof(double) * rows * ((size_t)p->nsteps + 1)));
     double *hist = h.hist.as<double>();
     pxb_ch_run_stats st{};
     PXB_TRY(initial_state(r, c0, hist));
@@ -356,7 +488,6 @@ extern "C" int pxb_ch_gradient(pxb_ctx *c, const pxb_ch_run_params *p, const dou
     double e = 0.0, dk = 0.0;
     double *g = h.Uold.as<double>(), *lam = h.dU.as<double>();
     PXB_TRY(energy(r, hist + rows * (size_t)p->nsteps, &e, &dk, g));
-    PXB_TRY(ensure_transpose(c));
     for (int s = p->nsteps; s >= 1; --s) {
         const double *Un = hist + rows * (size_t)s;
         // A = (K - J_M)^T at (U_n, U_{n-1}): fold the mobility derivative into K, then transpose the values
@@ -407,7 +538,7 @@ extern "C" int pxb_ch_energy(pxb_ctx *c, double kappa, double chi, const double 
     p.kappa = kappa;
     p.chi = chi;
     RunCtx r{c, c->g.n, 2LL * c->g.n, p};
-    PXB_TRY(alloc_run(r));
+    PXB_TRY(alloc_run(r, false, 0));
     ChState &h = c->ch;
     PXB_TRY(h2d(c, h.U.p, u, sizeof(double) * (size_t)r.rows));
     PXB_TRY(energy(r, h.U.as<double>(), E, nullptr, dE_du ? h.dU.as<double>() : nullptr));

@@ -507,6 +507,7 @@ enum BicgStatus : int { kBicgRunning = 0, kBicgDone = 2, kBicgBreakdown = 3, kBi
 constexpr int kBicgParts = 148 * 8;  // most blocks of the solve kernel (one partial sum slot each)
 struct BicgScalars {
     double relres;
+    double bnorm, dd, uu;                // Newton solve: |F|, |x|^2 and |U|^2 before the update
     int status, its;                     // status: kBicgRunning until the solve ends (then abort tells a timeout)
     unsigned int bar_count;              // grid barrier arrivals
     int abort;                           // set by a barrier wait that gave up
@@ -520,6 +521,41 @@ struct BicgArgs {
     BicgScalars *sc = nullptr;
     double *part = nullptr;  // 6 * kBicgParts doubles (two alternating sets of three)
 };
+// The Newton system of the implicit Cahn-Hilliard run on slices of 32 nodes (k_bicg.cu): pairs and columns at
+// 32 (row0[s] + k) + lane; bulk rows have the diagonal (d0, d1), ghost rows the scale (g0, g1)
+struct ChSlices {
+    int n = 0;
+    const int *row0 = nullptr;
+    int *col = nullptr;
+    double2 *pair = nullptr;
+    const int *mirror = nullptr;
+    const int *bptr = nullptr, *bcol = nullptr;  // fill only
+    double d0 = 0.0, d1 = -1.0, g0 = 1.0, g1 = 1.0;
+};
+struct ChSystemArgs {
+    int n = 0;
+    double kappa = 0, chi = 0, dt = 1, M0 = 0;
+    const int *off = nullptr, *nbr = nullptr, *mirror = nullptr, *row0 = nullptr;
+    const double *lap = nullptr, *lrv = nullptr, *vol = nullptr;
+    const uint8_t *bfl = nullptr, *bpos = nullptr, *spos = nullptr;
+    const double *u = nullptr, *uold = nullptr;  // u 16-byte aligned
+    double2 *pair = nullptr;
+    double *binv = nullptr, *rhs = nullptr;
+    BicgScalars *sc = nullptr;  // cleared for the solve that follows
+};
+struct ChNewton {
+    double *u = nullptr;      // U += x when the solve ends
+    double stop = 0.0;        // |F| <= stop: nothing to solve
+    int only_norm = 0;        // |F| only
+    double tol = 0.0;
+    int max_its = 0;
+};
+// scale of a ghost row: the magnitude of the element's own diagonal entry (1 when zero)
+inline __host__ __device__ double ghost_scale(double dt) { return 1.0 / dt > 0.0 ? 1.0 / dt : 1.0; }
+cudaError_t launch_ch_slices_fill(const ChSlices &a, cudaStream_t s);
+cudaError_t launch_ch_system(const ChSystemArgs &a, cudaStream_t s);
+// the solve and the update of one Newton iteration as one cooperative kernel (scalars cleared by launch_ch_system)
+cudaError_t launch_ch_newton(const BicgArgs &a, const ChSlices &m, const ChNewton &nw, cudaStream_t s);
 // Block view of a 2-dof CSR pattern (host arrays): false unless rows 2i and 2i+1 share one column list of pairs
 // (2j, 2j+1); then bptr[i] = rowptr[2i] / 4 and bcol lists node i's column nodes.
 bool block_view(int n, const int *rowptr, const int *cols, std::vector<int> &bptr, std::vector<int> &bcol);

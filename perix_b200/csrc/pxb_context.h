@@ -203,6 +203,7 @@ struct CsrState {
     bool blocked2 = false, transposed = false;
     std::vector<int> h_bptr, h_bcol;
     DevBuf bptr, bcol, tbptr, tbcol, tperm;
+    DevBuf sl_row0, sl_col, sl_pair;  // exact 2-dof pattern: the implicit run's slices (ChSlices), built by its first use
     DevBuf kvals, rhs, u, uold, fnode, mnode;
 };
 
