@@ -254,6 +254,8 @@ extern "C" int pxb_ctx_destroy(pxb_ctx *c) {
     drop_snapshot(c);
     destroy_graphs(c->epf);
     if (c->bond_ev) cudaEventDestroy(c->bond_ev);
+    for (cudaEvent_t e : c->newton_ev)
+        if (e) cudaEventDestroy(e);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
     return PXB_OK;

@@ -24,8 +24,8 @@ namespace pxb {
 namespace {
 
 constexpr double kUpdateTol = 1e-14;  // Newton stops when |dU| <= kUpdateTol |U|
-constexpr size_t kBicgScalarBytes = 128;  // BicgScalars, then the partial sums
-static_assert(sizeof(BicgScalars) <= kBicgScalarBytes, "BiCGStab scalar block");
+constexpr size_t kBicgScalarBytes = 256;  // two BicgScalars, 128 bytes apart, then the partial sums
+static_assert(sizeof(BicgScalars) <= kBicgScalarBytes / 2, "BiCGStab scalar block");
 constexpr int kHostDots = 4;  // dot products read back with a solve's outcome
 
 struct RunCtx {
@@ -261,12 +261,15 @@ int queue_readback(pxb_ctx *c, int ndots) {
     return PXB_OK;
 }
 
+int newton_unfinished(const RunCtx &r) {
+    return fail(PXB_ERR_STATE, "CH Newton did not reach the relative residual " + std::to_string(r.p.newton_rtol));
+}
+
 int bicg_timeout() {
     return fail(PXB_ERR_CUDA, "CH linear solve: a grid barrier of the BiCGStab kernel timed out");
 }
 
-int bicg_outcome(ChState &h, int *its, double *relres) {
-    const BicgScalars *hs = host_outcome(h);
+int bicg_outcome(const BicgScalars *hs, int *its, double *relres) {
     *its = hs->its;
     *relres = hs->relres;
     if (hs->status == kBicgDone) return PXB_OK;
@@ -283,9 +286,14 @@ int dot_into(RunCtx &r, long long len, const double *a, const double *b, int k) 
     return check(c, launch_dot(len, a, b, red, dev_dots(c->ch) + k, c->stream), "dot");
 }
 
-// one Newton iteration on the slices: the system at (U, Uold), then the solve and update in one kernel.  The outcome
-// (|F|, solve, update and state norms) is in host_outcome; `stop`: |F| that ends the step, `only_norm`: |F| only.
-int newton_iteration(RunCtx &r, double *U, const double *Uold, double stop, bool only_norm) {
+BicgScalars *newton_outcome(ChState &h, int it) {
+    return reinterpret_cast<BicgScalars *>(static_cast<char *>(h.bicg_h.p) + (it & 1) * (kBicgScalarBytes / 2));
+}
+
+// Queues Newton iteration `it` of a step on the slices: the system at (U, Uold), then the solve and update in one
+// kernel, whose outcome is in newton_outcome(it) when newton_ev[it & 1] has been reached.  Queued before the outcome of
+// iteration it - 1 is known, it does nothing if that one ended the step.
+int queue_newton(RunCtx &r, double *U, const double *Uold, int it) {
     pxb_ctx *c = r.c;
     ChState &h = c->ch;
     const CsrState &k = c->csr;
@@ -310,7 +318,9 @@ int newton_iteration(RunCtx &r, double *U, const double *Uold, double stop, bool
     s.pair = k.sl_pair.as<double2>();
     s.binv = h.binv.as<double>();
     s.rhs = h.rhs.as<double>();
-    s.sc = h.bicg.as<BicgScalars>();
+    auto scalars = [&](int k) { return reinterpret_cast<BicgScalars *>(h.bicg.as<char>() + (k & 1) * (kBicgScalarBytes / 2)); };
+    s.sc = scalars(it);
+    s.prev = it > 0 ? scalars(it - 1) : nullptr;
     PXB_TRY(check(c, launch_ch_system(s, c->stream), "ch system"));
     BicgArgs a = bicg_args(r, h.rhs.as<double>(), h.dU.as<double>());
     a.r0 = h.rhs.as<double>();  // the shadow residual is the right-hand side, which no phase writes
@@ -324,32 +334,34 @@ int newton_iteration(RunCtx &r, double *U, const double *Uold, double stop, bool
     m.g0 = ghost_scale(r.p.dt);
     ChNewton nw;
     nw.u = U;
-    nw.stop = stop;
-    nw.only_norm = only_norm ? 1 : 0;
+    nw.prev = s.prev;
+    nw.host = newton_outcome(h, it);
+    nw.rtol = r.p.newton_rtol;
+    nw.update_tol = kUpdateTol;
+    nw.only_norm = it == r.p.newton_max ? 1 : 0;
     nw.tol = r.p.lin_rtol;
     nw.max_its = r.p.lin_max;
+    a.sc = s.sc;
+    *nw.host = BicgScalars{};
     PXB_TRY(check(c, launch_ch_newton(a, m, nw, c->stream), "ch newton"));
-    PXB_TRY(queue_readback(c, 0));
-    return sync(c);
+    cudaEvent_t &ev = c->newton_ev[it & 1];
+    if (!ev) PXB_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    PXB_CUDA_TRY(cudaEventRecord(ev, c->stream));
+    return PXB_OK;
 }
 
-// one backward-Euler step: U (in: initial guess, out: converged state) from Uold
-int newton_step(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) {
+// One backward-Euler step on the slices.  The next iteration is queued before the host waits for the last one's
+// outcome, so the GPU does not wait for the host between iterations (a 256x256 run of 40: 9.7 -> 8.7 ms).
+int newton_step_slices(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) {
     pxb_ctx *c = r.c;
-    ChState &h = c->ch;
     double res0 = -1.0;
+    PXB_TRY(queue_newton(r, U, Uold, 0));
     for (int it = 0; it <= r.p.newton_max; ++it) {
-        double res = 0.0;
-        if (r.slices) {
-            PXB_TRY(newton_iteration(r, U, Uold, it > 0 ? r.p.newton_rtol * res0 : 0.0, it == r.p.newton_max));
-            if (host_outcome(h)->abort) return bicg_timeout();
-            res = host_outcome(h)->bnorm;
-        } else {
-            PXB_TRY(assemble(r, U, Uold));
-            double ff = 0.0;
-            PXB_TRY(dotp(r, r.rows, h.rhs.as<double>(), h.rhs.as<double>(), &ff));
-            res = std::sqrt(ff);
-        }
+        if (it < r.p.newton_max) PXB_TRY(queue_newton(r, U, Uold, it + 1));
+        PXB_CUDA_TRY(cudaEventSynchronize(c->newton_ev[it & 1]));
+        const BicgScalars &o = *newton_outcome(c->ch, it);
+        if (o.status == kBicgRunning) return bicg_timeout();
+        const double res = o.bnorm;
         if (!std::isfinite(res)) return fail(PXB_ERR_BLOWUP, "CH Newton: non-finite residual");
         if (it == 0) res0 = res;
         st->max_residual = std::max(st->max_residual, it == 0 ? 0.0 : res / std::max(res0, 1e-300));
@@ -358,24 +370,53 @@ int newton_step(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) 
             return PXB_OK;
         }
         if (it == r.p.newton_max) break;
-        if (!r.slices) {
-            PXB_TRY(check(c, launch_block_inv(r.n, c->csr.diag.as<int>(), h.kv.as<double>(), false, h.binv.as<double>(),
-                                              c->stream),
-                          "block inverse"));
-            PXB_TRY(bicgstab_launch(r, false, h.rhs.as<double>(), h.dU.as<double>()));
-            PXB_TRY(dot_into(r, r.rows, h.dU.as<double>(), h.dU.as<double>(), 0));
-            PXB_TRY(dot_into(r, r.rows, U, U, 1));
-            PXB_TRY(check(c, launch_axpby(r.rows, 1.0, h.dU.as<double>(), 1.0, U, c->stream), "update"));
-            PXB_TRY(queue_readback(c, 2));
-            PXB_TRY(sync(c));
-        }
         int lits = 0;
         double lres = 0.0;
-        PXB_TRY(bicg_outcome(h, &lits, &lres));
+        PXB_TRY(bicg_outcome(&o, &lits, &lres));
         st->lin_iters += lits;
         st->max_lin_relres = std::max(st->max_lin_relres, lres);
-        const double dd = r.slices ? host_outcome(h)->dd : host_dots(h)[0];
-        const double uu = r.slices ? host_outcome(h)->uu : host_dots(h)[1];
+        if (!o.go) {
+            st->newton_iters += it + 1;
+            return PXB_OK;
+        }
+    }
+    return newton_unfinished(r);
+}
+
+// one backward-Euler step: U (in: initial guess, out: converged state) from Uold
+int newton_step(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) {
+    if (r.slices) return newton_step_slices(r, U, Uold, st);
+    pxb_ctx *c = r.c;
+    ChState &h = c->ch;
+    double res0 = -1.0;
+    for (int it = 0; it <= r.p.newton_max; ++it) {
+        PXB_TRY(assemble(r, U, Uold));
+        double ff = 0.0;
+        PXB_TRY(dotp(r, r.rows, h.rhs.as<double>(), h.rhs.as<double>(), &ff));
+        const double res = std::sqrt(ff);
+        if (!std::isfinite(res)) return fail(PXB_ERR_BLOWUP, "CH Newton: non-finite residual");
+        if (it == 0) res0 = res;
+        st->max_residual = std::max(st->max_residual, it == 0 ? 0.0 : res / std::max(res0, 1e-300));
+        if (res == 0.0 || (it > 0 && res <= r.p.newton_rtol * res0)) {
+            st->newton_iters += it;
+            return PXB_OK;
+        }
+        if (it == r.p.newton_max) break;
+        PXB_TRY(check(c, launch_block_inv(r.n, c->csr.diag.as<int>(), h.kv.as<double>(), false, h.binv.as<double>(),
+                                          c->stream),
+                      "block inverse"));
+        PXB_TRY(bicgstab_launch(r, false, h.rhs.as<double>(), h.dU.as<double>()));
+        PXB_TRY(dot_into(r, r.rows, h.dU.as<double>(), h.dU.as<double>(), 0));
+        PXB_TRY(dot_into(r, r.rows, U, U, 1));
+        PXB_TRY(check(c, launch_axpby(r.rows, 1.0, h.dU.as<double>(), 1.0, U, c->stream), "update"));
+        PXB_TRY(queue_readback(c, 2));
+        PXB_TRY(sync(c));
+        int lits = 0;
+        double lres = 0.0;
+        PXB_TRY(bicg_outcome(host_outcome(h), &lits, &lres));
+        st->lin_iters += lits;
+        st->max_lin_relres = std::max(st->max_lin_relres, lres);
+        const double dd = host_dots(h)[0], uu = host_dots(h)[1];
         // an update at the rounding level of the state ends the iteration (the residual of a small step can sit
         // at its evaluation floor, far above newton_rtol times its initial value)
         if (std::sqrt(dd) <= kUpdateTol * std::sqrt(uu)) {
@@ -383,7 +424,7 @@ int newton_step(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) 
             return PXB_OK;
         }
     }
-    return fail(PXB_ERR_STATE, "CH Newton did not reach the relative residual " + std::to_string(r.p.newton_rtol));
+    return newton_unfinished(r);
 }
 
 // U0 = (c0, 0) with ghost c copied from the mirror bulk node
@@ -511,7 +552,7 @@ extern "C" int pxb_ch_gradient(pxb_ctx *c, const pxb_ch_run_params *p, const dou
         PXB_TRY(sync(c));
         int lits = 0;
         double lres = 0.0;
-        PXB_TRY(bicg_outcome(h, &lits, &lres));
+        PXB_TRY(bicg_outcome(host_outcome(h), &lits, &lres));
         st.lin_iters += lits;
         st.max_lin_relres = std::max(st.max_lin_relres, lres);
         dk += host_dots(h)[0];

@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM) bicg_solve_kernel(Bicg
 // nothing) but the L1 data pipe under the gathers and the grid barriers, about 3800 cycles each.  So 148 blocks of 512
 // threads (two of 512: 10.0 ms a run, one of 1024: 10.1, one of 512: 9.2), the preconditioned direction's
 // ph - omega vh formed once a node in phase C instead of at every gather, and the Newton iteration's other sums and its
-// update in the same kernel.  256x256, 10 steps (32 solves, 298 iterations): 18.3 ms with the CSR kernels -> 9.0 ms;
+// update in the same kernel.  256x256, 10 steps (32 solves, 298 iterations): 18.4 ms with the CSR kernels -> 9.7 ms;
 // 64x64: 10.8 (one lane a node) -> 5.9 ms with eight.
 
 // K (Picard Jacobian, Neumann ghost rows) and F at (U, Uold): value pairs, block-Jacobi inverse, right-hand side.  The
@@ -326,6 +326,7 @@ __device__ __forceinline__ double mobility(double M0, double c) {
 
 __global__ void __launch_bounds__(256) ch_system_kernel(ChSystemArgs a) {
     constexpr int LPN = kSystemLanes, GPW = kWarp / LPN, U = kSystemUnroll;
+    if (a.prev && !a.prev->go) return;
     if (blockIdx.x == 0 && threadIdx.x < sizeof(BicgScalars) / 4) reinterpret_cast<int *>(a.sc)[threadIdx.x] = 0;
     const int lane = threadIdx.x & 31, gl = lane & (LPN - 1);
     const int i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * GPW + lane / LPN;
@@ -548,6 +549,7 @@ __device__ bool grid_sum(const double (&val)[NV], double *part, BicgScalars *sc,
 template <int LPN>
 __global__ void __launch_bounds__(kSliceThreads, kSliceBlocks) ch_newton_kernel(BicgArgs a, ChSlices m, ChNewton nw) {
     BicgScalars *sc = a.sc;
+    if (nw.prev && !nw.prev->go) return;
     unsigned int epoch = 0;
     const int tid = blockIdx.x * kSliceThreads + threadIdx.x, nth = gridDim.x * kSliceThreads;
     double bb = 0.0;
@@ -564,8 +566,22 @@ __global__ void __launch_bounds__(kSliceThreads, kSliceBlocks) ch_newton_kernel(
     double t1[1], t2[2], t3[3];
     if (!grid_sum<1>({bb}, a.part, sc, epoch, t1)) return;
     const double bnorm = sqrt(t1[0]);
-    if (tid == 0) sc->bnorm = bnorm;
-    if (!(bnorm > nw.stop) || !isfinite(bnorm) || nw.only_norm) return finish(sc, kBicgDone, 0, 0.0);
+    const double res0 = nw.prev ? nw.prev->res0 : bnorm;
+    auto finish = [&](int status, int its, double rel, double dd, double uu, bool go) {
+        if (tid != 0) return;
+        BicgScalars *h = nw.host;
+        h->bnorm = bnorm;
+        h->dd = dd;
+        h->uu = uu;
+        h->relres = rel;
+        h->its = its;
+        h->go = go ? 1 : 0;
+        h->status = status;
+        sc->res0 = res0;
+        sc->go = go ? 1 : 0;
+    };
+    if (!(bnorm > (nw.prev ? nw.rtol * res0 : 0.0)) || !isfinite(bnorm) || nw.only_norm)
+        return finish(kBicgDone, 0, 0.0, 0.0, 0.0, false);
     double rho = 1.0, rho1 = t1[0], relres = 0.0;
     Scal c{1.0, t1[0], 1.0};
     int k = 1;
@@ -575,7 +591,7 @@ __global__ void __launch_bounds__(kSliceThreads, kSliceBlocks) ch_newton_kernel(
         double d[3] = {0.0, 0.0, 0.0};
         slices_phase<0, LPN>(a, m, c, phn, vhn, d);
         if (!grid_sum<1>({d[0]}, a.part, sc, epoch, t1)) return;
-        if (t1[0] == 0.0 || !isfinite(t1[0])) return finish(sc, kBicgBreakdown, k - 1, 0.0);
+        if (t1[0] == 0.0 || !isfinite(t1[0])) return finish(kBicgBreakdown, k - 1, 0.0, 0.0, 0.0, false);
         c.alpha = rho1 / t1[0];
         d[0] = d[1] = d[2] = 0.0;
         slices_phase<1, LPN>(a, m, c, phn, vhn, d);
@@ -604,10 +620,10 @@ __global__ void __launch_bounds__(kSliceThreads, kSliceBlocks) ch_newton_kernel(
         if (!grid_sum<2>({rr, r0r}, a.part, sc, epoch, t2)) return;
         relres = sqrt(t2[0]) / bnorm;
         if (relres <= nw.tol) break;
-        if (k >= nw.max_its) return finish(sc, kBicgMaxIts, k, relres);
+        if (k >= nw.max_its) return finish(kBicgMaxIts, k, relres, 0.0, 0.0, false);
         rho = rho1;
         rho1 = t2[1];
-        if (rho1 == 0.0 || !isfinite(rho1) || c.omega == 0.0) return finish(sc, kBicgBreakdown, k, relres);
+        if (rho1 == 0.0 || !isfinite(rho1) || c.omega == 0.0) return finish(kBicgBreakdown, k, relres, 0.0, 0.0, false);
         c.beta = (rho1 / rho) * (c.alpha / c.omega);
     }
     double dd = 0.0, uu = 0.0;
@@ -624,11 +640,9 @@ __global__ void __launch_bounds__(kSliceThreads, kSliceBlocks) ch_newton_kernel(
         uu += u.x * u.x + u.y * u.y;
     }
     if (!grid_sum<2>({dd, uu}, a.part, sc, epoch, t2)) return;
-    if (tid == 0) {
-        sc->dd = t2[0];
-        sc->uu = t2[1];
-    }
-    finish(sc, kBicgDone, k, relres);
+    // an update at the rounding level of the state ends the step (the residual of a small step can sit at its
+    // evaluation floor, far above rtol times its initial value)
+    finish(kBicgDone, k, relres, t2[0], t2[1], !(sqrt(t2[0]) <= nw.update_tol * sqrt(t2[1])));
 }
 
 // vt[q] = v[perm[q]]: the values of the transposed matrix

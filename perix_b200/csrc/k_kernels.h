@@ -508,9 +508,11 @@ constexpr int kBicgParts = 148 * 8;  // most blocks of the solve kernel (one par
 struct BicgScalars {
     double relres;
     double bnorm, dd, uu;                // Newton solve: |F|, |x|^2 and |U|^2 before the update
+    double res0;                         // |F| of the step's first Newton iteration
     int status, its;                     // status: kBicgRunning until the solve ends (then abort tells a timeout)
     unsigned int bar_count;              // grid barrier arrivals
     int abort;                           // set by a barrier wait that gave up
+    int go;                              // Newton solve: the step goes on with another iteration
 };
 struct BicgArgs {
     int n = 0;                                  // node blocks (rows 2i, 2i+1)
@@ -542,12 +544,17 @@ struct ChSystemArgs {
     double2 *pair = nullptr;
     double *binv = nullptr, *rhs = nullptr;
     BicgScalars *sc = nullptr;  // cleared for the solve that follows
+    const BicgScalars *prev = nullptr;  // as in ChNewton
 };
+// An iteration may be queued before the outcome of the one ahead of it is known: unless that one set `go`, it does
+// nothing.
 struct ChNewton {
-    double *u = nullptr;      // U += x when the solve ends
-    double stop = 0.0;        // |F| <= stop: nothing to solve
-    int only_norm = 0;        // |F| only
-    double tol = 0.0;
+    double *u = nullptr;                  // U += x when the solve ends
+    const BicgScalars *prev = nullptr;    // the iteration ahead (NULL: the step's first)
+    BicgScalars *host = nullptr;          // pinned host memory: the outcome (status stays kBicgRunning after a timeout)
+    double rtol = 0.0, update_tol = 0.0;  // |F| <= rtol res0 or |x| <= update_tol |U| end the step
+    int only_norm = 0;                    // |F| only
+    double tol = 0.0;                     // of the solve
     int max_its = 0;
 };
 // scale of a ghost row: the magnitude of the element's own diagonal entry (1 when zero)

@@ -242,6 +242,7 @@ struct pxb_ctx {
     // last use of ops.bond: another stream's use waits for it
     cudaEvent_t bond_ev = nullptr;
     cudaStream_t bond_stream = nullptr;
+    cudaEvent_t newton_ev[2] = {nullptr, nullptr};  // ends of the implicit run's queued Newton iterations
     size_t mem_limit = 0;  // device bytes the context may hold (0: no limit beyond the GPU's)
     int gbuild_schedule = -1;  // g-build: -1 by problem, 0 lane groups, 1 one warp per node, 2 the same with
                                // its products on the FP64 tensor cores
