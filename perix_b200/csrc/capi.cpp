@@ -29,9 +29,53 @@ int cuda_fail(cudaError_t e, const char *what) {
 }
 
 void DevBuf::release() {
-    if (p) cudaFree(p);
+    if (p && pool) pool->give(p, cap);
+    else if (p) cudaFree(p);
     p = nullptr;
+    pool = nullptr;
+    bytes = cap = 0;
+}
+
+void DevPool::trim() {
+    for (const Block &b : idle) cudaFree(b.p);
+    idle.clear();
     bytes = 0;
+}
+
+void DevPool::give(void *p, size_t cap) {
+    dirty = true;
+    size_t drop = 0;
+    while (drop < idle.size() && bytes + cap > kMax) {
+        cudaFree(idle[drop].p);
+        bytes -= idle[drop++].cap;
+    }
+    idle.erase(idle.begin(), idle.begin() + (ptrdiff_t)drop);
+    if (cap > kMax) {
+        cudaFree(p);
+        return;
+    }
+    idle.push_back({p, cap});
+    bytes += cap;
+}
+
+// the tightest block that wastes at most a quarter of what is wanted (or 64 KB), NULL without one
+void *DevPool::take(size_t want, size_t *cap) {
+    size_t best = idle.size();
+    for (size_t k = 0; k < idle.size(); ++k)
+        if (idle[k].cap >= want && idle[k].cap <= want + want / 4 + 65536 &&
+            (best == idle.size() || idle[k].cap < idle[best].cap))
+            best = k;
+    if (best == idle.size()) return nullptr;
+    if (dirty && cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    dirty = false;
+    void *p = idle[best].p;
+    *cap = idle[best].cap;
+    bytes -= idle[best].cap;
+    idle.erase(idle.begin() + (ptrdiff_t)best);
+    return p;
 }
 
 PinnedBuf::~PinnedBuf() {
@@ -70,7 +114,7 @@ static int malloc_dev(void **p, size_t bytes) {
     return cuda_fail(e, "cudaMalloc");
 }
 
-// What the context can do without gives way to what has to be there: the field transpose's scratch, then the
+// What the context can do without gives way to what has to be there: idle blocks, the field transpose's scratch, the
 // implicit run's slices (both are built again by a use that finds the memory).
 static void make_room(pxb_ctx *c, const DevBuf &b, size_t bytes) {
     CsrState &k = c->csr;
@@ -79,6 +123,8 @@ static void make_room(pxb_ctx *c, const DevBuf &b, size_t bytes) {
         size_t free_b = 0, total_b = 0;
         return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > free_b;
     };
+    const bool limited = c->mem_limit && ctx_bytes(c) - b.bytes + bytes + c->pool.bytes > c->mem_limit;
+    if (c->pool.bytes && (limited || short_of())) c->pool.trim();
     if (c->ops.bond.p && &b != &c->ops.bond && short_of()) c->ops.bond.release();
     if (k.sl_pair.p && &b != &k.sl_pair && &b != &k.sl_col && &b != &k.sl_row0 && short_of()) {
         k.sl_pair.release();
@@ -86,16 +132,44 @@ static void make_room(pxb_ctx *c, const DevBuf &b, size_t bytes) {
     }
 }
 
-int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
-    if (b.p && b.bytes == bytes) return PXB_OK;
-    if (c && bytes > b.bytes) make_room(c, b, bytes);
+static int over_limit(const pxb_ctx *c, const DevBuf &b, size_t bytes) {
     if (c && c->mem_limit && bytes > b.bytes && ctx_bytes(c) - b.bytes + bytes > c->mem_limit)
         return fail(PXB_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes would exceed the context's " +
                                      std::to_string(c->mem_limit) + "-byte limit (pxb_ctx_set_memory_limit)");
+    return PXB_OK;
+}
+
+int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
+    if (b.p && b.bytes == bytes) return PXB_OK;
+    if (c && bytes > b.bytes) make_room(c, b, bytes);
+    PXB_TRY(over_limit(c, b, bytes));
     b.release();
     if (bytes == 0) return PXB_OK;
-    PXB_TRY(malloc_dev(&b.p, bytes));
-    b.bytes = bytes;
+    int st = malloc_dev(&b.p, bytes);
+    if (st == PXB_ERR_OOM && c && c->pool.bytes) {
+        c->pool.trim();
+        st = malloc_dev(&b.p, bytes);
+    }
+    PXB_TRY(st);
+    b.bytes = b.cap = bytes;
+    return PXB_OK;
+}
+
+int pool_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
+    if (b.p && b.bytes == bytes) return PXB_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (bytes > 0 && cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+        !(c->mem_limit && ctx_bytes(c) - b.bytes + bytes + c->pool.bytes > c->mem_limit)) {
+        b.release();
+        if (void *p = c->pool.take(bytes, &b.cap)) {
+            b.p = p;
+            b.bytes = bytes;
+            b.pool = &c->pool;
+            return PXB_OK;
+        }
+    }
+    PXB_TRY(dev_alloc(c, b, bytes));
+    b.pool = &c->pool;
     return PXB_OK;
 }
 
@@ -113,6 +187,11 @@ int d2h(pxb_ctx *c, void *dst, const void *src, size_t bytes) {
 
 int dev_upload(pxb_ctx *c, DevBuf &b, const void *host, size_t bytes) {
     PXB_TRY(dev_alloc(c, b, bytes));
+    return h2d(c, b.p, host, bytes);
+}
+
+int pool_upload(pxb_ctx *c, DevBuf &b, const void *host, size_t bytes) {
+    PXB_TRY(pool_alloc(c, b, bytes));
     return h2d(c, b.p, host, bytes);
 }
 
@@ -310,10 +389,10 @@ static int geometry_reset(pxb_ctx *c, int n, int dim, const int *neigh_off, int 
     g.h_off.assign(neigh_off, neigh_off + n + 1);
     if (mirror) g.h_mirror.assign(mirror, mirror + n);
     g.ldb = ((nb + 16 + 15) / 16) * 16;
-    PXB_TRY(dev_alloc(c, g.off, sizeof(int) * (size_t)(n + 1 + 16)));
+    PXB_TRY(pool_alloc(c, g.off, sizeof(int) * (size_t)(n + 1 + 16)));
     PXB_CUDA_TRY(cudaMemsetAsync(g.off.p, 0, g.off.bytes, c->stream));
     PXB_TRY(h2d(c, g.off.p, neigh_off, sizeof(int) * (size_t)(n + 1)));
-    PXB_TRY(dev_alloc(c, g.nbr, sizeof(int) * (size_t)g.ldb));
+    PXB_TRY(pool_alloc(c, g.nbr, sizeof(int) * (size_t)g.ldb));
     PXB_CUDA_TRY(cudaMemsetAsync(g.nbr.p, 0, g.nbr.bytes, c->stream));
     return PXB_OK;
 }
@@ -322,12 +401,12 @@ static int geometry_reset(pxb_ctx *c, int n, int dim, const int *neigh_off, int 
 static int geometry_finish(pxb_ctx *c, const double *coords3_d, const double *vols, const int *mirror,
                            const int *layer_index) {
     Geometry &g = c->g;
-    PXB_TRY(dev_alloc(c, g.pos, (g.dim == 2 ? 16 : 32) * (size_t)g.n));
+    PXB_TRY(pool_alloc(c, g.pos, (g.dim == 2 ? 16 : 32) * (size_t)g.n));
     launch_pos_pack(g.n, g.dim, coords3_d, g.pos.p, c->stream);
     PXB_TRY(check_launch(c, "pos_pack"));
-    PXB_TRY(dev_upload(c, g.vol, vols, sizeof(double) * (size_t)g.n));
-    if (mirror) PXB_TRY(dev_upload(c, g.mirror, mirror, sizeof(int) * (size_t)g.n));
-    if (layer_index) PXB_TRY(dev_upload(c, g.layer, layer_index, sizeof(int) * (size_t)g.n));
+    PXB_TRY(pool_upload(c, g.vol, vols, sizeof(double) * (size_t)g.n));
+    if (mirror) PXB_TRY(pool_upload(c, g.mirror, mirror, sizeof(int) * (size_t)g.n));
+    if (layer_index) PXB_TRY(pool_upload(c, g.layer, layer_index, sizeof(int) * (size_t)g.n));
     PXB_TRY(sync(c));
     g.ready = true;
     return PXB_OK;
@@ -493,19 +572,17 @@ static int run_gbuild(pxb_ctx *c, int order, bool mixed, void *ops_out, void *G_
     PXB_TRY(scratch(c, 16, &tmp));
     unsigned int *nd = static_cast<unsigned int *>(tmp);
     int *first = reinterpret_cast<int *>(static_cast<char *>(tmp) + 8);
-    PXB_CUDA_TRY(cudaMemsetAsync(nd, 0, 4, c->stream));
-    const int big = std::numeric_limits<int>::max();
-    PXB_TRY(h2d(c, first, &big, sizeof(int)));
+    PXB_CUDA_TRY(cudaMemsetAsync(nd, 0, 8, c->stream));
+    PXB_CUDA_TRY(cudaMemsetAsync(first, 0x7f, 8, c->stream));  // above every node id
     const GBuildArgs a = gbuild_args(c, ops_out, G_out, deg_out, nd, first, defect);
     cudaError_t e = gbuild_launch(c, a, order, mixed);
     c->launches++;
     if (e != cudaSuccess) return cuda_fail(e, "gbuild launch");
-    unsigned int hnd = 0;
-    int hfirst = big;
-    PXB_TRY(d2h(c, &hnd, nd, 4));
-    PXB_TRY(d2h(c, &hfirst, first, 4));
+    int got[4] = {0, 0, 0, 0};
+    PXB_TRY(d2h(c, got, nd, sizeof(got)));
     PXB_TRY(sync(c));
-    if (n_degenerate) *n_degenerate = (int)hnd;
+    const int hnd = got[0], hfirst = got[2];
+    if (n_degenerate) *n_degenerate = hnd;
     if (first_degenerate) *first_degenerate = hnd ? hfirst + 1 : 0;
     if (hnd)
         return fail(PXB_ERR_DEGENERATE, "degenerate moment matrix at node " + std::to_string(hfirst + 1) + " (" +
@@ -522,8 +599,8 @@ extern "C" int pxb_gbuild(pxb_ctx *c, int order, int precision, int *n_degenerat
     int nop = 0;
     for (int k = 1; k <= order; ++k) nop += (c->g.dim == 3) ? (k + 1) * (k + 2) / 2 : (k + 1);
     const size_t es = precision == PXB_MIXED ? 4 : 8;
-    PXB_TRY(dev_alloc(c, o.ops, es * (size_t)nop * (size_t)std::max(1LL, c->g.nb)));
-    PXB_TRY(dev_alloc(c, o.degenerate, (size_t)c->g.n));
+    PXB_TRY(pool_alloc(c, o.ops, es * (size_t)nop * (size_t)std::max(1LL, c->g.nb)));
+    PXB_TRY(pool_alloc(c, o.degenerate, (size_t)c->g.n));
     o.order = order;
     o.nop = nop;
     o.precision = precision;
@@ -1617,6 +1694,7 @@ extern "C" int pxb_epf_advance_to(pxb_ctx *c, double t_end, int chunk, int *bad_
 extern "C" int pxb_ctx_set_memory_limit(pxb_ctx *c, size_t bytes) {
     if (!c) return fail(PXB_ERR_INVALID, "pxb_ctx_set_memory_limit: NULL context");
     c->mem_limit = bytes;
+    if (bytes && ctx_bytes(c) + c->pool.bytes > bytes) c->pool.trim();
     return PXB_OK;
 }
 
@@ -2111,7 +2189,7 @@ int csr_finish(pxb_ctx *c, const char *who, bool verify) {
     CsrState &k = c->csr;
     const int ndof = k.ndof, n = c->g.n;
     const size_t rows = (size_t)n * ndof, nb = (size_t)std::max(1LL, c->g.nb);
-    PXB_TRY(dev_alloc(c, k.diag, sizeof(int) * (size_t)n * ndof * ndof));
+    PXB_TRY(pool_alloc(c, k.diag, sizeof(int) * (size_t)n * ndof * ndof));
     void *tmp = nullptr;
     PXB_TRY(scratch(c, 8, &tmp));
     PXB_CUDA_TRY(cudaMemsetAsync(tmp, 0, 8, c->stream));
@@ -2119,9 +2197,9 @@ int csr_finish(pxb_ctx *c, const char *who, bool verify) {
     k.exact = false;
     int flags[2] = {0, 0};
     if (k.mmax <= kBlockMax) {
-        PXB_TRY(dev_alloc(c, k.bpos, nb));
-        PXB_TRY(dev_alloc(c, k.spos, (size_t)n));
-        PXB_TRY(dev_alloc(c, k.xpos, sizeof(int16_t) * (size_t)n));
+        PXB_TRY(pool_alloc(c, k.bpos, nb));
+        PXB_TRY(pool_alloc(c, k.spos, (size_t)n));
+        PXB_TRY(pool_alloc(c, k.xpos, sizeof(int16_t) * (size_t)n));
         BlockMapArgs m;
         m.n = n;
         m.ndof = ndof;
@@ -2165,10 +2243,10 @@ int csr_finish(pxb_ctx *c, const char *who, bool verify) {
         if (flags[1]) return fail(PXB_ERR_INVALID, std::string(who) + ": pattern lacks " + std::to_string(flags[1]) +
                                                        " entries required by the families");
     }
-    PXB_TRY(dev_alloc(c, k.kvals, sizeof(double) * (size_t)k.nnz));
-    PXB_TRY(dev_alloc(c, k.rhs, sizeof(double) * rows));
-    PXB_TRY(dev_alloc(c, k.u, sizeof(double) * rows));
-    PXB_TRY(dev_alloc(c, k.uold, sizeof(double) * rows));
+    PXB_TRY(pool_alloc(c, k.kvals, sizeof(double) * (size_t)k.nnz));
+    PXB_TRY(pool_alloc(c, k.rhs, sizeof(double) * rows));
+    PXB_TRY(pool_alloc(c, k.u, sizeof(double) * rows));
+    PXB_TRY(pool_alloc(c, k.uold, sizeof(double) * rows));
     k.ready = true;
     return PXB_OK;
 }
@@ -2205,11 +2283,12 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     CsrState &k = c->csr;
     k = CsrState{};
     k.ndof = ndof;
-    DevBuf count, first, bsum, small;
-    PXB_TRY(dev_alloc(c, count, sizeof(int) * (size_t)n));
-    PXB_TRY(dev_alloc(c, first, sizeof(long long) * ((size_t)n + 1)));
-    PXB_TRY(dev_alloc(c, bsum, sizeof(long long) * (size_t)pattern_scan_blocks(n)));
-    PXB_TRY(dev_alloc(c, small, 16));
+    DevBuf count, first, bsum, small, list;
+    PXB_TRY(pool_alloc(c, list, sizeof(int) * ((size_t)c->g.nb + 2 * (size_t)n)));
+    PXB_TRY(pool_alloc(c, count, sizeof(int) * (size_t)n));
+    PXB_TRY(pool_alloc(c, first, sizeof(long long) * ((size_t)n + 1)));
+    PXB_TRY(pool_alloc(c, bsum, sizeof(long long) * (size_t)scan_blocks(n)));
+    PXB_TRY(pool_alloc(c, small, 16));
     PXB_CUDA_TRY(cudaMemsetAsync(small.p, 0, 16, c->stream));
     PatternArgs a;
     a.n = n;
@@ -2220,7 +2299,9 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     a.count = count.as<int>();
     a.first = first.as<long long>();
     a.overflow = reinterpret_cast<int *>(small.as<char>() + 8);
-    PXB_CUDA_TRY(launch_pattern_count(a, bsum.as<long long>(), small.as<long long>(), c->stream));
+    a.list = list.as<int>();
+    PXB_CUDA_TRY(launch_pattern_count(a, c->stream));
+    PXB_CUDA_TRY(launch_scan(n, a.count, bsum.as<long long>(), small.as<long long>(), a.first, nullptr, c->stream));
     c->launches += 4;
     long long h[2] = {0, 0};
     PXB_TRY(d2h(c, h, small.p, 16));
@@ -2234,11 +2315,11 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     if (total > std::numeric_limits<int>::max())
         return fail(PXB_ERR_INVALID, "pxb_csr_build_pattern: nnz exceeds 2^31-1");
     k.nnz = total;
-    PXB_TRY(dev_alloc(c, k.rowptr, sizeof(int) * ((size_t)n * ndof + 1)));
-    PXB_TRY(dev_alloc(c, k.cols, sizeof(int) * (size_t)std::max(1LL, total)));
+    PXB_TRY(pool_alloc(c, k.rowptr, sizeof(int) * ((size_t)n * ndof + 1)));
+    PXB_TRY(pool_alloc(c, k.cols, sizeof(int) * (size_t)std::max(1LL, total)));
     if (ndof == 2) {
-        PXB_TRY(dev_alloc(c, k.bptr, sizeof(int) * ((size_t)n + 1)));
-        PXB_TRY(dev_alloc(c, k.bcol, sizeof(int) * (size_t)std::max(1LL, blocks)));
+        PXB_TRY(pool_alloc(c, k.bptr, sizeof(int) * ((size_t)n + 1)));
+        PXB_TRY(pool_alloc(c, k.bcol, sizeof(int) * (size_t)std::max(1LL, blocks)));
         a.bptr = k.bptr.as<int>();
         a.bcol = k.bcol.as<int>();
         k.blocked2 = true;

@@ -9,7 +9,7 @@
 namespace pxb {
 
 // count(): cells, members, candidate counts -> host offsets hoff[n+1], largest family, bond total.
-// fill(): keyed candidates and the per-family sort, written 0-based (+ id_base) at nbr_d[off_d[x] + k].
+// fill(): the families in the reference's order, written 0-based (+ id_base) at nbr_d[off_d[x] + k].
 // The device temporaries live until the builder is destroyed; fill() needs the count() of the same builder.
 class FamBuilder {
 public:
@@ -20,7 +20,7 @@ public:
 
 private:
     FamArgs a_;
-    DevBuf coords_, keys_, ccount_, cminid_, cstart_, cfill_, members_, cell_of_, cxyz_, pos_, fcount_, fkey_, fval_, err_;
+    DevBuf coords_, keys_, cminid_, cstart_, cfill_, members_, cell_of_, cxyz_, fcount_, votes_, off_, bsum_;
 };
 
 }  // namespace pxb

@@ -63,6 +63,7 @@ __host__ __device__ constexpr int unit_doubles(int mmax) {
 // are anything else (then the slot map of k_csr.cu serves the pattern).
 __global__ void __launch_bounds__(128) block_map_kernel(BlockMapArgs a) {
     __shared__ unsigned taken[4][kBlockMax / 32];
+    __shared__ int nodes[4][kBlockMax];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nd = a.ndof;
     for (int i = blockIdx.x * 4 + w; i < a.n; i += gridDim.x * 4) {
         const int lo = a.rowptr[i * nd], width = a.rowptr[i * nd + 1] - lo, m = width / nd;
@@ -86,8 +87,9 @@ __global__ void __launch_bounds__(128) block_map_kernel(BlockMapArgs a) {
         }
         if (ok) {
             if (lane < kBlockMax / 32) taken[w][lane] = 0;
+            for (int p = lane; p < m; p += kWarp) nodes[w][p] = a.cols[lo + p * nd] / nd;
             __syncwarp();
-            auto list = [&](int p) { return a.cols[lo + p * nd] / nd; };
+            auto list = [&](int p) { return nodes[w][p]; };
             const int mir = a.mirror ? a.mirror[i] - 1 : -1;
             bool has_mirror = mir == i, found = true;
             for (int k = lane; k < len; k += kWarp) {

@@ -8,10 +8,16 @@
 // and fam(x) lists the partners of x in increasing key.  A cell's rank is the order in which it was opened, i.e.
 // the order of its smallest node id, so that id stands in for the rank.
 //
-// Steps: cell coordinates and a hash table of cells (min node id, member count); members per cell, sorted by node
-// id (position = insertion order); per node, the candidates of the 3^dim surrounding cells with the reference's
-// distance test, counted, then written with their keys; finally each family is sorted by key (one warp per node,
-// bitonic in shared memory).
+// The partners that x finds in one cell are in key order when the cell's members are taken by node id, and no two
+// of the surrounding cells share (rank, phase).  So a family needs no sort of its own: the 3^dim cells are put in the
+// order of (rank, phase), and the members that pass the test are written as they come.
+//
+// Steps: cell coordinates and a hash table of cells (min node id, member count); members per cell, by node id; per
+// node: the surrounding cells in order, the reference's distance test on their members, counted, and in a second pass
+// written.
+// B200, 73,600 nodes in 3D (families of 113 from some 700 candidates): count 205 + write 150 + cells and scans 45 us; a
+// thread a node with keyed candidates and a bitonic sort of every family by key: 206 + 383 + 337 + 75 us, and 12 bytes
+// a bond of temporaries where the votes take 128 a node.
 #include <cstdint>
 
 #include "k_kernels.h"
@@ -22,6 +28,7 @@ namespace pxb {
 namespace {
 
 constexpr unsigned long long kEmpty = ~0ULL;
+constexpr int kFamRun = 4;  // nodes a warp looks after at a time
 
 __device__ __forceinline__ unsigned long long cell_key(long ix, long iy, long iz) {
     const long b = 1L << 20;
@@ -48,10 +55,24 @@ __device__ __forceinline__ int find_slot(const unsigned long long *keys, unsigne
     return -1;
 }
 
-// forward stencils of the reference (CreatePDMesh.cpp:1001-1010)
-__constant__ int c_st2[4][3] = {{1, -1, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}};
-__constant__ int c_st3[13][3] = {{1, -1, -1}, {1, -1, 0}, {1, -1, 1}, {1, 0, -1}, {1, 0, 0}, {1, 0, 1}, {1, 1, -1},
-                                 {1, 1, 0},   {1, 1, 1},  {0, 1, -1}, {0, 1, 0},  {0, 1, 1}, {0, 0, 1}};
+// Forward stencils of the reference (CreatePDMesh.cpp:1001-1010): offset (dx, dy, dz) has phase 1 + its index, the
+// opposite offset the same phase with the roles exchanged.
+constexpr int kSt2[4][3] = {{1, -1, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}};
+constexpr int kSt3[13][3] = {{1, -1, -1}, {1, -1, 0}, {1, -1, 1}, {1, 0, -1}, {1, 0, 0}, {1, 0, 1}, {1, 1, -1},
+                             {1, 1, 0},   {1, 1, 1},  {0, 1, -1}, {0, 1, 0},  {0, 1, 1}, {0, 0, 1}};
+struct Phases {
+    signed char v[27];  // cell (dx + 1) + 3 (dy + 1) + 9 (dz + 1): phase, negative where the other cell processes
+};
+constexpr Phases make_phases(bool is3d) {
+    Phases p{};
+    for (int o = 0; o < (is3d ? 13 : 4); ++o) {
+        const int x = is3d ? kSt3[o][0] : kSt2[o][0], y = is3d ? kSt3[o][1] : kSt2[o][1], z = is3d ? kSt3[o][2] : 0;
+        p.v[(x + 1) + 3 * (y + 1) + 9 * (z + 1)] = (signed char)(1 + o);
+        p.v[(1 - x) + 3 * (1 - y) + 9 * (1 - z)] = (signed char)(-1 - o);
+    }
+    return p;
+}
+__constant__ Phases c_phases[2] = {make_phases(false), make_phases(true)};
 
 }  // namespace
 
@@ -64,7 +85,7 @@ __global__ void fam_cells_kernel(FamArgs a) {
         const long iz = a.is3d ? (int)floor((p[2] - a.lo[2]) / a.radius) : 0;
         if (ix < -(1L << 20) || ix >= (1L << 20) || iy < -(1L << 20) || iy >= (1L << 20) || iz < -(1L << 20) ||
             iz >= (1L << 20)) {
-            atomicExch(a.err, 1);
+            atomicExch(&a.tot->err, 1);
             a.cell_of[i] = -1;
             continue;
         }
@@ -83,7 +104,7 @@ __global__ void fam_cells_kernel(FamArgs a) {
             s = (s + 1) & a.mask;
         }
         if (slot < 0) {
-            atomicExch(a.err, 2);
+            atomicExch(&a.tot->err, 2);
             a.cell_of[i] = -1;
             continue;
         }
@@ -93,136 +114,152 @@ __global__ void fam_cells_kernel(FamArgs a) {
     }
 }
 
-// members of every cell (unordered), then each cell's list sorted by node id and the positions written back
+// members of every cell as they come, then each to its place by node id (its rank among the cell's members)
 __global__ void fam_members_kernel(FamArgs a) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         const int s = a.cell_of[i];
         if (s < 0) continue;
         const int k = atomicAdd(a.cfill + s, 1);
-        a.members[a.cstart[s] + k] = i;
+        a.unsorted[a.cstart[s] + k] = i;
     }
 }
 
-__global__ void fam_sort_cells_kernel(FamArgs a) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s <= (int)a.mask; s += gridDim.x * blockDim.x) {
-        const int c = a.ccount[s];
-        if (c == 0) continue;
-        int *m = a.members + a.cstart[s];
-        for (int x = 1; x < c; ++x) {  // insertion sort: cells hold a few tens of nodes
-            const int v = m[x];
-            int y = x - 1;
-            while (y >= 0 && m[y] > v) {
-                m[y + 1] = m[y];
-                --y;
-            }
-            m[y + 1] = v;
-        }
-        for (int x = 0; x < c; ++x) a.pos[m[x]] = x;
+__global__ void fam_order_members_kernel(FamArgs a) {
+    if (a.tot->maxcell >= kFamCell) return;  // refused
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+        const int s = a.cell_of[i];
+        if (s < 0) continue;
+        const int b = a.cstart[s], c = a.ccount[s];
+        int rank = 0;
+        for (int k = 0; k < c; ++k) rank += a.unsorted[b + k] < i;
+        a.members[b + rank] = i;
     }
 }
 
-// per node x: visit the 3^dim cells around its own, test every member, count (pass 0) or write key + partner (1)
+// Warp per kFamRun nodes that follow each other in the cells' member lists, nearly always of one cell: the cell's
+// surroundings are looked up and put in order once, and every candidate that a lane loads is tested against all of
+// them.  The first pass counts, and keeps each pass of 32 candidates' votes (a word a pass and node, 32 words a node
+// at most); the second writes the partners from the votes, or, for a node with more passes, from the tests again.
+// What bounds it is instruction issue.  Cells with 16 members or more on average are taken one by one, a lane a
+// member; smaller ones (2D: 9) are laid end to end, a lane a candidate, its cell found by bisection.
 template <bool WRITE>
-__global__ void fam_candidates_kernel(FamArgs a) {
-    const int ns = a.is3d ? 13 : 4;
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < a.n; x += gridDim.x * blockDim.x) {
-        if (a.cell_of[x] < 0) continue;
-        const int cx = a.cxyz[3 * (size_t)x], cy = a.cxyz[3 * (size_t)x + 1], cz = a.cxyz[3 * (size_t)x + 2];
-        const double *px = a.coords + 3 * (size_t)x;
-        const int mycell = a.cell_of[x];
-        const int posx = a.pos[x];
-        int cnt = 0;
-        long long w = WRITE ? (long long)a.off[x] - a.off_base : 0;
-        for (int dz = (a.is3d ? -1 : 0); dz <= (a.is3d ? 1 : 0); ++dz)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int s = find_slot(a.keys, a.mask, cell_key(cx + dx, cy + dy, cz + dz));
-                    if (s < 0) continue;
-                    // which cell processes the pair, and in which phase
-                    int phase = -1;
-                    bool x_outer = true;
-                    if (dx == 0 && dy == 0 && dz == 0) {
-                        phase = 0;
-                    } else {
-                        for (int o = 0; o < ns; ++o) {
-                            const int *st = a.is3d ? c_st3[o] : c_st2[o];
-                            if (st[0] == dx && st[1] == dy && st[2] == dz) { phase = 1 + o; x_outer = true; }
-                            if (st[0] == -dx && st[1] == -dy && st[2] == -dz) { phase = 1 + o; x_outer = false; }
-                        }
-                    }
-                    const int *m = a.members + a.cstart[s];
-                    const int c = a.ccount[s];
-                    for (int q = 0; q < c; ++q) {
-                        const int j = m[q];
-                        if (j == x) continue;
-                        // the reference's test on (outer - inner); the squared differences do not depend on the order
-                        const double *pj = a.coords + 3 * (size_t)j;
-                        const double ddx = px[0] - pj[0], ddy = px[1] - pj[1], ddz = a.is3d ? (px[2] - pj[2]) : 0.0;
-                        // (dx^2 + dy^2) + dz^2 with separate roundings, as the host computes it (no contraction)
-                        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
-                        if (!(d2 <= a.r2 + a.r2tol)) continue;
-                        if (WRITE) {
-                            unsigned long long rank, outer, inner;
-                            if (phase == 0) {
-                                rank = (unsigned long long)a.cminid[mycell];
-                                outer = (unsigned long long)min(posx, q);
-                                inner = (unsigned long long)max(posx, q);
-                            } else if (x_outer) {
-                                rank = (unsigned long long)a.cminid[mycell];
-                                outer = (unsigned long long)posx;
-                                inner = (unsigned long long)q;
-                            } else {
-                                rank = (unsigned long long)a.cminid[s];
-                                outer = (unsigned long long)q;
-                                inner = (unsigned long long)posx;
-                            }
-                            a.fkey[w] = (rank << 32) | ((unsigned long long)phase << 24) | (outer << 12) | inner;
-                            a.fval[w] = j;
-                            ++w;
-                        }
-                        ++cnt;
-                    }
-                }
-        if (!WRITE) a.fcount[x] = cnt;
-    }
-}
-
-// one warp per node: bitonic sort of the family's (key, partner) pairs in shared memory, partners written 0-based
-__global__ void __launch_bounds__(128) fam_sort_kernel(FamArgs a) {
-    constexpr int WPB = 4, CAP = kFamMax;
-    __shared__ unsigned long long sk[WPB][CAP];
-    __shared__ int sv[WPB][CAP];
+__global__ void __launch_bounds__(128) fam_partners_kernel(FamArgs a) {
+    constexpr int WPB = 4, R = kFamRun;
+    __shared__ int s_start[WPB][kWarp], s_first[WPB][kWarp];
+    if (a.tot->err || a.tot->maxcell >= kFamCell) return;  // refused
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int x = blockIdx.x * WPB + w; x < a.n; x += gridDim.x * WPB) {
-        const long long b0 = a.off[x];
-        const int len = a.off[x + 1] - a.off[x];
-        for (int k = lane; k < CAP; k += 32) {
-            sk[w][k] = k < len ? a.fkey[b0 - a.off_base + k] : kEmpty;
-            sv[w][k] = k < len ? a.fval[b0 - a.off_base + k] : 0;
-        }
-        __syncwarp();
-        int size = 2;
-        while (size < len) size <<= 1;
-        for (int k = 2; k <= size; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = lane; i < size; i += 32) {
-                    const int l = i ^ j;
-                    if (l > i) {
-                        const bool up = (i & k) == 0;
-                        const unsigned long long ki = sk[w][i], kl = sk[w][l];
-                        if ((ki > kl) == up) {
-                            sk[w][i] = kl;
-                            sk[w][l] = ki;
-                            const int t = sv[w][i];
-                            sv[w][i] = sv[w][l];
-                            sv[w][l] = t;
-                        }
+    const int ncell = a.is3d ? 27 : 9, cell = a.is3d ? lane : 9 + lane;
+    const unsigned before = (1u << lane) - 1u;
+    for (int p0 = (blockIdx.x * WPB + w) * R; p0 < a.n; p0 += gridDim.x * WPB * R) {
+        const int xl = lane < R && p0 + lane < a.n ? a.members[p0 + lane] : -1;
+        const int sl = xl >= 0 ? a.cell_of[xl] : -1;
+        for (int r = 0, r1; r < R && p0 + r < a.n; r = r1) {
+            const int own = __shfl_sync(kFull, sl, r), x0 = __shfl_sync(kFull, xl, r);
+            r1 = r + __popc(__ballot_sync(kFull, lane >= r && xl >= 0 && sl == own));
+            // the cells around x0's, a lane a cell, in the order in which the reference processes them
+            unsigned long long order = kEmpty;
+            int start = 0, count = 0;
+            if (lane < ncell) {
+                const int dx = cell % 3 - 1, dy = cell / 3 % 3 - 1, dz = cell / 9 - 1, phase = c_phases[a.is3d].v[cell];
+                const int *c = a.cxyz + 3 * (size_t)x0;
+                const int s = find_slot(a.keys, a.mask, cell_key(c[0] + dx, c[1] + dy, c[2] + dz));
+                if (s >= 0) {
+                    start = a.cstart[s];
+                    count = a.ccount[s];
+                    const unsigned rank = (unsigned)a.cminid[phase < 0 ? s : own];
+                    order = (unsigned long long)rank << 8 | (unsigned)abs(phase);
+                }
+            }
+            int place = 0;  // the cells that are not there come last, empty
+            for (int k = 0; k < ncell; ++k) {
+                const unsigned long long o = __shfl_sync(kFull, order, k);
+                place += o < order || (o == order && k < lane);
+            }
+            if (lane >= ncell) place = lane;
+            __syncwarp();
+            s_start[w][place] = start;
+            s_first[w][place] = count;
+            __syncwarp();
+            start = s_start[w][lane];
+            count = s_first[w][lane];
+            int upto = count;
+#pragma unroll
+            for (int o = 1; o < kWarp; o <<= 1) {
+                const int v = __shfl_up_sync(kFull, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const int total = __shfl_sync(kFull, upto, kWarp - 1);
+            __syncwarp();
+            s_first[w][lane] = upto - count;
+            __syncwarp();
+            const bool by_cell = total >= 16 * ncell;
+            const int passes = by_cell ? __reduce_add_sync(kFull, (count + kWarp - 1) / kWarp) : (total + kWarp - 1) / kWarp;
+            const bool votes = passes <= kWarp;
+            double px[R], py[R], pz[R];
+            int x[R], found[R], *out[R];
+            unsigned vote[R];
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                x[q] = __shfl_sync(kFull, xl, q);
+                const bool in = q >= r && q < r1;
+                const double *c = a.coords + 3 * (size_t)(in ? x[q] : 0);
+                px[q] = in ? c[0] : __longlong_as_double(0x7ff8000000000000LL);  // no candidate passes
+                py[q] = c[1];
+                pz[q] = a.is3d ? c[2] : 0.0;
+                found[q] = 0;
+                vote[q] = WRITE && in && votes ? a.votes[(size_t)x[q] * kWarp + lane] : 0u;
+                out[q] = WRITE && in ? a.nbr + a.off[x[q]] : nullptr;
+            }
+            auto pass = [&](int it, bool in, int at) {
+                const int j = in ? __ldg(a.members + at) : -1;
+                unsigned got[R];
+                if (WRITE && votes) {
+#pragma unroll
+                    for (int q = 0; q < R; ++q) got[q] = __shfl_sync(kFull, vote[q], it);
+                } else {
+                    // the reference's test on (outer - inner); the squared differences do not depend on the order;
+                    // (dx^2 + dy^2) + dz^2 with separate roundings, as the host computes it (no contraction)
+                    const double *pj = a.coords + 3 * (size_t)(in ? j : 0);
+                    const double jx = __ldg(pj), jy = __ldg(pj + 1), jz = a.is3d ? __ldg(pj + 2) : 0.0;
+#pragma unroll
+                    for (int q = 0; q < R; ++q) {
+                        const double dx = px[q] - jx, dy = py[q] - jy, dz = pz[q] - jz;
+                        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+                        got[q] = __ballot_sync(kFull, in && j != x[q] && d2 <= a.r2 + a.r2tol);
+                        if (!WRITE && lane == it) vote[q] = got[q];
                     }
                 }
-                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    if (WRITE && (got[q] >> lane & 1u)) out[q][found[q] + __popc(got[q] & before)] = j + a.id_base;
+                    found[q] += __popc(got[q]);
+                }
+            };
+            int it = 0;
+            if (by_cell) {
+                for (int k = 0; k < ncell; ++k) {
+                    const int b = __shfl_sync(kFull, start, k), c = __shfl_sync(kFull, count, k);
+                    for (int m = lane; m - lane < c; m += kWarp) pass(it++, m < c, b + m);
+                }
+            } else {
+                for (int m = lane; m - lane < total; m += kWarp) {
+                    int k = 0;  // the last cell that starts at or before m
+#pragma unroll
+                    for (int h = kWarp / 2; h > 0; h >>= 1)
+                        if (s_first[w][k + h] <= m) k += h;
+                    pass(it++, m < total, s_start[w][k] + m - s_first[w][k]);
+                }
             }
-        for (int k = lane; k < len; k += 32) a.nbr[b0 + k] = sv[w][k] + a.id_base;
-        __syncwarp();
+            if (!WRITE) {
+#pragma unroll
+                for (int q = 0; q < R; ++q)
+                    if (q >= r && q < r1) {
+                        if (votes) a.votes[(size_t)x[q] * kWarp + lane] = vote[q];
+                        if (lane == 0) a.fcount[x[q]] = found[q];
+                    }
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -234,23 +271,13 @@ cudaError_t launch_fam_cells(const FamArgs &a, cudaStream_t s) {
 cudaError_t launch_fam_members(const FamArgs &a, cudaStream_t s) {
     const int g = (int)((a.n + 255) / 256 < 148 * 16 ? (a.n + 255) / 256 : 148 * 16);
     fam_members_kernel<<<g > 0 ? g : 1, 256, 0, s>>>(a);
+    fam_order_members_kernel<<<g > 0 ? g : 1, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
-cudaError_t launch_fam_sort_cells(const FamArgs &a, cudaStream_t s) {
-    const long long slots = (long long)a.mask + 1;
-    const int g = (int)((slots + 255) / 256 < 148 * 16 ? (slots + 255) / 256 : 148 * 16);
-    fam_sort_cells_kernel<<<g > 0 ? g : 1, 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-cudaError_t launch_fam_candidates(const FamArgs &a, bool write, cudaStream_t s) {
-    const int g = (int)((a.n + 127) / 128 < 148 * 32 ? (a.n + 127) / 128 : 148 * 32);
-    if (write) fam_candidates_kernel<true><<<g > 0 ? g : 1, 128, 0, s>>>(a);
-    else fam_candidates_kernel<false><<<g > 0 ? g : 1, 128, 0, s>>>(a);
-    return cudaGetLastError();
-}
-cudaError_t launch_fam_sort(const FamArgs &a, cudaStream_t s) {
-    const int g = (int)((a.n + 3) / 4 < 148 * 16 ? (a.n + 3) / 4 : 148 * 16);
-    fam_sort_kernel<<<g > 0 ? g : 1, 128, 0, s>>>(a);
+cudaError_t launch_fam_partners(const FamArgs &a, bool write, cudaStream_t s) {
+    const int per = 4 * kFamRun, g = (int)((a.n + per - 1) / per < 148 * 64 ? (a.n + per - 1) / per : 148 * 64);
+    if (write) fam_partners_kernel<true><<<g > 0 ? g : 1, 128, 0, s>>>(a);
+    else fam_partners_kernel<false><<<g > 0 ? g : 1, 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 

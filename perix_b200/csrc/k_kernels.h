@@ -47,6 +47,10 @@ bool gbuild_warp_supported(int dim, int order);
 // ------------------------------------------------------------------------------ families on the device (A1)
 constexpr int kFamMax = 256;   // largest family the device build sorts
 constexpr int kFamCell = 4096; // largest cell population (12-bit positions in the visit key)
+struct FamTotals {  // read back once per build
+    long long members, bonds;
+    int err, maxcell, maxfam, pad;
+};
 struct FamArgs {
     int n = 0, is3d = 0;
     const double *coords = nullptr;  // xyz per node
@@ -54,22 +58,25 @@ struct FamArgs {
     double radius = 0, r2 = 0, r2tol = 0;
     unsigned mask = 0;               // cell table size - 1 (power of two)
     unsigned long long *keys = nullptr;
-    int *ccount = nullptr, *cminid = nullptr, *cstart = nullptr, *cfill = nullptr, *members = nullptr;
-    int *cell_of = nullptr, *cxyz = nullptr, *pos = nullptr;
+    int *ccount = nullptr, *cminid = nullptr, *cstart = nullptr, *cfill = nullptr;
+    int *unsorted = nullptr, *members = nullptr;  // the cells' nodes as inserted, and by node id
+    int *cell_of = nullptr, *cxyz = nullptr;
     int *fcount = nullptr;
+    unsigned *votes = nullptr;  // [n][32] which candidates passed (fam_partners_kernel)
     const int *off = nullptr;  // family offsets (a batch cloud's slice: global bond indices)
-    int off_base = 0;          // off[0]: fkey / fval are indexed from it
-    unsigned long long *fkey = nullptr;
-    int *fval = nullptr;
-    int *nbr = nullptr;  // output, 0-based, plus id_base (a batch cloud's first node)
+    int *nbr = nullptr;        // output, 0-based, plus id_base (a batch cloud's first node)
     int id_base = 0;
-    int *err = nullptr;
+    FamTotals *tot = nullptr;
 };
 cudaError_t launch_fam_cells(const FamArgs &a, cudaStream_t s);
 cudaError_t launch_fam_members(const FamArgs &a, cudaStream_t s);
-cudaError_t launch_fam_sort_cells(const FamArgs &a, cudaStream_t s);
-cudaError_t launch_fam_candidates(const FamArgs &a, bool write, cudaStream_t s);
-cudaError_t launch_fam_sort(const FamArgs &a, cudaStream_t s);
+cudaError_t launch_fam_partners(const FamArgs &a, bool write, cudaStream_t s);
+// exclusive scan of count[0, n) into first[0, n] (first[n] = *total), 64-bit sums; *maxv (optional, zeroed by the
+// caller) = largest count.  bsum: scan_blocks(n) long longs of scratch. 
+int scan_blocks(int n);
+cudaError_t launch_scan(int n, const int *count, long long *bsum, long long *total, int *first, int *maxv, cudaStream_t s);
+cudaError_t launch_scan(int n, const int *count, long long *bsum, long long *total, long long *first, int *maxv,
+                        cudaStream_t s);
 
 // ------------------------------------------------------------------------------------------ batched clouds
 // Many independent clouds (2D and 3D mixed) in one node/bond numbering: cloud c owns nodes [node0, node0+n) and
@@ -494,13 +501,14 @@ struct PatternArgs {
     const int *off = nullptr, *nbr = nullptr;  // families, nbr 0-based
     const int *mirror = nullptr;               // 1-based mirror node, 0 none (may be NULL)
     int *count = nullptr;                      // [n] unique column nodes per node
+    int *list = nullptr;                       // [nb + 2 n] their lists, node i's at off[i] + 2 i
     long long *first = nullptr;                // [n+1] exclusive scan of count
     int *overflow = nullptr;                   // nodes whose list exceeds the sort capacity
     int *rowptr = nullptr, *cols = nullptr;    // fill: [n*ndof+1], [nnz]
     int *bptr = nullptr, *bcol = nullptr;      // fill, optional: block view [n+1], [sum count]
 };
-int pattern_scan_blocks(int n);  // long longs of the scan's block-sum scratch
-cudaError_t launch_pattern_count(const PatternArgs &a, long long *bsum, long long *total, cudaStream_t s);
+// count: the sorted lists (list) and their lengths (count); fill: rows from the lists and their scan (first)
+cudaError_t launch_pattern_count(const PatternArgs &a, cudaStream_t s);
 cudaError_t launch_pattern_fill(const PatternArgs &a, cudaStream_t s);
 // device-resident BiCGStab (k_bicg.cu): one cooperative kernel per solve, the host reads the outcome
 enum BicgStatus : int { kBicgRunning = 0, kBicgDone = 2, kBicgBreakdown = 3, kBicgMaxIts = 4 };

@@ -32,21 +32,58 @@ int cuda_fail(cudaError_t e, const char *what);
     } while (0)
 
 // ---- device buffer ---------------------------------------------------------------------------------------------
+// Device blocks that a context's setup has released (families, geometry, operators, pattern) and its next setup takes
+// again: cudaMalloc and cudaFree of the thirty buffers cost more than the kernels between them.  Bounded (kMax, the
+// oldest go first) and given back when memory or the context's limit runs short and with the context.  A block that was
+// given back may still be in use on any stream, as with cudaFree: the first take after a give waits for the device.
+struct DevPool {
+    static constexpr size_t kMax = size_t(1) << 30;
+    struct Block {
+        void *p;
+        size_t cap;
+    };
+    std::vector<Block> idle;
+    size_t bytes = 0;
+    bool dirty = false;
+    void give(void *p, size_t cap);
+    void *take(size_t want, size_t *cap);
+    void trim();
+    DevPool() = default;
+    DevPool(const DevPool &) = delete;
+    DevPool &operator=(const DevPool &) = delete;
+    ~DevPool() { trim(); }
+};
+
 struct DevBuf {
     void *p = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0, cap = 0;
+    DevPool *pool = nullptr;  // where the block goes on release (pool_alloc), else cudaFree
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes) { o.p = nullptr; o.bytes = 0; }
+    DevBuf(DevBuf &&o) noexcept { take(o); }
     DevBuf &operator=(DevBuf &&o) noexcept {
-        if (this != &o) { release(); p = o.p; bytes = o.bytes; o.p = nullptr; o.bytes = 0; }
+        if (this != &o) {
+            release();
+            take(o);
+        }
         return *this;
     }
     ~DevBuf() { release(); }
     void release();
     template <typename T>
     T *as() const { return static_cast<T *>(p); }
+
+private:
+    void take(DevBuf &o) {
+        p = o.p;
+        bytes = o.bytes;
+        cap = o.cap;
+        pool = o.pool;
+        o.p = nullptr;
+        o.bytes = o.cap = 0;
+        o.pool = nullptr;
+    }
 };
 
 // Pinned host staging buffer (grown on demand).
@@ -239,6 +276,7 @@ struct BatchState {
 
 struct pxb_ctx {
     int device = 0;
+    pxb::DevPool pool;  // before the buffers, which go back to it
     // last use of ops.bond: another stream's use waits for it
     cudaEvent_t bond_ev = nullptr;
     cudaStream_t bond_stream = nullptr;
@@ -266,6 +304,8 @@ struct pxb_ctx {
 namespace pxb {
 // device allocation helpers (track bytes per context)
 int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes);
+int pool_alloc(pxb_ctx *c, DevBuf &b, size_t bytes);  // as dev_alloc, from and back to the context's pool
+int pool_upload(pxb_ctx *c, DevBuf &b, const void *host, size_t bytes);
 int dev_upload(pxb_ctx *c, DevBuf &b, const void *host, size_t bytes);
 int h2d(pxb_ctx *c, void *dst, const void *src, size_t bytes);
 int d2h(pxb_ctx *c, void *dst, const void *src, size_t bytes);
