@@ -1099,8 +1099,16 @@ static int rate_plan(pxb_ctx *c) {
 
 // pinned: both host buffers page-locked (copies from pageable memory are staged synchronously, so chunking them
 // only adds per-chunk overhead)
+// The sliced kernels write the acceleration of page-locked buffers straight to the host, while they compute: a copy
+// after them would cost the bus time again.
 static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStream_t s, bool pinned) {
     EpfState &e = c->epf;
+    double *direct = nullptr;
+    if (pinned && runs_sliced(e)) {
+        void *p = nullptr;
+        if (cudaHostGetDevicePointer(&p, accel, 0) == cudaSuccess) direct = static_cast<double *>(p);
+        else cudaGetLastError();
+    }
     const size_t nd = (size_t)c->g.n * c->g.dim;
     unsigned long long *cnt = e.counters.as<unsigned long long>();
     // (a per-bond critical stretch runs the lane-group kernel, which computes every node: no chunking then)
@@ -1133,7 +1141,7 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
             err = cudaMemcpyAsync(cnt + 4, cnt, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
         EpfArgs a = epf_args(c);
         a.u = ud;
-        a.accel = e.accel.as<double>();
+        a.accel = direct ? direct : e.accel.as<double>();
         for (int k = 0; k < K && err == cudaSuccess; ++k) {
             err = cudaStreamWaitEvent(s, ev[2 + e.rate_need[(size_t)k]], 0);
             a.node0 = b[k];
@@ -1141,7 +1149,7 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
             if (err == cudaSuccess) err = epf_launch(c, a, EPF_RATE, e.variant, s);
             if (err == cudaSuccess) err = cudaEventRecord(ev[2 + K + k], s);
             if (err == cudaSuccess) err = cudaStreamWaitEvent(e.rate_down, ev[2 + K + k], 0);
-            if (err == cudaSuccess)
+            if (err == cudaSuccess && !direct)
                 err = cudaMemcpyAsync(accel + (size_t)b[k] * dim, e.accel.as<double>() + (size_t)b[k] * dim, span(k),
                                       cudaMemcpyDeviceToHost, e.rate_down);
         }
@@ -1159,9 +1167,9 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
     if (err != cudaSuccess) return err;
     EpfArgs a = epf_args(c);
     a.u = e.u[e.cur].as<double>();
-    a.accel = e.accel.as<double>();
+    a.accel = direct ? direct : e.accel.as<double>();
     err = epf_launch(c, a, EPF_RATE, e.variant, s);
-    if (err == cudaSuccess)
+    if (err == cudaSuccess && !direct)
         err = cudaMemcpyAsync(accel, e.accel.p, sizeof(double) * nd, cudaMemcpyDeviceToHost, s);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(e.rate_h.p, cnt, sizeof(unsigned long long) * 5, cudaMemcpyDeviceToHost, s);

@@ -118,6 +118,32 @@ __device__ __forceinline__ void load_u(const double *u, size_t i, double *v) {
     }
 }
 
+// The nodes' vectors of a warp (lane = node i) as whole 16- or 8-byte pieces of consecutive addresses: the rate call may
+// point `out` at pinned host memory, where strided pieces would cross the bus one by one.
+template <int DIM>
+__device__ __forceinline__ void store_nodes(double *out, int i, bool act, const double (&v)[DIM]) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (DIM == 2) {
+        if ((reinterpret_cast<unsigned long long>(out) & 15) == 0) {
+            if (act) reinterpret_cast<double2 *>(out)[i] = make_double2(v[0], v[1]);
+            return;
+        }
+    }
+    const unsigned live = __ballot_sync(kFull, act);
+    double *base = out + (size_t)(i - lane) * DIM;  // (lane 0's node may be out of range: never written then)
+#pragma unroll
+    for (int q = 0; q < DIM; ++q) {
+        const int e = q * 32 + lane, node = e / DIM, d = e % DIM;
+        double x = 0.0;
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) {
+            const double y = __shfl_sync(kFull, v[c], node);
+            if (c == d) x = y;
+        }
+        if (live >> node & 1u) base[e] = x;
+    }
+}
+
 }  // namespace
 
 // KW warps a slice, SPB slices a block, U rows in flight a lane.  The loop has no bounds of its own: short families are
@@ -272,12 +298,17 @@ __global__ void __launch_bounds__(KW * SPB * 32, MINB) epf_sliced_kernel(EpfArgs
 #pragma unroll
             for (int d = 0; d < DIM; ++d) L[d] += part[sub][q][d][lane];
     }
+    if (a.rate == kEpfRate) {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) L[d] = __ddiv_rn(__dadd_rn(L[d], a.b[d]), a.rho);
+        store_nodes<DIM>(a.accel, i, act, L);
+        return;
+    }
     double umax = 0.0, un[DIM];
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
         const double acc = __ddiv_rn(__dadd_rn(L[d], a.b[d]), a.rho);
         un[d] = 0.0;
-        if (act && a.rate == kEpfRate) a.accel[(size_t)i * DIM + d] = acc;
         if (act && a.rate == kEpfStart) {
             const double v = a.v0 ? a.v0[(size_t)i * DIM + d] : 0.0;
             a.u_other[(size_t)i * DIM + d] = __dadd_rn(__dsub_rn(ui[d], __dmul_rn(a.dt, v)), __dmul_rn(a.dt2, acc));
