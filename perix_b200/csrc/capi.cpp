@@ -1103,11 +1103,21 @@ static int rate_plan(pxb_ctx *c) {
 // after them would cost the bus time again.
 static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStream_t s, bool pinned) {
     EpfState &e = c->epf;
-    double *direct = nullptr;
-    if (pinned && runs_sliced(e)) {
-        void *p = nullptr;
-        if (cudaHostGetDevicePointer(&p, accel, 0) == cudaSuccess) direct = static_cast<double *>(p);
-        else cudaGetLastError();
+    bool writes = false;  // the kernel writes to the host itself
+    double *direct = nullptr, *direct_u = nullptr;
+    unsigned long long *direct_n = nullptr;
+    if (pinned) {
+        void *p[3] = {nullptr, nullptr, nullptr};
+        if (cudaHostGetDevicePointer(&p[0], accel, 0) == cudaSuccess &&
+            cudaHostGetDevicePointer(&p[1], const_cast<double *>(u), 0) == cudaSuccess &&
+            cudaHostGetDevicePointer(&p[2], e.rate_h.p, 0) == cudaSuccess) {
+            direct = static_cast<double *>(p[0]);
+            writes = runs_sliced(e);
+            direct_u = static_cast<double *>(p[1]);
+            direct_n = static_cast<unsigned long long *>(p[2]);
+        } else {
+            cudaGetLastError();
+        }
     }
     const size_t nd = (size_t)c->g.n * c->g.dim;
     unsigned long long *cnt = e.counters.as<unsigned long long>();
@@ -1141,7 +1151,7 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
             err = cudaMemcpyAsync(cnt + 4, cnt, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
         EpfArgs a = epf_args(c);
         a.u = ud;
-        a.accel = direct ? direct : e.accel.as<double>();
+        a.accel = writes ? direct : e.accel.as<double>();
         for (int k = 0; k < K && err == cudaSuccess; ++k) {
             err = cudaStreamWaitEvent(s, ev[2 + e.rate_need[(size_t)k]], 0);
             a.node0 = b[k];
@@ -1149,7 +1159,7 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
             if (err == cudaSuccess) err = epf_launch(c, a, EPF_RATE, e.variant, s);
             if (err == cudaSuccess) err = cudaEventRecord(ev[2 + K + k], s);
             if (err == cudaSuccess) err = cudaStreamWaitEvent(e.rate_down, ev[2 + K + k], 0);
-            if (err == cudaSuccess && !direct)
+            if (err == cudaSuccess && !writes)
                 err = cudaMemcpyAsync(accel + (size_t)b[k] * dim, e.accel.as<double>() + (size_t)b[k] * dim, span(k),
                                       cudaMemcpyDeviceToHost, e.rate_down);
         }
@@ -1160,16 +1170,22 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
         if (err == cudaSuccess) err = cudaStreamWaitEvent(s, ev[1], 0);
         return err;
     }
+    EpfArgs a = epf_args(c);
+    a.u = e.u[e.cur].as<double>();
+    a.accel = writes ? direct : e.accel.as<double>();
+    if (direct) {
+        cudaError_t err = launch_rate_up(nd, direct_u, e.u[e.cur].as<double>(), cnt, s);
+        if (err == cudaSuccess) err = epf_launch(c, a, EPF_RATE, e.variant, s);
+        if (err == cudaSuccess) err = launch_rate_down(cnt, direct_n, writes ? 0 : nd, a.accel, direct, s);
+        return err;
+    }
     cudaError_t err = cudaMemcpyAsync(e.u[e.cur].p, u, sizeof(double) * nd, cudaMemcpyHostToDevice, s);
     // the broken-bond count before the kernel, snapshot on the device: one host synchronisation per call
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(cnt + 4, cnt, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
     if (err != cudaSuccess) return err;
-    EpfArgs a = epf_args(c);
-    a.u = e.u[e.cur].as<double>();
-    a.accel = direct ? direct : e.accel.as<double>();
     err = epf_launch(c, a, EPF_RATE, e.variant, s);
-    if (err == cudaSuccess && !direct)
+    if (err == cudaSuccess)
         err = cudaMemcpyAsync(accel, e.accel.p, sizeof(double) * nd, cudaMemcpyDeviceToHost, s);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(e.rate_h.p, cnt, sizeof(unsigned long long) * 5, cudaMemcpyDeviceToHost, s);

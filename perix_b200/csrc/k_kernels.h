@@ -335,6 +335,10 @@ cudaError_t launch_apply(const ApplyArgs &a, bool mixed, int grid, cudaStream_t 
 bool apply_has_rows(const ApplyArgs &a);  // the operator row has kernels of its own
 // bond: one double a bond of scratch for the two-pass transpose, NULL for the kernel that needs none
 cudaError_t launch_apply_adjoint(const ApplyArgs &a, bool mixed, double *bond, int grid, cudaStream_t s);
+// the rate call's page-locked ends (k_epf_sliced.cu): u up with cnt[4] = cnt[0], cnt[0..4] and n values of accel down
+cudaError_t launch_rate_up(size_t n, const double *host_u, double *u, unsigned long long *cnt, cudaStream_t s);
+cudaError_t launch_rate_down(const unsigned long long *cnt, unsigned long long *host, size_t n, const double *accel,
+                             double *host_a, cudaStream_t s);
 struct AdjPrepArgs {
     int n = 0, dim = 2, nop = 0, nk = 0, next = 0;
     int slots[32], ext[32];
