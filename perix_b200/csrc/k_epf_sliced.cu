@@ -734,9 +734,9 @@ cudaError_t launch_sliced_health(int n, const int *off, const int *row0, const u
 
 // ---- the rate call's ends for page-locked buffers ------------------------------------------------------------------
 // The displacement up and the broken-bond count before the kernel, and the counters (and, unless the kernel wrote it
-// there itself, the acceleration) down after it, by threads that read and write the host's memory: a copy-engine node each costs the call several microseconds of hand-over.
-// A call on a plate of 81,200 nodes: 81 us with the
-// copies, 75 with these; on one of 2,600 nodes 35 and 19.
+// there itself, the acceleration) down after it, by threads that read and write the host's memory: a copy-engine node
+// each costs the call several microseconds of hand-over.  A call on a plate of 81,200 nodes: 81 us with the copies, 75
+// with these; on one of 2,600 nodes 35 and 19.
 __global__ void __launch_bounds__(256) rate_up_kernel(size_t n, const double *host_u, double *u, unsigned long long *cnt,
                                                       bool wide) {
     const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;

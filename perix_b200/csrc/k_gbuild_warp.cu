@@ -16,7 +16,7 @@
 //           the per-node first moments of the stored second-derivative operators (GBuildArgs::defect).
 // With TC (up to nine monomials, the default there) the same three phases use the FP64 tensor cores
 // (mma.sync.m8n8k4.f64): pass 1 accumulates the (0,0) tile of A = (W M)^T M from each chunk's transposed monomials
-// (the ninth row per lane on the CUDA cores), the solve is Gauss-Jordan on [A | diag(q!)] with a row per lane in
+// (the ninth row per lane on the CUDA cores), the solve is Gauss-Jordan on [A | diag(q!)], a few lanes a row, in
 // registers and its residual D - A X a tensor-core product, and pass 2 forms operators 0-7 as 8-bond tiles (the
 // ninth per lane) staged in shared memory and stored as one coalesced block per chunk.
 // Per-node horizons (GBuildArgs::node_delta / node_dxc) follow the reference's variable-horizon path: node i
@@ -107,6 +107,13 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
+}
+
+// largest of the warp's non-negative values, a NaN above all: their bit patterns are ordered as the values are
+__device__ __forceinline__ double warp_max_magnitude(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), top = __reduce_max_sync(kFull, hi);
+    const unsigned lo = __reduce_max_sync(kFull, hi == top ? (unsigned)__double2loint(v) : 0u);
+    return __hiloint2double((int)top, (int)lo);
 }
 
 struct BondGeo {
@@ -317,7 +324,7 @@ __device__ __forceinline__ void gbuild_warp_node(const GBuildArgs &a, int i, int
         }
     }
     }
-    usable = group_sum_int<kWarp>(usable);
+    usable = __reduce_add_sync(kFull, usable);
     if constexpr (TC) {  // the tiles' upper triangle, mirrored (the matrix stays exactly symmetric)
         auto put = [&](int p, int q, double v) {
             if (p <= q && q < NOP) {
@@ -355,37 +362,54 @@ __device__ __forceinline__ void gbuild_warp_node(const GBuildArgs &a, int i, int
     double res = 0.0, maxA = 0.0, maxX = 0.0;
     bool degenerate;
     if constexpr (TC) {
-        // ---- solve (up to nine monomials): Gauss-Jordan on [A | diag(q!)] with row r in lane r's registers; the
-        // pivot row is broadcast by shuffles, so no shared-memory round trip or warp barrier per column.  A is
-        // symmetric positive definite for a usable family (no pivoting, as in the L D L^T path); before step j the
-        // right-hand side of row j is zero past column j.  Lane p < NOP ends with row p of X = A^-1 diag(q!).
-        double ra[NOP], rb[NOP];
+        // ---- solve (up to nine monomials): Gauss-Jordan on [A | diag(q!)] in registers, CG lanes a row, lane (row, c)
+        // with the columns c, c + CG, ... of both halves; the pivot row and the column of factors are broadcast by
+        // shuffles, so no shared-memory round trip or warp barrier per column.  With a row a lane and nine lanes at
+        // work the nine steps took twice the shuffles and three times the products: 8.3 million bonds in 3D 418 us, here
+        // 378 (with the maxima below by integer reductions).
+        // A is symmetric positive definite for a usable family (no pivoting, as in the L D L^T path); before step j the
+        // right-hand side of row j is zero past column j, and columns of A up to j are not read again.
+        constexpr int CG = NOP <= 5 ? NOP : 3, MC = (NOP + CG - 1) / CG;
+        static_assert(NOP * CG <= kWarp, "a lane for every part of a row");
+        const bool part = lane < NOP * CG;
+        const int row = part ? lane / CG : 0, cg = lane % CG;
+        double ra[MC], rb[MC], fr = 0.0;
 #pragma unroll
-        for (int k = 0; k < NOP; ++k) {
-            ra[k] = lane < NOP ? lds(&sm.A[(lane < NOP ? lane : 0) * NOP + k]) : 0.0;
-            rb[k] = (k == lane) ? Q.fact[k] : 0.0;
+        for (int q = 0; q < NOP; ++q)
+            if (q == row) fr = Q.fact[q];
+#pragma unroll
+        for (int m = 0; m < MC; ++m) {
+            const int k = cg + CG * m;
+            ra[m] = k < NOP ? lds(&sm.A[row * NOP + (k < NOP ? k : 0)]) : 0.0;
+            rb[m] = k == row ? fr : 0.0;
         }
 #pragma unroll
         for (int j = 0; j < NOP; ++j) {
-            double pa[NOP], pb[NOP];
+            const double pj = __shfl_sync(kFull, ra[j / CG], j * CG + j % CG);
+            const double aj = __shfl_sync(kFull, ra[j / CG], row * CG + j % CG);
+            const double inv = 1.0 / pj, f = aj * inv;
+            const bool piv = row == j;
 #pragma unroll
-            for (int k = j; k < NOP; ++k) pa[k] = __shfl_sync(kFull, ra[k], j);
-#pragma unroll
-            for (int k = 0; k <= j; ++k) pb[k] = __shfl_sync(kFull, rb[k], j);
-            const double inv = 1.0 / pa[j];
-            const bool piv = lane == j;
-            const double f = ra[j] * inv;
-#pragma unroll
-            for (int k = j + 1; k < NOP; ++k) ra[k] = piv ? pa[k] * inv : fma(-f, pa[k], ra[k]);
-#pragma unroll
-            for (int k = 0; k <= j; ++k) rb[k] = piv ? pb[k] * inv : fma(-f, pb[k], rb[k]);
+            for (int m = 0; m < MC; ++m) {
+                if (CG * m + CG - 1 > j) {
+                    const double pa = __shfl_sync(kFull, ra[m], j * CG + cg);
+                    ra[m] = piv ? pa * inv : fma(-f, pa, ra[m]);
+                }
+                if (CG * m <= j) {
+                    const double pb = __shfl_sync(kFull, rb[m], j * CG + cg);
+                    rb[m] = piv ? pb * inv : fma(-f, pb, rb[m]);
+                }
+            }
         }
         // the consistency test's residual D - A X on the tensor cores (X rows through shared memory, 8x8 tiles)
-        if (lane < NOP) {
+        if (part) {
+            if (NP > NOP && cg == 0) sm.X[row * NP + NOP] = 0.0;
 #pragma unroll
-            for (int k = 0; k < NP; ++k) sm.X[lane * NP + k] = k < NOP ? rb[k < NOP ? k : 0] : 0.0;
-#pragma unroll
-            for (int k = 0; k < NOP; ++k) maxX = max_nan(maxX, fabs(rb[k]));
+            for (int m = 0; m < MC; ++m)
+                if (cg + CG * m < NOP) {
+                    sm.X[row * NP + cg + CG * m] = rb[m];
+                    maxX = max_nan(maxX, fabs(rb[m]));
+                }
         }
         __syncwarp();
         constexpr int RT = NOP > 8 ? 2 : 1, KS = (NOP + 3) / 4;
@@ -425,9 +449,9 @@ __device__ __forceinline__ void gbuild_warp_node(const GBuildArgs &a, int i, int
                         res = max_nan(res, fabs(dv - rt[u][v][h]));
                     }
                 }
-        maxA = group_max<kWarp>(maxA);
-        res = group_max_nan<kWarp>(res);
-        maxX = group_max_nan<kWarp>(maxX);
+        maxA = warp_max_magnitude(maxA);
+        res = warp_max_magnitude(res);
+        maxX = warp_max_magnitude(maxX);
         double maxB = 0.0;
 #pragma unroll
         for (int q = 0; q < NOP; ++q) maxB = fmax(maxB, Q.fact[q]);
@@ -436,14 +460,17 @@ __device__ __forceinline__ void gbuild_warp_node(const GBuildArgs &a, int i, int
         degenerate = (usable < NOP) || !consistent;
         __syncwarp();  // X is written again below, scaled
         // column k carries the operator's scale 1/delta^|q_k|, so that pass 2 only multiplies by the bond weight
-        if (lane < NOP) {
+        if (part) {
 #pragma unroll
-            for (int k = 0; k < NOP; ++k) {
+            for (int m = 0; m < MC; ++m) {
+                const int k = cg + CG * m;
                 double cs = inv_delta;
 #pragma unroll
-                for (int t2 = 1; t2 < Q.p[k] + Q.q[k] + Q.r[k]; ++t2) cs *= inv_delta;
-                sm.X[lane * NP + k] = degenerate ? 0.0 : rb[k] * cs;
-                if (k == 8) sm.c8[lane < NOP ? lane : 0] = degenerate ? 0.0 : rb[k] * cs;
+                for (int o = 1; o < ORDER; ++o)
+                    if (k >= nop_of(DIM, o)) cs *= inv_delta;
+                const double v = degenerate ? 0.0 : rb[m] * cs;
+                if (k < NOP) sm.X[row * NP + k] = v;
+                if (k == 8) sm.c8[row] = v;
             }
         }
     } else {
