@@ -52,7 +52,7 @@ int pxb_ctx_destroy(pxb_ctx *ctx);
  * To share the legacy default stream (torch's default stream, handle 0) pass cudaStreamLegacy ((void*)1). */
 int pxb_ctx_set_stream(pxb_ctx *ctx, void *stream);
 int pxb_ctx_synchronize(pxb_ctx *ctx);
-/* Device bytes currently held by the context. */
+/* Device bytes in use by the context (idle blocks that its next set-up may take again, at most 1 GiB, not counted). */
 int pxb_ctx_device_bytes(pxb_ctx *ctx, size_t *bytes);
 /* Caps the device bytes the context may hold (0 = no cap beyond the GPU's own memory), e.g. to share a GPU with
  * other work: an allocation past the cap fails with PXB_ERR_OOM before reaching the driver, like one the driver
@@ -302,7 +302,8 @@ int pxb_epf_snapshot(pxb_ctx *ctx);
 int pxb_epf_restore(pxb_ctx *ctx);
 /* Schedule variants of the explicit kernel: 0-2 lane groups (lanes per node x bonds per lane per pass), 3-4
  * CSR-stream tiles, 5-16 TMA-staged tiles, 17-20 sliced (time step and rate call, in FP64 the start and the frozen
- * force too; the other modes of a staged or sliced variant run variant 1).  A sliced variant keeps a second, neighbour-sorted copy of the bond streams (about
+ * force too; the other modes of a staged or sliced variant run variant 1).
+ * A sliced variant keeps a second, neighbour-sorted copy of the bond streams (about
  * 54 bytes a bond in 3D FP64, 30 mixed), built when it is first selected; without room for it pxb_epf_set_variant
  * fails with PXB_ERR_OOM and the autotuners skip it.  pxb_epf_variant_count() gives their number.  pxb_epf_autotune
  * times every variant that fits for `steps` steps from a private copy of the current state (L2 flushed before each

@@ -234,7 +234,8 @@ size_t ctx_bytes(const pxb_ctx *c) {
     s += bufsz(bt.clouds) + bufsz(bt.tasks) + bufsz(bt.off) + bufsz(bt.nbr) + bufsz(bt.pos) + bufsz(bt.vol) +
          bufsz(bt.ops) + bufsz(bt.degenerate) + bufsz(bt.counters) + bufsz(bt.defect);
     const CsrState &k = c->csr;
-    s += bufsz(k.rowptr) + bufsz(k.cols) + bufsz(k.slot) + bufsz(k.bpos) + bufsz(k.spos) + bufsz(k.xpos) + bufsz(k.diag) + bufsz(k.kvals) + bufsz(k.rhs) +
+    s += bufsz(k.rowptr) + bufsz(k.cols) + bufsz(k.slot) + bufsz(k.bpos) + bufsz(k.spos) + bufsz(k.xpos) +
+         bufsz(k.diag) + bufsz(k.kvals) + bufsz(k.rhs) +
          bufsz(k.u) + bufsz(k.uold) + bufsz(k.fnode) + bufsz(k.mnode) + bufsz(k.sl_row0) + bufsz(k.sl_col) +
          bufsz(k.sl_pair);
     s += bufsz(c->ch.rev) + bufsz(c->ch.lap) + bufsz(c->ch.ghost) + bufsz(c->ch.lrv) + bufsz(c->ch.bfl) +

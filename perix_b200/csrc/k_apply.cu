@@ -259,8 +259,12 @@ template <typename F>
 static bool with_rows(const ApplyArgs &a, bool mixed, F f) {
     auto lanes = [&](auto nop) {
         using N = decltype(nop);
-        if (a.dim == 3) mixed ? f(std::true_type{}, N{}, std::integral_constant<int, 16>{}) : f(std::false_type{}, N{}, std::integral_constant<int, 16>{});
-        else mixed ? f(std::true_type{}, N{}, std::integral_constant<int, 8>{}) : f(std::false_type{}, N{}, std::integral_constant<int, 8>{});
+        auto by_type = [&](auto lpn) {
+            if (mixed) f(std::true_type{}, N{}, lpn);
+            else f(std::false_type{}, N{}, lpn);
+        };
+        if (a.dim == 3) by_type(std::integral_constant<int, 16>{});
+        else by_type(std::integral_constant<int, 8>{});
     };
     switch (a.nop) {
         case 2: lanes(std::integral_constant<int, 2>{}); return true;
