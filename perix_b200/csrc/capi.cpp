@@ -2206,25 +2206,35 @@ extern "C" int pxb_epf_force_adjoint(pxb_ctx *c, const double *u, const double *
     return PXB_OK;
 }
 
+// the longest block list that an exact pattern can have: own block, family, a mirror outside it
+static int longest_list(const pxb_ctx *c) { return c->g.max_family + 2; }
+
+static int alloc_positions(pxb_ctx *c) {
+    CsrState &k = c->csr;
+    const size_t n = (size_t)c->g.n;
+    PXB_TRY(pool_alloc(c, k.diag, sizeof(int) * n * k.ndof * k.ndof));
+    if (k.mmax > kBlockMax) return PXB_OK;
+    PXB_TRY(pool_alloc(c, k.bpos, (size_t)std::max(1LL, c->g.nb)));
+    PXB_TRY(pool_alloc(c, k.spos, n));
+    return pool_alloc(c, k.xpos, sizeof(int16_t) * n);
+}
+
+
 // ============================================================================================== CSR assembly
 namespace pxb {
-// the block positions (exact block patterns) or the slot map, the diagonal slots and the value buffers of the pattern
-// in c->csr (rowptr, cols, ndof, nnz set on the device); verify: the rows come from the caller and are checked
+// the block positions (exact block patterns) or the slot map, the diagonal slots (unless k.exact says that the pattern's
+// sort has left both) and the value buffers of the pattern in c->csr (rowptr, cols, ndof, nnz, mmax set); verify: the rows
+// come from the caller and are checked
 int csr_finish(pxb_ctx *c, const char *who, bool verify) {
     CsrState &k = c->csr;
     const int ndof = k.ndof, n = c->g.n;
     const size_t rows = (size_t)n * ndof, nb = (size_t)std::max(1LL, c->g.nb);
-    PXB_TRY(pool_alloc(c, k.diag, sizeof(int) * (size_t)n * ndof * ndof));
     void *tmp = nullptr;
     PXB_TRY(scratch(c, 8, &tmp));
     PXB_CUDA_TRY(cudaMemsetAsync(tmp, 0, 8, c->stream));
-    k.mmax = c->g.max_family + 2;  // own block, family, a mirror outside it
-    k.exact = false;
     int flags[2] = {0, 0};
-    if (k.mmax <= kBlockMax) {
-        PXB_TRY(pool_alloc(c, k.bpos, nb));
-        PXB_TRY(pool_alloc(c, k.spos, (size_t)n));
-        PXB_TRY(pool_alloc(c, k.xpos, sizeof(int16_t) * (size_t)n));
+    if (!k.exact) PXB_TRY(alloc_positions(c));
+    if (!k.exact && k.mmax <= kBlockMax) {
         BlockMapArgs m;
         m.n = n;
         m.ndof = ndof;
@@ -2289,6 +2299,7 @@ extern "C" int pxb_csr_set_pattern(pxb_ctx *c, int ndof, const int *rowptr, cons
     k = CsrState{};
     k.ndof = ndof;
     k.nnz = nnz;
+    k.mmax = longest_list(c);
     const size_t rows = (size_t)c->g.n * ndof;
     PXB_TRY(dev_upload(c, k.rowptr, rowptr, sizeof(int) * (rows + 1)));
     PXB_TRY(dev_upload(c, k.cols, cols, sizeof(int) * (size_t)nnz));
@@ -2308,6 +2319,7 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     CsrState &k = c->csr;
     k = CsrState{};
     k.ndof = ndof;
+    k.mmax = longest_list(c);
     DevBuf count, first, bsum, small, list;
     PXB_TRY(pool_alloc(c, list, sizeof(int) * ((size_t)c->g.nb + 2 * (size_t)n)));
     PXB_TRY(pool_alloc(c, count, sizeof(int) * (size_t)n));
@@ -2325,6 +2337,15 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     a.first = first.as<long long>();
     a.overflow = reinterpret_cast<int *>(small.as<char>() + 8);
     a.list = list.as<int>();
+    const bool positions = k.mmax <= kBlockMax && n < kPackedNodes;
+    if (positions) {
+        PXB_TRY(alloc_positions(c));
+        a.bpos = k.bpos.as<uint8_t>();
+        a.spos = k.spos.as<uint8_t>();
+        a.xpos = k.xpos.as<int16_t>();
+        a.diag = k.diag.as<int>();
+        a.inexact = reinterpret_cast<int *>(small.as<char>() + 12);
+    }
     PXB_CUDA_TRY(launch_pattern_count(a, c->stream));
     PXB_CUDA_TRY(launch_scan(n, a.count, bsum.as<long long>(), small.as<long long>(), a.first, nullptr, c->stream));
     c->launches += 4;
@@ -2353,6 +2374,7 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     a.cols = k.cols.as<int>();
     PXB_CUDA_TRY(launch_pattern_fill(a, c->stream));
     c->launches++;
+    k.exact = positions && (h[1] >> 32) == 0;
     PXB_TRY(csr_finish(c, "pxb_csr_build_pattern", false));
     if (nnz) *nnz = total;
     return PXB_OK;

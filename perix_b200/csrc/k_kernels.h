@@ -510,7 +510,13 @@ struct PatternArgs {
     int *overflow = nullptr;                   // nodes whose list exceeds the sort capacity
     int *rowptr = nullptr, *cols = nullptr;    // fill: [n*ndof+1], [nnz]
     int *bptr = nullptr, *bcol = nullptr;      // fill, optional: block view [n+1], [sum count]
+    // optional (n <= kPackedNodes, families + 2 <= kBlockMax): the block positions of BlockMapArgs as the sort leaves
+    // them, *inexact counting the nodes whose family lists a node twice or the node itself; fill: diag
+    uint8_t *bpos = nullptr, *spos = nullptr;
+    int16_t *xpos = nullptr;
+    int *inexact = nullptr, *diag = nullptr;
 };
+constexpr int kPackedNodes = 1 << 23;  // node ids that leave room for a list index of 8 bits in a positive int
 // count: the sorted lists (list) and their lengths (count); fill: rows from the lists and their scan (first)
 cudaError_t launch_pattern_count(const PatternArgs &a, cudaStream_t s);
 cudaError_t launch_pattern_fill(const PatternArgs &a, cudaStream_t s);

@@ -52,8 +52,9 @@ __device__ __forceinline__ void sort_values(int (&v)[E]) {
         }
 }
 
-// node i's own, family and mirror nodes, sorted and unique, to out; returns how many
-template <int E>
+// node i's own, family and mirror nodes, sorted and unique, to out; returns how many.  PACKED: a value is node << 8 | index
+// in the unsorted list, so that every entry's position in the sorted one is known when it is written (bpos, spos, xpos).
+template <int E, bool PACKED>
 __device__ __forceinline__ int node_list(const PatternArgs &a, int i, int b0, int len, int mir, int *out) {
     const int lane = threadIdx.x & 31, tot = len + 1 + (mir >= 0 ? 1 : 0);
     int v[E];
@@ -61,22 +62,42 @@ __device__ __forceinline__ int node_list(const PatternArgs &a, int i, int b0, in
     for (int q = 0; q < E; ++q) {
         const int k = 32 * q + lane;
         v[q] = k < len ? a.nbr[b0 + k] : (k == len ? i : (k < tot ? mir : INT_MAX));
+        if (PACKED && k < tot) v[q] = v[q] << 8 | k;
     }
     sort_values<E>(v);
-    int m = 0, last = -1;  // last: the value before element 32 q
+    int m = 0, last = -1;  // last: the node before element 32 q
+    bool own_kept = true;
+    int at_mirror = -1;
 #pragma unroll
     for (int q = 0; q < E; ++q) {
-        int before = __shfl_up_sync(kFull, v[q], 1);
+        const int node = PACKED ? v[q] >> 8 : v[q], k = v[q] & 255;
+        int before = __shfl_up_sync(kFull, node, 1);
         if (lane == 0) before = last;
-        const bool keep = 32 * q + lane < tot && v[q] != before;
+        const bool in = 32 * q + lane < tot, keep = in && node != before;
         const unsigned ball = __ballot_sync(kFull, keep);
-        if (keep) out[m + __popc(ball & ((1u << lane) - 1u))] = v[q];
+        const int at = m + __popc(ball & ((1u << lane) - 1u));
+        if (keep) out[at] = node;
+        if (PACKED && in) {  // of a node listed twice the family's entry comes first, the mirror's last
+            if (k < len) a.bpos[b0 + k] = (uint8_t)at;
+            else if (k == len) a.spos[i] = (uint8_t)at;
+            else if (keep) at_mirror = at;
+            if (k <= len && !keep) own_kept = false;
+        }
         m += __popc(ball);
-        last = __shfl_sync(kFull, v[q], 31);
+        last = __shfl_sync(kFull, node, 31);
+    }
+    if constexpr (PACKED) {
+        at_mirror = __reduce_max_sync(kFull, at_mirror);
+        own_kept = __all_sync(kFull, own_kept);
+        if (lane == 0) {
+            a.xpos[i] = (int16_t)at_mirror;
+            if (!own_kept) atomicAdd(a.inexact, 1);
+        }
     }
     return m;
 }
 
+template <bool PACKED>
 __global__ void __launch_bounds__(kPatWarps * 32) pattern_list_kernel(PatternArgs a) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int i = blockIdx.x * kPatWarps + w; i < a.n; i += gridDim.x * kPatWarps) {
@@ -84,10 +105,10 @@ __global__ void __launch_bounds__(kPatWarps * 32) pattern_list_kernel(PatternArg
         const int mir = m0 >= 1 && m0 <= a.n ? m0 - 1 : -1, tot = len + 1 + (mir >= 0 ? 1 : 0);
         int *out = a.list + ((size_t)b0 + 2 * (size_t)i);
         int m = -1;
-        if (tot <= 32) m = node_list<1>(a, i, b0, len, mir, out);
-        else if (tot <= 64) m = node_list<2>(a, i, b0, len, mir, out);
-        else if (tot <= 128) m = node_list<4>(a, i, b0, len, mir, out);
-        else if (tot <= kPatCap) m = node_list<8>(a, i, b0, len, mir, out);
+        if (tot <= 32) m = node_list<1, PACKED>(a, i, b0, len, mir, out);
+        else if (tot <= 64) m = node_list<2, PACKED>(a, i, b0, len, mir, out);
+        else if (tot <= 128) m = node_list<4, PACKED>(a, i, b0, len, mir, out);
+        else if (tot <= kPatCap) m = node_list<8, PACKED>(a, i, b0, len, mir, out);
         if (lane == 0) {
             if (m < 0) atomicAdd(a.overflow, 1);
             a.count[i] = m < 0 ? 0 : m;
@@ -113,6 +134,9 @@ __global__ void __launch_bounds__(kPatWarps * 32) pattern_rows_kernel(PatternArg
                 for (int b = 0; b < nd; ++b) a.cols[row0 + (long long)k * nd + b] = node * nd + b;
             }
         }
+        if (a.diag && lane < nd * nd)
+            a.diag[(size_t)i * nd * nd + lane] =
+                (int)((long long)nd * nd * first + (long long)(lane / nd) * m * nd + a.spos[i] * nd + lane % nd);
         if (lane < nd) a.rowptr[(size_t)i * nd + lane] = (int)((long long)nd * nd * first + (long long)lane * m * nd);
         if (a.bptr && lane == 0) a.bptr[i] = (int)first;
     }
@@ -210,7 +234,8 @@ cudaError_t launch_scan(int n, const int *count, long long *bsum, long long *tot
 }
 
 cudaError_t launch_pattern_count(const PatternArgs &a, cudaStream_t s) {
-    pattern_list_kernel<<<pattern_grid(a.n), kPatWarps * 32, 0, s>>>(a);
+    if (a.bpos) pattern_list_kernel<true><<<pattern_grid(a.n), kPatWarps * 32, 0, s>>>(a);
+    else pattern_list_kernel<false><<<pattern_grid(a.n), kPatWarps * 32, 0, s>>>(a);
     return cudaGetLastError();
 }
 
