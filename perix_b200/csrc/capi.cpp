@@ -114,35 +114,38 @@ static int malloc_dev(void **p, size_t bytes) {
     return cuda_fail(e, "cudaMalloc");
 }
 
-// What the context can do without gives way to what has to be there: idle blocks, the field transpose's scratch, the
-// implicit run's slices (both are built again by a use that finds the memory).
-static void make_room(pxb_ctx *c, const DevBuf &b, size_t bytes) {
+// What the context can do without gives way to buffer b: the implicit run's slices and the field transpose's scratch
+// (both are built again by a use that finds the memory); true when anything was there.
+static bool drop_optional(pxb_ctx *c, const DevBuf &b) {
     CsrState &k = c->csr;
-    auto short_of = [&]() {
-        if (c->mem_limit && ctx_bytes(c) - b.bytes + bytes > c->mem_limit) return true;
-        size_t free_b = 0, total_b = 0;
-        return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > free_b;
-    };
-    const bool limited = c->mem_limit && ctx_bytes(c) - b.bytes + bytes + c->pool.bytes > c->mem_limit;
-    if (c->pool.bytes && (limited || short_of())) c->pool.trim();
-    if (c->ops.bond.p && &b != &c->ops.bond && short_of()) c->ops.bond.release();
-    if (k.sl_pair.p && &b != &k.sl_pair && &b != &k.sl_col && &b != &k.sl_row0 && short_of()) {
+    const bool any = (c->ops.bond.p && &b != &c->ops.bond) || (k.sl_pair.p && &b != &k.sl_pair && &b != &k.sl_col);
+    if (&b != &c->ops.bond) c->ops.bond.release();
+    if (&b != &k.sl_pair && &b != &k.sl_col && &b != &k.sl_row0) {
         k.sl_pair.release();
         k.sl_col.release();
     }
+    return any;
 }
 
-static int over_limit(const pxb_ctx *c, const DevBuf &b, size_t bytes) {
-    if (c && c->mem_limit && bytes > b.bytes && ctx_bytes(c) - b.bytes + bytes > c->mem_limit)
-        return fail(PXB_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes would exceed the context's " +
-                                     std::to_string(c->mem_limit) + "-byte limit (pxb_ctx_set_memory_limit)");
-    return PXB_OK;
+// under stream capture, or not to be told
+static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+static bool over_limit(const pxb_ctx *c, const DevBuf &b, size_t bytes, size_t idle) {
+    return c && c->mem_limit && bytes > b.bytes && ctx_bytes(c) - b.bytes + bytes + idle > c->mem_limit;
 }
 
 int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
     if (b.p && b.bytes == bytes) return PXB_OK;
-    if (c && bytes > b.bytes) make_room(c, b, bytes);
-    PXB_TRY(over_limit(c, b, bytes));
+    if (c && over_limit(c, b, bytes, c->pool.bytes)) c->pool.trim();
+    if (c && over_limit(c, b, bytes, 0)) drop_optional(c, b);
+    if (over_limit(c, b, bytes, 0))
+        return fail(PXB_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes would exceed the context's " +
+                                     std::to_string(c->mem_limit) + "-byte limit (pxb_ctx_set_memory_limit)");
     b.release();
     if (bytes == 0) return PXB_OK;
     int st = malloc_dev(&b.p, bytes);
@@ -150,6 +153,7 @@ int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
         c->pool.trim();
         st = malloc_dev(&b.p, bytes);
     }
+    if (st == PXB_ERR_OOM && c && drop_optional(c, b)) st = malloc_dev(&b.p, bytes);
     PXB_TRY(st);
     b.bytes = b.cap = bytes;
     return PXB_OK;
@@ -157,9 +161,7 @@ int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
 
 int pool_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
     if (b.p && b.bytes == bytes) return PXB_OK;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (bytes > 0 && cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
-        !(c->mem_limit && ctx_bytes(c) - b.bytes + bytes + c->pool.bytes > c->mem_limit)) {
+    if (bytes > 0 && !capturing(c->stream) && !over_limit(c, b, bytes, c->pool.bytes)) {
         b.release();
         if (void *p = c->pool.take(bytes, &b.cap)) {
             b.p = p;
@@ -739,10 +741,7 @@ extern "C" int pxb_apply(pxb_ctx *c, const double *u, int nk, const int *slots, 
 // its own, when the memory (limit) does not hold it, and under stream capture, whose graph would keep a pointer
 // to a buffer that the context may give up.
 static double *adjoint_scratch(pxb_ctx *c, const ApplyArgs &a) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!apply_has_rows(a) || c->g.nb == 0 || cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess ||
-        cap != cudaStreamCaptureStatusNone)
-        return nullptr;
+    if (!apply_has_rows(a) || c->g.nb == 0 || capturing(c->stream)) return nullptr;
     const size_t need = sizeof(double) * (size_t)c->g.nb;
     if (c->ops.bond.bytes != need && dev_alloc(c, c->ops.bond, need) != PXB_OK) return nullptr;
     if (!c->bond_ev && cudaEventCreateWithFlags(&c->bond_ev, cudaEventDisableTiming) != cudaSuccess) return nullptr;
