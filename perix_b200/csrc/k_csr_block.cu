@@ -9,10 +9,10 @@
 //     memory and leave as one coalesced copy, every entry written once: no zeroing pass, no 8-byte stores scattered
 //     over the rows (each of which cost a 32-byte L2 sector);
 //   * the operator rows of a family are one contiguous span too, read coalesced into shared memory.
-// B200: 38,912 nodes in 3D with five unknowns (4.29 M bonds, 1.30 GB necessary) 783 us with slots -> 428 us; 81,200
-// nodes in 2D with two unknowns (2.25 M bonds, 171 MB) 96 -> 66 us.  What bounds both now is the L1 data pipe (65 % of
-// its peak: the values pass through shared memory once, with bank conflicts where a family's positions are not
-// consecutive), then DRAM latency (24-31 % occupancy, limited by registers and the tile's shared memory).
+// B200: 38,912 nodes in 3D with five unknowns (4.29 M bonds, 1.30 GB necessary) 783 us with slots -> 391 us; 81,200
+// nodes in 2D with two unknowns (2.25 M bonds, 171 MB) 96 -> 64 us.  What bounds both is the L1 data pipe (65 % of
+// its peak at 428 and 66 us: the values pass through shared memory once, with bank conflicts where a family's positions are not
+// consecutive), then DRAM latency (24-31 % occupancy there, limited by registers and the tile's shared memory; MINB below).
 #include <type_traits>
 
 #include "k_kernels.h"
@@ -305,7 +305,9 @@ template <int DIM>
 struct StressChEl {
     static constexpr int ND = DIM + 2, NOP = DIM == 3 ? 9 : 5, TN = DIM == 3 ? 1 : 4, P = DIM == 3 ? 1 : 4;
     // nodal values: u[ND], V, M, 1/V, (c_old, -, u - u_old - v dt)[ND]
-    static constexpr int NQ = 2 * ND + 3, MINB = 4;
+    // resident blocks: 3D (128 threads) 5 against 4 391 us of 427 at the size above, 3 506, 6 455; 2D (one warp a block) 12,
+    // against 4 blocks of two warps 181 us of 188 on 56,000 nodes
+    static constexpr int NQ = 2 * ND + 3, MINB = DIM == 3 ? 5 : 12;
     // operator slots in the multi-index order: first derivatives, then xx xy [xz] yy [yz zz]
     static constexpr int SXX = DIM, SXY = DIM + 1, SXZ = 5, SYY = DIM == 3 ? 6 : 4, SYZ = 7, SZZ = 8;
     StressChAsmArgs a;
@@ -417,7 +419,7 @@ template <int DIM>
 struct CachedEl {
     static constexpr int ND = DIM, NOP = DIM == 3 ? 9 : 5, NP = DIM == 3 ? 6 : 3, TN = DIM == 3 ? 1 : 4, P = DIM == 3 ? 1 : 4;
     static constexpr int NQ = 2 * ND;  // u, u - u_old - v dt
-    static constexpr int MINB = DIM == 3 ? 6 : 5;
+    static constexpr int MINB = DIM == 3 ? 6 : 10;  // 2D, two warps a block: 64 us against 66 with 5 blocks of four
     static constexpr int SXX = DIM, SXY = DIM + 1, SXZ = 5, SYY = DIM == 3 ? 6 : 4, SYZ = 7, SZZ = 8;
     CachedAsmArgs a;
     struct Bond {
@@ -633,11 +635,11 @@ cudaError_t launch_nodes(const El &el, const BlockPattern &bp, int mmax, cudaStr
 
 cudaError_t launch_stress_ch_block(const StressChAsmArgs &a, const BlockPattern &bp, int mmax, cudaStream_t s) {
     if (a.dim == 3) return launch_nodes<128, 1>(StressChEl<3>{a}, bp, mmax, s);
-    return launch_nodes<32, 2>(StressChEl<2>{a}, bp, mmax, s);
+    return launch_nodes<32, 1>(StressChEl<2>{a}, bp, mmax, s);
 }
 cudaError_t launch_cached_block(const CachedAsmArgs &a, const BlockPattern &bp, int mmax, cudaStream_t s) {
     if (a.dim == 3) return launch_nodes<128, 1>(CachedEl<3>{a}, bp, mmax, s);
-    return launch_nodes<32, 4>(CachedEl<2>{a}, bp, mmax, s);
+    return launch_nodes<32, 2>(CachedEl<2>{a}, bp, mmax, s);
 }
 cudaError_t launch_ch_block(const ChAsmArgs &a, const BlockPattern &bp, cudaStream_t s) {
     constexpr int LPN = 8;
