@@ -658,8 +658,9 @@ cudaError_t launch_sliced(const EpfArgs &a, const SlicedArgs &sl, cudaStream_t s
 
 // Sliced configurations (the autotuner picks): warps a slice, slices a block, rows in flight, minimum resident blocks.
 // Measured in a captured 50-step loop, FP64 / mixed us a step: the 44.2 M-bond slab 4,1,2,6 352 / 246, 4,1,3,4 359 / 278,
-// 4,1,1,8 356 / 269, 8,1,2,3 412 / 285; the 2.25 M-bond plate 4,1,2,8 16.1 / 13.6, 2,2,4,5 16.4 / 13.7, 2,2,2,8 16.9 /
-// 14.2, 1,4,2,8 23.5 / 20.3.  The last of each dimension, eight warps a slice, is for meshes of a few hundred slices.
+// 4,1,1,8 356 / 269, 8,1,2,3 412 / 285, 3,1,2,8 376 / 245, 5,1,2,4 362 / 285; the 2.25 M-bond plate 3,1,2,10 14.2 / 12.4,
+// 4,1,2,8 14.9 / 12.9, 2,2,4,5 15.2 / 13.0, 2,2,2,8 15.7 / 13.4, 5,1,2,6 15.1 / 13.1, 3,1,2,11 18.3 / 13.5, 1,2,4,10
+// 17.4 / 14.0.  The last of each dimension, eight warps a slice, is for meshes of a few hundred slices.
 template <int DIM, bool MIXED>
 cudaError_t launch_cfg(const EpfArgs &a, const SlicedArgs &sl, int which, cudaStream_t s) {
     if constexpr (DIM == 3) {
@@ -673,7 +674,7 @@ cudaError_t launch_cfg(const EpfArgs &a, const SlicedArgs &sl, int which, cudaSt
         switch (which) {
             case 0: return launch_sliced<2, MIXED, 4, 1, 2, 8>(a, sl, s);
             case 1: return launch_sliced<2, MIXED, 2, 2, 4, 5>(a, sl, s);
-            case 2: return launch_sliced<2, MIXED, 2, 2, 2, 8>(a, sl, s);
+            case 2: return launch_sliced<2, MIXED, 3, 1, 2, 10>(a, sl, s);
             default: return launch_sliced<2, MIXED, 8, 1, 2, 4>(a, sl, s);
         }
     }
