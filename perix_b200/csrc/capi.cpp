@@ -745,8 +745,7 @@ static double *adjoint_scratch(pxb_ctx *c, const ApplyArgs &a) {
     const size_t need = sizeof(double) * (size_t)c->g.nb;
     if (c->ops.bond.bytes != need && dev_alloc(c, c->ops.bond, need) != PXB_OK) return nullptr;
     if (!c->bond_ev && cudaEventCreateWithFlags(&c->bond_ev, cudaEventDisableTiming) != cudaSuccess) return nullptr;
-    if (c->bond_stream && c->bond_stream != c->stream && cudaStreamWaitEvent(c->stream, c->bond_ev, 0) != cudaSuccess)
-        return nullptr;
+    if (c->bond_used && cudaStreamWaitEvent(c->stream, c->bond_ev, 0) != cudaSuccess) return nullptr;
     return c->ops.bond.as<double>();
 }
 
@@ -792,7 +791,7 @@ extern "C" int pxb_apply_adjoint_d(pxb_ctx *c, const double *ybar_d, int nk, con
     if (bond) {
         c->launches++;
         PXB_CUDA_TRY(cudaEventRecord(c->bond_ev, c->stream));
-        c->bond_stream = c->stream;
+        c->bond_used = true;
     }
     return PXB_OK;
 }

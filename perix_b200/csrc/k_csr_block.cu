@@ -570,7 +570,8 @@ __global__ void __launch_bounds__(256) ch_block_kernel(ChAsmArgs a, BlockPattern
 }
 
 // ---- Poisson / diffusion (see assemble_scalar_kernel in k_csr.cu): one warp a node, one value a bond ---------------
-template <bool MIXED, int DIM>
+// (U bonds of a lane in flight)
+template <bool MIXED, int DIM, int U>
 __global__ void __launch_bounds__(128) scalar_block_kernel(ScalarAsmArgs a, BlockPattern bp) {
     using GT = typename std::conditional<MIXED, float, double>::type;
     const int lane = threadIdx.x & 31;
@@ -589,6 +590,7 @@ __global__ void __launch_bounds__(128) scalar_block_kernel(ScalarAsmArgs a, Bloc
     }
     const double coef = a.type == 0 ? a.coef : -a.coef;
     double rsum = 0.0, dsum = 0.0;
+#pragma unroll U
     for (int t = b0 + lane; t < b1; t += kWarp) {
         const int j = __ldg(a.nbr + t);
         const GT *g = static_cast<const GT *>(a.ops) + (size_t)t * a.nop;
@@ -649,16 +651,20 @@ cudaError_t launch_ch_block(const ChAsmArgs &a, const BlockPattern &bp, cudaStre
     else ch_block_kernel<LPN, false><<<grid, 256, 0, s>>>(a, bp);
     return cudaGetLastError();
 }
-cudaError_t launch_scalar_block(const ScalarAsmArgs &a, const BlockPattern &bp, cudaStream_t s) {
+template <bool MIXED, int DIM>
+static cudaError_t launch_scalar(const ScalarAsmArgs &a, const BlockPattern &bp, cudaStream_t s) {
     const int g = (a.n + 3) / 4;
-    if (a.dim == 3) {
-        if (a.mixed) scalar_block_kernel<true, 3><<<g, 128, 0, s>>>(a, bp);
-        else scalar_block_kernel<false, 3><<<g, 128, 0, s>>>(a, bp);
-    } else {
-        if (a.mixed) scalar_block_kernel<true, 2><<<g, 128, 0, s>>>(a, bp);
-        else scalar_block_kernel<false, 2><<<g, 128, 0, s>>>(a, bp);
-    }
+    // two bonds in flight where the blocks outnumber what the chip holds (16 an SM): 45,600 nodes in 3D FP64 78 -> 72 us,
+    // 157,000 mixed 183 -> 150, 151,600 in 2D 68 -> 61; below that the second bond only lengthens the one wave (64x64: 4.1
+    // us against 6.0)
+    if (g > 148 * 16) scalar_block_kernel<MIXED, DIM, 2><<<g, 128, 0, s>>>(a, bp);
+    else scalar_block_kernel<MIXED, DIM, 1><<<g, 128, 0, s>>>(a, bp);
     return cudaGetLastError();
+}
+
+cudaError_t launch_scalar_block(const ScalarAsmArgs &a, const BlockPattern &bp, cudaStream_t s) {
+    if (a.dim == 3) return a.mixed ? launch_scalar<true, 3>(a, bp, s) : launch_scalar<false, 3>(a, bp, s);
+    return a.mixed ? launch_scalar<true, 2>(a, bp, s) : launch_scalar<false, 2>(a, bp, s);
 }
 
 }  // namespace pxb

@@ -277,9 +277,9 @@ struct BatchState {
 struct pxb_ctx {
     int device = 0;
     pxb::DevPool pool;  // before the buffers, which go back to it
-    // last use of ops.bond: another stream's use waits for it
+    // last use of ops.bond: the next one waits for it, whatever its stream
     cudaEvent_t bond_ev = nullptr;
-    cudaStream_t bond_stream = nullptr;
+    bool bond_used = false;
     cudaEvent_t newton_ev[2] = {nullptr, nullptr};  // ends of the implicit run's queued Newton iterations
     size_t mem_limit = 0;  // device bytes the context may hold (0: no limit beyond the GPU's)
     int gbuild_schedule = -1;  // g-build: -1 by problem, 0 lane groups, 1 one warp per node, 2 the same with
