@@ -124,11 +124,13 @@ int timed_steps(pxb_ctx *c, int nsteps, size_t flush_bytes, int restore_every, c
     return PXB_OK;
 }
 
-// makes `variant` the context's schedule; a sliced one that cannot be built leaves the schedule as it was
+// makes `variant` the context's schedule; a sliced one that cannot be built leaves the schedule as it was.  What that
+// queues is waited for: the caller may put the context on another stream before the first step.
 int select_variant(pxb_ctx *c, int variant) {
     const int before = c->epf.variant;
     c->epf.variant = variant;
-    const int st = epf_ready(c);
+    int st = epf_ready(c);
+    if (st == PXB_OK && epf_is_sliced(variant)) st = sync(c);
     if (st != PXB_OK) c->epf.variant = before;
     return st;
 }
