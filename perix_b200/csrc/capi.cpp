@@ -966,13 +966,12 @@ int epf_ready(pxb_ctx *c) {
     EpfState &e = c->epf;
     if (!runs_sliced(e)) return PXB_OK;
     if (!e.sl_ready) PXB_TRY(sliced_build(c));
-    if (!e.sl_P_stale && !e.sl_stale) return PXB_OK;
-    if (e.sl_P_stale) PXB_TRY(sliced_fill(c, e.P.p, nullptr, nullptr, e.sl_P.p));
-    if (e.sl_stale) PXB_TRY(sliced_health(c, nullptr, e.sl_word.as<int>()));
-    // (captured by a caller, these launches have not run: the next call queues them again)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    PXB_CUDA_TRY(cudaStreamIsCapturing(c->stream, &cap));
-    if (cap == cudaStreamCaptureStatusNone) e.sl_P_stale = e.sl_stale = false;
+    // A caller's capture always holds the refresh: health and constants may change between its replays.  (It has not run
+    // when this returns, so the flags stay as they are.)
+    const bool cap = capturing(c->stream);
+    if (e.sl_P_stale || cap) PXB_TRY(sliced_fill(c, e.P.p, nullptr, nullptr, e.sl_P.p));
+    if (e.sl_stale || cap) PXB_TRY(sliced_health(c, nullptr, e.sl_word.as<int>()));
+    if (!cap) e.sl_P_stale = e.sl_stale = false;
     return PXB_OK;
 }
 
@@ -1773,14 +1772,18 @@ extern "C" int pxb_epf_broken_count(pxb_ctx *c, long long *n_broken) {
 extern "C" int pxb_epf_force_frozen_d(pxb_ctx *c, const double *u_d, double *a_d) {
     PXB_TRY(need_epf(c, "pxb_epf_force_frozen"));
     if (!u_d || !a_d) return fail(PXB_ERR_INVALID, "pxb_epf_force_frozen: NULL buffer");
-    PXB_TRY(epf_ready(c));
+    EpfState &e = c->epf;
     EpfArgs a = epf_args(c);
     a.u = u_d;
     a.accel = a_d;
     a.damage = 0;
-    // (the sliced kernel reads 2D displacements as 16-byte pairs)
+    // The sliced kernel (FP64) reads 2D displacements as 16-byte pairs, and health from the slices' words; a captured call
+    // runs the lane-group kernel, which reads the health bytes as they are at the replay.
     const bool pairs = c->g.dim == 3 || (reinterpret_cast<uintptr_t>(u_d) & 15u) == 0;
-    const cudaError_t err = epf_launch(c, a, EPF_FORCE_FROZEN, pairs ? c->epf.variant : 1, c->stream);
+    const bool sliced = runs_sliced(e) && e.precision == PXB_FP64 && pairs && !capturing(c->stream);
+    if (sliced) PXB_TRY(epf_ready(c));
+    const int variant = epf_is_sliced(e.variant) && !sliced ? 1 : e.variant;
+    const cudaError_t err = epf_launch(c, a, EPF_FORCE_FROZEN, variant, c->stream);
     if (err != cudaSuccess) return cuda_fail(err, "epf force (frozen mask)");
     return check_launch(c, "epf force (frozen mask)");
 }

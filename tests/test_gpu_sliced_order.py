@@ -1,0 +1,90 @@
+"""The sliced schedules' copy of health and constants where a program changes streams, or captures, between the calls that
+write it and those that read it.  Each result is compared with the lane-group kernel (variant 1) on the same state, which
+reads the health bytes and the operators themselves.
+
+Tolerance: both kernels add the same bond forces in another order, at most (m + 8) eps sum |P| |e| / rho apart, m the family
+size; a wrong mask or coefficient moves an acceleration by whole bond forces."""
+import numpy as np
+import pytest
+
+import perix_b200 as px
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+H, RHO = 1e-3, 2440.0
+
+
+class Case:
+    def __init__(self, dim, shape):
+        self.torch = pytest.importorskip("torch")
+        rng = np.random.default_rng(sum(shape))
+        q = np.indices(shape).reshape(dim, -1)[::-1].T.astype(np.float64)
+        x = np.zeros((len(q), 3))
+        x[:, :dim] = (q + 0.5 + rng.uniform(-0.2, 0.2, q.shape)) * H
+        off, ids = px.families(x, 3.015 * H, dim == 3)
+        self.C = px.elastic_constants(dim, False, 72e9, 0.22)
+        self.nb, self.dim, self.n = int(off[-1]), dim, len(x)
+        self.masks = [(rng.uniform(size=self.nb) > f).astype(np.uint8) for f in (0.1, 0.6)]
+        self.u = self.torch.tensor((rng.standard_normal(len(x) * dim) * 4e-6), device="cuda")
+        self.ctxs = []
+        for variant in (1, 17):
+            c = px.Context(0)
+            c.set_geometry(x, np.full(len(x), H ** dim), off, ids, 3.015 * H, H, dim)
+            c.epf_setup(*self.C, RHO, sc=4e-3, tension_only=True, health0=self.masks[0])
+            c.epf_set_bcs([])
+            c.epf_set_variant(variant)
+            self.ctxs.append(c)
+        c = self.ctxs[0]
+        c.gbuild(2, 0)
+        g = np.abs(c.get_ops())[:, dim:].sum(1)
+        i = np.repeat(np.arange(len(off) - 1), np.diff(off))
+        F = np.zeros(len(x))
+        np.add.at(F, i, 1.5 * (self.C[0] + self.C[1] + 2 * self.C[2]) * g * 2 * float(self.u.abs().max()))
+        self.tol = (int(np.diff(off).max()) + 8) * EPS * F.max() / RHO
+        self.torch.cuda.synchronize()
+
+    def state(self, c, mask):
+        z = np.zeros(self.n * self.dim)
+        c.epf_set_state(z, z, self.masks[mask], 0.0)
+
+    def force(self, c, out=None):
+        a = self.torch.empty_like(self.u) if out is None else out
+        c.epf_force_frozen_d(self.u.data_ptr(), a.data_ptr())
+        return a
+
+    def close_to(self, a, b):
+        assert float((a - b).abs().max()) <= self.tol
+
+    def reference(self, mask, scale=1.0):
+        c = self.ctxs[0]
+        self.state(c, mask)
+        c.epf_set_constants(*[scale * v for v in self.C], RHO)
+        a = self.force(c)
+        c.synchronize()
+        return a
+
+
+SHAPES = [(2, (23, 29)), (3, (7, 6, 9))]
+
+
+@pytest.mark.parametrize("dim,shape", SHAPES)
+def test_captured_force_follows_health(dim, shape):
+    k = Case(dim, shape)
+    torch, c = k.torch, k.ctxs[1]
+    ref = [k.reference(0), k.reference(1)]
+    assert float((ref[0] - ref[1]).abs().max()) > 1e6 * k.tol
+    k.force(c)
+    c.synchronize()
+    out = torch.empty_like(k.u)
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=s):
+        c.set_stream(s.cuda_stream)
+        k.force(c, out)
+    for mask in (1, 0, 1):
+        k.state(c, mask)
+        graph.replay()
+        torch.cuda.synchronize()
+        k.close_to(out, ref[mask])
+    k.state(c, 0)
+    k.close_to(k.force(c), ref[0])  # and uncaptured calls go on as before
+    c.set_stream(None)
