@@ -336,6 +336,7 @@ extern "C" int pxb_ctx_destroy(pxb_ctx *c) {
     drop_snapshot(c);
     destroy_graphs(c->epf);
     if (c->bond_ev) cudaEventDestroy(c->bond_ev);
+    if (c->epf_ev) cudaEventDestroy(c->epf_ev);
     for (cudaEvent_t e : c->newton_ev)
         if (e) cudaEventDestroy(e);
     if (c->own) cudaStreamDestroy(c->own);
@@ -962,8 +963,32 @@ SlicedArgs sliced_args(const EpfState &e) {
 
 }  // namespace
 
+// The context stream goes on after the asynchronous explicit calls queued so far (see pxb_ctx::epf_ev), which costs
+// nothing on the stream they are on; epf_mark ends such a call.  Neither has a place in a caller's capture.
+static int epf_order(pxb_ctx *c) {
+    if (!c->epf_queued || capturing(c->stream)) return PXB_OK;
+    const cudaError_t q = cudaEventQuery(c->epf_ev);
+    if (q == cudaSuccess) {
+        c->epf_queued = false;
+        return PXB_OK;
+    }
+    if (q != cudaErrorNotReady) return cuda_fail(q, "explicit calls in flight");
+    cudaGetLastError();
+    PXB_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->epf_ev, 0));
+    return PXB_OK;
+}
+
+static int epf_mark(pxb_ctx *c) {
+    if (capturing(c->stream)) return PXB_OK;
+    if (!c->epf_ev) PXB_CUDA_TRY(cudaEventCreateWithFlags(&c->epf_ev, cudaEventDisableTiming));
+    PXB_CUDA_TRY(cudaEventRecord(c->epf_ev, c->stream));
+    c->epf_queued = true;
+    return PXB_OK;
+}
+
 int epf_ready(pxb_ctx *c) {
     EpfState &e = c->epf;
+    PXB_TRY(epf_order(c));
     if (!runs_sliced(e)) return PXB_OK;
     if (!e.sl_ready) PXB_TRY(sliced_build(c));
     // A caller's capture always holds the refresh: health and constants may change between its replays.  (It has not run
@@ -1785,7 +1810,8 @@ extern "C" int pxb_epf_force_frozen_d(pxb_ctx *c, const double *u_d, double *a_d
     const int variant = epf_is_sliced(e.variant) && !sliced ? 1 : e.variant;
     const cudaError_t err = epf_launch(c, a, EPF_FORCE_FROZEN, variant, c->stream);
     if (err != cudaSuccess) return cuda_fail(err, "epf force (frozen mask)");
-    return check_launch(c, "epf force (frozen mask)");
+    PXB_TRY(check_launch(c, "epf force (frozen mask)"));
+    return sliced ? epf_mark(c) : PXB_OK;
 }
 
 // s_c from the fracture energy (reference include/ElmtSystem/FractureCriterion.h:30-43): 3D 5 G0 / (6 E delta),
@@ -1826,6 +1852,7 @@ extern "C" int pxb_epf_set_constants(pxb_ctx *c, double C11, double C12, double 
     PXB_TRY(need_epf(c, "pxb_epf_set_constants"));
     if (!(rho > 0.0)) return fail(PXB_ERR_INVALID, "pxb_epf_set_constants: rho must be > 0");
     EpfState &e = c->epf;
+    PXB_TRY(epf_order(c));
     destroy_graphs(e);  // captured launches carry the old constants
     e.C11 = C11;
     e.C12 = C12;
@@ -1834,7 +1861,8 @@ extern "C" int pxb_epf_set_constants(pxb_ctx *c, double C11, double C12, double 
     e.sl_P_stale = true;
     PXB_CUDA_TRY(launch_navier_pack(e.G.p, e.P.p, (long long)c->g.ldb, c->g.dim, e.precision == PXB_MIXED, C11, C12,
                                     C66, c->stream));
-    return check_launch(c, "navier pack");
+    PXB_TRY(check_launch(c, "navier pack"));
+    return epf_mark(c);
 }
 
 extern "C" int pxb_epf_force_adjoint_d(pxb_ctx *c, const double *u_d, const double *abar_d, double *ubar_d,
@@ -2052,7 +2080,7 @@ extern "C" int pxb_epf_record_d(pxb_ctx *c, const double *u0_d, const double *v0
     e.rec_K = K;
     e.rec_all = all;
     e.rec_seg = all ? -1 : nseg - 1;
-    return PXB_OK;
+    return epf_mark(c);
 }
 
 extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, const double *ubar_Nm1_d,
@@ -2176,7 +2204,7 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
         PXB_TRY(check_launch(c, "dC collect"));
     }
     if (dC_d) PXB_TRY(d2d(dC_d, e.adj_dC.p, 3 * sizeof(double)));
-    return PXB_OK;
+    return epf_mark(c);
 }
 
 extern "C" int pxb_epf_adjoint_d(pxb_ctx *c, const double *u0_d, const double *v0_d, double dt, int nsteps,

@@ -280,6 +280,10 @@ struct pxb_ctx {
     // last use of ops.bond: the next one waits for it, whatever its stream
     cudaEvent_t bond_ev = nullptr;
     bool bond_used = false;
+    // end of what the explicit element's asynchronous calls (constants, frozen force, recording, reverse sweep) have queued:
+    // the next explicit call waits for it, whatever its stream, because they share the slices' words and coefficients
+    cudaEvent_t epf_ev = nullptr;
+    bool epf_queued = false;
     cudaEvent_t newton_ev[2] = {nullptr, nullptr};  // ends of the implicit run's queued Newton iterations
     size_t mem_limit = 0;  // device bytes the context may hold (0: no limit beyond the GPU's)
     int gbuild_schedule = -1;  // g-build: -1 by problem, 0 lane groups, 1 one warp per node, 2 the same with
@@ -316,7 +320,8 @@ size_t ctx_bytes(const pxb_ctx *c);
 int l2_flush(pxb_ctx *c, size_t bytes);  // writes `bytes` through the L2 on the context stream (0: nothing)
 // the explicit kernel of schedule `variant` (mode EpfMode) on stream s; a sliced variant must be ready (epf_ready)
 cudaError_t epf_launch(pxb_ctx *c, const EpfArgs &a, int mode, int variant, cudaStream_t s);
-// before launches of the current variant on the context stream: a sliced variant's streams built and up to date
+// before launches of the current variant on the context stream: in order after what other streams hold, a sliced variant's
+// streams built and up to date
 int epf_ready(pxb_ctx *c);
 int wait_failure(pxb_ctx *c, unsigned int werr, const char *what);  // report (and clear) a staged wait that ran out
 }  // namespace pxb

@@ -88,3 +88,74 @@ def test_captured_force_follows_health(dim, shape):
     k.state(c, 0)
     k.close_to(k.force(c), ref[0])  # and uncaptured calls go on as before
     c.set_stream(None)
+
+
+@pytest.mark.parametrize("dim,shape", SHAPES)
+def test_force_on_another_stream_waits_for_the_refresh(dim, shape):
+    """The words are refreshed by a call on one stream, late; a call on another stream needs them, and the constants that a
+    third one writes."""
+    k = Case(dim, shape)
+    torch, c = k.torch, k.ctxs[1]
+    ref = [k.reference(0), k.reference(1), k.reference(1, 1.5)]
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    outs = [torch.empty_like(k.u) for _ in range(5)]
+    torch.cuda.synchronize()
+    late = lambda s: torch.cuda._sleep(20_000_000)  # noqa: E731
+    k.force(c, outs[0])
+    c.synchronize()
+    k.close_to(outs[0], ref[0])
+    k.state(c, 1)
+    c.set_stream(a.cuda_stream)
+    with torch.cuda.stream(a):
+        late(a)
+    k.force(c, outs[1])  # refreshes the words, once the stream gets there
+    c.set_stream(b.cuda_stream)
+    k.force(c, outs[2])
+    c.set_stream(a.cuda_stream)
+    with torch.cuda.stream(a):
+        late(a)
+    c.epf_set_constants(*[1.5 * v for v in k.C], RHO)
+    c.set_stream(b.cuda_stream)
+    k.force(c, outs[3])
+    with torch.cuda.stream(b):
+        late(b)
+    k.force(c, outs[4])  # reads coefficients that the next call may write
+    c.set_stream(a.cuda_stream)
+    c.epf_set_constants(*k.C, RHO)
+    k.force(c, outs[0])
+    torch.cuda.synchronize()
+    for o, r in zip(outs, (ref[1], ref[1], ref[1], ref[2], ref[2])):
+        k.close_to(o, r)
+    c.set_stream(None)
+
+
+@pytest.mark.parametrize("dim,shape", SHAPES)
+def test_recording_and_sweep_on_changing_streams(dim, shape):
+    """Recordings and reverse sweeps on two streams in turn, the first of each pair late, give what one stream gives: the
+    same kernels on the same values, but for dC, whose blocks are added in any order."""
+    import ctypes as C
+    k = Case(dim, shape)
+    torch, c = k.torch, k.ctxs[1]
+    g = torch.randn_like(k.u)
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    s = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    dt = 0.4 * H / np.sqrt(k.C[0] / RHO)
+    got = []
+    for order in ((0, 0), (0, 1), (1, 0), (1, 1)):
+        uN, ub, vb = (torch.empty_like(k.u) for _ in range(3))
+        dC = torch.zeros(3, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        c.set_stream(s[order[0]].cuda_stream)
+        with torch.cuda.stream(s[order[0]]):
+            torch.cuda._sleep(20_000_000)
+        assert c.L.pxb_epf_record_d(c.h, p(k.u), None, C.c_double(dt), 6, 4, p(uN), None) == 0
+        c.set_stream(s[order[1]].cuda_stream)
+        assert c.L.pxb_epf_adjoint_recorded_d(c.h, p(g), None, p(ub), p(vb), p(dC)) == 0
+        torch.cuda.synchronize()
+        got.append((uN, ub, vb, dC))
+    for o in got[1:]:
+        for x, y in zip(o[:3], got[0]):
+            assert torch.equal(x, y)
+        assert float((o[3] - got[0][3]).abs().max()) <= 1e-9 * float(got[0][3].abs().max())
+    c.set_stream(None)
