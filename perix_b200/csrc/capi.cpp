@@ -7,6 +7,9 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+
+#include "host_range.h"
 #include "k_kernels.h"
 #include "pxb_context.h"
 #include "tune_internal.h"
@@ -1120,7 +1123,7 @@ static int rate_plan(pxb_ctx *c) {
     return PXB_OK;
 }
 
-// pinned: both host buffers page-locked (copies from pageable memory are staged synchronously, so chunking them
+// pinned: both host buffers page-locked from end to end (copies from pageable memory are staged synchronously, so chunking them
 // only adds per-chunk overhead)
 // The sliced kernels write the acceleration of page-locked buffers straight to the host, while they compute: a copy
 // after them would cost the bus time again.
@@ -1215,13 +1218,23 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
     return err;
 }
 
-static bool pinned_host(const void *p) {
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+// all of [p, p + bytes) is page-locked and in reach of the GPU
+static bool pinned_host(const void *p, size_t bytes) {
+    using GetAttributes = CUresult (*)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr);
+    static const GetAttributes get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            f = nullptr;
         cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeHost;
+        return reinterpret_cast<GetAttributes>(f);
+    }();
+    HostRange r;
+    CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[4] = {&r.type, &r.managed, &r.start, &r.size};
+    return get && get(4, what, to, (CUdeviceptr)reinterpret_cast<uintptr_t>(p)) == CUDA_SUCCESS && range_holds(r, p, bytes);
 }
 
 // Captures rate_ops for the current buffers on the context's own stream (never the legacy default stream); the
@@ -1266,13 +1279,15 @@ extern "C" int pxb_epf_rate(pxb_ctx *c, const double *u, double *accel, long lon
     e.rate_last_u = u;
     e.rate_last_a = accel;
     e.rate_last_variant = e.variant;
-    if (again && pinned_host(u) && pinned_host(accel)) {
+    const size_t bytes = sizeof(double) * (size_t)c->g.n * c->g.dim;
+    const bool pinned = pinned_host(u, bytes) && pinned_host(accel, bytes);
+    if (again && pinned) {
         if (!e.rate_graph || e.rate_u != u || e.rate_a != accel || e.rate_cur != e.cur || e.rate_variant != e.variant)
             PXB_TRY(capture_rate(c, u, accel));
         PXB_CUDA_TRY(cudaGraphLaunch(e.rate_graph, c->stream));
         c->launches++;
     } else {
-        const cudaError_t err = rate_ops(c, u, accel, c->stream, pinned_host(u) && pinned_host(accel));
+        const cudaError_t err = rate_ops(c, u, accel, c->stream, pinned);
         if (err != cudaSuccess) return cuda_fail(err, "epf rate");
         PXB_TRY(check_launch(c, "epf rate"));
     }
