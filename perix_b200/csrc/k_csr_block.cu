@@ -615,15 +615,22 @@ __global__ void __launch_bounds__(128) scalar_block_kernel(ScalarAsmArgs a, Bloc
 
 // ---- launchers ------------------------------------------------------------------------------------------------
 namespace {
+constexpr size_t kTileShared = 112 * 1024;  // of a block of several units
+
 // resident blocks: the grid is what the chip holds, at most one tile a unit
 template <int NT, int UPB, typename El>
 cudaError_t launch_nodes(const El &el, const BlockPattern &bp, int mmax, cudaStream_t s) {
     const size_t smem = sizeof(double) * (size_t)UPB * unit_doubles<El>(mmax);
     if constexpr (UPB > 1)  // long families: one unit's tile may need most of an SM's shared memory
-        if (smem > 112 * 1024) return launch_nodes<NT, 1>(el, bp, mmax, s);
+        if (smem > kTileShared) return launch_nodes<NT, 1>(el, bp, mmax, s);
     auto kernel = node_rows_kernel<El, NT, UPB>;
+    // The limit belongs to the kernel, which contexts in other threads launch too: always the most that this one may be
+    // launched with, so that no call lowers what another has set.
+    constexpr size_t longest = sizeof(double) * (size_t)UPB * unit_doubles<El>(kBlockMax);
+    constexpr size_t most = UPB > 1 && longest > kTileShared ? kTileShared : longest;
+    static_assert(most <= 227 * 1024, "shared memory of a block");
     cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     int dev = 0, sms = 148, res = 1;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
