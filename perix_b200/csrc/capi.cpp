@@ -46,30 +46,37 @@ void DevPool::trim() {
 }
 
 void DevPool::give(void *p, size_t cap) {
-    dirty = true;
+    if (foreign || cap > kMax) {
+        cudaFree(p);
+        return;
+    }
     size_t drop = 0;
     while (drop < idle.size() && bytes + cap > kMax) {
         cudaFree(idle[drop].p);
         bytes -= idle[drop++].cap;
     }
     idle.erase(idle.begin(), idle.begin() + (ptrdiff_t)drop);
-    if (cap > kMax) {
+    try {
+        idle.push_back({p, cap});
+    } catch (...) {  // (called from destructors)
         cudaFree(p);
         return;
     }
-    idle.push_back({p, cap});
+    dirty = true;
     bytes += cap;
 }
 
 // the tightest block that wastes at most a quarter of what is wanted (or 64 KB), NULL without one
-void *DevPool::take(size_t want, size_t *cap) {
+void *DevPool::take(size_t want, size_t *cap, cudaStream_t stream, cudaStream_t own) {
+    if (foreign) return nullptr;
     size_t best = idle.size();
     for (size_t k = 0; k < idle.size(); ++k)
         if (idle[k].cap >= want && idle[k].cap <= want + want / 4 + 65536 &&
             (best == idle.size() || idle[k].cap < idle[best].cap))
             best = k;
     if (best == idle.size()) return nullptr;
-    if (dirty && cudaDeviceSynchronize() != cudaSuccess) {
+    if (dirty && (cudaStreamSynchronize(stream) != cudaSuccess ||
+                  (own != stream && cudaStreamSynchronize(own) != cudaSuccess))) {
         cudaGetLastError();
         return nullptr;
     }
@@ -166,7 +173,7 @@ int pool_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
     if (b.p && b.bytes == bytes) return PXB_OK;
     if (bytes > 0 && !capturing(c->stream) && !over_limit(c, b, bytes, c->pool.bytes)) {
         b.release();
-        if (void *p = c->pool.take(bytes, &b.cap)) {
+        if (void *p = c->pool.take(bytes, &b.cap, c->stream, c->own)) {
             b.p = p;
             b.bytes = bytes;
             b.pool = &c->pool;
@@ -351,6 +358,7 @@ extern "C" int pxb_ctx_set_stream(pxb_ctx *c, void *stream) {
     if (!c) return fail(PXB_ERR_INVALID, "pxb_ctx_set_stream: NULL context");
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->own;
     if (s != c->stream) destroy_graphs(c->epf);
+    if (s != c->stream && c->stream != c->own) c->pool.foreign = true;
     c->stream = s;
     return PXB_OK;
 }
@@ -386,6 +394,10 @@ static int geometry_reset(pxb_ctx *c, int n, int dim, const int *neigh_off, int 
     c->ch = ChState{};
     Geometry &g = c->g;
     g = Geometry{};
+    if (c->pool.foreign) {  // what the stream left behind used is released
+        c->pool.trim();
+        c->pool.foreign = false;
+    }
     const long long nb = neigh_off[n];
     g.n = n;
     g.dim = dim;
