@@ -52,11 +52,13 @@ int pxb_ctx_destroy(pxb_ctx *ctx);
  * To share the legacy default stream (torch's default stream, handle 0) pass cudaStreamLegacy ((void*)1). */
 int pxb_ctx_set_stream(pxb_ctx *ctx, void *stream);
 int pxb_ctx_synchronize(pxb_ctx *ctx);
-/* Device bytes in use by the context (idle blocks that its next set-up may take again, at most 1 GiB, not counted). */
+/* Device bytes in use by the context.  Idle blocks that its next set-up may take again (at most 1 GiB) are not counted;
+ * pxb_ctx_set_memory_limit, with any limit, gives them back to the GPU. */
 int pxb_ctx_device_bytes(pxb_ctx *ctx, size_t *bytes);
 /* Caps the device bytes the context may hold (0 = no cap beyond the GPU's own memory), e.g. to share a GPU with
  * other work: an allocation past the cap fails with PXB_ERR_OOM before reaching the driver, like one the driver
- * refuses (cudaErrorMemoryAllocation is also reported as PXB_ERR_OOM).  No counterpart in the reference. */
+ * refuses (cudaErrorMemoryAllocation is also reported as PXB_ERR_OOM).  Every call gives the context's idle blocks back
+ * (cudaFree), also one that leaves the limit as it is.  No counterpart in the reference. */
 int pxb_ctx_set_memory_limit(pxb_ctx *ctx, size_t bytes);
 /* Kernel launches issued by this context since creation (graph replays count each captured launch). */
 int pxb_ctx_launch_count(pxb_ctx *ctx, long long *count);

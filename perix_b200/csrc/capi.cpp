@@ -66,12 +66,13 @@ void DevPool::give(void *p, size_t cap) {
     bytes += cap;
 }
 
-// the tightest block that wastes at most a quarter of what is wanted (or 64 KB), NULL without one
-void *DevPool::take(size_t want, size_t *cap, cudaStream_t stream, cudaStream_t own) {
+// the tightest block that wastes at most a quarter of what is wanted (or 64 KB; exact: nothing), NULL without one
+void *DevPool::take(size_t want, size_t *cap, bool exact, cudaStream_t stream, cudaStream_t own) {
     if (foreign) return nullptr;
+    const size_t most = exact ? want : want + want / 4 + 65536;
     size_t best = idle.size();
     for (size_t k = 0; k < idle.size(); ++k)
-        if (idle[k].cap >= want && idle[k].cap <= want + want / 4 + 65536 &&
+        if (idle[k].cap >= want && idle[k].cap <= most &&
             (best == idle.size() || idle[k].cap < idle[best].cap))
             best = k;
     if (best == idle.size()) return nullptr;
@@ -146,7 +147,7 @@ static bool capturing(cudaStream_t s) {
 }
 
 static bool over_limit(const pxb_ctx *c, const DevBuf &b, size_t bytes, size_t idle) {
-    return c && c->mem_limit && bytes > b.bytes && ctx_bytes(c) - b.bytes + bytes + idle > c->mem_limit;
+    return c && c->mem_limit && bytes > b.cap && ctx_bytes(c) - b.cap + bytes + idle > c->mem_limit;
 }
 
 int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
@@ -173,7 +174,8 @@ int pool_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
     if (b.p && b.bytes == bytes) return PXB_OK;
     if (bytes > 0 && !capturing(c->stream) && !over_limit(c, b, bytes, c->pool.bytes)) {
         b.release();
-        if (void *p = c->pool.take(bytes, &b.cap, c->stream, c->own)) {
+        // (under a limit nothing is held beyond what was asked for, so that what fits without the pool fits with it)
+        if (void *p = c->pool.take(bytes, &b.cap, c->mem_limit != 0, c->stream, c->own)) {
             b.p = p;
             b.bytes = bytes;
             b.pool = &c->pool;
@@ -227,7 +229,7 @@ int wait_failure(pxb_ctx *c, unsigned int werr, const char *what) {
     return fail(PXB_ERR_CUDA, std::string(what) + ": a staged-copy wait ran out (" + std::to_string(werr) + " blocks)");
 }
 
-static size_t bufsz(const DevBuf &b) { return b.bytes; }
+static size_t bufsz(const DevBuf &b) { return b.cap; }
 
 size_t ctx_bytes(const pxb_ctx *c) {
     size_t s = 0;
@@ -1768,7 +1770,7 @@ extern "C" int pxb_epf_advance_to(pxb_ctx *c, double t_end, int chunk, int *bad_
 extern "C" int pxb_ctx_set_memory_limit(pxb_ctx *c, size_t bytes) {
     if (!c) return fail(PXB_ERR_INVALID, "pxb_ctx_set_memory_limit: NULL context");
     c->mem_limit = bytes;
-    if (bytes && ctx_bytes(c) + c->pool.bytes > bytes) c->pool.trim();
+    c->pool.trim();
     return PXB_OK;
 }
 

@@ -34,11 +34,11 @@ int cuda_fail(cudaError_t e, const char *what);
 // ---- device buffer ---------------------------------------------------------------------------------------------
 // Device blocks that a context's setup has released (families, geometry, operators, pattern) and its next setup takes
 // again: cudaMalloc and cudaFree of the thirty buffers cost more than the kernels between them.  Bounded (kMax, the
-// oldest go first) and given back when memory or the context's limit runs short and with the context.  A block that was
-// given back may still be in use on the context's streams: the first take after a give waits for them, and for nothing
-// else of the device (a wait for the whole device would break a capture that another thread has under way).  A caller's
-// stream that the context has left cannot be waited for (it may be gone): while its work may use a block (`foreign`,
-// until the next geometry has released them all), blocks go to cudaFree and none is taken.
+// oldest go first) and given back when memory or the context's limit runs short, when a limit is set or lifted, and with
+// the context.  A block that was given back may still be in use on the context's streams: the first take after a give
+// waits for them, and for nothing else of the device (a wait for the whole device would break a capture that another
+// thread has under way).  A caller's stream that the context has left cannot be waited for (it may be gone): while its
+// work may use a block (`foreign`, until the next geometry has released them all), blocks go to cudaFree and none is taken.
 struct DevPool {
     static constexpr size_t kMax = size_t(1) << 30;
     struct Block {
@@ -49,7 +49,7 @@ struct DevPool {
     size_t bytes = 0;
     bool dirty = false, foreign = false;
     void give(void *p, size_t cap);
-    void *take(size_t want, size_t *cap, cudaStream_t stream, cudaStream_t own);
+    void *take(size_t want, size_t *cap, bool exact, cudaStream_t stream, cudaStream_t own);
     void trim();
     DevPool() = default;
     DevPool(const DevPool &) = delete;
