@@ -305,9 +305,10 @@ int pxb_epf_restore(pxb_ctx *ctx);
 /* Schedule variants of the explicit kernel: 0-2 lane groups (lanes per node x bonds per lane per pass), 3-4
  * CSR-stream tiles, 5-16 TMA-staged tiles, 17-20 sliced (time step and rate call, in FP64 the start and the frozen
  * force too; the other modes of a staged or sliced variant run variant 1).
- * A sliced variant keeps a second, neighbour-sorted copy of the bond streams (about
- * 54 bytes a bond in 3D FP64, 30 mixed), built when it is first selected; without room for it pxb_epf_set_variant
- * fails with PXB_ERR_OOM and the autotuners skip it.  pxb_epf_variant_count() gives their number.  pxb_epf_autotune
+ * A sliced variant has a second, neighbour-sorted copy of the bond streams (54 bytes a bond and some padding in 3D FP64,
+ * 30 mixed), built when it is selected and held while it is current; without room for it pxb_epf_set_variant fails with
+ * PXB_ERR_OOM and the autotuners skip it.  Where a later allocation has no room beside it, the copy is given up and the
+ * last other schedule that was selected (the autotuner: its fastest other) takes over; pxb_epf_get_variant tells.  pxb_epf_variant_count() gives their number.  pxb_epf_autotune
  * times every variant that fits for `steps` steps from a private copy of the current state (L2 flushed before each
  * step), restores the state, selects the fastest and caches the choice per problem signature (dim, precision, nodes,
  * bonds, largest family); where the streams fit in the L2, the schedules within a tenth of the fastest are timed in a

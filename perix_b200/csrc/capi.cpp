@@ -126,7 +126,8 @@ static int malloc_dev(void **p, size_t bytes) {
 }
 
 // What the context can do without gives way to buffer b: the implicit run's slices and the field transpose's scratch
-// (both are built again by a use that finds the memory); true when anything was there.
+// (both are built again by a use that finds the memory), then, for a buffer that has to be there, the sliced step's
+// streams (another schedule takes over).  True when anything was there.
 static bool drop_optional(pxb_ctx *c, const DevBuf &b) {
     CsrState &k = c->csr;
     const bool any = (c->ops.bond.p && &b != &c->ops.bond) || (k.sl_pair.p && &b != &k.sl_pair && &b != &k.sl_col);
@@ -136,6 +137,18 @@ static bool drop_optional(pxb_ctx *c, const DevBuf &b) {
         k.sl_col.release();
     }
     return any;
+}
+
+static bool drop_step_slices(pxb_ctx *c, const DevBuf &b) {
+    EpfState &e = c->epf;
+    const CsrState &k = c->csr;
+    const DevBuf *without[] = {&c->ops.bond, &k.sl_row0, &k.sl_col, &k.sl_pair, &e.sl_row0, &e.sl_src, &e.sl_word, &e.sl_P,
+                               &e.sl_aword, &e.sl_GR, &e.adj_GR, &e.adj_HR, &e.adj_SG, &e.adj_UW};
+    for (const DevBuf *w : without)
+        if (&b == w) return false;
+    if (!e.sl_word.p) return false;
+    epf_drop_slices(c);
+    return true;
 }
 
 // under stream capture, or not to be told
@@ -154,6 +167,7 @@ int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
     if (b.p && b.bytes == bytes) return PXB_OK;
     if (c && over_limit(c, b, bytes, c->pool.bytes)) c->pool.trim();
     if (c && over_limit(c, b, bytes, 0)) drop_optional(c, b);
+    if (c && over_limit(c, b, bytes, 0)) drop_step_slices(c, b);
     if (over_limit(c, b, bytes, 0))
         return fail(PXB_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes would exceed the context's " +
                                      std::to_string(c->mem_limit) + "-byte limit (pxb_ctx_set_memory_limit)");
@@ -165,6 +179,7 @@ int dev_alloc(pxb_ctx *c, DevBuf &b, size_t bytes) {
         st = malloc_dev(&b.p, bytes);
     }
     if (st == PXB_ERR_OOM && c && drop_optional(c, b)) st = malloc_dev(&b.p, bytes);
+    if (st == PXB_ERR_OOM && c && drop_step_slices(c, b)) st = malloc_dev(&b.p, bytes);
     PXB_TRY(st);
     b.bytes = b.cap = bytes;
     return PXB_OK;
@@ -957,6 +972,22 @@ int sliced_build(pxb_ctx *c) {
     e.sl_stale = true;
     return PXB_OK;
 }
+
+}  // namespace
+
+void epf_drop_slices(pxb_ctx *c) {
+    EpfState &e = c->epf;
+    if (epf_is_sliced(e.variant)) e.variant = e.plain;
+    e.sl_ready = false;
+    if (e.sl_word.p) destroy_graphs(e);  // (captured sliced steps hold the streams' addresses)
+    e.sl_word.release();
+    e.sl_P.release();
+    if (e.sl_GR.p) return;  // the reverse sweep's streams are laid out alike
+    e.sl_src.release();
+    e.sl_row0.release();
+}
+
+namespace {
 
 int sliced_health(pxb_ctx *c, const int *rev, int *word) {
     EpfState &e = c->epf;

@@ -221,6 +221,7 @@ struct EpfState {
     std::map<GraphKey, cudaGraphExec_t> graphs;
     int graph_chunk = 0;
     int variant = 1;   // schedule variant of the explicit kernel (set by the autotuner or pxb_epf_set_variant)
+    int plain = 1;     // the variant that takes over where a sliced one has to give up its streams: the last other one
     bool evict_first = false;  // the step's bond streams exceed the L2: stage them with an evict-first policy
     int wait_tries = -1;       // staged kernels' consumer waits: try_wait calls allowed (-1: the default bound)
 };
@@ -326,5 +327,7 @@ cudaError_t epf_launch(pxb_ctx *c, const EpfArgs &a, int mode, int variant, cuda
 // before launches of the current variant on the context stream: in order after what other streams hold, a sliced variant's
 // streams built and up to date
 int epf_ready(pxb_ctx *c);
+// frees the sliced step's streams; a sliced variant gives way to EpfState::plain
+void epf_drop_slices(pxb_ctx *c);
 int wait_failure(pxb_ctx *c, unsigned int werr, const char *what);  // report (and clear) a staged wait that ran out
 }  // namespace pxb

@@ -135,6 +135,15 @@ int select_variant(pxb_ctx *c, int variant) {
     return st;
 }
 
+// select_variant to stay: another schedule than a sliced one keeps no slices (`plain`: the best of those, for later)
+int settle_variant(pxb_ctx *c, int variant, int plain) {
+    EpfState &e = c->epf;
+    e.plain = plain;
+    const int st = select_variant(c, variant);
+    if ((st != PXB_OK || !epf_is_sliced(variant)) && !epf_is_sliced(e.variant)) epf_drop_slices(c);
+    return st;
+}
+
 // milliseconds of a captured run of kLoopSteps steps of the current schedule from `from` (the better of two)
 constexpr int kLoopSteps = 24;
 int loop_time(pxb_ctx *c, const Snapshot &from, float *ms) {
@@ -155,8 +164,11 @@ int loop_time(pxb_ctx *c, const Snapshot &from, float *ms) {
     return PXB_OK;
 }
 
-// process-wide cache of autotuned schedule choices, keyed by problem signature
-std::map<std::string, int> g_tuned;
+// process-wide cache of autotuned schedule choices (the fastest, the fastest without slices), keyed by problem signature
+struct Choice {
+    int variant, plain;
+};
+std::map<std::string, Choice> g_tuned;
 
 std::string signature(const pxb_ctx *c) {
     return std::to_string(c->g.dim) + ":" + std::to_string(c->epf.precision) + ":" + std::to_string(c->g.n) + ":" +
@@ -198,7 +210,7 @@ extern "C" int pxb_epf_set_variant(pxb_ctx *c, int variant) {
     if (variant < 0 || variant >= kEpfVariants) return fail(PXB_ERR_INVALID, "pxb_epf_set_variant: no such variant");
     if (!epf_variant_fits(c->g.dim, variant, c->g.max_family))
         return fail(PXB_ERR_UNSUPPORTED, "pxb_epf_set_variant: families too large for this tile size");
-    return select_variant(c, variant);
+    return settle_variant(c, variant, epf_is_sliced(variant) ? c->epf.plain : variant);
 }
 
 extern "C" int pxb_epf_variant_count(void) { return kEpfVariants; }
@@ -218,15 +230,15 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
     if (steps <= 0) return fail(PXB_ERR_INVALID, "pxb_epf_autotune: steps must be > 0");
     const std::string key = signature(c);
     auto hit = g_tuned.find(key);
-    if (use_cache && hit != g_tuned.end() && select_variant(c, hit->second) == PXB_OK) {
-        if (best) *best = hit->second;
+    if (use_cache && hit != g_tuned.end() && settle_variant(c, hit->second.variant, hit->second.plain) == PXB_OK) {
+        if (best) *best = hit->second.variant;
         return PXB_OK;
     }
     Snapshot keep;
     PXB_TRY(save_state(c, keep));
     std::vector<float> ms((size_t)std::max(steps, 2)), step_ms(kEpfVariants, 1e30f);
-    float best_ms = 1e30f;
-    int best_v = c->epf.variant;
+    float best_ms = 1e30f, plain_ms = 1e30f;
+    int best_v = c->epf.variant, plain_v = c->epf.plain;
     for (int v = 0; v < kEpfVariants; ++v) {
         if (!epf_variant_fits(c->g.dim, v, c->g.max_family)) {
             if (ms_per_variant) ms_per_variant[v] = -1.f;
@@ -241,6 +253,10 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
         PXB_TRY(timed_steps(c, 2, 0, 0, nullptr, ms.data()));
         PXB_TRY(load_state(c, keep));
         PXB_TRY(timed_steps(c, steps, flush_bytes, 0, nullptr, ms.data()));
+        if (c->epf.variant != v) {  // its streams gave way to the flush buffer
+            if (ms_per_variant) ms_per_variant[v] = -1.f;
+            continue;
+        }
         float mean = 0.f;
         for (int k = 0; k < steps; ++k) mean += ms[(size_t)k];
         mean /= (float)steps;
@@ -248,6 +264,7 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
         std::nth_element(ms.begin(), ms.begin() + steps / 2, ms.begin() + steps);
         step_ms[(size_t)v] = ms[(size_t)(steps / 2)];  // the median decides: one late step must not
         if (step_ms[(size_t)v] < best_ms) { best_ms = step_ms[(size_t)v]; best_v = v; }
+        if (!epf_is_sliced(v) && step_ms[(size_t)v] < plain_ms) { plain_ms = step_ms[(size_t)v]; plain_v = v; }
     }
     // Streams that stay in L2 from one step to the next: a run's captured steps are faster than the flushed ones timed
     // above, and not by the same factor for every schedule (the 2.25 M-bond plate, mixed: 24.5 and 25.3 us flushed, 13.6
@@ -263,14 +280,11 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
     }
     PXB_TRY(load_state(c, keep));
     PXB_TRY(sync(c));
-    c->epf.variant = best_v;
-    g_tuned[key] = best_v;
+    if (settle_variant(c, best_v, plain_v) != PXB_OK) PXB_TRY(settle_variant(c, best_v = plain_v, plain_v));
+    g_tuned[key] = {best_v, plain_v};
     if (best) *best = best_v;
     return PXB_OK;
 }
-
-
-
 
 // Times the per-step rate call's kernel (RATE epilogue: damage, force, acceleration out) of every schedule variant
 // that fits, at the caller's displacement u (host, n*dim), reps launches each after one untimed launch; the bond
@@ -283,8 +297,8 @@ extern "C" int pxb_epf_autotune_rate(pxb_ctx *c, const double *u, int reps, int 
     EpfState &e = c->epf;
     const std::string key = signature(c) + ":rate";
     auto hit = g_tuned.find(key);
-    if (use_cache && hit != g_tuned.end() && select_variant(c, hit->second) == PXB_OK) {
-        if (best) *best = hit->second;
+    if (use_cache && hit != g_tuned.end() && settle_variant(c, hit->second.variant, hit->second.plain) == PXB_OK) {
+        if (best) *best = hit->second.variant;
         return PXB_OK;
     }
     DevBuf health, counters;
@@ -302,8 +316,8 @@ extern "C" int pxb_epf_autotune_rate(pxb_ctx *c, const double *u, int reps, int 
     Events ev;
     PXB_TRY(ev.make(2 * (size_t)reps));
     const int keep = e.variant;
-    float best_ms = 1e30f;
-    int best_v = keep;
+    float best_ms = 1e30f, plain_ms = 1e30f;
+    int best_v = keep, plain_v = e.plain;
     for (int v = 0; v < kEpfVariants; ++v) {
         if (!epf_variant_fits(c->g.dim, v, c->g.max_family)) {
             if (ms_per_variant) ms_per_variant[v] = -1.f;
@@ -343,11 +357,12 @@ extern "C" int pxb_epf_autotune_rate(pxb_ctx *c, const double *u, int reps, int 
         mean /= (float)reps;
         if (ms_per_variant) ms_per_variant[v] = mean;
         if (mean < best_ms) { best_ms = mean; best_v = v; }
+        if (!epf_is_sliced(v) && mean < plain_ms) { plain_ms = mean; plain_v = v; }
     }
     PXB_TRY(restore());
     PXB_TRY(sync(c));
-    e.variant = best_v;
-    g_tuned[key] = best_v;
+    if (settle_variant(c, best_v, plain_v) != PXB_OK) PXB_TRY(settle_variant(c, best_v = plain_v, plain_v));
+    g_tuned[key] = {best_v, plain_v};
     if (best) *best = best_v;
     return PXB_OK;
 }
