@@ -22,7 +22,7 @@ namespace {
 struct Snapshot {
     DevBuf u0, u1, health;
     int cur = 0;
-    double t = 0.0;
+    double t = 0.0, dt_prev = 0.0;
     long long step = 0;
     bool valid = false;
 };
@@ -67,6 +67,7 @@ int save_state(pxb_ctx *c, Snapshot &s) {
     PXB_TRY(d2d(c, s.health.p, e.health.p, e.health.bytes));
     s.cur = e.cur;
     s.t = e.t;
+    s.dt_prev = e.dt_prev;  // the length of the step between u^{n-1} and u^n
     s.step = e.step;
     s.valid = true;
     return sync(c);
@@ -80,6 +81,7 @@ int load_state(pxb_ctx *c, const Snapshot &s) {
     e.sl_stale = true;
     e.cur = s.cur;
     e.t = s.t;
+    e.dt_prev = s.dt_prev;
     e.step = s.step;
     e.umax_hist.resize((size_t)std::min<long long>(s.step, (long long)e.umax_hist.size()));
     return PXB_OK;
