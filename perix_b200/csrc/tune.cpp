@@ -9,6 +9,7 @@
 #include "k_kernels.h"
 #include "pxb_context.h"
 #include "tune_internal.h"
+#include "tune_pick.h"
 
 namespace pxb {
 int step_args(pxb_ctx *c, int par, EpfArgs *out);
@@ -271,15 +272,11 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
     // Streams that stay in L2 from one step to the next: a run's captured steps are faster than the flushed ones timed
     // above, and not by the same factor for every schedule (the 2.25 M-bond plate, mixed: 24.5 and 25.3 us flushed, 13.6
     // and 16.1 us in the loop).  The schedules within a tenth of the best are timed in a loop too, and that decides.
-    if (!c->epf.evict_first && flush_bytes > 0) {
-        float loop_best = 1e30f;
-        for (int v = 0; v < kEpfVariants; ++v) {
-            float t = 0.f;
-            if (step_ms[(size_t)v] > 1.1f * best_ms || select_variant(c, v) != PXB_OK) continue;
-            if (loop_time(c, keep, &t) != PXB_OK) break;  // (a run that blows up within the loop: the flushed choice stands)
-            if (t < loop_best) { loop_best = t; best_v = v; }
-        }
-    }
+    if (!c->epf.evict_first && flush_bytes > 0 && best_ms < 1e30f)
+        best_v = pick_by_loop(step_ms, best_v, [&](int v, float *t) {
+            if (select_variant(c, v) != PXB_OK) return 0;
+            return loop_time(c, keep, t) == PXB_OK ? 1 : -1;  // (a run that blows up within the loop)
+        });
     PXB_TRY(load_state(c, keep));
     PXB_TRY(sync(c));
     if (settle_variant(c, best_v, plain_v) != PXB_OK) PXB_TRY(settle_variant(c, best_v = plain_v, plain_v));
