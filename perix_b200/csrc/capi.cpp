@@ -807,6 +807,8 @@ extern "C" int pxb_apply_adjoint_d(pxb_ctx *c, const double *ybar_d, int nk, con
             if (!have) p.ext[p.next++] = m;
         }
         if (p.next > 20) return fail(PXB_ERR_INVALID, "pxb_apply_adjoint: too many slots with the defect correction");
+        for (int q = 0; q < p.next; ++q)
+            if (p.ext[q] < p.dim && std::find(p.ext, p.ext + q, p.ext[q]) == p.ext + q) p.once |= 1u << q;
         const size_t need = sizeof(double) * (size_t)a.n * (size_t)p.next;
         if (c->ops.yeff.bytes < need) PXB_TRY(dev_alloc(c, c->ops.yeff, need));
         p.defect = a.defect;

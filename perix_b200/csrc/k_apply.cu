@@ -64,8 +64,9 @@ __global__ void __launch_bounds__(kApplyThreads) apply_kernel(ApplyArgs a) {
 
 // Transpose of the defect correction, ahead of the transpose scatter: the corrected forward is
 // D = G u - C (G1 u) with G1 the first-derivative rows, so ubar = G^T ybar' where ybar' equals ybar on the
-// requested slots and every first-derivative slot m additionally receives -sum_k C[k][m] ybar[k].  p.ext lists
-// the scatter's slots (the requested ones, then any first-derivative slot not requested); yeff is N x next.
+// requested slots and every first-derivative slot m additionally receives -sum_k C[k][m] ybar[k], once however often
+// it is requested.  p.ext lists the scatter's slots (the requested ones, then any first-derivative slot not requested);
+// yeff is N x next.
 __global__ void apply_adjoint_prep_kernel(AdjPrepArgs p) {
     const int nd = (p.nop - p.dim) * p.dim;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += gridDim.x * blockDim.x) {
@@ -77,7 +78,7 @@ __global__ void apply_adjoint_prep_kernel(AdjPrepArgs p) {
             const double yk = p.ybar[(size_t)i * p.nk + s];
             const float *dv = p.defect + (size_t)i * nd + (k - p.dim) * p.dim;
             for (int e = 0; e < p.next; ++e)
-                if (p.ext[e] < p.dim) y[e] -= (double)dv[p.ext[e]] * yk;
+                if (p.once >> e & 1u) y[e] -= (double)dv[p.ext[e]] * yk;
         }
     }
 }

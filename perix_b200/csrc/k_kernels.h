@@ -342,6 +342,7 @@ cudaError_t launch_rate_down(const unsigned long long *cnt, unsigned long long *
 struct AdjPrepArgs {
     int n = 0, dim = 2, nop = 0, nk = 0, next = 0;
     int slots[32], ext[32];
+    unsigned int once = 0;  // bit e: ext[e] is a first-derivative slot that no earlier entry names
     const float *defect = nullptr;
     const double *ybar = nullptr;
     double *yeff = nullptr;
