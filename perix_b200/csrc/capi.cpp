@@ -770,11 +770,11 @@ extern "C" int pxb_apply(pxb_ctx *c, const double *u, int nk, const int *slots, 
     return sync(c);
 }
 
-// Scratch of the two-pass transpose, or NULL for the one-pass kernel: where the operator row has no kernels of
-// its own, when the memory (limit) does not hold it, and under stream capture, whose graph would keep a pointer
-// to a buffer that the context may give up.
+// Scratch of the two-pass transpose, or NULL for the one-pass kernel: where that is the faster one or the operator row has
+// no kernels of its own, when the memory (limit) does not hold it, and under stream capture, whose graph would keep a
+// pointer to a buffer that the context may give up.
 static double *adjoint_scratch(pxb_ctx *c, const ApplyArgs &a) {
-    if (!apply_has_rows(a) || c->g.nb == 0 || capturing(c->stream)) return nullptr;
+    if (!apply_two_pass(a, c->g.nb) || capturing(c->stream)) return nullptr;
     const size_t need = sizeof(double) * (size_t)c->g.nb;
     if (c->ops.bond.bytes != need && dev_alloc(c, c->ops.bond, need) != PXB_OK) return nullptr;
     if (!c->bond_ev && cudaEventCreateWithFlags(&c->bond_ev, cudaEventDisableTiming) != cudaSuccess) return nullptr;

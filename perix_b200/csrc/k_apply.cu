@@ -89,8 +89,8 @@ cudaError_t launch_apply_adjoint_prep(const AdjPrepArgs &p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// One pass, no scratch: rows of other lengths, and every row where the scratch of the two passes below is not to be
-// had (memory, stream capture).
+// One pass, no scratch: rows of other lengths, small meshes (apply_two_pass), and every row where the scratch of the two
+// passes below is not to be had (memory, stream capture).
 template <bool MIXED>
 __global__ void __launch_bounds__(kApplyThreads) apply_adjoint_kernel(ApplyArgs a) {
     constexpr int WPB = kApplyThreads / kWarp;
@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(kApplyThreads) apply_rows_kernel(ApplyArgs a, 
 // Transpose in two passes.  The first streams the operators in their own order and keeps one scalar a bond,
 // s_t = sum_k g^k_t ybar_i^k (8 bytes), and the node's -sum_t s_t in out; the second adds the s of the reverse
 // bonds.  Gathering the reverse bonds' operator rows instead reads 72 bytes a bond a second time, out of order.
+// (apply_two_pass: the sizes where this pays.)
 // Same mesh: 197 + 61 us (1.19 and 0.17 GB) against 717 us for the gather of rows (apply_adjoint_kernel).
 template <bool MIXED, int NOP, int LPN>
 __global__ void __launch_bounds__(kApplyThreads) adjoint_bonds_kernel(ApplyArgs a, unsigned int used, double *bond) {
@@ -276,7 +277,21 @@ static bool with_rows(const ApplyArgs &a, bool mixed, F f) {
     }
 }
 
-bool apply_has_rows(const ApplyArgs &a) { return a.nop == 2 || a.nop == 3 || a.nop == 5 || a.nop == 9; }
+// The two passes are two launches and two event calls, and the first call on a mesh allocates their scratch (0.3-0.6 ms);
+// the one pass gathers reverse rows, which costs little while they stay in L2.  In 3D what it costs goes with the operators
+// asked for, in 2D hardly.  One pass against two, FP64, us a call among others:
+//   3D, nine operators   142 K bonds 14.4 / 14.4, 363 K 26.6 / 17.5, 1.3 M 69 / 35;   one operator 363 K 10.3 / 13.4,
+//   1.3 M 32.7 / 26.0, 3.2 M 67.7 / 60.9
+//   2D, five operators   106 K 8.3 / 12.3, 431 K 16.5 / 14.1, 1.7 M 67.6 / 31.1;      one operator 431 K 11.8 / 12.3,
+//   1.7 M 47.2 / 26.1
+// The lines below lie where a call saves 5 to 10 us, so that some tens of calls pay for the scratch.
+bool apply_two_pass(const ApplyArgs &a, long long nb) {
+    if (a.nop != 2 && a.nop != 3 && a.nop != 5 && a.nop != 9) return false;
+    if (a.dim == 2) return nb >= 800000;
+    ApplyArgs b = a;
+    b.defect = nullptr;
+    return nb * (2 + __builtin_popcount(used_ops(b))) >= 2900000;
+}
 
 cudaError_t launch_apply(const ApplyArgs &a, bool mixed, int grid, cudaStream_t s) {
     if (a.nk > kMaxK) return cudaErrorInvalidValue;
