@@ -86,7 +86,9 @@ def test_captured_force_follows_health(dim, shape):
         torch.cuda.synchronize()
         k.close_to(out, ref[mask])
     k.state(c, 0)
-    k.close_to(k.force(c), ref[0])  # and uncaptured calls go on as before
+    k.force(c, out)  # and uncaptured calls go on as before
+    c.synchronize()
+    k.close_to(out, ref[0])
     c.set_stream(None)
 
 
