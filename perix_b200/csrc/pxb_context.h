@@ -49,7 +49,7 @@ struct DevPool {
     size_t bytes = 0;
     bool dirty = false, foreign = false;
     void give(void *p, size_t cap);
-    void *take(size_t want, size_t *cap, bool exact, cudaStream_t stream, cudaStream_t own);
+    void *take(size_t want, size_t *cap, size_t slack, cudaStream_t stream, cudaStream_t own);
     void trim();
     DevPool() = default;
     DevPool(const DevPool &) = delete;
