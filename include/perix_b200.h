@@ -283,9 +283,10 @@ int pxb_epf_set_rate_chunks(pxb_ctx *ctx, int chunks);
  * tiles' ids, reverse health and node rows staged by bulk copies through a shared-memory ring (bounded waits: a wait that
  * runs out fails the sweep with PXB_ERR_CUDA) and each reverse bond's source node gathered as one interleaved (u, adjoint)
  * row, in three launch configurations (3D: 2, 1 or 3 reverse bonds a lane per pass at 16 lanes a node; 2D: 4, 4 or 8 lanes
- * a node); 5 (and -1, the default) the reverse-only sums on the slices of the sliced step, with a neighbour-sorted copy of
- * the reverse operators (without room for it: 4).  The reverse-only kernels apply when every bond has its reverse
- * (symmetric families); other meshes fall back to 0.  Results agree to rounding.  No counterpart in the reference. */
+ * a node); 5 the reverse-only sums on the slices of the sliced step, with a neighbour-sorted copy of the reverse operators
+ * (without room for it: 4); -1, the default, is 5, and 4 on 3D meshes of fewer than 4,736 nodes.  The reverse-only
+ * kernels apply when every bond has its reverse (symmetric families); other meshes fall back to 0.  Results agree to
+ * rounding.  No counterpart in the reference. */
 int pxb_epf_set_adjoint_schedule(pxb_ctx *ctx, int schedule);
 /* The reverse sweep of the last pxb_epf_record_d (PXB_ERR_STATE when there is none); arguments as pxb_epf_adjoint_d. */
 int pxb_epf_adjoint_recorded_d(pxb_ctx *ctx, const double *ubar_N_d, const double *ubar_Nm1_d, double *u0bar_d,

@@ -141,11 +141,11 @@ static bool drop_optional(pxb_ctx *c, const DevBuf &b) {
 static bool drop_step_slices(pxb_ctx *c, const DevBuf &b) {
     EpfState &e = c->epf;
     const CsrState &k = c->csr;
-    const DevBuf *without[] = {&c->ops.bond, &k.sl_row0, &k.sl_col, &k.sl_pair, &e.sl_row0, &e.sl_src, &e.sl_word, &e.sl_P,
-                               &e.sl_aword, &e.sl_GR, &e.adj_GR, &e.adj_HR, &e.adj_SG, &e.adj_UW};
+    const DevBuf *without[] = {&c->ops.bond, &k.sl_row0, &k.sl_col, &k.sl_pair, &e.sl_topo, &e.sl_step,
+                               &e.sl_rev,    &e.adj_GR,  &e.adj_HR, &e.adj_SG,  &e.adj_UW};
     for (const DevBuf *w : without)
         if (&b == w) return false;
-    if (!e.sl_word.p) return false;
+    if (!e.sl_step.p) return false;
     epf_drop_slices(c);
     return true;
 }
@@ -258,8 +258,8 @@ size_t ctx_bytes(const pxb_ctx *c) {
     s += bufsz(c->ops.ops) + bufsz(c->ops.degenerate) + bufsz(c->ops.defect) + bufsz(c->ops.yeff) + bufsz(c->ops.bond);
     const EpfState &e = c->epf;
     s += bufsz(e.G) + bufsz(e.P) + bufsz(e.xib) + bufsz(e.health) + bufsz(e.u[0]) + bufsz(e.u[1]) + bufsz(e.accel) + bufsz(e.counters) +
-         bufsz(e.umax) + bufsz(e.tsched) + bufsz(e.sc_bond) + bufsz(e.sl_row0) + bufsz(e.sl_word) + bufsz(e.sl_P) +
-         bufsz(e.sl_src) + bufsz(e.sl_GR) + bufsz(e.sl_aword);
+         bufsz(e.umax) + bufsz(e.tsched) + bufsz(e.sc_bond) + bufsz(e.sl_topo) + bufsz(e.sl_step) +
+         bufsz(e.sl_rev);
     s += bufsz(e.adj_ckpt) + bufsz(e.adj_seg) + bufsz(e.adj_p[0]) + bufsz(e.adj_p[1]) + bufsz(e.adj_A) + bufsz(e.adj_R) +
          bufsz(e.adj_W) + bufsz(e.adj_t) + bufsz(e.adj_dC) + bufsz(e.adj_umax) + bufsz(e.adj_GR) + bufsz(e.adj_HR) + bufsz(e.adj_u0) + bufsz(e.adj_SG) + bufsz(e.adj_UW);
     s += bufsz(e.bc.own) + bufsz(e.bc.src_off) + bufsz(e.bc.tgt) + bufsz(e.bc.comp) + bufsz(e.bc.form) +
@@ -690,8 +690,13 @@ extern "C" int pxb_gbuild_set_schedule(pxb_ctx *c, int schedule) {
     return PXB_OK;
 }
 
-// the recorded sweep's adjoint schedule asked for (-1: the sliced reverse-only kernel, schedule 5)
-static int adj_sched(const pxb_ctx *c) { return c->adj_schedule < 0 ? 5 : c->adj_schedule; }
+// The recorded sweep's adjoint schedule asked for.  -1: the sliced reverse-only kernel (5), and in 3D with less than a slice
+// of 32 nodes an SM the staged one (4), whose 16 lanes a node then fill the chip better.  A 10-step sweep, staged and sliced:
+// 3D 1,728 nodes 200 / 230 us, 4,096 242 / 229, 13,824 376 / 311; 2D 100 nodes 168 / 160, 90,000 476 / 385.
+static int adj_sched(const pxb_ctx *c) {
+    if (c->adj_schedule >= 0) return c->adj_schedule;
+    return c->g.dim == 3 && c->g.n < 32 * 148 ? 4 : 5;
+}
 
 extern "C" int pxb_epf_set_rate_chunks(pxb_ctx *c, int chunks) {
     if (!c) return fail(PXB_ERR_INVALID, "pxb_epf_set_rate_chunks: NULL context");
@@ -902,13 +907,18 @@ namespace {
 
 bool runs_sliced(const EpfState &e) { return epf_is_sliced(e.variant) && !e.sc_bond.p; }
 
-size_t sliced_entries(const EpfState &e) { return e.sl_src.bytes / sizeof(uint16_t); }
+size_t coef_bytes(const pxb_ctx *c) {
+    return (c->epf.precision == PXB_MIXED ? 4 : 8) * (c->g.dim == 3 ? 6 : 3) * c->epf.sl_entries;
+}
+uint16_t *slice_src(const EpfState &e) { return e.sl_topo.as<uint16_t>(); }
+int *slice_row0(const EpfState &e) { return reinterpret_cast<int *>(e.sl_topo.as<uint16_t>() + e.sl_entries); }
+int *slice_words(const pxb_ctx *c, const DevBuf &b) { return reinterpret_cast<int *>(b.as<char>() + coef_bytes(c)); }
 
 // slices, places in the families and length classes of the geometry
 int sliced_topology(pxb_ctx *c) {
     EpfState &e = c->epf;
     const Geometry &g = c->g;
-    if (e.sl_src.p) return PXB_OK;
+    if (e.sl_topo.p) return PXB_OK;
     const int n = g.n, slices = (n + 31) / 32;
     std::vector<int> row0((size_t)slices + 1, 0);
     for (int s = 0; s < slices; ++s) {
@@ -919,13 +929,9 @@ int sliced_topology(pxb_ctx *c) {
             return fail(PXB_ERR_UNSUPPORTED, "sliced step: more than 2^30 stream entries");
         row0[(size_t)s + 1] = row0[(size_t)s] + rows;
     }
-    const size_t entries = 32 * (size_t)std::max(1, row0.back());
-    PXB_TRY(dev_alloc(c, e.sl_src, sizeof(uint16_t) * entries));
-    const int st = dev_upload(c, e.sl_row0, row0.data(), sizeof(int) * row0.size());
-    if (st != PXB_OK) {
-        e.sl_src.release();
-        return st;
-    }
+    e.sl_entries = 32 * (size_t)std::max(1, row0.back());
+    PXB_TRY(dev_alloc(c, e.sl_topo, sizeof(uint16_t) * e.sl_entries + sizeof(int) * row0.size()));
+    PXB_TRY(h2d(c, slice_row0(e), row0.data(), sizeof(int) * row0.size()));
     int idbits = 1;
     while (idbits < 31 && (n - 1) >> idbits) ++idbits;
     const int qbits = std::min(7, 31 - idbits);
@@ -933,47 +939,41 @@ int sliced_topology(pxb_ctx *c) {
     e.sl_shift = 31 - qbits;
     unsigned long long *key = e.counters.as<unsigned long long>() + 5;  // the set-up's scratch counter
     PXB_CUDA_TRY(cudaMemsetAsync(key, 0, sizeof(*key), c->stream));
-    PXB_CUDA_TRY(launch_sliced_rank(n, g.dim, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, e.sl_row0.as<int>(),
-                                    e.sl_src.as<uint16_t>(), key, c->stream));
+    PXB_CUDA_TRY(launch_sliced_rank(n, g.dim, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, slice_row0(e), slice_src(e), key,
+                                    c->stream));
     c->launches++;
     unsigned long long k2 = 0;
     PXB_TRY(d2h(c, &k2, key, sizeof(k2)));
     PXB_TRY(sync(c));  // (row0 leaves scope here too)
     double r2 = 0.0;
     std::memcpy(&r2, &k2, sizeof(double));
-    e.sl_step = std::isfinite(r2) ? std::sqrt(r2) / (1 << qbits) : 0.0;
+    e.sl_step_len = std::isfinite(r2) ? std::sqrt(r2) / (1 << qbits) : 0.0;
     return PXB_OK;
 }
 
-// words and coefficients (bond-ordered source Pc; rev: the reverse bonds') of the slices; word NULL: coefficients only
-int sliced_fill(pxb_ctx *c, const void *Pc, const int *rev, int *word, void *P) {
+// words and coefficients (bond-ordered source Pc; rev: the reverse bonds') of the slices in `to`; words false:
+// coefficients only
+int sliced_fill(pxb_ctx *c, const void *Pc, const int *rev, const DevBuf &to, bool words) {
     EpfState &e = c->epf;
     const Geometry &g = c->g;
     PXB_CUDA_TRY(launch_sliced_fill(g.n, g.dim, e.precision == PXB_MIXED, g.off.as<int>(), g.nbr.as<int>(), g.pos.p,
-                                    e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(), e.sl_shift,
-                                    e.sl_step > 0.0 ? 1.0 / e.sl_step : 0.0, (1 << (31 - e.sl_shift)) - 1, Pc,
-                                    (long long)g.ldb, rev, word, P, c->stream));
+                                    slice_row0(e), slice_src(e), e.sl_shift,
+                                    e.sl_step_len > 0.0 ? 1.0 / e.sl_step_len : 0.0, (1 << (31 - e.sl_shift)) - 1, Pc,
+                                    (long long)g.ldb, rev, words ? slice_words(c, to) : nullptr, to.p, c->stream));
     c->launches++;
     return PXB_OK;
 }
 
-int sliced_alloc(pxb_ctx *c, DevBuf &word, DevBuf &P) {
-    const EpfState &e = c->epf;
-    const size_t entries = sliced_entries(e), nc = c->g.dim == 3 ? 6 : 3;
-    int st = dev_alloc(c, word, sizeof(int) * (entries + 32 * kSlicedSlack));
-    if (st == PXB_OK) st = dev_alloc(c, P, (e.precision == PXB_MIXED ? 4 : 8) * nc * entries);
-    if (st != PXB_OK) {
-        word.release();
-        P.release();
-    }
-    return st;
+// (one allocation for both streams: the first use of either pays for it)
+int sliced_alloc(pxb_ctx *c, DevBuf &b) {
+    return dev_alloc(c, b, coef_bytes(c) + sizeof(int) * (c->epf.sl_entries + 32 * kSlicedSlack));
 }
 
 int sliced_build(pxb_ctx *c) {
     EpfState &e = c->epf;
     PXB_TRY(sliced_topology(c));
-    PXB_TRY(sliced_alloc(c, e.sl_word, e.sl_P));
-    PXB_TRY(sliced_fill(c, e.P.p, nullptr, e.sl_word.as<int>(), e.sl_P.p));
+    PXB_TRY(sliced_alloc(c, e.sl_step));
+    PXB_TRY(sliced_fill(c, e.P.p, nullptr, e.sl_step, true));
     e.sl_ready = true;
     e.sl_P_stale = false;
     e.sl_stale = true;
@@ -986,33 +986,31 @@ void epf_drop_slices(pxb_ctx *c) {
     EpfState &e = c->epf;
     if (epf_is_sliced(e.variant)) e.variant = e.plain;
     e.sl_ready = false;
-    if (e.sl_word.p) destroy_graphs(e);  // (captured sliced steps hold the streams' addresses)
-    e.sl_word.release();
-    e.sl_P.release();
-    if (e.sl_GR.p) return;  // the reverse sweep's streams are laid out alike
-    e.sl_src.release();
-    e.sl_row0.release();
+    if (e.sl_step.p) destroy_graphs(e);  // (captured sliced steps hold the streams' addresses)
+    e.sl_step.release();
+    if (!e.sl_rev.p) e.sl_topo.release();  // (the reverse sweep's streams are laid out alike)
 }
 
 namespace {
 
 int sliced_health(pxb_ctx *c, const int *rev, int *word) {
     EpfState &e = c->epf;
-    PXB_CUDA_TRY(launch_sliced_health(c->g.n, c->g.off.as<int>(), e.sl_row0.as<int>(), e.sl_src.as<uint16_t>(),
+    PXB_CUDA_TRY(launch_sliced_health(c->g.n, c->g.off.as<int>(), slice_row0(e), slice_src(e),
                                       e.health.as<uint8_t>(), rev, word, c->stream));
     c->launches++;
     return PXB_OK;
 }
 
-SlicedArgs sliced_args(const EpfState &e) {
+SlicedArgs sliced_args(const pxb_ctx *c, const DevBuf &streams) {
+    const EpfState &e = c->epf;
     SlicedArgs s;
-    s.row0 = e.sl_row0.as<int>();
-    s.word = e.sl_word.as<int>();
-    s.P = e.sl_P.p;
-    s.src = e.sl_src.as<uint16_t>();
+    s.row0 = slice_row0(e);
+    s.word = slice_words(c, streams);
+    s.P = streams.p;
+    s.src = slice_src(e);
     s.shift = e.sl_shift;
     const double m = e.sc * (1.0 - 1.0e-6) - 1.0e-12;
-    s.clear = m > 0.0 ? m * m * e.sl_step * e.sl_step : 0.0;
+    s.clear = m > 0.0 ? m * m * e.sl_step_len * e.sl_step_len : 0.0;
     return s;
 }
 
@@ -1049,8 +1047,8 @@ int epf_ready(pxb_ctx *c) {
     // A caller's capture always holds the refresh: health and constants may change between its replays.  (It has not run
     // when this returns, so the flags stay as they are.)
     const bool cap = capturing(c->stream);
-    if (e.sl_P_stale || cap) PXB_TRY(sliced_fill(c, e.P.p, nullptr, nullptr, e.sl_P.p));
-    if (e.sl_stale || cap) PXB_TRY(sliced_health(c, nullptr, e.sl_word.as<int>()));
+    if (e.sl_P_stale || cap) PXB_TRY(sliced_fill(c, e.P.p, nullptr, e.sl_step, false));
+    if (e.sl_stale || cap) PXB_TRY(sliced_health(c, nullptr, slice_words(c, e.sl_step)));
     if (!cap) e.sl_P_stale = e.sl_stale = false;
     return PXB_OK;
 }
@@ -1065,7 +1063,7 @@ cudaError_t epf_launch(pxb_ctx *c, const EpfArgs &a, int mode, int variant, cuda
         EpfArgs r = a;
         r.rate = mode == EPF_STEP ? kEpfStep : mode == EPF_START ? kEpfStart : kEpfRate;
         if (mode == EPF_FORCE_FROZEN) r.damage = 0;
-        return launch_epf_sliced(r, sliced_args(e), c->g.dim, mixed, variant - 5 - kEpfTmaConfigs, s);
+        return launch_epf_sliced(r, sliced_args(c, e.sl_step), c->g.dim, mixed, variant - 5 - kEpfTmaConfigs, s);
     }
     if (a.damage && mode != EPF_FORCE_FROZEN) e.sl_stale = true;
     return launch_epf(a, c->g.dim, mixed, mode, variant, s);
@@ -2026,12 +2024,7 @@ int adj_kernel(pxb_ctx *c, const double *u, const double *w, double scale, doubl
         a.evict_first = e.evict_first ? 1 : 0;
         a.UW = uw;
         a.dC = e.adj_dC.as<double>() + 4;
-        SlicedArgs sl;
-        sl.row0 = e.sl_row0.as<int>();
-        sl.word = e.sl_aword.as<int>();
-        sl.P = e.sl_GR.p;
-        sl.shift = e.sl_shift;
-        const cudaError_t err = launch_adjoint_sliced(a, sl, c->g.dim, e.precision == PXB_MIXED, c->stream);
+        const cudaError_t err = launch_adjoint_sliced(a, sliced_args(c, e.sl_rev), c->g.dim, e.precision == PXB_MIXED, c->stream);
         if (err != cudaSuccess) return cuda_fail(err, "sliced adjoint step");
         return check_launch(c, "sliced adjoint step");
     }
@@ -2181,14 +2174,13 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
         sums = nmiss == 0;
     }
     if (sums && adj_sched(c) == 5) {  // the slices' reverse streams (without room for them: schedule 4)
-        bool built = e.sl_GR.p && e.sl_aword.p;
-        if (!built && c->g.max_family <= 0xffff && sliced_topology(c) == PXB_OK &&
-            sliced_alloc(c, e.sl_aword, e.sl_GR) == PXB_OK) {
-            PXB_TRY(sliced_fill(c, e.G.p, c->g.rev.as<int>(), e.sl_aword.as<int>(), e.sl_GR.p));
+        bool built = e.sl_rev.p;
+        if (!built && c->g.max_family <= 0xffff && sliced_topology(c) == PXB_OK && sliced_alloc(c, e.sl_rev) == PXB_OK) {
+            PXB_TRY(sliced_fill(c, e.G.p, c->g.rev.as<int>(), e.sl_rev, true));
             built = true;
         }
         if (built) {
-            PXB_TRY(sliced_health(c, c->g.rev.as<int>(), e.sl_aword.as<int>()));
+            PXB_TRY(sliced_health(c, c->g.rev.as<int>(), slice_words(c, e.sl_rev)));
             e.adj_sliced = e.adj_sg_on = true;
         }
     }

@@ -161,14 +161,16 @@ struct EpfState {
     DevBuf G;          // SoA Navier operators [c][ldb], double or float (c = 3 in 2D, 6 in 3D)
     DevBuf P;          // SoA packed Navier coefficients [c][ldb] (same type): the staged step kernels' stream
     DevBuf xib;        // mixed: FP32 reference bond vectors [dim][ldb] (the staged kernels' stretch pre-test)
-    // the sliced step's copy of the streams (k_epf_sliced.cu), built when a sliced variant is first selected: rows of
-    // the slices, words, coefficients, places in the family; sl_P_stale: the constants changed since they were filled,
-    // sl_stale: something other than a sliced launch may have written health since the words' broken bits were set
-    // sl_GR, sl_aword: the reverse sweep's (operators in reverse-bond order; words whose broken bits are the reverse bonds')
-    DevBuf sl_row0, sl_word, sl_P, sl_src, sl_GR, sl_aword;
+    // the sliced step's copy of the streams (k_epf_sliced.cu), held while a sliced variant is current: the bonds' places in
+    // the families, then the rows of the slices (sl_topo); coefficients, then words (sl_step); the reverse sweep's, laid out
+    // alike (sl_rev: operators in reverse-bond order, words whose broken bits are the reverse bonds').  sl_P_stale: the
+    // constants changed since the coefficients were filled, sl_stale: something other than a sliced launch may have written
+    // health since the words' broken bits were set
+    DevBuf sl_topo, sl_step, sl_rev;
+    size_t sl_entries = 0;
     bool sl_ready = false, sl_P_stale = false, sl_stale = true;
     int sl_shift = 31;
-    double sl_step = 0.0;
+    double sl_step_len = 0.0;  // of a length class
     DevBuf sc_bond;    // variable horizon: per-bond critical stretch s_c(0.5 (delta_i + delta_j)) [ldb]
     // explicit-loop adjoint (pxb_epf_adjoint_d): checkpoints, a segment's states, the two ping-pong states, the
     // adjoint vectors A (dJ/du^n), R (dJ/du^{n-1} carried), W (BC-transposed A), step times, dC accumulator
@@ -292,7 +294,7 @@ struct pxb_ctx {
     size_t mem_limit = 0;  // device bytes the context may hold (0: no limit beyond the GPU's)
     int gbuild_schedule = -1;  // g-build: -1 by problem, 0 lane groups, 1 one warp per node, 2 the same with
                                // its products on the FP64 tensor cores
-    int adj_schedule = -1;     // recorded reverse sweep: -1 default (5; 4 without room for its streams), 0 both operator
+    int adj_schedule = -1;     // recorded reverse sweep: -1 default (5, 4 on small 3D meshes; adj_sched), 0 both operator
                                // streams, 1 reverse-only, 2-4 reverse-only staged (bulk-copy ring) in three launch
                                // configurations, 5 reverse-only on the slices
     int rate_chunks = -1;      // pipelined rate call: -1 by mesh size, 1 off, 2..8 node chunks
