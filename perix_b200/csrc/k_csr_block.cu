@@ -11,7 +11,7 @@
 //   * the operator rows of a family are one contiguous span too, read coalesced into shared memory.
 // B200: 38,912 nodes in 3D with five unknowns (4.29 M bonds, 1.30 GB necessary) 783 us with slots -> 391 us; 81,200
 // nodes in 2D with two unknowns (2.25 M bonds, 171 MB) 96 -> 64 us.  What bounds both is the L1 data pipe (65 % of
-// its peak at 428 and 66 us: the values pass through shared memory once, with bank conflicts where a family's positions are not
+// its peak at 428 and 66 us, four nodes a tile in 2D: the values pass through shared memory once, with bank conflicts where a family's positions are not
 // consecutive), then DRAM latency (24-31 % occupancy there, limited by registers and the tile's shared memory; MINB below).
 #include <type_traits>
 
@@ -43,15 +43,15 @@ __device__ __forceinline__ void copy8_async(void *dst, const void *src) {
 __device__ __forceinline__ void copy_fence() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <int NT>
-__device__ __forceinline__ void unit_sync() {
+__device__ __forceinline__ void tile_sync() {
     if constexpr (NT == kWarp) __syncwarp();
     else __syncthreads();
 }
 
-// doubles of one unit's shared memory: the values of its nodes' rows, the bonds' residual terms, the operator rows,
-// the nodal words and values
+// doubles of a tile's shared memory: the values of its nodes' rows, the bonds' residual terms, the operator rows, the nodal
+// words and values
 template <typename El>
-__host__ __device__ constexpr int unit_doubles(int mmax) {
+__host__ __device__ constexpr int tile_doubles(int mmax) {
     return El::TN * (mmax * (El::ND * El::ND + El::ND + El::NOP) + El::NQ + 3) + 2;
 }
 
@@ -128,8 +128,12 @@ cudaError_t launch_block_map(const BlockMapArgs &a, cudaStream_t s) {
 }
 
 // ---- the assembly skeleton ---------------------------------------------------------------------------------------
-// A unit of NT threads (a warp in 2D, a block of four warps in 3D) takes TN consecutive nodes at a time: about 115
-// bonds, whose ids, operator rows and values are contiguous.  Per tile:
+// A block of NT threads (a warp in 2D, four warps in 3D) takes TN consecutive nodes at a time, two in 2D and one in 3D, whose
+// bonds' ids, operator rows and values are contiguous.  A long tile is a long chain for a mesh that does not fill the chip, a
+// short one has fewer bonds than threads.  2D with one, two and four nodes a tile, us a call (kernels with slots last):
+//   stress-CH         1,024 nodes 10.7 / 10.3 / 14.4 (10.3), 22,500 64 / 64 / 76 (113), 90,000 228 / 218 / 272 (425)
+//   dynamic fracture  1,024 nodes 6.2 / 6.2 / 8.2 (6.2), 22,500 24.6 / 18.5 / 20.5 (22.6), 90,000 109 / 69 / 72 (102)
+// Per tile:
 //   bonds     a bond a thread and pass: -K_IJ into the tile's rows in shared memory, the residual terms beside them;
 //   ahead     the next tile's bond words (registers), nodal values and operator rows (asynchronous copies) start out;
 //   nodes     one entry of a diagonal block or right-hand side a thread (SEG threads where there are enough): the sum
@@ -137,19 +141,19 @@ cudaError_t launch_block_map(const BlockMapArgs &a, cudaStream_t s) {
 //   store     the rows leave as one contiguous copy.
 // El: the element.  Bond: what a thread holds of a bond; nodal(): the NQ values of a node the bonds and the epilogue
 // read; bond(): -K_IJ at kb (row r at kb + r W) and the ND residual terms; diag() / rhs(): the entry from its sum.
-template <typename El, int NT, int UPB>
-__global__ void __launch_bounds__(NT * UPB, El::MINB) node_rows_kernel(El el, BlockPattern bp, int mmax) {
+template <typename El, int NT>
+__global__ void __launch_bounds__(NT, El::MINB) node_rows_kernel(El el, BlockPattern bp, int mmax) {
     constexpr int ND = El::ND, TN = El::TN, NQ = El::NQ, P = El::P, NE = ND * ND + ND, NOP = El::NOP;
     constexpr int SEG = NT / (TN * NE) >= 16 ? 16 : NT / (TN * NE) >= 8 ? 8 : NT / (TN * NE) >= 4 ? 4 : NT / (TN * NE) >= 2 ? 2 : 1;
     extern __shared__ __align__(16) double sm_blk[];
-    const int unit = threadIdx.x / NT, tid = threadIdx.x % NT;
-    double *rows = sm_blk + (size_t)unit * unit_doubles<El>(mmax);  // [values of the tile]
-    double *res = rows + TN * mmax * ND * ND;                       // [bond][ND]
-    double *ops = res + TN * mmax * ND;                             // [bond][NOP]
-    double *nq = ops + TN * mmax * NOP;                             // [node][NQ]
-    int *so = reinterpret_cast<int *>(nq + TN * NQ);                // bond offsets within the tile [TN + 1]
+    const int tid = threadIdx.x;
+    double *rows = sm_blk;                            // [values of the tile]
+    double *res = rows + TN * mmax * ND * ND;         // [bond][ND]
+    double *ops = res + TN * mmax * ND;               // [bond][NOP]
+    double *nq = ops + TN * mmax * NOP;               // [node][NQ]
+    int *so = reinterpret_cast<int *>(nq + TN * NQ);  // bond offsets within the tile [TN + 1]
     int *sw = so + TN + 1, *sp = sw + TN;                           // row length; own block | (mirror block + 1) << 8 | dead << 24
-    const int n = el.a.n, stride = gridDim.x * UPB, ntiles = (n + TN - 1) / TN;
+    const int n = el.a.n, stride = gridDim.x, ntiles = (n + TN - 1) / TN;
 
     // the tile being fetched: bond range, bond words, and (thread k < TN) the words of node k
     int f0 = 0, f1 = 0, flo = 0, fo = 0, fw = 0, fp = 0;
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(NT * UPB, El::MINB) node_rows_kernel(El el, Bl
         }
     };
 
-    int tile = blockIdx.x * UPB + unit;
+    int tile = blockIdx.x;
     int n0, n1;  // bond range of the tile after the one being fetched
     range(tile, n0, n1);
     fetch(tile, n0, n1);
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(NT * UPB, El::MINB) node_rows_kernel(El el, Bl
     for (; tile < ntiles; tile += stride) {
         const int b0 = f0, nb = f1 - f0, i0 = tile * TN;
         const size_t lo = flo;
-        unit_sync<NT>();  // the previous tile's rows have left
+        tile_sync<NT>();  // the previous tile's rows have left
         if (tid < TN) {
             so[tid] = fo - b0;
             sw[tid] = fw;
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(NT * UPB, El::MINB) node_rows_kernel(El el, Bl
         }
         if (tid == 0) so[TN] = nb;
         copy_fence();
-        unit_sync<NT>();  // words, values and operator rows of this tile are here
+        tile_sync<NT>();  // words, values and operator rows of this tile are here
         int rbase[TN];  // first value of each node's rows
         int len = 0;
 #pragma unroll
@@ -233,7 +237,7 @@ __global__ void __launch_bounds__(NT * UPB, El::MINB) node_rows_kernel(El el, Bl
         for (int p = 0; p < P; ++p)
             if (tid + p * NT < nb) bond(tid + p * NT, bq[p]);
         for (int q = tid + P * NT; q < nb; q += NT) bond(q, el.load(b0 + q));
-        unit_sync<NT>();
+        tile_sync<NT>();
         fetch(tile + stride, n0, n1);
         range(tile + 2 * stride, n0, n1);
         // diagonal blocks, mirror blocks and right-hand sides
@@ -286,7 +290,7 @@ __global__ void __launch_bounds__(NT * UPB, El::MINB) node_rows_kernel(El el, Bl
                 }
             }
         }
-        unit_sync<NT>();
+        tile_sync<NT>();
         double *dst = el.a.kvals + lo;
         int k = tid;
         for (; k + 3 * NT < len; k += 4 * NT) {
@@ -303,10 +307,10 @@ __global__ void __launch_bounds__(NT * UPB, El::MINB) node_rows_kernel(El el, Bl
 // ---- stress-coupled Cahn-Hilliard (rows c, mu, u; see assemble_stress_ch_kernel in k_csr.cu for the terms) -------
 template <int DIM>
 struct StressChEl {
-    static constexpr int ND = DIM + 2, NOP = DIM == 3 ? 9 : 5, TN = DIM == 3 ? 1 : 4, P = DIM == 3 ? 1 : 4;
+    static constexpr int ND = DIM + 2, NOP = DIM == 3 ? 9 : 5, TN = DIM == 3 ? 1 : 2, P = TN;
     // nodal values: u[ND], V, M, 1/V, (c_old, -, u - u_old - v dt)[ND]
-    // resident blocks: 3D (128 threads) 5 against 4 391 us of 427 at the size above, 3 506, 6 455; 2D (one warp a block) 12,
-    // against 4 blocks of two warps 181 us of 188 on 56,000 nodes
+    // resident blocks: 3D (128 threads) 5, against 4 391 us of 427 at the size above, 3 506, 6 455; in 2D (one warp a block)
+    // the bound leaves the registers free
     static constexpr int NQ = 2 * ND + 3, MINB = DIM == 3 ? 5 : 12;
     // operator slots in the multi-index order: first derivatives, then xx xy [xz] yy [yz zz]
     static constexpr int SXX = DIM, SXY = DIM + 1, SXZ = 5, SYY = DIM == 3 ? 6 : 4, SYZ = 7, SZZ = 8;
@@ -417,9 +421,9 @@ struct StressChEl {
 // ---- implicit dynamic fracture (rows u; see assemble_cached_kernel in k_csr.cu) ------------------------------------
 template <int DIM>
 struct CachedEl {
-    static constexpr int ND = DIM, NOP = DIM == 3 ? 9 : 5, NP = DIM == 3 ? 6 : 3, TN = DIM == 3 ? 1 : 4, P = DIM == 3 ? 1 : 4;
+    static constexpr int ND = DIM, NOP = DIM == 3 ? 9 : 5, NP = DIM == 3 ? 6 : 3, TN = DIM == 3 ? 1 : 2, P = TN;
     static constexpr int NQ = 2 * ND;  // u, u - u_old - v dt
-    static constexpr int MINB = DIM == 3 ? 6 : 10;  // 2D, two warps a block: 64 us against 66 with 5 blocks of four
+    static constexpr int MINB = DIM == 3 ? 6 : 10;  // (2D: the bound leaves the registers free)
     static constexpr int SXX = DIM, SXY = DIM + 1, SXZ = 5, SYY = DIM == 3 ? 6 : 4, SYZ = 7, SZZ = 8;
     CachedAsmArgs a;
     struct Bond {
@@ -615,40 +619,35 @@ __global__ void __launch_bounds__(128) scalar_block_kernel(ScalarAsmArgs a, Bloc
 
 // ---- launchers ------------------------------------------------------------------------------------------------
 namespace {
-constexpr size_t kTileShared = 112 * 1024;  // of a block of several units
-
-// resident blocks: the grid is what the chip holds, at most one tile a unit
-template <int NT, int UPB, typename El>
+// resident blocks: the grid is what the chip holds, at most one tile a block
+template <int NT, typename El>
 cudaError_t launch_nodes(const El &el, const BlockPattern &bp, int mmax, cudaStream_t s) {
-    const size_t smem = sizeof(double) * (size_t)UPB * unit_doubles<El>(mmax);
-    if constexpr (UPB > 1)  // long families: one unit's tile may need most of an SM's shared memory
-        if (smem > kTileShared) return launch_nodes<NT, 1>(el, bp, mmax, s);
-    auto kernel = node_rows_kernel<El, NT, UPB>;
-    // The limit belongs to the kernel, which contexts in other threads launch too: always the most that this one may be
-    // launched with, so that no call lowers what another has set.
-    constexpr size_t longest = sizeof(double) * (size_t)UPB * unit_doubles<El>(kBlockMax);
-    constexpr size_t most = UPB > 1 && longest > kTileShared ? kTileShared : longest;
+    const size_t smem = sizeof(double) * (size_t)tile_doubles<El>(mmax);
+    auto kernel = node_rows_kernel<El, NT>;
+    // The limit belongs to the kernel, which contexts in other threads launch too: always the most that it may be launched
+    // with, so that no call lowers what another has set.
+    constexpr size_t most = sizeof(double) * (size_t)tile_doubles<El>(kBlockMax);
     static_assert(most <= 227 * 1024, "shared memory of a block");
     cudaError_t e = cudaSuccess;
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     int dev = 0, sms = 148, res = 1;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, kernel, NT * UPB, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, kernel, NT, smem);
     if (e != cudaSuccess) return e;
-    const long long need = ((long long)el.a.n + El::TN * UPB - 1) / (El::TN * UPB), have = (long long)sms * (res > 0 ? res : 1);
-    kernel<<<(int)(need < have ? need : have), NT * UPB, smem, s>>>(el, bp, mmax);
+    const long long need = ((long long)el.a.n + El::TN - 1) / El::TN, have = (long long)sms * (res > 0 ? res : 1);
+    kernel<<<(int)(need < have ? need : have), NT, smem, s>>>(el, bp, mmax);
     return cudaGetLastError();
 }
 }  // namespace
 
 cudaError_t launch_stress_ch_block(const StressChAsmArgs &a, const BlockPattern &bp, int mmax, cudaStream_t s) {
-    if (a.dim == 3) return launch_nodes<128, 1>(StressChEl<3>{a}, bp, mmax, s);
-    return launch_nodes<32, 1>(StressChEl<2>{a}, bp, mmax, s);
+    if (a.dim == 3) return launch_nodes<128>(StressChEl<3>{a}, bp, mmax, s);
+    return launch_nodes<32>(StressChEl<2>{a}, bp, mmax, s);
 }
 cudaError_t launch_cached_block(const CachedAsmArgs &a, const BlockPattern &bp, int mmax, cudaStream_t s) {
-    if (a.dim == 3) return launch_nodes<128, 1>(CachedEl<3>{a}, bp, mmax, s);
-    return launch_nodes<32, 2>(CachedEl<2>{a}, bp, mmax, s);
+    if (a.dim == 3) return launch_nodes<128>(CachedEl<3>{a}, bp, mmax, s);
+    return launch_nodes<32>(CachedEl<2>{a}, bp, mmax, s);
 }
 cudaError_t launch_ch_block(const ChAsmArgs &a, const BlockPattern &bp, cudaStream_t s) {
     constexpr int LPN = 8;
