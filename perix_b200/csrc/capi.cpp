@@ -1249,7 +1249,9 @@ static cudaError_t rate_ops(pxb_ctx *c, const double *u, double *accel, cudaStre
     EpfArgs a = epf_args(c);
     a.u = e.u[e.cur].as<double>();
     a.accel = writes ? direct : e.accel.as<double>();
-    if (direct) {
+    // (without a kernel that writes to the host itself, the copy engines win from some megabytes on: variant 1, copies / kernels
+    // at the ends, 90,000 nodes in 2D 107 / 101 us, 490,000 483 / 510, a million 943 / 976; 110,592 in 3D 341 / 333)
+    if (direct && (writes || nd * sizeof(double) <= (size_t(4) << 20))) {
         cudaError_t err = launch_rate_up(nd, direct_u, e.u[e.cur].as<double>(), cnt, s);
         if (err == cudaSuccess) err = epf_launch(c, a, EPF_RATE, e.variant, s);
         if (err == cudaSuccess) err = launch_rate_down(cnt, direct_n, writes ? 0 : nd, a.accel, direct, s);
