@@ -147,7 +147,9 @@ int settle_variant(pxb_ctx *c, int variant, int plain) {
     return st;
 }
 
-// milliseconds of a captured run of kLoopSteps steps of the current schedule from `from` (the better of two)
+// milliseconds of a captured run of kLoopSteps steps of the current schedule from `from` (the better of two), with what a
+// schedule has to do first after a change of state: on small meshes, where the steps of all schedules take the same time,
+// the refresh of the slices' words (3 us) decides
 constexpr int kLoopSteps = 24;
 int loop_time(pxb_ctx *c, const Snapshot &from, float *ms) {
     Events ev;
@@ -155,7 +157,6 @@ int loop_time(pxb_ctx *c, const Snapshot &from, float *ms) {
     *ms = 1e30f;
     for (int r = 0; r < 3; ++r) {  // the first one captures
         PXB_TRY(load_state(c, from));
-        PXB_TRY(epf_ready(c));
         PXB_CUDA_TRY(cudaEventRecord(ev.ev[0], c->stream));
         PXB_TRY(pxb_epf_advance(c, kLoopSteps, kLoopSteps, nullptr));
         PXB_CUDA_TRY(cudaEventRecord(ev.ev[1], c->stream));
