@@ -914,7 +914,31 @@ uint16_t *slice_src(const EpfState &e) { return e.sl_topo.as<uint16_t>(); }
 int *slice_row0(const EpfState &e) { return reinterpret_cast<int *>(e.sl_topo.as<uint16_t>() + e.sl_entries); }
 int *slice_words(const pxb_ctx *c, const DevBuf &b) { return reinterpret_cast<int *>(b.as<char>() + coef_bytes(c)); }
 
-// slices, places in the families and length classes of the geometry
+// places in the families and length classes, into sl_topo (rows set)
+int sliced_places(pxb_ctx *c, const std::vector<int> &row0) {
+    EpfState &e = c->epf;
+    const Geometry &g = c->g;
+    PXB_TRY(h2d(c, slice_row0(e), row0.data(), sizeof(int) * row0.size()));
+    int idbits = 1;
+    while (idbits < 31 && (g.n - 1) >> idbits) ++idbits;
+    const int qbits = std::min(7, 31 - idbits);
+    static_assert(kSlicedClasses == 1 << 7, "length classes");
+    e.sl_shift = 31 - qbits;
+    unsigned long long *key = e.counters.as<unsigned long long>() + 5;  // the set-up's scratch counter
+    PXB_CUDA_TRY(cudaMemsetAsync(key, 0, sizeof(*key), c->stream));
+    PXB_CUDA_TRY(launch_sliced_rank(g.n, g.dim, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, slice_row0(e), slice_src(e), key,
+                                    c->stream));
+    c->launches++;
+    unsigned long long k2 = 0;
+    PXB_TRY(d2h(c, &k2, key, sizeof(k2)));
+    PXB_TRY(sync(c));  // (row0 is the caller's)
+    double r2 = 0.0;
+    std::memcpy(&r2, &k2, sizeof(double));
+    e.sl_step_len = std::isfinite(r2) ? std::sqrt(r2) / (1 << qbits) : 0.0;
+    return PXB_OK;
+}
+
+// the slices of the geometry; what could not be filled is not kept
 int sliced_topology(pxb_ctx *c) {
     EpfState &e = c->epf;
     const Geometry &g = c->g;
@@ -931,24 +955,9 @@ int sliced_topology(pxb_ctx *c) {
     }
     e.sl_entries = 32 * (size_t)std::max(1, row0.back());
     PXB_TRY(dev_alloc(c, e.sl_topo, sizeof(uint16_t) * e.sl_entries + sizeof(int) * row0.size()));
-    PXB_TRY(h2d(c, slice_row0(e), row0.data(), sizeof(int) * row0.size()));
-    int idbits = 1;
-    while (idbits < 31 && (n - 1) >> idbits) ++idbits;
-    const int qbits = std::min(7, 31 - idbits);
-    static_assert(kSlicedClasses == 1 << 7, "length classes");
-    e.sl_shift = 31 - qbits;
-    unsigned long long *key = e.counters.as<unsigned long long>() + 5;  // the set-up's scratch counter
-    PXB_CUDA_TRY(cudaMemsetAsync(key, 0, sizeof(*key), c->stream));
-    PXB_CUDA_TRY(launch_sliced_rank(n, g.dim, g.off.as<int>(), g.nbr.as<int>(), g.pos.p, slice_row0(e), slice_src(e), key,
-                                    c->stream));
-    c->launches++;
-    unsigned long long k2 = 0;
-    PXB_TRY(d2h(c, &k2, key, sizeof(k2)));
-    PXB_TRY(sync(c));  // (row0 leaves scope here too)
-    double r2 = 0.0;
-    std::memcpy(&r2, &k2, sizeof(double));
-    e.sl_step_len = std::isfinite(r2) ? std::sqrt(r2) / (1 << qbits) : 0.0;
-    return PXB_OK;
+    const int st = sliced_places(c, row0);
+    if (st != PXB_OK) e.sl_topo.release();
+    return st;
 }
 
 // words and coefficients (bond-ordered source Pc; rev: the reverse bonds') of the slices in `to`; words false:
@@ -2178,7 +2187,11 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
     if (sums && adj_sched(c) == 5) {  // the slices' reverse streams (without room for them: schedule 4)
         bool built = e.sl_rev.p;
         if (!built && c->g.max_family <= 0xffff && sliced_topology(c) == PXB_OK && sliced_alloc(c, e.sl_rev) == PXB_OK) {
-            PXB_TRY(sliced_fill(c, e.G.p, c->g.rev.as<int>(), e.sl_rev, true));
+            const int st = sliced_fill(c, e.G.p, c->g.rev.as<int>(), e.sl_rev, true);
+            if (st != PXB_OK) {  // (not to be taken for filled by the next sweep)
+                e.sl_rev.release();
+                return st;
+            }
             built = true;
         }
         if (built) {
