@@ -14,6 +14,7 @@
 // g_{n-1} = (dF_n/dU_{n-1})^T lambda_n (the c_old term), and accumulates dE/dkappa += lambda_n . dF_n/dkappa.  The
 // converged states are kept on the device (one per step).
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -24,7 +25,13 @@ namespace pxb {
 namespace {
 
 constexpr double kUpdateTol = 1e-14;  // Newton stops when |dU| <= kUpdateTol |U|
-constexpr size_t kBicgScalarBytes = 256;  // two BicgScalars, 128 bytes apart, then the partial sums
+constexpr size_t kBicgScalarBytes = 256;  // two BicgScalars, 128 bytes apart
+// Two pages for the scalars, then the partial sums.  A barrier's counter costs 1.7 us more a barrier on some pages of 4 KB
+// than on others (which half of the chip's L2 holds it), and of two neighbours one is of each kind: a 256x256 run of 10
+// steps takes 8.1 or 9.8 ms by nothing but the place of this block.  So a context's first Newton iterations use the two in
+// turn, timed, and the others the faster one.
+constexpr size_t kPage = 4096;
+constexpr int kPageRuns = 3;
 static_assert(sizeof(BicgScalars) <= kBicgScalarBytes / 2, "BiCGStab scalar block");
 constexpr int kHostDots = 4;  // dot products read back with a solve's outcome
 
@@ -132,7 +139,7 @@ int alloc_buffers(RunCtx &r, bool values) {
     PXB_TRY(dev_alloc(c, h.red, sizeof(double) * (size_t)(dot_scratch_doubles() + 8)));
     PXB_TRY(dev_alloc(c, h.nodal, sizeof(double) * 2 * n));
     for (auto &w : h.w) PXB_TRY(dev_alloc(c, w, sizeof(double) * rows));
-    PXB_TRY(dev_alloc(c, h.bicg, kBicgScalarBytes + sizeof(double) * 6 * kBicgParts));
+    PXB_TRY(dev_alloc(c, h.bicg, 4 * kPage + sizeof(double) * 6 * kBicgParts));
     return PXB_OK;
 }
 
@@ -209,6 +216,25 @@ ChAdjArgs adj_args(RunCtx &r, const double *U, const double *x, double *y) {
     return a;
 }
 
+char *bicg_pages(const ChState &h) {
+    return reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(h.bicg.p) + 2 * kPage - 1) / (2 * kPage) * (2 * kPage));
+}
+// scalars of Newton iteration k (single solves: 0)
+BicgScalars *bicg_scalars(const ChState &h, int k) {
+    const size_t at = h.sc_page < 0 ? (k & 1) * kPage : h.sc_page * kPage + (k & 1) * (kBicgScalarBytes / 2);
+    return reinterpret_cast<BicgScalars *>(bicg_pages(h) + at);
+}
+void time_page(ChState &h, int it, double seconds, int lits) {
+    if (h.sc_page >= 0) return;
+    double &t = h.page_time[it & 1];
+    t = std::min(t, seconds / (lits + 3));  // (assembly and start are worth some three iterations)
+    h.page_runs[it & 1]++;
+}
+void choose_page(ChState &h) {
+    if (h.sc_page < 0 && h.page_runs[0] >= kPageRuns && h.page_runs[1] >= kPageRuns)
+        h.sc_page = h.page_time[1] < h.page_time[0] ? 1 : 0;
+}
+
 // Right-preconditioned BiCGStab for A x = b (x starts at 0) on the device, one cooperative kernel (k_bicg.cu); A = K
 // (ch.kv) or, for adjoint solves, K'^T (ch.kvt through the transposed block view); the block-Jacobi inverse of A must
 // be in ch.binv.  Launches only; bicg_outcome reads the result after the caller's next synchronisation.
@@ -230,8 +256,8 @@ BicgArgs bicg_args(RunCtx &r, const double *b, double *x) {
     a.ph[1] = h.w[8].as<double>();
     a.vh[0] = h.w[9].as<double>();
     a.vh[1] = h.w[10].as<double>();
-    a.sc = h.bicg.as<BicgScalars>();
-    a.part = reinterpret_cast<double *>(h.bicg.as<char>() + kBicgScalarBytes);
+    a.sc = bicg_scalars(h, 0);
+    a.part = reinterpret_cast<double *>(bicg_pages(h) + 2 * kPage);
     return a;
 }
 
@@ -254,7 +280,7 @@ double *dev_dots(ChState &h) { return h.red.as<double>() + dot_scratch_doubles()
 
 int queue_readback(pxb_ctx *c, int ndots) {
     ChState &h = c->ch;
-    PXB_CUDA_TRY(cudaMemcpyAsync(host_outcome(h), h.bicg.p, sizeof(BicgScalars), cudaMemcpyDeviceToHost, c->stream));
+    PXB_CUDA_TRY(cudaMemcpyAsync(host_outcome(h), bicg_scalars(h, 0), sizeof(BicgScalars), cudaMemcpyDeviceToHost, c->stream));
     if (ndots > 0)
         PXB_CUDA_TRY(cudaMemcpyAsync(host_dots(h), dev_dots(h), sizeof(double) * ndots, cudaMemcpyDeviceToHost,
                                      c->stream));
@@ -318,9 +344,8 @@ int queue_newton(RunCtx &r, double *U, const double *Uold, int it) {
     s.pair = k.sl_pair.as<double2>();
     s.binv = h.binv.as<double>();
     s.rhs = h.rhs.as<double>();
-    auto scalars = [&](int k) { return reinterpret_cast<BicgScalars *>(h.bicg.as<char>() + (k & 1) * (kBicgScalarBytes / 2)); };
-    s.sc = scalars(it);
-    s.prev = it > 0 ? scalars(it - 1) : nullptr;
+    s.sc = bicg_scalars(h, it);
+    s.prev = it > 0 ? bicg_scalars(h, it - 1) : nullptr;
     PXB_TRY(check(c, launch_ch_system(s, c->stream), "ch system"));
     BicgArgs a = bicg_args(r, h.rhs.as<double>(), h.dU.as<double>());
     a.r0 = h.rhs.as<double>();  // the shadow residual is the right-hand side, which no phase writes
@@ -353,12 +378,18 @@ int queue_newton(RunCtx &r, double *U, const double *Uold, int it) {
 // One backward-Euler step on the slices.  The next iteration is queued before the host waits for the last one's
 // outcome, so the GPU does not wait for the host between iterations (a 256x256 run of 40: 9.7 -> 8.7 ms).
 int newton_step_slices(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) {
+    using Clock = std::chrono::steady_clock;
     pxb_ctx *c = r.c;
     double res0 = -1.0;
+    choose_page(c->ch);
     PXB_TRY(queue_newton(r, U, Uold, 0));
+    Clock::time_point last;
     for (int it = 0; it <= r.p.newton_max; ++it) {
         if (it < r.p.newton_max) PXB_TRY(queue_newton(r, U, Uold, it + 1));
         PXB_CUDA_TRY(cudaEventSynchronize(c->newton_ev[it & 1]));
+        const Clock::time_point now = Clock::now();
+        const double took = std::chrono::duration<double>(now - last).count();
+        last = now;
         const BicgScalars &o = *newton_outcome(c->ch, it);
         if (o.status == kBicgRunning) return bicg_timeout();
         const double res = o.bnorm;
@@ -373,6 +404,7 @@ int newton_step_slices(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stat
         int lits = 0;
         double lres = 0.0;
         PXB_TRY(bicg_outcome(&o, &lits, &lres));
+        if (it > 0) time_page(c->ch, it, took, lits);
         st->lin_iters += lits;
         st->max_lin_relres = std::max(st->max_lin_relres, lres);
         if (!o.go) {

@@ -260,6 +260,11 @@ struct ChState {
     DevBuf nodal;  // per-node scratch (energy, dkappa terms)
     DevBuf kvt;         // values of K^T (adjoint solves)
     DevBuf bicg;        // BiCGStab scalars and partial sums (k_bicg.cu)
+    // the page of the scalars with the grid barrier's counter (ch_solver.cpp): -1 not known yet; per page the fastest
+    // Newton iteration so far and how many were timed
+    int sc_page = -1;
+    double page_time[2] = {1e30, 1e30};
+    int page_runs[2] = {0, 0};
     PinnedBuf bicg_h;   // host copy of the scalars
 };
 
