@@ -2477,9 +2477,13 @@ extern "C" int pxb_csr_build_pattern(pxb_ctx *c, int ndof, long long *nnz) {
     a.cols = k.cols.as<int>();
     PXB_CUDA_TRY(launch_pattern_fill(a, c->stream));
     c->launches++;
-    for (DevBuf *b : {&list, &count, &first, &bsum, &small}) b->release();  // room for the value buffers
     k.exact = positions && (h[1] >> 32) == 0;
-    PXB_TRY(csr_finish(c, "pxb_csr_build_pattern", false));
+    int st = csr_finish(c, "pxb_csr_build_pattern", false);
+    if (st == PXB_ERR_OOM) {  // the temporaries make room for the value buffers
+        for (DevBuf *b : {&list, &count, &first, &bsum, &small}) b->release();
+        st = csr_finish(c, "pxb_csr_build_pattern", false);
+    }
+    PXB_TRY(st);
     PXB_TRY(sync(c));  // the caller may put the context on another stream before the pattern is used
     if (nnz) *nnz = total;
     return PXB_OK;

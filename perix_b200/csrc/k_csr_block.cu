@@ -10,7 +10,7 @@
 //     over the rows (each of which cost a 32-byte L2 sector);
 //   * the operator rows of a family are one contiguous span too, read coalesced into shared memory.
 // B200: 38,912 nodes in 3D with five unknowns (4.29 M bonds, 1.30 GB necessary) 783 us with slots -> 391 us; 81,200
-// nodes in 2D with two unknowns (2.25 M bonds, 171 MB) 96 -> 64 us.  What bounds both is the L1 data pipe (65 % of
+// nodes in 2D with two unknowns (2.25 M bonds, 171 MB) 96 -> 63 us.  What bounds both is the L1 data pipe (65 % of
 // its peak at 428 and 66 us, four nodes a tile in 2D: the values pass through shared memory once, with bank conflicts where a family's positions are not
 // consecutive), then DRAM latency (24-31 % occupancy there, limited by registers and the tile's shared memory; MINB below).
 #include <type_traits>
@@ -131,8 +131,8 @@ cudaError_t launch_block_map(const BlockMapArgs &a, cudaStream_t s) {
 // A block of NT threads (a warp in 2D, four warps in 3D) takes TN consecutive nodes at a time, two in 2D and one in 3D, whose
 // bonds' ids, operator rows and values are contiguous.  A long tile is a long chain for a mesh that does not fill the chip, a
 // short one has fewer bonds than threads.  2D with one, two and four nodes a tile, us a call (kernels with slots last):
-//   stress-CH         1,024 nodes 10.7 / 10.3 / 14.4 (10.3), 22,500 64 / 64 / 76 (113), 90,000 228 / 218 / 272 (425)
-//   dynamic fracture  1,024 nodes 6.2 / 6.2 / 8.2 (6.2), 22,500 24.6 / 18.5 / 20.5 (22.6), 90,000 109 / 69 / 72 (102)
+//   stress-CH         1,024 nodes 10.7 / 10.3 / 14.4 (10.3), 22,500 64 / 63 / 76 (113), 90,000 228 / 208 / 272 (425)
+//   dynamic fracture  1,024 nodes 6.2 / 6.2 / 8.2 (6.2), 22,500 24.6 / 18.5 / 20.5 (22.6), 90,000 109 / 67 / 72 (102)
 // Per tile:
 //   bonds     a bond a thread and pass: -K_IJ into the tile's rows in shared memory, the residual terms beside them;
 //   ahead     the next tile's bond words (registers), nodal values and operator rows (asynchronous copies) start out;
@@ -309,9 +309,9 @@ template <int DIM>
 struct StressChEl {
     static constexpr int ND = DIM + 2, NOP = DIM == 3 ? 9 : 5, TN = DIM == 3 ? 1 : 2, P = TN;
     // nodal values: u[ND], V, M, 1/V, (c_old, -, u - u_old - v dt)[ND]
-    // resident blocks: 3D (128 threads) 5, against 4 391 us of 427 at the size above, 3 506, 6 455; in 2D (one warp a block)
-    // the bound leaves the registers free
-    static constexpr int NQ = 2 * ND + 3, MINB = DIM == 3 ? 5 : 12;
+    // resident blocks: 3D (128 threads) 5, against 4 391 us of 427 at the size above, 3 506, 6 455; 2D (one warp a block) 14,
+    // against 12 208 us of 217 on 90,000 nodes, 18 221
+    static constexpr int NQ = 2 * ND + 3, MINB = DIM == 3 ? 5 : 14;
     // operator slots in the multi-index order: first derivatives, then xx xy [xz] yy [yz zz]
     static constexpr int SXX = DIM, SXY = DIM + 1, SXZ = 5, SYY = DIM == 3 ? 6 : 4, SYZ = 7, SZZ = 8;
     StressChAsmArgs a;
@@ -423,7 +423,7 @@ template <int DIM>
 struct CachedEl {
     static constexpr int ND = DIM, NOP = DIM == 3 ? 9 : 5, NP = DIM == 3 ? 6 : 3, TN = DIM == 3 ? 1 : 2, P = TN;
     static constexpr int NQ = 2 * ND;  // u, u - u_old - v dt
-    static constexpr int MINB = DIM == 3 ? 6 : 10;  // (2D: the bound leaves the registers free)
+    static constexpr int MINB = DIM == 3 ? 6 : 28;  // 2D: 66.7 us on 90,000 nodes against 69.2 with 10, 68.0 with 24, 67.7 with 32
     static constexpr int SXX = DIM, SXY = DIM + 1, SXZ = 5, SYY = DIM == 3 ? 6 : 4, SYZ = 7, SZZ = 8;
     CachedAsmArgs a;
     struct Bond {
