@@ -101,3 +101,19 @@ def test_slices_give_way_to_a_recording():
         c.synchronize()
         got.append((uN, ub))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+def test_pattern_temporaries_make_room():
+    """A limit that holds the built pattern and its value buffers, but not the build's temporaries beside them."""
+    c = px.Context(0)
+    _set_up(c, 120)
+    rows, cols = c.csr_get_pattern()
+    held = c.device_bytes()
+    x, vol, delta, h = _mesh(120)
+    d = px.Context(0)
+    d.set_geometry_points(x, vol, delta, delta, h, 2)
+    d.gbuild(2, px.FP64)
+    d.set_memory_limit(held + 4096)  # the build's lists take 4 bytes a bond more
+    assert d.csr_build_pattern(1) == cols.size
+    r, k = d.csr_get_pattern()
+    assert np.array_equal(r, rows) and np.array_equal(k, cols)
