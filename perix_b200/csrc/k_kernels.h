@@ -188,7 +188,8 @@ struct EpfArgs {
 constexpr int kEpfTmaConfigs = 12;                // staged (TMA) configurations per dimension
 constexpr int kEpfSlicedConfigs = 4;              // sliced configurations per dimension (k_epf_sliced.cu)
 // 0-2 lane groups, 3-4 CSR tiles, then staged, then sliced
-constexpr int kEpfVariants = 5 + kEpfTmaConfigs + kEpfSlicedConfigs;
+constexpr int kEpfLaneVariants = 5;                // lane groups and CSR tiles
+constexpr int kEpfVariants = kEpfLaneVariants + kEpfTmaConfigs + kEpfSlicedConfigs;
 // (a sliced variant is launched by launch_epf_sliced)
 cudaError_t launch_epf(const EpfArgs &a, int dim, bool mixed, int mode, int variant, cudaStream_t s);
 // P[c][t] from G[c][t] (t < ldb, SoA stride ldb): 2D p11 = C11 Gxx + C66 Gyy, p22 = C66 Gxx + C11 Gyy,

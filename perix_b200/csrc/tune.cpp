@@ -273,8 +273,11 @@ extern "C" int pxb_epf_autotune(pxb_ctx *c, int steps, size_t flush_bytes, int u
     // Streams that stay in L2 from one step to the next: a run's captured steps are faster than the flushed ones timed
     // above, and not by the same factor for every schedule (the 2.25 M-bond plate, mixed: 24.5 and 25.3 us flushed, 13.6
     // and 16.1 us in the loop).  The schedules within a tenth of the best are timed in a loop too, and that decides.
+    // In mixed precision the lane groups form their coefficients from the FP32 operators in FP64, the others read packed ones
+    // that were rounded once more: on meshes of some 5,000 nodes and less, where a loop takes as long with all of them, the
+    // tie goes to the lane groups.
     if (!c->epf.evict_first && flush_bytes > 0 && best_ms < 1e30f)
-        best_v = pick_by_loop(step_ms, best_v, [&](int v, float *t) {
+        best_v = pick_by_loop(step_ms, best_v, c->epf.precision == PXB_MIXED ? kEpfLaneVariants : 0, [&](int v, float *t) {
             if (select_variant(c, v) != PXB_OK) return 0;
             return loop_time(c, keep, t) == PXB_OK ? 1 : -1;  // (a run that blows up within the loop)
         });

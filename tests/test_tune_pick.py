@@ -9,8 +9,9 @@ MAIN = r"""
 #include "tune_pick.h"
 #include <cstdio>
 static int bad = 0;
-static void expect(int want, int flushed, std::vector<float> step, std::vector<float> loop, const char *what) {
-    const int got = pxb::pick_by_loop(step, flushed, [&](int v, float *t) {
+static void expect(int want, int flushed, std::vector<float> step, std::vector<float> loop, const char *what,
+                   int exact = 0) {
+    const int got = pxb::pick_by_loop(step, flushed, exact, [&](int v, float *t) {
         if (loop[v] == -2.f) { std::printf("%s: schedule %d timed\n", what, v); ++bad; }
         *t = loop[v];
         return loop[v] < 0.f ? -1 : loop[v] == 0.f ? 0 : 1;
@@ -23,6 +24,12 @@ int main() {
     expect(1, 1, {1.05f, 1.0f, 1.09f}, {-1.f, -2.f, -2.f}, "the first loop fails");
     expect(0, 1, {1.05f, 1.0f, 1.09f}, {3.f, 4.f, 0.f}, "one is not to be had");
     expect(1, 1, {1.05f, 1.0f, 1e30f}, {0.f, 0.f, -2.f}, "none is");
+    // the first two are the more accurate ones
+    expect(1, 2, {1.05f, 1.0f, 1.0f, 1.09f}, {3.f, 2.03f, 2.1f, 2.f}, "a tie goes to them", 2);
+    expect(3, 2, {1.05f, 1.0f, 1.0f, 1.09f}, {3.f, 2.2f, 2.1f, 2.f}, "more than a tie does not", 2);
+    expect(3, 2, {1.5f, 1.4f, 1.0f, 1.09f}, {-2.f, -2.f, 2.1f, 2.f}, "they are far off", 2);
+    expect(2, 2, {1.05f, 1.0f, 1.0f}, {2.f, -1.f, 2.f}, "one of their loops fails", 2);
+    expect(0, 2, {1.05f, 1.0f, 1.0f}, {2.f, 0.f, 2.01f}, "one is not to be had", 2);
     return bad;
 }
 """
