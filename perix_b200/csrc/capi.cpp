@@ -784,11 +784,14 @@ extern "C" int pxb_apply(pxb_ctx *c, const double *u, int nk, const int *slots, 
 // no kernels of its own, when the memory (limit) does not hold it, and under stream capture, whose graph would keep a
 // pointer to a buffer that the context may give up.
 static double *adjoint_scratch(pxb_ctx *c, const ApplyArgs &a) {
-    if (!apply_two_pass(a, c->g.nb) || capturing(c->stream)) return nullptr;
+    if (!apply_two_pass(a, c->ops.precision == PXB_MIXED, c->g.nb) || capturing(c->stream)) return nullptr;
     const size_t need = sizeof(double) * (size_t)c->g.nb;
     if (c->ops.bond.bytes != need && dev_alloc(c, c->ops.bond, need) != PXB_OK) return nullptr;
     if (!c->bond_ev && cudaEventCreateWithFlags(&c->bond_ev, cudaEventDisableTiming) != cudaSuccess) return nullptr;
-    if (c->bond_used && cudaStreamWaitEvent(c->stream, c->bond_ev, 0) != cudaSuccess) return nullptr;
+    if (c->bond_used && c->bond_stream != c->stream) {
+        if (!c->bond_marked && cudaEventRecord(c->bond_ev, c->bond_stream) != cudaSuccess) return nullptr;
+        if (cudaStreamWaitEvent(c->stream, c->bond_ev, 0) != cudaSuccess) return nullptr;
+    }
     return c->ops.bond.as<double>();
 }
 
@@ -835,8 +838,10 @@ extern "C" int pxb_apply_adjoint_d(pxb_ctx *c, const double *ybar_d, int nk, con
     PXB_TRY(check_launch(c, "apply_adjoint"));
     if (bond) {
         c->launches++;
-        PXB_CUDA_TRY(cudaEventRecord(c->bond_ev, c->stream));
         c->bond_used = true;
+        c->bond_stream = c->stream;
+        c->bond_marked = c->stream != c->own && c->stream != cudaStreamLegacy;
+        if (c->bond_marked) PXB_CUDA_TRY(cudaEventRecord(c->bond_ev, c->stream));
     }
     return PXB_OK;
 }

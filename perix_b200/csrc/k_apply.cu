@@ -277,20 +277,22 @@ static bool with_rows(const ApplyArgs &a, bool mixed, F f) {
     }
 }
 
-// The two passes are two launches and two event calls, and the first call on a mesh allocates their scratch (0.3-0.6 ms);
-// the one pass gathers reverse rows, which costs little while they stay in L2.  In 3D what it costs goes with the operators
-// asked for, in 2D hardly.  One pass against two, FP64, us a call among others:
+// The two passes are two launches, and the first call on a mesh allocates their scratch (0.3-0.6 ms); the one pass gathers
+// reverse rows, which costs little while they stay in L2.  In 3D what it costs goes with the operators asked for, in 2D
+// hardly.  One pass against two, FP64, us a call among others:
 //   3D, nine operators   142 K bonds 14.4 / 14.4, 363 K 26.6 / 17.5, 1.3 M 69 / 35;   one operator 363 K 10.3 / 13.4,
 //   1.3 M 32.7 / 26.0, 3.2 M 67.7 / 60.9
 //   2D, five operators   106 K 8.3 / 12.3, 431 K 16.5 / 14.1, 1.7 M 67.6 / 31.1;      one operator 431 K 11.8 / 12.3,
 //   1.7 M 47.2 / 26.1
-// The lines below lie where a call saves 5 to 10 us, so that some tens of calls pay for the scratch.
-bool apply_two_pass(const ApplyArgs &a, long long nb) {
+// The lines below lie where a call saves 5 to 10 us, so that some tens of calls pay for the scratch.  Mixed 3D calls, whose
+// rows are half as long and whose one pass is hidden behind the host's work up to there (363 K bonds 32.8 / 24.4, 1.3 M
+// 61.5 / 34.7 of some 120 us for both directions through torch): later.
+bool apply_two_pass(const ApplyArgs &a, bool mixed, long long nb) {
     if (a.nop != 2 && a.nop != 3 && a.nop != 5 && a.nop != 9) return false;
     if (a.dim == 2) return nb >= 800000;
     ApplyArgs b = a;
     b.defect = nullptr;
-    return nb * (2 + __builtin_popcount(used_ops(b))) >= 2900000;
+    return nb * (2 + __builtin_popcount(used_ops(b))) >= (mixed ? 8000000 : 2900000);
 }
 
 cudaError_t launch_apply(const ApplyArgs &a, bool mixed, int grid, cudaStream_t s) {

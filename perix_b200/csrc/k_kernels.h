@@ -333,7 +333,7 @@ struct ApplyArgs {
     int dim = 2;
 };
 cudaError_t launch_apply(const ApplyArgs &a, bool mixed, int grid, cudaStream_t s);
-bool apply_two_pass(const ApplyArgs &a, long long nb);  // the two-pass transpose is the faster one
+bool apply_two_pass(const ApplyArgs &a, bool mixed, long long nb);  // the two-pass transpose is the faster one
 // bond: one double a bond of scratch for the two-pass transpose, NULL for the kernel that needs none
 cudaError_t launch_apply_adjoint(const ApplyArgs &a, bool mixed, double *bond, int grid, cudaStream_t s);
 // the rate call's page-locked ends (k_epf_sliced.cu): u up with cnt[4] = cnt[0], cnt[0..4] and n values of accel down

@@ -288,9 +288,12 @@ struct BatchState {
 struct pxb_ctx {
     int device = 0;
     pxb::DevPool pool;  // before the buffers, which go back to it
-    // last use of ops.bond: the next one waits for it, whatever its stream
+    // last use of ops.bond: a use on another stream waits for it (a handle is not given to a new stream while the old one has
+    // work).  bond_ev has been recorded behind it (a caller's stream), or is when it is wanted (the context's own stream and
+    // the legacy one are always there)
     cudaEvent_t bond_ev = nullptr;
-    bool bond_used = false;
+    cudaStream_t bond_stream = nullptr;
+    bool bond_used = false, bond_marked = false;
     // end of what the explicit element's asynchronous calls (constants, frozen force, recording, reverse sweep) have queued:
     // the next explicit call waits for it, whatever its stream, because they share the slices' words and coefficients
     cudaEvent_t epf_ev = nullptr;
