@@ -376,7 +376,7 @@ int queue_newton(RunCtx &r, double *U, const double *Uold, int it) {
 }
 
 // One backward-Euler step on the slices.  The next iteration is queued before the host waits for the last one's
-// outcome, so the GPU does not wait for the host between iterations (a 256x256 run of 40: 9.7 -> 8.7 ms).
+// outcome, so the GPU does not wait for the host between iterations (a 256x256 run of 40: 9.7 -> 8.7 ms on the same page).
 int newton_step_slices(RunCtx &r, double *U, const double *Uold, pxb_ch_run_stats *st) {
     using Clock = std::chrono::steady_clock;
     pxb_ctx *c = r.c;

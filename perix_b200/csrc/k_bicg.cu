@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM) bicg_solve_kernel(Bicg
 // nothing) but the L1 data pipe under the gathers and the grid barriers, about 3800 cycles each.  So 148 blocks of 512
 // threads (two of 512: 10.0 ms a run, one of 1024: 10.1, one of 512: 9.2), the preconditioned direction's
 // ph - omega vh formed once a node in phase C instead of at every gather, and the Newton iteration's other sums and its
-// update in the same kernel.  256x256, 10 steps (32 solves, 298 iterations): 18.4 ms with the CSR kernels -> 9.7 ms;
+// update in the same kernel.  256x256, 10 steps (32 solves, 298 iterations): 18.4 ms with the CSR kernels -> 9.7 ms, and
+// 8.1 ms with the next iteration queued ahead and the barrier's counter on the faster page (ch_solver.cpp);
 // 64x64: 10.8 (one lane a node) -> 5.9 ms with eight.
 
 // K (Picard Jacobian, Neumann ghost rows) and F at (U, Uold): value pairs, block-Jacobi inverse, right-hand side.  The
