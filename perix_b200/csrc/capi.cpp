@@ -66,26 +66,31 @@ void DevPool::give(void *p, size_t cap) {
     bytes += cap;
 }
 
-// the tightest block that wastes at most `slack`, NULL without one
-void *DevPool::take(size_t want, size_t *cap, size_t slack, cudaStream_t stream, cudaStream_t own) {
-    if (foreign) return nullptr;
-    size_t best = idle.size();
+// index of the tightest block that wastes at most `slack`, -1 without one
+int DevPool::find(size_t want, size_t slack) const {
+    if (foreign) return -1;
+    int best = -1;
     for (size_t k = 0; k < idle.size(); ++k)
-        if (idle[k].cap >= want && idle[k].cap <= want + slack &&
-            (best == idle.size() || idle[k].cap < idle[best].cap))
-            best = k;
-    if (best == idle.size()) return nullptr;
+        if (idle[k].cap >= want && idle[k].cap <= want + slack && (best < 0 || idle[k].cap < idle[(size_t)best].cap))
+            best = (int)k;
+    return best;
+}
+
+// that block, NULL without one
+void *DevPool::take(size_t want, size_t *cap, size_t slack, cudaStream_t stream, cudaStream_t own) {
+    const int best = find(want, slack);
+    if (best < 0) return nullptr;
     if (dirty && (cudaStreamSynchronize(stream) != cudaSuccess ||
                   (own != stream && cudaStreamSynchronize(own) != cudaSuccess))) {
         cudaGetLastError();
         return nullptr;
     }
     dirty = false;
-    void *p = idle[best].p;
-    *cap = idle[best].cap;
-    bytes -= idle[best].cap;
-    idle.erase(idle.begin() + (ptrdiff_t)best);
-    return p;
+    const Block b = idle[(size_t)best];
+    *cap = b.cap;
+    bytes -= b.cap;
+    idle.erase(idle.begin() + best);
+    return b.p;
 }
 
 PinnedBuf::~PinnedBuf() {
@@ -165,7 +170,8 @@ static bool over_limit(const pxb_ctx *c, const DevBuf &b, size_t bytes, size_t i
 // b from the pool's idle blocks; whether there is one that wastes at most `slack`.  Under a limit none is wasted, so that
 // what fits without the pool fits with it.
 static bool take_idle(pxb_ctx *c, DevBuf &b, size_t bytes, size_t slack) {
-    if (!c || !bytes || c->pool.idle.empty() || capturing(c->stream) || over_limit(c, b, bytes, c->pool.bytes)) return false;
+    if (!c || !bytes || !c->pool.fits(bytes, c->mem_limit ? 0 : slack)) return false;
+    if (capturing(c->stream) || over_limit(c, b, bytes, c->pool.bytes)) return false;
     size_t cap = 0;
     void *p = c->pool.take(bytes, &cap, c->mem_limit ? 0 : slack, c->stream, c->own);
     if (!p) return false;
@@ -232,6 +238,27 @@ int pool_upload(pxb_ctx *c, DevBuf &b, const void *host, size_t bytes) {
 int sync(pxb_ctx *c) {
     PXB_CUDA_TRY(cudaStreamSynchronize(c->stream));
     return PXB_OK;
+}
+
+cudaError_t StreamOrder::before(cudaStream_t s, cudaStream_t own) {
+    if (!used || last == s) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (!ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess && !marked) e = cudaEventRecord(ev, last);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev, 0);
+    return e == cudaSuccess ? after(s, own) : e;  // (s is behind the last use now)
+}
+
+cudaError_t StreamOrder::after(cudaStream_t s, cudaStream_t own) {
+    used = true;
+    last = s;
+    marked = s != own && s != cudaStreamLegacy;
+    if (!marked) return cudaSuccess;
+    if (!ev) {
+        const cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaEventRecord(ev, s);
 }
 
 int check_launch(pxb_ctx *c, const char *what) {
@@ -367,8 +394,8 @@ extern "C" int pxb_ctx_destroy(pxb_ctx *c) {
     cudaStreamSynchronize(c->stream);
     drop_snapshot(c);
     destroy_graphs(c->epf);
-    if (c->bond_ev) cudaEventDestroy(c->bond_ev);
-    if (c->epf_ev) cudaEventDestroy(c->epf_ev);
+    for (StreamOrder *o : {&c->bond_order, &c->epf_order})
+        if (o->ev) cudaEventDestroy(o->ev);
     for (cudaEvent_t e : c->newton_ev)
         if (e) cudaEventDestroy(e);
     if (c->own) cudaStreamDestroy(c->own);
@@ -403,10 +430,10 @@ extern "C" int pxb_ctx_launch_count(pxb_ctx *c, long long *count) {
 }
 
 // ==================================================================================================== geometry
-// drop every state that depends on the geometry, then store the CSR offsets (host copy + device) and allocate
-// the zeroed neighbour array (ldb = nb rounded up to 16, plus 16)
+// drop every state that depends on the geometry, then store the CSR offsets (host copy + device; off_d: where the device has
+// them already) and allocate the zeroed neighbour array (ldb = nb rounded up to 16, plus 16)
 static int geometry_reset(pxb_ctx *c, int n, int dim, const int *neigh_off, int maxf, double delta, double dx_char,
-                          const int *mirror) {
+                          const int *mirror, const int *off_d = nullptr) {
     PXB_CUDA_TRY(cudaSetDevice(c->device));
     PXB_CUDA_TRY(cudaStreamSynchronize(c->stream));
     destroy_graphs(c->epf);
@@ -432,7 +459,8 @@ static int geometry_reset(pxb_ctx *c, int n, int dim, const int *neigh_off, int 
     g.ldb = ((nb + 16 + 15) / 16) * 16;
     PXB_TRY(pool_alloc(c, g.off, sizeof(int) * (size_t)(n + 1 + 16)));
     PXB_CUDA_TRY(cudaMemsetAsync(g.off.p, 0, g.off.bytes, c->stream));
-    PXB_TRY(h2d(c, g.off.p, neigh_off, sizeof(int) * (size_t)(n + 1)));
+    PXB_CUDA_TRY(cudaMemcpyAsync(g.off.p, off_d ? off_d : neigh_off, sizeof(int) * (size_t)(n + 1),
+                                 off_d ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream));
     PXB_TRY(pool_alloc(c, g.nbr, sizeof(int) * (size_t)g.ldb));
     PXB_CUDA_TRY(cudaMemsetAsync(g.nbr.p, 0, g.nbr.bytes, c->stream));
     return PXB_OK;
@@ -498,7 +526,7 @@ extern "C" int pxb_set_geometry_points(pxb_ctx *c, int n, int dim, const double 
     int maxf = 0;
     long long tot = 0;
     PXB_TRY(fb.count(c, n, dim == 3, coords3, radius, hoff, maxf, tot));
-    PXB_TRY(geometry_reset(c, n, dim, hoff.data(), maxf, delta, dx_char, mirror));
+    PXB_TRY(geometry_reset(c, n, dim, hoff.data(), maxf, delta, dx_char, mirror, fb.offsets_d()));
     PXB_TRY(fb.fill(c, c->g.off.as<int>(), c->g.nbr.as<int>(), 0));
     if (nbtot) *nbtot = tot;
     return geometry_finish(c, fb.coords_d(), vols, mirror, layer_index);
@@ -787,11 +815,7 @@ static double *adjoint_scratch(pxb_ctx *c, const ApplyArgs &a) {
     if (!apply_two_pass(a, c->ops.precision == PXB_MIXED, c->g.nb) || capturing(c->stream)) return nullptr;
     const size_t need = sizeof(double) * (size_t)c->g.nb;
     if (c->ops.bond.bytes != need && dev_alloc(c, c->ops.bond, need) != PXB_OK) return nullptr;
-    if (!c->bond_ev && cudaEventCreateWithFlags(&c->bond_ev, cudaEventDisableTiming) != cudaSuccess) return nullptr;
-    if (c->bond_used && c->bond_stream != c->stream) {
-        if (!c->bond_marked && cudaEventRecord(c->bond_ev, c->bond_stream) != cudaSuccess) return nullptr;
-        if (cudaStreamWaitEvent(c->stream, c->bond_ev, 0) != cudaSuccess) return nullptr;
-    }
+    if (c->bond_order.before(c->stream, c->own) != cudaSuccess) return nullptr;
     return c->ops.bond.as<double>();
 }
 
@@ -838,10 +862,7 @@ extern "C" int pxb_apply_adjoint_d(pxb_ctx *c, const double *ybar_d, int nk, con
     PXB_TRY(check_launch(c, "apply_adjoint"));
     if (bond) {
         c->launches++;
-        c->bond_used = true;
-        c->bond_stream = c->stream;
-        c->bond_marked = c->stream != c->own && c->stream != cudaStreamLegacy;
-        if (c->bond_marked) PXB_CUDA_TRY(cudaEventRecord(c->bond_ev, c->stream));
+        PXB_CUDA_TRY(c->bond_order.after(c->stream, c->own));
     }
     return PXB_OK;
 }
@@ -1030,32 +1051,20 @@ SlicedArgs sliced_args(const pxb_ctx *c, const DevBuf &streams) {
 
 }  // namespace
 
-// The context stream goes on after the asynchronous explicit calls queued so far (see pxb_ctx::epf_ev), which costs
-// nothing on the stream they are on; epf_mark ends such a call.  Neither has a place in a caller's capture.
-static int epf_order(pxb_ctx *c) {
-    if (!c->epf_queued || capturing(c->stream)) return PXB_OK;
-    const cudaError_t q = cudaEventQuery(c->epf_ev);
-    if (q == cudaSuccess) {
-        c->epf_queued = false;
-        return PXB_OK;
-    }
-    if (q != cudaErrorNotReady) return cuda_fail(q, "explicit calls in flight");
-    cudaGetLastError();
-    PXB_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->epf_ev, 0));
+// around an asynchronous explicit call (not in a caller's capture)
+static int epf_begin(pxb_ctx *c) {
+    if (!capturing(c->stream)) PXB_CUDA_TRY(c->epf_order.before(c->stream, c->own));
     return PXB_OK;
 }
 
-static int epf_mark(pxb_ctx *c) {
-    if (capturing(c->stream)) return PXB_OK;
-    if (!c->epf_ev) PXB_CUDA_TRY(cudaEventCreateWithFlags(&c->epf_ev, cudaEventDisableTiming));
-    PXB_CUDA_TRY(cudaEventRecord(c->epf_ev, c->stream));
-    c->epf_queued = true;
+static int epf_end(pxb_ctx *c) {
+    if (!capturing(c->stream)) PXB_CUDA_TRY(c->epf_order.after(c->stream, c->own));
     return PXB_OK;
 }
 
 int epf_ready(pxb_ctx *c) {
     EpfState &e = c->epf;
-    PXB_TRY(epf_order(c));
+    PXB_TRY(epf_begin(c));
     if (!runs_sliced(e)) return PXB_OK;
     if (!e.sl_ready) PXB_TRY(sliced_build(c));
     // A caller's capture always holds the refresh: health and constants may change between its replays.  (It has not run
@@ -1892,7 +1901,7 @@ extern "C" int pxb_epf_force_frozen_d(pxb_ctx *c, const double *u_d, double *a_d
     const cudaError_t err = epf_launch(c, a, EPF_FORCE_FROZEN, variant, c->stream);
     if (err != cudaSuccess) return cuda_fail(err, "epf force (frozen mask)");
     PXB_TRY(check_launch(c, "epf force (frozen mask)"));
-    return sliced ? epf_mark(c) : PXB_OK;
+    return sliced ? epf_end(c) : PXB_OK;
 }
 
 // s_c from the fracture energy (reference include/ElmtSystem/FractureCriterion.h:30-43): 3D 5 G0 / (6 E delta),
@@ -1933,7 +1942,7 @@ extern "C" int pxb_epf_set_constants(pxb_ctx *c, double C11, double C12, double 
     PXB_TRY(need_epf(c, "pxb_epf_set_constants"));
     if (!(rho > 0.0)) return fail(PXB_ERR_INVALID, "pxb_epf_set_constants: rho must be > 0");
     EpfState &e = c->epf;
-    PXB_TRY(epf_order(c));
+    PXB_TRY(epf_begin(c));
     destroy_graphs(e);  // captured launches carry the old constants
     e.C11 = C11;
     e.C12 = C12;
@@ -1943,7 +1952,7 @@ extern "C" int pxb_epf_set_constants(pxb_ctx *c, double C11, double C12, double 
     PXB_CUDA_TRY(launch_navier_pack(e.G.p, e.P.p, (long long)c->g.ldb, c->g.dim, e.precision == PXB_MIXED, C11, C12,
                                     C66, c->stream));
     PXB_TRY(check_launch(c, "navier pack"));
-    return epf_mark(c);
+    return epf_end(c);
 }
 
 extern "C" int pxb_epf_force_adjoint_d(pxb_ctx *c, const double *u_d, const double *abar_d, double *ubar_d,
@@ -2156,7 +2165,7 @@ extern "C" int pxb_epf_record_d(pxb_ctx *c, const double *u0_d, const double *v0
     e.rec_K = K;
     e.rec_all = all;
     e.rec_seg = all ? -1 : nseg - 1;
-    return epf_mark(c);
+    return epf_end(c);
 }
 
 extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, const double *ubar_Nm1_d,
@@ -2283,7 +2292,7 @@ extern "C" int pxb_epf_adjoint_recorded_d(pxb_ctx *c, const double *ubar_N_d, co
         PXB_TRY(check_launch(c, "dC collect"));
     }
     if (dC_d) PXB_TRY(d2d(dC_d, e.adj_dC.p, 3 * sizeof(double)));
-    return epf_mark(c);
+    return epf_end(c);
 }
 
 extern "C" int pxb_epf_adjoint_d(pxb_ctx *c, const double *u0_d, const double *v0_d, double dt, int nsteps,
@@ -2338,10 +2347,12 @@ int csr_finish(pxb_ctx *c, const char *who, bool verify) {
     const int ndof = k.ndof, n = c->g.n;
     const size_t rows = (size_t)n * ndof, nb = (size_t)std::max(1LL, c->g.nb);
     void *tmp = nullptr;
-    PXB_TRY(scratch(c, 8, &tmp));
-    PXB_CUDA_TRY(cudaMemsetAsync(tmp, 0, 8, c->stream));
     int flags[2] = {0, 0};
-    if (!k.exact) PXB_TRY(alloc_positions(c));
+    if (!k.exact) {
+        PXB_TRY(scratch(c, 8, &tmp));
+        PXB_CUDA_TRY(cudaMemsetAsync(tmp, 0, 8, c->stream));
+        PXB_TRY(alloc_positions(c));
+    }
     if (!k.exact && k.mmax <= kBlockMax) {
         BlockMapArgs m;
         m.n = n;

@@ -17,6 +17,7 @@ public:
               int &maxf, long long &tot);
     int fill(pxb_ctx *c, const int *off_d, int *nbr_d, int id_base);
     const double *coords_d() const { return coords_.as<double>(); }
+    const int *offsets_d() const { return off_.as<int>(); }  // hoff on the device
 
 private:
     FamArgs a_;

@@ -49,6 +49,8 @@ struct DevPool {
     size_t bytes = 0;
     bool dirty = false, foreign = false;
     void give(void *p, size_t cap);
+    int find(size_t want, size_t slack) const;
+    bool fits(size_t want, size_t slack) const { return find(want, slack) >= 0; }
     void *take(size_t want, size_t *cap, size_t slack, cudaStream_t stream, cudaStream_t own);
     void trim();
     DevPool() = default;
@@ -285,19 +287,27 @@ struct BatchState {
 };
 }  // namespace pxb
 
+namespace pxb {
+// Puts uses of something in order that may be queued on changing streams.  On one stream they are in order as they are, and
+// a handle is not given to a new stream while the old one has work; on another stream a use waits for the event behind the
+// last one.  A caller's stream may be gone by then, so the event is recorded at once there; the context's own stream and
+// the legacy one are always there, and it is recorded when it is wanted.  Nothing of this has a place in a caller's capture.
+struct StreamOrder {
+    cudaEvent_t ev = nullptr;
+    cudaStream_t last = nullptr;
+    bool used = false, marked = false;
+    cudaError_t before(cudaStream_t s, cudaStream_t own);  // a use on s may be queued after this
+    cudaError_t after(cudaStream_t s, cudaStream_t own);   // and has been
+};
+}  // namespace pxb
+
 struct pxb_ctx {
     int device = 0;
     pxb::DevPool pool;  // before the buffers, which go back to it
-    // last use of ops.bond: a use on another stream waits for it (a handle is not given to a new stream while the old one has
-    // work).  bond_ev has been recorded behind it (a caller's stream), or is when it is wanted (the context's own stream and
-    // the legacy one are always there)
-    cudaEvent_t bond_ev = nullptr;
-    cudaStream_t bond_stream = nullptr;
-    bool bond_used = false, bond_marked = false;
-    // end of what the explicit element's asynchronous calls (constants, frozen force, recording, reverse sweep) have queued:
-    // the next explicit call waits for it, whatever its stream, because they share the slices' words and coefficients
-    cudaEvent_t epf_ev = nullptr;
-    bool epf_queued = false;
+    pxb::StreamOrder bond_order;  // uses of ops.bond
+    // the explicit element's asynchronous calls (constants, frozen force, recording, reverse sweep), which share the slices'
+    // words and coefficients
+    pxb::StreamOrder epf_order;
     cudaEvent_t newton_ev[2] = {nullptr, nullptr};  // ends of the implicit run's queued Newton iterations
     size_t mem_limit = 0;  // device bytes the context may hold (0: no limit beyond the GPU's)
     int gbuild_schedule = -1;  // g-build: -1 by problem, 0 lane groups, 1 one warp per node, 2 the same with

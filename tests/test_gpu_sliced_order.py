@@ -92,14 +92,15 @@ def test_captured_force_follows_health(dim, shape):
     c.set_stream(None)
 
 
+@pytest.mark.parametrize("legacy", [False, True])
 @pytest.mark.parametrize("dim,shape", SHAPES)
-def test_force_on_another_stream_waits_for_the_refresh(dim, shape):
+def test_force_on_another_stream_waits_for_the_refresh(dim, shape, legacy):
     """The words are refreshed by a call on one stream, late; a call on another stream needs them, and the constants that a
-    third one writes."""
+    third one writes.  The late stream is torch's default (the legacy) one or another."""
     k = Case(dim, shape)
     torch, c = k.torch, k.ctxs[1]
     ref = [k.reference(0), k.reference(1), k.reference(1, 1.5)]
-    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    a, b = torch.cuda.default_stream() if legacy else torch.cuda.Stream(), torch.cuda.Stream()
     outs = [torch.empty_like(k.u) for _ in range(5)]
     torch.cuda.synchronize()
     late = lambda s: torch.cuda._sleep(20_000_000)  # noqa: E731
